@@ -151,7 +151,8 @@ double ternaspmm_debug_int8_mma_rate(int iters, ternaspmm_stream_t stream);
 /* Test hook: shape of the most recent kernel launch made by this thread.
  * out6 = {kernel (1 = small-batch kernel, one fat CTA per SM; 2 = small-batch
  * kernel, thin CTAs; 3 = tcgen05 kernel; 4 = output head; 5 = work list; 6 = tcgen05 kernel
- * on dense weights from the workspace, single CTAs; 7 = the same on CTA pairs), tokens per pass, K split (cluster
+ * on dense weights from the workspace, single CTAs; 7 = the same on CTA pairs; 8 = small-batch kernel
+ * on two-bit weights: splits = 1, row tiles = strips of 16 rows per CTA), tokens per pass, K split (cluster
  * size), warps per CTA, 64-row tiles per CTA, CTAs}. */
 void ternaspmm_last_launch_shape(int* out6);
 
@@ -262,6 +263,25 @@ void ternaspmm_tp_allreduce_finish(float** bufs, unsigned int** flags, ternaspmm
                                    int world, unsigned int* counters, ternaspmm_bf16* ws, float eps,
                                    int full_width, int M, int N, ternaspmm_bf16* residual,
                                    ternaspmm_stream_t stream);
+
+/* ---- linears on weights laid out once in two bits -----------------------------------------------
+ * For programs that keep a weight for many calls: ternaspmm_w2_relayout() rewrites the packed arrays
+ * (which it does not change) as fixed-rate two-bit codes, ternaspmm_w2_bytes(N, K) bytes at w2 (N*K/4, K
+ * rounded up to a multiple of 128; 16-byte aligned), in the order in which the kernels consume them; the linear then decodes with one AND and at most one shift
+ * per four weights instead of the packed format's popcount prefixes and table look-ups.
+ * ternaspmm_w2_linear() is ternaspmm_linear_segments / bitlinear_TernaSpMM_residual on such weights:
+ * same contraction, epilogue and roundings (seg1 = seg2 = seg3 = 0: the reference's segment rules).
+ * front_end 0: x is int8 [M][K] with its scales s.  1: x is bf16 [M][K], quantised per token in the
+ * same kernel (ternaspmm_quant).  2: RMSNorm with norm_weight and eps first (ternaspmm_rmsnorm_quant).
+ * 3: x is bf16 [M][2K], gate + RMSNorm first (ternaspmm_relu2_gate_rmsnorm_quant).  Front-ends 1-3
+ * ignore s and take at most ternaspmm_w2_fused_rows(K) tokens.  K below 2^18. */
+void ternaspmm_w2_relayout(uint64_t* bitmap, int* tile_offsets, uint16_t* quarter_offsets, uint32_t* sign_words,
+                           int N, int K, void* w2, ternaspmm_stream_t stream);
+long long ternaspmm_w2_bytes(int N, int K);
+int ternaspmm_w2_fused_rows(int K);
+void ternaspmm_w2_linear(void* x, int front_end, ternaspmm_bf16* norm_weight, float eps, void* w2, ternaspmm_bf16* out,
+                         ternaspmm_bf16* s, ternaspmm_bf16* ws, int ws_num, int M, int N, int K, int seg1, int seg2,
+                         int seg3, int prefill_form, ternaspmm_bf16* residual, ternaspmm_stream_t stream);
 
 /* ---- work lists: many independent small-batch linears in one persistent launch ------------------
  * One item is what one call of bitlinear_TernaSpMM / ternaspmm_linear_segments /

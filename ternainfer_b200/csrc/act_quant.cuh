@@ -5,8 +5,9 @@
 // per linear input:
 //   norm_quant       x -> RMSNorm(x) * w -> per-token absmax int8 + scale
 //   gated_norm_quant [x1 | x3] -> relu(x1)^2 * x3 -> RMSNorm * w -> int8 + scale
-// One CTA per token row; the row is staged once in shared memory as bf16, so
-// HBM traffic is one read of the activations and one write of int8 + scale.
+// One CTA per token row; the row is held in registers (up to 8192 elements) or
+// staged once in shared memory as bf16, so HBM traffic is one read of the
+// activations and one write of int8 + scale.
 // Rounding points follow the eager PyTorch evaluation of the same expressions
 // (bf16 after the norm, bf16(1/amax) * 127 for the scale, bf16(x*s) before the
 // round-half-even).  The fp32 sum of squares has a FIXED order, so the result is
@@ -29,18 +30,21 @@ constexpr int kActMaxThreads = 1024;   // one 8-element vector per thread up to 
 
 __device__ __forceinline__ float bf16_round_f(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
+// Maximum that keeps a NaN, as torch's does: a row that holds one gets a NaN scale.
+__device__ __forceinline__ float nan_max(float a, float b) { return (b > a || b != b) ? b : a; }
+
 __device__ __forceinline__ float block_reduce(float v, float* scratch, bool is_max) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
         const float o = __shfl_xor_sync(0xffffffffu, v, d);
-        v = is_max ? fmaxf(v, o) : v + o;
+        v = is_max ? nan_max(v, o) : v + o;
     }
     __syncthreads();   // scratch may still be read from the previous reduction
     if (lane == 0) scratch[warp] = v;
     __syncthreads();
     float r = scratch[0];
-    for (int i = 1; i < (int)(blockDim.x >> 5); ++i) r = is_max ? fmaxf(r, scratch[i]) : r + scratch[i];
+    for (int i = 1; i < (int)(blockDim.x >> 5); ++i) r = is_max ? nan_max(r, scratch[i]) : r + scratch[i];
     return r;
 }
 
@@ -51,8 +55,142 @@ __device__ __forceinline__ float block_reduce(float v, float* scratch, bool is_m
 // model's final norm in the same fixed summation order.
 enum ActMode : int { ACT_RMSNORM = 0, ACT_SCALE_SUMSQ = 1, ACT_PLAIN = 2, ACT_NORM_ONLY = 3 };
 
+// One row in registers: thread `tid` of `nthreads` holds the elements of virtual threads tid + j * nthreads, j < NV (eight
+// consecutive elements each; NV * nthreads >= T, K <= 8192 so that T covers the row), from the load to the int8 store.
+// What remains is one chain of latencies - load, butterfly, barrier, square root, barrier, reciprocal -, so nothing
+// goes through shared memory but one float per warp and reduction, and the maximum (of magnitudes, whose bit patterns
+// order like the values, NaN above all) is a redux.sync.  `part` and `mxp`: 32 words each, 16-byte aligned; the caller
+// may reuse them after its next barrier.  store(k0, q) takes eight int8 values (or, NORM_ONLY, eight bf16).  Returns the scale s.
+__device__ __forceinline__ uint32_t warp_max_u32(uint32_t v) {
+    uint32_t r;
+    asm volatile("redux.sync.max.u32 %0, %1, 0xffffffff;" : "=r"(r) : "r"(v));
+    return r;
+}
+
+template <int NV, bool GATED, int MODE, typename Store>
+__device__ __forceinline__ float row_front_end(const __nv_bfloat16* xr, const uint4 (&nw)[NV], float eps, int K, int T, float* part,
+                                               uint32_t* mxp, float* ss_out, Store store) {
+    const int tid = threadIdx.x, lane = tid & 31, nthreads = blockDim.x, vwarps = T >> 5;
+    uint4 a[NV], b[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int k0 = (tid + j * nthreads) * 8;
+        a[j] = k0 < K ? ld_cg_128(xr + k0) : make_uint4(0, 0, 0, 0);
+        if (GATED) b[j] = k0 < K ? ld_cg_128(xr + K + k0) : make_uint4(0, 0, 0, 0);
+    }
+    float f[NV][8], ss[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const uint32_t av[4] = {a[j].x, a[j].y, a[j].z, a[j].w};
+        const uint32_t bv[4] = {b[j].x, b[j].y, b[j].z, b[j].w};
+        ss[j] = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            f[j][i] = __uint_as_float((i & 1) ? (av[i >> 1] & 0xFFFF0000u) : (av[i >> 1] << 16));
+            if (GATED) {
+                const float r = fmaxf(f[j][i], 0.f);
+                const float x3 = __uint_as_float((i & 1) ? (bv[i >> 1] & 0xFFFF0000u) : (bv[i >> 1] << 16));
+                f[j][i] = bf16_round_f(bf16_round_f(r * r) * x3);   // relu(x1) ** 2, bf16; * x3, bf16
+            }
+            ss[j] = __fadd_rn(ss[j], __fmul_rn(f[j][i], f[j][i]));
+        }
+    }
+    if (MODE != ACT_PLAIN) {
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1)
+#pragma unroll
+            for (int j = 0; j < NV; ++j) ss[j] += __shfl_xor_sync(0xffffffffu, ss[j], d);
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const int vw = (tid + j * nthreads) >> 5;
+            if (lane == 0 && vw < vwarps) part[vw] = ss[j];
+        }
+        __syncthreads();
+        float sum = 0.f;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            if (4 * c >= vwarps) break;
+            const float4 v = *reinterpret_cast<const float4*>(part + 4 * c);
+            sum = c == 0 ? v.x : sum + v.x;      // (T is at least 64: two warps or more)
+            if (4 * c + 1 < vwarps) sum += v.y;
+            if (4 * c + 2 < vwarps) sum += v.z;
+            if (4 * c + 3 < vwarps) sum += v.w;
+        }
+        if (MODE == ACT_SCALE_SUMSQ && tid == 0) *ss_out = sum;
+        const float rstd = (MODE == ACT_RMSNORM || MODE == ACT_NORM_ONLY)
+                               ? __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)K), eps))) : 1.f;
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const uint32_t wv[4] = {nw[j].x, nw[j].y, nw[j].z, nw[j].w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float w = __uint_as_float((i & 1) ? (wv[i >> 1] & 0xFFFF0000u) : (wv[i >> 1] << 16));
+                f[j][i] = bf16_round_f(__fmul_rn(MODE == ACT_SCALE_SUMSQ ? f[j][i] : __fmul_rn(f[j][i], rstd), w));
+            }
+        }
+    }
+    if (MODE == ACT_NORM_ONLY) {
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const int k0 = (tid + j * nthreads) * 8;
+            uint32_t o[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) o[i] = (__float_as_uint(f[j][2 * i]) >> 16) | (__float_as_uint(f[j][2 * i + 1]) & 0xFFFF0000u);
+            if (k0 < K) store(k0, make_uint4(o[0], o[1], o[2], o[3]));
+        }
+        return 0.f;
+    }
+    uint32_t mx[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        mx[j] = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) mx[j] = max(mx[j], __float_as_uint(f[j][i]) & 0x7FFFFFFFu);
+        mx[j] = warp_max_u32(mx[j]);
+        const int vw = (tid + j * nthreads) >> 5;
+        if (lane == 0 && vw < vwarps) mxp[vw] = mx[j];
+    }
+    __syncthreads();
+    const float top = __uint_as_float(warp_max_u32(lane < vwarps ? mxp[lane] : 0u));
+    const float amax = bf16_round_f(top < 1e-5f ? 1e-5f : top);
+    const float s = bf16_round_f(bf16_round_f(1.0f / amax) * 127.0f);   // 127 / amax as reciprocal * 127, in bf16
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int k0 = (tid + j * nthreads) * 8;
+        uint32_t o[2] = {0u, 0u};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int v = max(min(__float2int_rn(bf16_round_f(f[j][i] * s)), 127), -128);
+            o[i >> 2] |= (uint32_t)(v & 0xFF) << (8 * (i & 3));
+        }
+        if (k0 < K) store(k0, make_uint4(o[0], o[1], 0u, 0u));
+    }
+    return s;
+}
+
+// Rows of at most 8192 elements: one CTA per row, T threads with one vector each (row_front_end).
 // x: [M][ld] bf16 (GATED: the row holds [x1 (K) | x3 (K)], ld = 2K), w: [K] bf16 norm weight,
-// q: [M][K] int8, s_out: [M] bf16, ss_out: [M] fp32 (MODE 1).  Dynamic shared memory: K bf16.
+// q: [M][K] int8, s_out: [M] bf16, ss_out: [M] fp32 (MODE 1).
+template <bool GATED, int MODE>
+__global__ void __launch_bounds__(kActMaxThreads) norm_quant_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                                                                        float eps, int K, int8_t* __restrict__ q,
+                                                                        __nv_bfloat16* __restrict__ s_out, float* __restrict__ ss_out) {
+    __shared__ __align__(16) float part[32];
+    __shared__ uint32_t mxp[32];
+    griddep_launch_dependents();
+    const int t = blockIdx.x, tid = threadIdx.x;
+    uint4 nw[1] = {make_uint4(0, 0, 0, 0)};
+    if (MODE != ACT_PLAIN && tid * 8 < K) nw[0] = __ldg(reinterpret_cast<const uint4*>(w) + tid);   // weights: before the wait
+    griddep_wait();   // the activations come from the previous kernel
+    const float s = row_front_end<1, GATED, MODE>(x + (size_t)t * (GATED ? 2 * K : K), nw, eps, K, (int)blockDim.x, part, mxp,
+                                                  MODE == ACT_SCALE_SUMSQ ? ss_out + t : nullptr, [&](int k0, const uint4& v) {
+        if (MODE == ACT_NORM_ONLY) *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(q) + (size_t)t * K + k0) = v;
+        else *reinterpret_cast<uint2*>(q + (size_t)t * K + k0) = make_uint2(v.x, v.y);
+    });
+    if (MODE != ACT_NORM_ONLY && tid == 0) s_out[t] = __float2bfloat16_rn(s);
+}
+
+// Longer rows, staged in shared memory: same arguments, dynamic shared memory K bf16.
 template <bool GATED, int MODE>
 __global__ void __launch_bounds__(kActMaxThreads) norm_quant_kernel(const __nv_bfloat16* __restrict__ x,
                                                                   const __nv_bfloat16* __restrict__ w, float eps,
@@ -118,11 +256,11 @@ __global__ void __launch_bounds__(kActMaxThreads) norm_quant_kernel(const __nv_b
             else *reinterpret_cast<uint4*>(row + k0) = a;
         }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(__bfloat162float(av[i])));
+        for (int i = 0; i < 8; ++i) amax = nan_max(amax, fabsf(__bfloat162float(av[i])));
     }
     if (MODE == ACT_NORM_ONLY) return;
     amax = block_reduce(amax, scratch, true);
-    amax = bf16_round_f(fmaxf(amax, 1e-5f));
+    amax = bf16_round_f(amax < 1e-5f ? 1e-5f : amax);
     const float s = bf16_round_f(bf16_round_f(1.0f / amax) * 127.0f);   // 127 / amax as reciprocal * 127, in bf16
     if (tid == 0) s_out[t] = __float2bfloat16_rn(s);
 
@@ -132,7 +270,7 @@ __global__ void __launch_bounds__(kActMaxThreads) norm_quant_kernel(const __nv_b
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             const float p = bf16_round_f(__bfloat162float(row[k0 + i]) * s);
-            o[i] = (int8_t)fminf(fmaxf(rintf(p), -128.f), 127.f);
+            o[i] = (int8_t)max(min(__float2int_rn(p), 127), -128);
         }
         *reinterpret_cast<uint4*>(q + (size_t)t * K + k0) = *reinterpret_cast<const uint4*>(o);
     }

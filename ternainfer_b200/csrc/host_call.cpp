@@ -1,0 +1,273 @@
+// The call site of one ternary linear as a CPython extension type.
+//
+// An eager call of a small layer costs a few microseconds on the GPU; done in
+// Python - shape checks, torch.empty, the current stream, fifteen ctypes
+// arguments, the quantiser as eight torch operators - its host side took 18 us
+// (int8 input) to 85 us (bf16 input).  `Layer` does all of it in one native call.
+//
+// A Layer also keeps the module's weights in the two-bit layout of w2_small.cuh, which
+// is laid out once from the packed checkpoint tensors and again whenever those have
+// changed: their addresses and version counters are compared on every call (tensors
+// made in inference mode have no version counter; SpBitLinear drops the layout when
+// a state dict is loaded into it).  A layout that is out of date while the stream is
+// being captured is not rebuilt there: that call reads the packed tensors.
+//
+// Every method returns None where the native path does not apply (other devices,
+// types or sizes); the caller then takes the general path in linear.py.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <cuda_runtime_api.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include "ternaspmm.h"
+
+namespace {
+
+constexpr int64_t kSmallTokens = 32;   // the mma.sync kernel on two-bit weights; above it the tensor-core paths of the library
+
+PyObject* g_keys[5];                   // interned parameter names, in the order of Weights
+
+struct Weights {
+    const at::Tensor *signs, *tile_offsets, *quarter_offsets, *bitmap, *scale;
+};
+
+struct Layer {
+    PyObject_HEAD
+    int in_features, out_features, ws_num, seg[3];
+    bool valid;                        // w2 was laid out from the tensors recorded below
+    const void* src_ptr[4];
+    int64_t src_version[4];
+    at::Tensor* w2;
+};
+
+int64_t version_of(const at::Tensor& t) { return t.is_inference() ? 0 : t._version(); }
+
+bool get_weights(PyObject* params, Weights& w) {
+    const at::Tensor** dst[5] = {&w.signs, &w.tile_offsets, &w.quarter_offsets, &w.bitmap, &w.scale};
+    for (int i = 0; i < 5; ++i) {
+        PyObject* o = PyDict_GetItem(params, g_keys[i]);   // borrowed
+        if (!o || !THPVariable_Check(o)) return false;
+        *dst[i] = &THPVariable_Unpack(o);
+        if (!(*dst[i])->is_cuda() || !(*dst[i])->is_contiguous()) return false;
+    }
+    return w.scale->scalar_type() == at::kBFloat16 && w.scale->numel() >= 4;
+}
+
+bool capturing(cudaStream_t stream) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
+}
+
+// The two-bit weights, up to date; null where there are none (wrong sizes, out of date during a capture).
+void* two_bit(Layer* self, const Weights& w, cudaStream_t stream) {
+    const at::Tensor* src[4] = {w.signs, w.tile_offsets, w.quarter_offsets, w.bitmap};
+    bool fresh = self->valid;
+    for (int i = 0; i < 4 && fresh; ++i)
+        fresh = src[i]->data_ptr() == self->src_ptr[i] && version_of(*src[i]) == self->src_version[i];
+    if (fresh) return self->w2->data_ptr();
+    self->valid = false;
+    const int64_t N = self->out_features, K = self->in_features;
+    if (N < 64 || K < 64 || N % 64 || K % 64 || K >= (1 << 18) || w.bitmap->nbytes() < (size_t)(N * K / 8) ||
+        w.tile_offsets->numel() < N * K / 4096 + 1 || capturing(stream))
+        return nullptr;
+    if (!self->w2->defined() || self->w2->device() != w.bitmap->device())
+        *self->w2 = at::empty({ternaspmm_w2_bytes((int)N, (int)K)}, w.bitmap->options().dtype(at::kByte));
+    ternaspmm_w2_relayout(static_cast<uint64_t*>(w.bitmap->data_ptr()), static_cast<int*>(w.tile_offsets->data_ptr()),
+                          static_cast<uint16_t*>(w.quarter_offsets->data_ptr()), static_cast<uint32_t*>(w.signs->data_ptr()), (int)N,
+                          (int)K, self->w2->data_ptr(), stream);
+    if (cudaStreamSynchronize(stream) != cudaSuccess) return nullptr;   // other streams may use the layer next
+    for (int i = 0; i < 4; ++i) self->src_ptr[i] = src[i]->data_ptr(), self->src_version[i] = version_of(*src[i]);
+    self->valid = true;
+    return self->w2->data_ptr();
+}
+
+at::Tensor output_like(const at::Tensor& x, int64_t N) {
+    c10::SmallVector<int64_t, 5> shape(x.sizes().begin(), x.sizes().end());
+    shape.back() = N;
+    return at::empty(shape, x.options().dtype(at::kBFloat16));
+}
+
+// A contiguous, 16-byte aligned CUDA tensor of this type whose last dimension is K.
+bool usable(PyObject* o, at::ScalarType type, int64_t K) {
+    if (!THPVariable_Check(o)) return false;
+    const at::Tensor& t = THPVariable_Unpack(o);
+    return t.is_cuda() && t.scalar_type() == type && t.dim() >= 1 && t.size(-1) == K && t.numel() > 0 && t.is_contiguous() &&
+           !(reinterpret_cast<uintptr_t>(t.data_ptr()) & 15);
+}
+
+void run_linear(Layer* self, const Weights& w, void* w2, void* x, int front_end, void* norm_w, float eps, at::Tensor& out, void* s,
+                int64_t M, void* residual, cudaStream_t stream) {
+    ternaspmm_w2_linear(x, front_end, static_cast<ternaspmm_bf16*>(norm_w), eps, w2, static_cast<ternaspmm_bf16*>(out.data_ptr()),
+                        static_cast<ternaspmm_bf16*>(s), static_cast<ternaspmm_bf16*>(w.scale->data_ptr()), self->ws_num, (int)M,
+                        self->out_features, self->in_features, self->seg[0], self->seg[1], self->seg[2], -1,
+                        static_cast<ternaspmm_bf16*>(residual), stream);
+}
+
+void* residual_ptr(PyObject* o, int64_t M, int64_t N, bool& ok) {   // None, or contiguous bf16 of M*N values
+    ok = true;
+    if (o == Py_None) return nullptr;
+    ok = usable(o, at::kBFloat16, N) && THPVariable_Unpack(o).numel() == M * N;
+    return ok ? THPVariable_Unpack(o).data_ptr() : nullptr;
+}
+
+// int8 rows and scales in one allocation: [M][K] int8, then [M] bf16.
+at::Tensor quantised_buffer(const at::Tensor& x, int64_t M, int64_t K) {
+    return at::empty({M * K + 2 * M}, x.options().dtype(at::kByte));
+}
+
+// front-end + linear of bf16 activations: in one kernel for the smallest calls, else as two launches
+PyObject* front_and_linear(Layer* self, PyObject* params, PyObject* xo, int front_end, PyObject* norm_o, float eps, PyObject* res_o) {
+    const int64_t K = self->in_features;
+    const bool gated = front_end == 3;
+    if (!usable(xo, at::kBFloat16, gated ? 2 * K : K)) Py_RETURN_NONE;
+    const at::Tensor& x = THPVariable_Unpack(xo);
+    const int64_t M = x.numel() / x.size(-1);
+    if (M > kSmallTokens) Py_RETURN_NONE;
+    void* norm_w = nullptr;
+    if (norm_o) {
+        if (!usable(norm_o, at::kBFloat16, K) || THPVariable_Unpack(norm_o).numel() != K) Py_RETURN_NONE;
+        norm_w = THPVariable_Unpack(norm_o).data_ptr();
+    }
+    bool ok;
+    void* residual = residual_ptr(res_o, M, self->out_features, ok);
+    Weights w;
+    if (!ok || !get_weights(params, w) || w.bitmap->device() != x.device()) Py_RETURN_NONE;
+    c10::cuda::OptionalCUDAGuard guard(x.device());
+    cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
+    void* w2 = two_bit(self, w, stream);
+    if (!w2) Py_RETURN_NONE;
+    at::Tensor out = output_like(x, self->out_features);
+    if (M <= ternaspmm_w2_fused_rows((int)K) && M <= (front_end == 1 ? 4 : 1)) {
+        run_linear(self, w, w2, x.data_ptr(), front_end, norm_w, eps, out, nullptr, M, residual, stream);
+        return THPVariable_Wrap(std::move(out));
+    }
+    if (K > 56 * 1024) Py_RETURN_NONE;
+    at::Tensor buf = quantised_buffer(x, M, K);
+    int8_t* q = static_cast<int8_t*>(buf.data_ptr());
+    ternaspmm_bf16* s = reinterpret_cast<ternaspmm_bf16*>(q + M * K);
+    ternaspmm_bf16* xp = static_cast<ternaspmm_bf16*>(x.data_ptr());
+    if (front_end == 1) ternaspmm_quant(xp, (int)M, (int)K, q, s, stream);
+    else if (gated) ternaspmm_relu2_gate_rmsnorm_quant(xp, static_cast<ternaspmm_bf16*>(norm_w), eps, (int)M, (int)K, q, s, stream);
+    else ternaspmm_rmsnorm_quant(xp, static_cast<ternaspmm_bf16*>(norm_w), eps, (int)M, (int)K, q, s, stream);
+    run_linear(self, w, w2, q, 0, nullptr, 0.f, out, s, M, residual, stream);
+    return THPVariable_Wrap(std::move(out));
+}
+
+// forward(params, x): per-token int8 quantiser, then the linear
+PyObject* layer_forward(PyObject* o, PyObject* const* args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 2) return PyErr_Format(PyExc_TypeError, "forward(params, x)");
+    return front_and_linear(reinterpret_cast<Layer*>(o), args[0], args[1], 1, nullptr, 0.f, Py_None);
+    END_HANDLE_TH_ERRORS
+}
+
+// forward_normed(params, x, norm_weight, eps, gated, residual): (gate,) RMSNorm, quantiser, linear, residual add
+PyObject* layer_forward_normed(PyObject* o, PyObject* const* args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 6) return PyErr_Format(PyExc_TypeError, "forward_normed(params, x, norm_weight, eps, gated, residual)");
+    const double eps = PyFloat_AsDouble(args[3]);
+    if (PyErr_Occurred()) return nullptr;
+    return front_and_linear(reinterpret_cast<Layer*>(o), args[0], args[1], PyObject_IsTrue(args[4]) ? 3 : 2, args[2], (float)eps, args[5]);
+    END_HANDLE_TH_ERRORS
+}
+
+// forward_quantized(params, x_q, s, residual): int8 activations and their scales in hand
+PyObject* layer_forward_quantized(PyObject* o, PyObject* const* args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 4) return PyErr_Format(PyExc_TypeError, "forward_quantized(params, x_q, s, residual)");
+    Layer* self = reinterpret_cast<Layer*>(o);
+    const int64_t K = self->in_features;
+    if (!usable(args[1], at::kChar, K) || !THPVariable_Check(args[2])) Py_RETURN_NONE;
+    const at::Tensor &x = THPVariable_Unpack(args[1]), &s = THPVariable_Unpack(args[2]);
+    const int64_t M = x.numel() / K;
+    if (M > kSmallTokens || s.scalar_type() != at::kBFloat16 || !s.is_contiguous() || s.numel() != M || s.device() != x.device())
+        Py_RETURN_NONE;
+    bool ok;
+    void* residual = residual_ptr(args[3], M, self->out_features, ok);
+    Weights w;
+    if (!ok || !get_weights(args[0], w) || w.bitmap->device() != x.device()) Py_RETURN_NONE;
+    c10::cuda::OptionalCUDAGuard guard(x.device());
+    cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
+    void* w2 = two_bit(self, w, stream);
+    if (!w2) Py_RETURN_NONE;
+    at::Tensor out = output_like(x, self->out_features);
+    run_linear(self, w, w2, x.data_ptr(), 0, nullptr, 0.f, out, s.data_ptr(), M, residual, stream);
+    return THPVariable_Wrap(std::move(out));
+    END_HANDLE_TH_ERRORS
+}
+
+// prepare(params): lay the weights out now instead of in the first call
+PyObject* layer_prepare(PyObject* o, PyObject* params) {
+    HANDLE_TH_ERRORS
+    Weights w;
+    if (!get_weights(params, w)) Py_RETURN_FALSE;
+    c10::cuda::OptionalCUDAGuard guard(w.bitmap->device());
+    return PyBool_FromLong(two_bit(reinterpret_cast<Layer*>(o), w, c10::cuda::getCurrentCUDAStream().stream()) != nullptr);
+    END_HANDLE_TH_ERRORS
+}
+
+PyObject* layer_invalidate(PyObject* o, PyObject*) {
+    reinterpret_cast<Layer*>(o)->valid = false;
+    Py_RETURN_NONE;
+}
+
+// copies and pickles carry the sizes; the weights are laid out again where they are used
+PyObject* layer_reduce(PyObject* o, PyObject*) {
+    Layer* self = reinterpret_cast<Layer*>(o);
+    return Py_BuildValue("O(iiiiii)", Py_TYPE(o), self->in_features, self->out_features, self->ws_num, self->seg[0], self->seg[1], self->seg[2]);
+}
+
+PyObject* layer_new(PyTypeObject* type, PyObject* args, PyObject*) {
+    Layer* self = reinterpret_cast<Layer*>(type->tp_alloc(type, 0));
+    if (!self) return nullptr;
+    self->w2 = new at::Tensor();
+    self->valid = false;
+    if (!PyArg_ParseTuple(args, "iiiiii", &self->in_features, &self->out_features, &self->ws_num, &self->seg[0], &self->seg[1], &self->seg[2])) {
+        Py_DECREF(self);
+        return nullptr;
+    }
+    return reinterpret_cast<PyObject*>(self);
+}
+
+void layer_dealloc(PyObject* o) {
+    delete reinterpret_cast<Layer*>(o)->w2;
+    Py_TYPE(o)->tp_free(o);
+}
+
+PyMethodDef layer_methods[] = {
+    {"forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(layer_forward)), METH_FASTCALL, nullptr},
+    {"forward_normed", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(layer_forward_normed)), METH_FASTCALL, nullptr},
+    {"forward_quantized", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(layer_forward_quantized)), METH_FASTCALL, nullptr},
+    {"prepare", layer_prepare, METH_O, nullptr},
+    {"invalidate", layer_invalidate, METH_NOARGS, nullptr},
+    {"__reduce__", layer_reduce, METH_NOARGS, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+
+PyTypeObject layer_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
+
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host_call", "Native call site of the ternary linears.", -1, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host_call() {
+    static const char* const names[5] = {"weight_compressed_val", "weight_TileOffsets_global", "weight_TileOffsets_median", "weight_bitmap",
+                                         "weight_scale"};
+    for (int i = 0; i < 5; ++i) g_keys[i] = PyUnicode_InternFromString(names[i]);
+    layer_type.tp_name = "_host_call.Layer";
+    layer_type.tp_basicsize = sizeof(Layer);
+    layer_type.tp_flags = Py_TPFLAGS_DEFAULT;
+    layer_type.tp_new = layer_new;
+    layer_type.tp_dealloc = layer_dealloc;
+    layer_type.tp_methods = layer_methods;
+    if (PyType_Ready(&layer_type) < 0) return nullptr;
+    PyObject* m = PyModule_Create(&module_def);
+    if (!m) return nullptr;
+    Py_INCREF(&layer_type);
+    PyModule_AddObject(m, "Layer", reinterpret_cast<PyObject*>(&layer_type));
+    return m;
+}

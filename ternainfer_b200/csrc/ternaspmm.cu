@@ -24,6 +24,7 @@
 #include "spmm_large_m.cuh"
 #include "spmm_list.cuh"
 #include "spmm_small_m.cuh"
+#include "w2_small.cuh"
 
 namespace tsp {
 
@@ -359,6 +360,23 @@ static cudaError_t launch_dense_pair(const SpmmParams& p_in, cudaStream_t stream
     return cudaLaunchKernelEx(&cfg, kern, p, map, wmap);
 }
 
+// Scale-segment boundaries of a call (see ws_group): explicit ones, or the reference's rules.
+static void set_segments(SpmmParams& p, const int* seg_bounds) {
+    if (seg_bounds) {
+        for (int i = 0; i < 3; ++i) p.seg_b[i] = (i + 1 < p.ws_num) ? seg_bounds[i] : INT_MAX;
+        p.seg_gran = 1;
+        return;
+    }
+    const bool prefill = p.epilogue == EPI_PREFILL;
+    p.seg_gran = prefill ? 128 : 8;
+    if (p.N == 3840 && (prefill || p.ws_num == 3)) {
+        p.seg_b[0] = 2560, p.seg_b[1] = 3200, p.seg_b[2] = INT_MAX;
+    } else {
+        const int gw = p.ws_num > 0 ? p.N / p.ws_num : p.N;
+        p.seg_b[0] = gw, p.seg_b[1] = 2 * gw, p.seg_b[2] = 3 * gw;
+    }
+}
+
 static void run_spmm(int8_t* x, uint64_t* bitmap, int* tile_off, uint16_t* quarter_off, uint32_t* signs, void* out,
                      __nv_bfloat16* s, __nv_bfloat16* ws, int ws_num, int M, int N, int K, int epilogue,
                      cudaStream_t stream, const int* seg_bounds = nullptr, const __nv_bfloat16* residual = nullptr) {
@@ -392,19 +410,7 @@ static void run_spmm(int8_t* x, uint64_t* bitmap, int* tile_off, uint16_t* quart
     p.N = N;
     p.K = K;
     p.epilogue = epilogue;
-    if (seg_bounds) {   // explicit segment boundaries
-        for (int i = 0; i < 3; ++i) p.seg_b[i] = (i + 1 < ws_num) ? seg_bounds[i] : INT_MAX;
-        p.seg_gran = 1;
-    } else {            // the reference's rules, see ws_group()
-        const bool prefill = epilogue == EPI_PREFILL;
-        p.seg_gran = prefill ? 128 : 8;
-        if (N == 3840 && (prefill || ws_num == 3)) {
-            p.seg_b[0] = 2560, p.seg_b[1] = 3200, p.seg_b[2] = INT_MAX;
-        } else {
-            const int gw = ws_num > 0 ? N / ws_num : N;
-            p.seg_b[0] = gw, p.seg_b[1] = 2 * gw, p.seg_b[2] = 3 * gw;
-        }
-    }
+    set_segments(p, seg_bounds);
     p.status = status_device_ptr();
     if (!p.status) {
         t_host_status = ST_LAUNCH;
@@ -576,16 +582,7 @@ extern "C" void bitlinear_TernaSpMM_ws(int8_t* x, uint64_t* bitmap, int* tile_of
     p.x = x, p.bitmap = reinterpret_cast<const uint32_t*>(bitmap), p.tile_off = tile_offsets, p.quarter_off = quarter_offsets;
     p.signs = sign_words, p.out = out, p.s = s, p.ws = ws, p.residual = residual;
     p.ws_num = ws_num, p.M = M, p.N = N, p.K = K, p.epilogue = epilogue, p.splits = 1;
-    {   // the reference's scale-segment rules (see ws_group in spmm_small_m.cuh)
-        const bool prefill = epilogue == EPI_PREFILL;
-        p.seg_gran = prefill ? 128 : 8;
-        if (N == 3840 && (prefill || ws_num == 3)) {
-            p.seg_b[0] = 2560, p.seg_b[1] = 3200, p.seg_b[2] = INT_MAX;
-        } else {
-            const int gw = N / ws_num;
-            p.seg_b[0] = gw, p.seg_b[1] = 2 * gw, p.seg_b[2] = 3 * gw;
-        }
-    }
+    set_segments(p, nullptr);
     p.status = status_device_ptr();
     if (!p.status) {
         t_host_status = ST_LAUNCH;
@@ -631,6 +628,138 @@ extern "C" void ternaspmm_linear_segments(int8_t* x, uint64_t* bitmap, int* tile
     checkLastCudaError(__LINE__);
 }
 
+// ---- linears on two-bit weights (w2_small.cuh) -----------------------------------------------------
+constexpr int kW2MaxSmem = 227 * 1024;
+
+template <int MT, int RG, int U, int FE, bool XS>
+static cudaError_t launch_w2_small(W2Params& p, cudaStream_t stream) {
+    static bool attr_done[64] = {false};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) dev = 0;
+    auto kern = w2_small_kernel<MT, RG, U, FE, XS>;
+    if (!attr_done[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kW2MaxSmem);
+        if (e != cudaSuccess) return e;
+        attr_done[dev] = true;
+    }
+    const int K = p.e.K, KP = w2_pairs(K);
+    const int blocks = (p.e.M + MT * 8 - 1) / (MT * 8), tokens = std::min(p.e.M, MT * 8);
+    // CTAs: one per SM (fewer when there are fewer strips), so that every SM gets the same share within a strip
+    const int strips = p.e.N / 16, ctas = std::min(strips, std::max(1, device_sm_count() / blocks)), R = (strips + ctas - 1) / ctas;
+    p.strips_q = strips / ctas, p.strips_r = strips % ctas;
+    // warps: as many as have a block pair of their own, at most ten (two CTAs of that size share the register file, so
+    // the next launch's CTA starts beside this one), evenly loaded; at least four for the front-end and the epilogue
+    const int per = (KP + kW2MaxWarps - 1) / kW2MaxWarps, W = std::max(4, (KP + per - 1) / per);
+    p.pairs_q = KP / W, p.pairs_r = KP % W;
+    // ring: all of the CTA's weights when they fit 64 KB (two launches' prefetches fit an SM side by side), otherwise
+    // slots of about 32 KB per CTA and up to four of them
+    const int groups = (R + RG - 1) / RG;
+    p.chunk_pairs = std::max(1, std::min(per, 32 * 1024 / (W * RG * 512)));
+    const int chunks = groups * ((per + p.chunk_pairs - 1) / p.chunk_pairs), slot_bytes = RG * p.chunk_pairs * 512;
+    const int fit = 64 * 1024 / (W * slot_bytes);
+    p.slots = std::min(chunks, chunks <= fit && chunks <= kW2MaxSlots ? chunks : 4);
+    p.smem = w2_smem(R, MT, tokens, K, W, p.slots, slot_bytes, XS);
+    while (p.smem.total > kW2MaxSmem && p.slots > 1) {
+        --p.slots;
+        p.smem = w2_smem(R, MT, tokens, K, W, p.slots, slot_bytes, XS);
+    }
+    if (p.smem.total > kW2MaxSmem) return cudaErrorInvalidValue;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas, blocks, 1);
+    cfg.blockDim = dim3(W * 32, 1, 1);
+    cfg.dynamicSmemBytes = p.smem.total;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = tuning().pdl ? 1 : 0;
+    t_echo = {8, MT * 8, 1, W, R, (int)(cfg.gridDim.x * cfg.gridDim.y)};
+    return cudaLaunchKernelEx(&cfg, kern, p);
+}
+
+// RG: strips whose accumulators a warp holds at a time; one where a CTA has one or two strips.  XS: activations in shared
+// memory while they leave room for the ring.
+template <int FE>
+static cudaError_t launch_w2_fused(W2Params& p, cudaStream_t stream) {
+    return p.e.N / 16 <= 2 * device_sm_count() ? launch_w2_small<1, 1, 2, FE, true>(p, stream) : launch_w2_small<1, 3, 2, FE, true>(p, stream);
+}
+
+static cudaError_t launch_w2_int8(W2Params& p, cudaStream_t stream) {
+    const int M = p.e.M;
+    const bool xs = (long long)std::min(M, 32) * (p.e.K + 64) <= 96 * 1024;
+    if (M <= 8) return xs ? launch_w2_fused<W2_INT8>(p, stream) : launch_w2_small<1, 3, 1, W2_INT8, false>(p, stream);
+    if (M <= 16) return xs ? launch_w2_small<2, 2, 2, W2_INT8, true>(p, stream) : launch_w2_small<2, 2, 1, W2_INT8, false>(p, stream);
+    return xs ? launch_w2_small<4, 2, 1, W2_INT8, true>(p, stream) : launch_w2_small<4, 2, 1, W2_INT8, false>(p, stream);
+}
+
+// Bytes of a weight's two-bit layout.
+extern "C" long long ternaspmm_w2_bytes(int N, int K) { return N < 16 || K < 64 ? 0 : (long long)(N / 16) * w2_pairs(K) * 512; }
+
+extern "C" void ternaspmm_w2_relayout(uint64_t* bitmap, int* tile_offsets, uint16_t* quarter_offsets, uint32_t* sign_words,
+                                      int N, int K, void* w2, cudaStream_t stream) {
+    t_host_status = ST_OK;
+    if (N < 64 || K < 64 || (N % 64) || (K % 64)) {
+        t_host_status = ST_BAD_SHAPE;
+        return;
+    }
+    if (!bitmap || !tile_offsets || !quarter_offsets || !sign_words || !w2 || (reinterpret_cast<uintptr_t>(bitmap) & 15) ||
+        (reinterpret_cast<uintptr_t>(w2) & 15)) {
+        t_host_status = ST_BAD_POINTER;
+        return;
+    }
+    SpmmParams p = {};
+    p.bitmap = reinterpret_cast<const uint32_t*>(bitmap), p.tile_off = tile_offsets, p.quarter_off = quarter_offsets;
+    p.signs = sign_words, p.N = N, p.K = K;
+    const long long tiles = (long long)(N / 64) * (K / 64);
+    relayout_w2_kernel<<<(unsigned)((tiles + 7) / 8), 256, 0, stream>>>(p, static_cast<uint8_t*>(w2));
+    checkLastCudaError(__LINE__);
+}
+
+// Rows that a front-end inside the kernel takes: a thread holds at most two eight-element vectors of a row.
+extern "C" int ternaspmm_w2_fused_rows(int K) { return K < 64 || K > 8 * kActMaxThreads ? 0 : kW2MaxFusedRows; }
+
+extern "C" void ternaspmm_w2_linear(void* x, int front_end, __nv_bfloat16* norm_weight, float eps, void* w2, __nv_bfloat16* out,
+                                    __nv_bfloat16* s, __nv_bfloat16* ws, int ws_num, int M, int N, int K, int seg1, int seg2,
+                                    int seg3, int prefill_form, __nv_bfloat16* residual, cudaStream_t stream) {
+    t_host_status = ST_OK;
+    if (M < 1 || N < 64 || K < 64 || (N % 64) || (K % 64) || K >= (1 << 18) || ws_num < 1 || ws_num > 4 || front_end < W2_INT8 ||
+        front_end > W2_GATED || (front_end != W2_INT8 && M > ternaspmm_w2_fused_rows(K))) {
+        fprintf(stderr, "ternaspmm: w2_linear: unsupported shape M=%d N=%d K=%d ws_num=%d front_end=%d\n", M, N, K, ws_num, front_end);
+        t_host_status = ST_BAD_SHAPE;
+        return;
+    }
+    if (!x || !w2 || !out || !ws || (front_end == W2_INT8 && !s) || (front_end >= W2_NORM && !norm_weight) ||
+        (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(w2) & 15) || (reinterpret_cast<uintptr_t>(norm_weight) & 15)) {
+        fprintf(stderr, "ternaspmm: w2_linear: null or misaligned pointer (x, w2, norm_weight: 16 bytes)\n");
+        t_host_status = ST_BAD_POINTER;
+        return;
+    }
+    W2Params p = {};
+    p.e.x = static_cast<const int8_t*>(x), p.xb = static_cast<const __nv_bfloat16*>(x);
+    p.norm_w = norm_weight, p.eps = eps, p.w = static_cast<const uint8_t*>(w2);
+    p.e.out = out, p.e.s = s, p.e.ws = ws, p.e.residual = residual, p.e.ws_num = ws_num, p.e.M = M, p.e.N = N, p.e.K = K;
+    p.e.epilogue = prefill_form < 0 ? (M <= 64 ? EPI_DECODE : EPI_PREFILL) : (prefill_form ? EPI_PREFILL : EPI_DECODE);
+    const int seg[3] = {seg1, seg2, seg3};
+    set_segments(p.e, seg1 | seg2 | seg3 ? seg : nullptr);
+    p.e.status = status_device_ptr();
+    if (!p.e.status) {
+        t_host_status = ST_LAUNCH;
+        return;
+    }
+    cudaError_t e;
+    if (front_end == W2_PLAIN) e = launch_w2_fused<W2_PLAIN>(p, stream);
+    else if (front_end == W2_NORM) e = launch_w2_fused<W2_NORM>(p, stream);
+    else if (front_end == W2_GATED) e = launch_w2_fused<W2_GATED>(p, stream);
+    else e = launch_w2_int8(p, stream);
+    if (e != cudaSuccess) {
+        fprintf(stderr, "ternaspmm: launch failed: %s\n", cudaGetErrorString(e));
+        t_host_status = ST_LAUNCH;
+    }
+    checkLastCudaError(__LINE__);
+}
+
 static void run_norm_quant(bool gated, int mode, __nv_bfloat16* x, __nv_bfloat16* w, float eps, int M, int K,
                            int8_t* q, __nv_bfloat16* s_out, float* ss_out, cudaStream_t stream) {
     t_host_status = ST_OK;
@@ -647,24 +776,29 @@ static void run_norm_quant(bool gated, int mode, __nv_bfloat16* x, __nv_bfloat16
         return;
     }
     typedef void (*Kern)(const __nv_bfloat16*, const __nv_bfloat16*, float, int, int8_t*, __nv_bfloat16*, float*);
-    Kern kern = gated ? (mode == ACT_RMSNORM ? norm_quant_kernel<true, ACT_RMSNORM> : norm_quant_kernel<true, ACT_SCALE_SUMSQ>)
-                      : mode == ACT_NORM_ONLY ? norm_quant_kernel<false, ACT_NORM_ONLY>
-                      : (mode == ACT_RMSNORM ? norm_quant_kernel<false, ACT_RMSNORM>
-                                             : (mode == ACT_SCALE_SUMSQ ? norm_quant_kernel<false, ACT_SCALE_SUMSQ>
-                                                                        : norm_quant_kernel<false, ACT_PLAIN>));
+    static const Kern in_regs[5] = {norm_quant_row_kernel<false, ACT_RMSNORM>, norm_quant_row_kernel<false, ACT_SCALE_SUMSQ>,
+                                    norm_quant_row_kernel<false, ACT_PLAIN>, norm_quant_row_kernel<false, ACT_NORM_ONLY>, nullptr};
+    static const Kern in_smem[5] = {norm_quant_kernel<false, ACT_RMSNORM>, norm_quant_kernel<false, ACT_SCALE_SUMSQ>,
+                                    norm_quant_kernel<false, ACT_PLAIN>, norm_quant_kernel<false, ACT_NORM_ONLY>, nullptr};
+    const bool row_in_regs = K <= 8 * kActMaxThreads;   // one eight-element vector per thread
+    Kern kern = row_in_regs ? in_regs[mode] : in_smem[mode];
+    if (gated) {
+        if (mode == ACT_RMSNORM) kern = row_in_regs ? norm_quant_row_kernel<true, ACT_RMSNORM> : norm_quant_kernel<true, ACT_RMSNORM>;
+        else kern = row_in_regs ? norm_quant_row_kernel<true, ACT_SCALE_SUMSQ> : norm_quant_kernel<true, ACT_SCALE_SUMSQ>;
+    }
     static bool attr_done[64][8] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) dev = 0;
     const int slot = (gated ? 4 : 0) + mode;
-    if (!attr_done[dev][slot]) {
+    if (!row_in_regs && !attr_done[dev][slot]) {
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 56 * 1024);
         attr_done[dev][slot] = true;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(M, 1, 1);
     cfg.blockDim = dim3(std::min(kActMaxThreads, std::max(64, (K / 8 + 31) / 32 * 32)), 1, 1);   // one vector per thread
-    cfg.dynamicSmemBytes = (size_t)K * 2;
+    cfg.dynamicSmemBytes = row_in_regs ? 0 : (size_t)K * 2;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

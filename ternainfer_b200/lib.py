@@ -9,12 +9,14 @@ There is no fallback: if the library is missing, loading raises.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 import subprocess
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 _CSRC = os.path.join(_HERE, "csrc")
 _LIB = None
+_HOST = None
 
 _P = ctypes.c_void_p
 _I = ctypes.c_int
@@ -111,6 +113,14 @@ def load_library() -> ctypes.CDLL:
     lib.bitlinear_TernaSpMM_ws.restype = None
     lib.bitlinear_TernaSpMM_residual.argtypes = [_P] * 8 + [_I] * 4 + [_P, _P]
     lib.bitlinear_TernaSpMM_residual.restype = None
+    lib.ternaspmm_w2_relayout.argtypes = [_P, _P, _P, _P, _I, _I, _P, _P]
+    lib.ternaspmm_w2_relayout.restype = None
+    lib.ternaspmm_w2_bytes.argtypes = [_I, _I]
+    lib.ternaspmm_w2_bytes.restype = ctypes.c_longlong
+    lib.ternaspmm_w2_fused_rows.argtypes = [_I]
+    lib.ternaspmm_w2_fused_rows.restype = _I
+    lib.ternaspmm_w2_linear.argtypes = [_P, _I, _P, ctypes.c_float, _P, _P, _P, _P] + [_I] * 8 + [_P, _P]
+    lib.ternaspmm_w2_linear.restype = None
     lib.ternaspmm_pack_i8.argtypes = [_P, _I, _I, _P, _P, _P, _P]
     lib.ternaspmm_pack_i8.restype = ctypes.c_longlong
     lib.ternaspmm_unpack_i8.argtypes = [_P, _P, _P, _I, _I, _P]
@@ -119,6 +129,21 @@ def load_library() -> ctypes.CDLL:
     lib.ternaspmm_transcode_reference_layout.restype = _I
     _LIB = lib
     return lib
+
+
+def load_host_call():
+    """The native call site (``_host_call.so``: the extension type behind ``SpBitLinear``); raises if it has not been built."""
+    global _HOST
+    if _HOST is None:
+        import torch  # noqa: F401  (its libraries are what the extension links against)
+        load_library()
+        path = os.path.join(_CSRC, "_host_call.so")
+        if not os.path.exists(path):
+            raise OSError(f"{path} not found: build it with `make -C {_CSRC}` (or __graft_entry__.build())")
+        spec = importlib.util.spec_from_file_location("_host_call", path)
+        _HOST = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(_HOST)
+    return _HOST
 
 
 EXPORTED_SYMBOLS = (
@@ -130,5 +155,6 @@ EXPORTED_SYMBOLS = (
     "ternaspmm_list_plan", "ternaspmm_list_create", "ternaspmm_list_run", "ternaspmm_list_destroy",
     "ternaspmm_accumulate_i32", "ternaspmm_linear_segments", "bitlinear_TernaSpMM_residual", "bitlinear_TernaSpMM_ws", "ternaspmm_quant",
     "ternaspmm_scale_quant_sumsq", "ternaspmm_partial_f32", "ternaspmm_tp_finish", "ternaspmm_tp_allreduce_finish", "ternaspmm_rmsnorm_quant", "ternaspmm_relu2_gate_rmsnorm_quant", "ternaspmm_rmsnorm", "ternaspmm_pack_i8",
+    "ternaspmm_w2_relayout", "ternaspmm_w2_bytes", "ternaspmm_w2_fused_rows", "ternaspmm_w2_linear",
     "ternaspmm_unpack_i8", "ternaspmm_transcode_reference_layout",
 )

@@ -19,7 +19,7 @@ import ctypes
 import torch
 from torch import nn
 
-from .lib import load_library
+from .lib import load_host_call, load_library
 
 _GLOBAL_WORKSPACE = {}
 _WORKSPACE_BYTES = 13824 * 2560      # the largest BitNet-2B layer as dense int8, as model.py:34 of the reference sizes it
@@ -48,7 +48,18 @@ def get_global_workspace(device="cuda"):
 
 def quant_input(input: torch.Tensor):
     """Per-token absmax int8 quantisation (model.py:120-123):
-    s = 127 / clamp(max|x|, 1e-5); x_q = clamp(round(x*s), -128, 127)."""
+    s = 127 / clamp(max|x|, 1e-5); x_q = clamp(round(x*s), -128, 127).  bf16 activations on the GPU take one
+    kernel (the same values bit for bit; eight torch operators cost 60 us of launches for one token)."""
+    K = input.shape[-1]
+    if (input.is_cuda and input.dtype == torch.bfloat16 and K % 16 == 0 and K <= 57344 and input.numel() > 0
+            and not (input.requires_grad and torch.is_grad_enabled())):
+        x = input.contiguous()
+        if x.data_ptr() % 16 == 0:
+            q = torch.empty(x.shape, dtype=torch.int8, device=x.device)
+            s = torch.empty((*x.shape[:-1], 1), dtype=torch.bfloat16, device=x.device)
+            load_library().ternaspmm_quant(x.data_ptr(), x.numel() // K, K, q.data_ptr(), s.data_ptr(),
+                                           torch.cuda.current_stream(x.device).cuda_stream)
+            return q, s
     s = 127 / input.abs().max(dim=-1, keepdim=True).values.clamp_(min=1e-5)
     return (input * s).round().clamp(-128, 127).to(torch.int8), s
 
@@ -220,18 +231,43 @@ class SpBitLinear(nn.Module):
         self.segments = [int(v) for v in seg] if seg is not None else None
         if self.segments is not None:
             assert sum(self.segments) == out_features and len(self.segments) == self.ws_num
+        bounds = [0, 0, 0]
+        if not _builtin_segments(self.segments, out_features, self.ws_num):
+            bounds = [sum(self.segments[:i + 1]) for i in range(len(self.segments) - 1)] + [2 ** 31 - 1] * 3
+        # native call site; it keeps the weights in the layout of the small-batch kernel, laid out here once
+        self._native = load_host_call().Layer(in_features, out_features, self.ws_num, *bounds[:3])
+        self._native.prepare(self._parameters)
 
     quant_input = staticmethod(quant_input)
 
+    def _load_from_state_dict(self, *args, **kwargs):
+        super()._load_from_state_dict(*args, **kwargs)
+        self._native.invalidate()
+
     def forward_quantized(self, input_q, s, residual=None):
         """Already quantised input (int8 + per-token scale), optional fused residual add."""
+        out = self._native.forward_quantized(self._parameters, input_q, s, residual)
+        if out is not None:
+            return out
         return TernaInfer_linear(
             input_q,
             self.weight_compressed_val, self.weight_TileOffsets_global, self.weight_TileOffsets_median,
             self.weight_bitmap, get_global_workspace(input_q.device), s, self.weight_scale, self.ws_num, self.out_features,
             residual=residual, segments=self.segments)
 
+    def forward_normed(self, x, norm_weight, eps, gated=False, residual=None):
+        """forward_quantized(*rmsnorm_quant(x, norm_weight, eps, gated), residual): the front-end runs inside the
+        linear's kernel for the smallest calls."""
+        out = self._native.forward_normed(self._parameters, x, norm_weight, eps, gated, residual)
+        if out is not None:
+            return out
+        xq, s = rmsnorm_quant(x, norm_weight, eps, gated)
+        return self.forward_quantized(xq, s, residual=residual)
+
     def forward(self, input):
+        out = self._native.forward(self._parameters, input)
+        if out is not None:
+            return out
         input, s = quant_input(input)
         return TernaInfer_linear(
             input,

@@ -20,7 +20,7 @@ import torch
 from torch import nn
 from torch.nn import functional as F
 
-from .linear import SpBitLinear, quant_input, rmsnorm, rmsnorm_quant, lm_head_argmax
+from .linear import SpBitLinear, quant_input, rmsnorm, lm_head_argmax
 
 
 @dataclass
@@ -105,10 +105,10 @@ class Attention(nn.Module):
                 self.attn_sub_norm.weight.copy_(dic[prefix + ".attn_sub_norm.weight"])
 
     def forward(self, x, cache: LayerCache, pos, cos, sin, mask, fused=None):
-        """``fused`` = (x_q, s, residual, eps): quantised input of wqkv and the residual for wo's epilogue."""
+        """``fused`` = (norm weight, eps): the norm in front of wqkv runs in its front-end, x is wo's residual."""
         B, T = x.shape[0], x.shape[1]
         H, Hkv, D = self.n_heads, self.n_kv_heads, self.head_dim
-        qkv = self.wqkv(x) if fused is None else self.wqkv.forward_quantized(fused[0], fused[1])
+        qkv = self.wqkv(x) if fused is None else self.wqkv.forward_normed(x, fused[0], fused[1])
         q = qkv[..., : H * D].view(B, T, H, D)
         k = qkv[..., H * D: (H + Hkv) * D].view(B, T, Hkv, D)
         v = qkv[..., (H + Hkv) * D:].view(B, T, Hkv, D)
@@ -118,7 +118,7 @@ class Attention(nn.Module):
         cv.index_copy_(2, pos, v.transpose(1, 2))
         o = F.scaled_dot_product_attention(q.transpose(1, 2), ck, cv, attn_mask=mask, enable_gqa=True)
         o = o.transpose(1, 2).reshape(B, T, H * D)
-        return self._project(o, fused)
+        return self._project(o, x, fused)
 
     def forward_flash(self, x, cache: LayerCache, seqlens, cos_tab, sin_tab, fused):
         """Attention glue through flash_attn's kv-cache kernel (library code, not part of the
@@ -127,18 +127,17 @@ class Attention(nn.Module):
         from flash_attn import flash_attn_with_kvcache
         B, T = x.shape[0], x.shape[1]
         H, Hkv, D = self.n_heads, self.n_kv_heads, self.head_dim
-        qkv = self.wqkv(x) if fused is None else self.wqkv.forward_quantized(fused[0], fused[1])
+        qkv = self.wqkv(x) if fused is None else self.wqkv.forward_normed(x, fused[0], fused[1])
         q = qkv[..., : H * D].view(B, T, H, D)
         k = qkv[..., H * D: (H + Hkv) * D].view(B, T, Hkv, D)
         v = qkv[..., (H + Hkv) * D:].view(B, T, Hkv, D)
         o = flash_attn_with_kvcache(q, cache[0], cache[1], k=k, v=v, rotary_cos=cos_tab, rotary_sin=sin_tab,
                                     cache_seqlens=seqlens, causal=True, rotary_interleaved=True)
-        return self._project(o.reshape(B, T, H * D), fused)
+        return self._project(o.reshape(B, T, H * D), x, fused)
 
-    def _project(self, o, fused):
+    def _project(self, o, x, fused):
         if fused is not None:
-            oq, os_ = rmsnorm_quant(o, self.attn_sub_norm.weight, fused[3])
-            return self.wo.forward_quantized(oq, os_, residual=fused[2])
+            return self.wo.forward_normed(o, self.attn_sub_norm.weight, fused[1], residual=x)
         if self.attn_sub_norm is not None:
             o = self.attn_sub_norm(o)
         return self.wo(o)
@@ -160,10 +159,9 @@ class FeedForward(nn.Module):
             with torch.no_grad():
                 self.ffn_sub_norm.weight.copy_(dic[prefix + ".ffn_sub_norm.weight"])
 
-    def forward_fused(self, xq, s, residual, eps):
-        x13 = self.w13.forward_quantized(xq, s)
-        iq, is_ = rmsnorm_quant(x13, self.ffn_sub_norm.weight, eps, gated=True)
-        return self.w2.forward_quantized(iq, is_, residual=residual)
+    def forward_fused(self, h, norm_weight, eps):
+        x13 = self.w13.forward_normed(h, norm_weight, eps)
+        return self.w2.forward_normed(x13, self.ffn_sub_norm.weight, eps, gated=True, residual=h)
 
     def forward(self, x):
         x1, x3 = self.w13(x).chunk(2, -1)
@@ -187,13 +185,12 @@ class TransformerBlock(nn.Module):
     def forward(self, x, cache, pos, cos, sin, mask, fused: bool = False, flash=None):
         if fused:
             eps = self.attention_norm.eps
-            xq, s = rmsnorm_quant(x, self.attention_norm.weight, eps)
+            fused = (self.attention_norm.weight, eps)
             if flash is not None:
-                h = self.attention.forward_flash(x, cache, flash[0], flash[1], flash[2], (xq, s, x, eps))
+                h = self.attention.forward_flash(x, cache, flash[0], flash[1], flash[2], fused)
             else:
-                h = self.attention(x, cache, pos, cos, sin, mask, fused=(xq, s, x, eps))
-            hq, hs = rmsnorm_quant(h, self.ffn_norm.weight, eps)
-            return self.feed_forward.forward_fused(hq, hs, h, eps)
+                h = self.attention(x, cache, pos, cos, sin, mask, fused=fused)
+            return self.feed_forward.forward_fused(h, self.ffn_norm.weight, eps)
         if flash is not None:
             h = x + self.attention.forward_flash(self.attention_norm(x), cache, flash[0], flash[1], flash[2], None)
         else:

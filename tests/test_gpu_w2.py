@@ -1,0 +1,107 @@
+"""GPU: linears on two-bit weights (the layout SpBitLinear keeps) against the CPU oracle, bit for bit, at the edges of
+the kernel's tiles: odd numbers of 64-column blocks, fewer blocks than warps, one strip group too many, token blocks with
+one row, weights larger than the shared-memory ring."""
+import copy
+
+import numpy as np
+import pytest
+import torch
+
+import ternaspmm_oracle as o
+import c_oracle
+from gpu_util import Packed, dev
+from ternainfer_b200.convert import compress_weight
+from ternainfer_b200.linear import SpBitLinear, quant_input, rmsnorm_quant
+
+pytestmark = pytest.mark.gpu
+
+
+def w2_of(lib, pk):
+    w2 = torch.empty(lib.ternaspmm_w2_bytes(pk.N, pk.K), dtype=torch.uint8, device="cuda")
+    lib.ternaspmm_w2_relayout(pk.bm.data_ptr(), pk.tg.data_ptr(), pk.tm.data_ptr(), pk.cv.data_ptr(), pk.N, pk.K, w2.data_ptr(),
+                              torch.cuda.current_stream().cuda_stream)
+    return w2
+
+
+@pytest.mark.parametrize("N,K,ws_num", [(64, 64, 1), (128, 192, 2), (192, 1088, 1), (3840, 2560, 3), (2560, 6912, 1), (64, 28672, 1),
+                                        (13824, 320, 2), (38464, 128, 2), (9536, 8192, 1)])
+@pytest.mark.parametrize("M", [1, 7, 9, 17, 33, 64, 65, 130])
+def test_linear_on_two_bit_weights(lib, M, N, K, ws_num):
+    w = o.make_ternary(N, K, 0.45, N + K)
+    pk = Packed(w, [t.cpu().numpy() for t in compress_weight(torch.from_numpy(w).cuda())])
+    xq, s = o.make_activations(M, K, M + 1)
+    xq[0, :64] = -128
+    ws = o.make_ws(ws_num, M + 2)
+    sb, wb = o.f32_to_bf16_bits(s.reshape(-1)), o.f32_to_bf16_bits(ws)
+    _, want = c_oracle.ternaspmm(xq, w, sb, wb, ws_num, -1)
+    w2, x_d, s_d, ws_d = w2_of(lib, pk), dev(xq), dev(sb), dev(wb)
+    for residual, skew in ((False, 0), (True, 0), (True, 3)):
+        res_d, exp = None, want
+        if residual:
+            res = o.bf16_round(np.random.default_rng(M).standard_normal((M, N)).astype(np.float32))
+            res_d, exp = dev(o.f32_to_bf16_bits(res)), o.f32_to_bf16_bits(res + o.bf16_bits_to_f32(want))
+        out = torch.full((M * N + 128,), 0x7B7B, dtype=torch.int16, device="cuda")
+        lib.ternaspmm_w2_linear(x_d.data_ptr(), 0, None, 0.0, w2.data_ptr(), out.data_ptr() + 2 * skew, s_d.data_ptr(), ws_d.data_ptr(),
+                                ws_num, M, N, K, 0, 0, 0, -1, res_d.data_ptr() if residual else None,
+                                torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert lib.ternaspmm_last_status() == 0
+        got = out.cpu().numpy().view(np.uint16)
+        assert (got[:skew] == 0x7B7B).all() and (got[skew + M * N:] == 0x7B7B).all(), "wrote outside the output"
+        assert (got[skew:skew + M * N].reshape(M, N) == exp).all()
+
+
+def make_layer(N, K, ws_num, seed, segments=None):
+    w = o.make_ternary(N, K, 0.45, seed)
+    cv, tg, tm, bm = compress_weight(torch.from_numpy(w))
+    dic = {"l.weight_compressed_val": cv, "l.weight_TileOffsets_global": tg, "l.weight_TileOffsets_median": tm, "l.weight_bitmap": bm,
+           "l.weight_scale": torch.from_numpy(o.make_ws(ws_num, seed)).to(torch.bfloat16)}
+    if segments:
+        dic["l.weight_segments"] = torch.tensor(segments)
+    return SpBitLinear(K, N, dic, "l"), dic
+
+
+@pytest.mark.parametrize("N,K", [(2560, 2560), (64, 64), (192, 6912), (128, 28672), (64, 8256)])
+@pytest.mark.parametrize("M", [1, 2, 3, 8, 20, 64, 70])
+@pytest.mark.parametrize("kind", ["plain", "norm", "gated"])
+def test_front_end_inside_the_linear(lib, M, N, K, kind):
+    """bf16 activations: one kernel or two, always the values of the separate front-end followed by the linear."""
+    layer, _ = make_layer(N, K, 1, N + K)
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.randn((M, 2 * K if kind == "gated" else K), generator=g, device="cuda").to(torch.bfloat16)
+    w = (1 + 0.1 * torch.randn(K, generator=g, device="cuda")).to(torch.bfloat16)
+    res = torch.randn((M, N), generator=g, device="cuda").to(torch.bfloat16)
+    if kind == "plain":
+        xf = (127 / x.abs().max(dim=-1, keepdim=True).values.clamp_(min=1e-5))
+        xq, s = (x * xf).round().clamp(-128, 127).to(torch.int8), xf
+        assert all(torch.equal(a, b) for a, b in zip(quant_input(x), (xq, s)))
+        got, want = layer(x), layer.forward_quantized(xq, s)
+    else:
+        xq, s = rmsnorm_quant(x, w, 1e-5, gated=kind == "gated")
+        got = layer.forward_normed(x, w, 1e-5, gated=kind == "gated", residual=res)
+        want = layer.forward_quantized(xq, s, residual=res)
+    assert torch.equal(got, want)
+
+
+def test_layer_follows_its_weights(lib):
+    """New values in place, a loaded state dict, a replaced parameter and copies: the layout is never stale."""
+    layer, dic = make_layer(128, 192, 2, 1, segments=[64, 64])
+    other, dic2 = make_layer(128, 192, 2, 1, segments=[64, 64])
+    x = torch.randn((5, 192), generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).cuda()
+    y = layer(x)
+    twin = copy.deepcopy(layer)
+    assert torch.equal(twin(x), y)
+    signs = layer.weight_compressed_val
+    layer.weight_compressed_val.data.view(torch.int32).copy_(~signs.data.view(torch.int32))      # every sign flipped (seen: same storage ...)
+    layer.weight_compressed_val.view(torch.int32).add_(0)                                        # ... and a version bump)
+    assert torch.equal(layer(x), -y)
+    assert torch.equal(twin(x), y)
+    layer.load_state_dict(other.state_dict())
+    assert torch.equal(layer(x), y)
+    layer.weight_compressed_val = torch.nn.Parameter((~dic["l.weight_compressed_val"].view(torch.int32)).view(torch.uint32).cuda(),
+                                                     requires_grad=False)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):                  # not laid out again inside a capture: reads the packed tensors
+        z = layer(x)
+    graph.replay()
+    assert torch.equal(z, -y) and torch.equal(layer(x), -y)
