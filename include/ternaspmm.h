@@ -283,6 +283,16 @@ void ternaspmm_w2_linear(void* x, int front_end, ternaspmm_bf16* norm_weight, fl
                          ternaspmm_bf16* s, ternaspmm_bf16* ws, int ws_num, int M, int N, int K, int seg1, int seg2,
                          int seg3, int prefill_form, ternaspmm_bf16* residual, ternaspmm_stream_t stream);
 
+/* Attention glue of one decode step in one launch: qkv bf16 [batch][(heads + 2 kv_heads) * head_dim] are
+ * the new token's projections (queries, keys, values); rotates queries and keys (RoPE on adjacent pairs,
+ * cosines and sines of the new position: bf16 [head_dim/2] each), writes key and value into row *pos of the caches (bf16
+ * [batch][max_len][kv_heads][head_dim]) and attends over rows 0 .. *pos; out bf16 [batch][heads *
+ * head_dim].  pos: device int64, the same position for every sequence, below max_len.  head_dim 128,
+ * heads / kv_heads 4 or 8; other shapes return status 1 without a launch.  qkv and caches 16-byte aligned. */
+int ternaspmm_attn_decode(ternaspmm_bf16* qkv, ternaspmm_bf16* k_cache, ternaspmm_bf16* v_cache,
+                          ternaspmm_bf16* cos_row, ternaspmm_bf16* sin_row, long long* pos, ternaspmm_bf16* out,
+                          int batch, int heads, int kv_heads, int head_dim, int max_len, ternaspmm_stream_t stream);
+
 /* ---- work lists: many independent small-batch linears in one persistent launch ------------------
  * One item is what one call of bitlinear_TernaSpMM / ternaspmm_linear_segments /
  * bitlinear_TernaSpMM_residual computes, for 1 <= M <= 16 tokens.  A list runs all its items in ONE

@@ -5,9 +5,8 @@
 // per linear input:
 //   norm_quant       x -> RMSNorm(x) * w -> per-token absmax int8 + scale
 //   gated_norm_quant [x1 | x3] -> relu(x1)^2 * x3 -> RMSNorm * w -> int8 + scale
-// One CTA per token row; the row is held in registers (up to 8192 elements) or
-// staged once in shared memory as bf16, so HBM traffic is one read of the
-// activations and one write of int8 + scale.
+// One CTA per token row; the row is staged once in shared memory as bf16, so
+// HBM traffic is one read of the activations and one write of int8 + scale.
 // Rounding points follow the eager PyTorch evaluation of the same expressions
 // (bf16 after the norm, bf16(1/amax) * 127 for the scale, bf16(x*s) before the
 // round-half-even).  The fp32 sum of squares has a FIXED order, so the result is
@@ -55,135 +54,153 @@ __device__ __forceinline__ float block_reduce(float v, float* scratch, bool is_m
 // model's final norm in the same fixed summation order.
 enum ActMode : int { ACT_RMSNORM = 0, ACT_SCALE_SUMSQ = 1, ACT_PLAIN = 2, ACT_NORM_ONLY = 3 };
 
-// One row in registers: thread `tid` of `nthreads` holds the elements of virtual threads tid + j * nthreads, j < NV (eight
-// consecutive elements each; NV * nthreads >= T, K <= 8192 so that T covers the row), from the load to the int8 store.
-// What remains is one chain of latencies - load, butterfly, barrier, square root, barrier, reciprocal -, so nothing
-// goes through shared memory but one float per warp and reduction, and the maximum (of magnitudes, whose bit patterns
-// order like the values, NaN above all) is a redux.sync.  `part` and `mxp`: 32 words each, 16-byte aligned; the caller
-// may reuse them after its next barrier.  store(k0, q) takes eight int8 values (or, NORM_ONLY, eight bf16).  Returns the scale s.
+// One row by one CTA.  Virtual thread vt of T owns the elements 8 vt .. 8 vt + 7 (K <= 8192, so that T covers the row); a
+// thread takes vt = tid, tid + blockDim, ....  What is left of this work at decode sizes is a chain of latencies -
+// load, butterfly, barrier, square root, barrier, reciprocal - and the instruction fetches of code that runs once, so
+// it is kept short: copies to shared memory by cp.async (every vector of a thread in flight at once, no registers
+// held), loops that are not unrolled, packed bf16 arithmetic where its single rounding is the eager one.
+//   act_row_prefetch_weight  norm weight -> shared memory (before the dependency wait: weights are immutable)
+//   act_row_load             the row (gated: both halves) -> shared memory
+//   act_row_finish           norm, maximum, int8 values through store(k0, int8 x 8) (NORM_ONLY: bf16 x 8)
+// `row`: K bf16 (gated: 2K), `wrow`: K bf16, both shared addresses; `part`, `mxp`: 32 words each.  The caller may reuse them
+// after its next barrier.  Returns the scale s.
+__device__ __forceinline__ void act_row_copy(uint32_t dst, const __nv_bfloat16* src, int K) {
+#pragma unroll 1
+    for (int i = threadIdx.x; i * 8 < K; i += blockDim.x) cp_async_16(dst + i * 16, src + i * 8);
+}
+
 __device__ __forceinline__ uint32_t warp_max_u32(uint32_t v) {
     uint32_t r;
     asm volatile("redux.sync.max.u32 %0, %1, 0xffffffff;" : "=r"(r) : "r"(v));
     return r;
 }
+__device__ __forceinline__ float act_lo(uint32_t v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float act_hi(uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); }
+__device__ __forceinline__ uint32_t act_mul2(uint32_t a, uint32_t b) {   // bf16 products, rounded once each
+    uint32_t r;
+    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ uint32_t act_pack(float lo, float hi) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
 
-template <int NV, bool GATED, int MODE, typename Store>
-__device__ __forceinline__ float row_front_end(const __nv_bfloat16* xr, const uint4 (&nw)[NV], float eps, int K, int T, float* part,
-                                               uint32_t* mxp, float* ss_out, Store store) {
+template <bool GATED, int MODE, typename Store>
+__device__ __forceinline__ float act_row_finish(uint32_t row, uint32_t wrow, float eps, int K, int T, float* part, uint32_t* mxp,
+                                                float* ss_out, Store store) {
     const int tid = threadIdx.x, lane = tid & 31, nthreads = blockDim.x, vwarps = T >> 5;
-    uint4 a[NV], b[NV];
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-        const int k0 = (tid + j * nthreads) * 8;
-        a[j] = k0 < K ? ld_cg_128(xr + k0) : make_uint4(0, 0, 0, 0);
-        if (GATED) b[j] = k0 < K ? ld_cg_128(xr + K + k0) : make_uint4(0, 0, 0, 0);
-    }
-    float f[NV][8], ss[NV];
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-        const uint32_t av[4] = {a[j].x, a[j].y, a[j].z, a[j].w};
-        const uint32_t bv[4] = {b[j].x, b[j].y, b[j].z, b[j].w};
-        ss[j] = 0.f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            f[j][i] = __uint_as_float((i & 1) ? (av[i >> 1] & 0xFFFF0000u) : (av[i >> 1] << 16));
-            if (GATED) {
-                const float r = fmaxf(f[j][i], 0.f);
-                const float x3 = __uint_as_float((i & 1) ? (bv[i >> 1] & 0xFFFF0000u) : (bv[i >> 1] << 16));
-                f[j][i] = bf16_round_f(bf16_round_f(r * r) * x3);   // relu(x1) ** 2, bf16; * x3, bf16
-            }
-            ss[j] = __fadd_rn(ss[j], __fmul_rn(f[j][i], f[j][i]));
-        }
-    }
+    cp_async_wait_all();
+    // (a thread reads only vectors that it copied itself, so no barrier follows the wait)
+    float rstd = 1.f;
     if (MODE != ACT_PLAIN) {
+#pragma unroll 1
+        for (int vt = tid; vt < T; vt += nthreads) {
+            float ss = 0.f;
+            if (vt * 8 < K) {
+                uint4 a = lds128(row + vt * 16);
+                uint32_t* av = reinterpret_cast<uint32_t*>(&a);
+                if (GATED) {
+                    const uint4 b = lds128(row + K * 2 + vt * 16);
+                    const uint32_t bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1)
+                    for (int i = 0; i < 4; ++i) {   // relu(x1) ** 2, bf16; * x3, bf16
+                        uint32_t r;
+                        asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(av[i]), "r"(0u));
+                        av[i] = act_mul2(act_mul2(r, r), bv[i]);
+                    }
+                    sts128(row + vt * 16, a);
+                }
 #pragma unroll
-            for (int j = 0; j < NV; ++j) ss[j] += __shfl_xor_sync(0xffffffffu, ss[j], d);
+                for (int i = 0; i < 4; ++i) {
+                    const float lo = act_lo(av[i]), hi = act_hi(av[i]);
+                    ss = __fadd_rn(ss, __fmul_rn(lo, lo));
+                    ss = __fadd_rn(ss, __fmul_rn(hi, hi));
+                }
+            }
 #pragma unroll
-        for (int j = 0; j < NV; ++j) {
-            const int vw = (tid + j * nthreads) >> 5;
-            if (lane == 0 && vw < vwarps) part[vw] = ss[j];
+            for (int d = 16; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+            if (lane == 0) part[vt >> 5] = ss;
         }
         __syncthreads();
-        float sum = 0.f;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            if (4 * c >= vwarps) break;
-            const float4 v = *reinterpret_cast<const float4*>(part + 4 * c);
-            sum = c == 0 ? v.x : sum + v.x;      // (T is at least 64: two warps or more)
-            if (4 * c + 1 < vwarps) sum += v.y;
-            if (4 * c + 2 < vwarps) sum += v.z;
-            if (4 * c + 3 < vwarps) sum += v.w;
-        }
+        float sum = part[0];
+#pragma unroll 4
+        for (int i = 1; i < vwarps; ++i) sum += part[i];
         if (MODE == ACT_SCALE_SUMSQ && tid == 0) *ss_out = sum;
-        const float rstd = (MODE == ACT_RMSNORM || MODE == ACT_NORM_ONLY)
-                               ? __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)K), eps))) : 1.f;
+        if (MODE != ACT_SCALE_SUMSQ) rstd = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)K), eps)));
+    }
+#pragma unroll 1
+    for (int vt = tid; vt < T; vt += nthreads) {
+        uint32_t mx = 0;
+        if (vt * 8 < K) {
+            uint4 a = lds128(row + vt * 16);
+            uint32_t* av = reinterpret_cast<uint32_t*>(&a);
+            if (MODE != ACT_PLAIN) {
+                const uint4 w = lds128(wrow + vt * 16);
+                const uint32_t wv[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-        for (int j = 0; j < NV; ++j) {
-            const uint32_t wv[4] = {nw[j].x, nw[j].y, nw[j].z, nw[j].w};
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float w = __uint_as_float((i & 1) ? (wv[i >> 1] & 0xFFFF0000u) : (wv[i >> 1] << 16));
-                f[j][i] = bf16_round_f(__fmul_rn(MODE == ACT_SCALE_SUMSQ ? f[j][i] : __fmul_rn(f[j][i], rstd), w));
+                for (int i = 0; i < 4; ++i) {
+                    const float lo = MODE == ACT_SCALE_SUMSQ ? act_lo(av[i]) : __fmul_rn(act_lo(av[i]), rstd);
+                    const float hi = MODE == ACT_SCALE_SUMSQ ? act_hi(av[i]) : __fmul_rn(act_hi(av[i]), rstd);
+                    av[i] = act_pack(__fmul_rn(lo, act_lo(wv[i])), __fmul_rn(hi, act_hi(wv[i])));
+                }
+                if (MODE == ACT_NORM_ONLY) store(vt * 8, a);
+                else sts128(row + vt * 16, a);
             }
+            // magnitudes: their bit patterns order like the values, NaN above all
+#pragma unroll
+            for (int i = 0; i < 4; ++i) mx = max(mx, max(av[i] & 0x7FFFu, (av[i] >> 16) & 0x7FFFu));
+        }
+        if (MODE != ACT_NORM_ONLY) {
+            mx = warp_max_u32(mx);
+            if (lane == 0) mxp[vt >> 5] = mx;
         }
     }
-    if (MODE == ACT_NORM_ONLY) {
-#pragma unroll
-        for (int j = 0; j < NV; ++j) {
-            const int k0 = (tid + j * nthreads) * 8;
-            uint32_t o[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) o[i] = (__float_as_uint(f[j][2 * i]) >> 16) | (__float_as_uint(f[j][2 * i + 1]) & 0xFFFF0000u);
-            if (k0 < K) store(k0, make_uint4(o[0], o[1], o[2], o[3]));
-        }
-        return 0.f;
-    }
-    uint32_t mx[NV];
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-        mx[j] = 0;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) mx[j] = max(mx[j], __float_as_uint(f[j][i]) & 0x7FFFFFFFu);
-        mx[j] = warp_max_u32(mx[j]);
-        const int vw = (tid + j * nthreads) >> 5;
-        if (lane == 0 && vw < vwarps) mxp[vw] = mx[j];
-    }
+    if (MODE == ACT_NORM_ONLY) return 0.f;
     __syncthreads();
-    const float top = __uint_as_float(warp_max_u32(lane < vwarps ? mxp[lane] : 0u));
+    const float top = __uint_as_float(warp_max_u32(lane < vwarps ? mxp[lane] : 0u) << 16);
     const float amax = bf16_round_f(top < 1e-5f ? 1e-5f : top);
     const float s = bf16_round_f(bf16_round_f(1.0f / amax) * 127.0f);   // 127 / amax as reciprocal * 127, in bf16
+    const uint32_t s2 = (__float_as_uint(s) >> 16) * 0x10001u;
+#pragma unroll 1
+    for (int vt = tid; vt * 8 < K; vt += nthreads) {
+        const uint4 a = lds128(row + vt * 16);
+        const uint32_t av[4] = {a.x, a.y, a.z, a.w};
+        uint32_t o[4];
 #pragma unroll
-    for (int j = 0; j < NV; ++j) {
-        const int k0 = (tid + j * nthreads) * 8;
-        uint32_t o[2] = {0u, 0u};
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int v = max(min(__float2int_rn(bf16_round_f(f[j][i] * s)), 127), -128);
-            o[i >> 2] |= (uint32_t)(v & 0xFF) << (8 * (i & 3));
+        for (int i = 0; i < 4; ++i) {
+            uint32_t pr = act_mul2(av[i], s2);
+            asm("min.bf16x2 %0, %1, %2;" : "=r"(pr) : "r"(pr), "r"(0x42FE42FEu));   // 127: only +128 can lie outside of int8
+            // adding 1.5 * 2^23 leaves the value rounded half to even in the low bits
+            const uint32_t lo = __float_as_uint(__fadd_rn(act_lo(pr), 12582912.f)), hi = __float_as_uint(__fadd_rn(act_hi(pr), 12582912.f));
+            o[i] = __byte_perm(lo, hi, 0x0040);
         }
-        if (k0 < K) store(k0, make_uint4(o[0], o[1], 0u, 0u));
+        store(vt * 8, make_uint4(__byte_perm(o[0], o[1], 0x5410), __byte_perm(o[2], o[3], 0x5410), 0u, 0u));
     }
     return s;
 }
 
-// Rows of at most 8192 elements: one CTA per row, T threads with one vector each (row_front_end).
-// x: [M][ld] bf16 (GATED: the row holds [x1 (K) | x3 (K)], ld = 2K), w: [K] bf16 norm weight,
-// q: [M][K] int8, s_out: [M] bf16, ss_out: [M] fp32 (MODE 1).
+// Rows of at most 8192 elements: one CTA of T threads per row, one vector per thread.  Dynamic shared memory: the row (gated:
+// both halves) and the norm weight.  x: [M][ld] bf16 (GATED: the row holds [x1 (K) | x3 (K)], ld = 2K), w: [K] bf16 norm
+// weight, q: [M][K] int8, s_out: [M] bf16, ss_out: [M] fp32 (MODE 1).
 template <bool GATED, int MODE>
 __global__ void __launch_bounds__(kActMaxThreads) norm_quant_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                                                                         float eps, int K, int8_t* __restrict__ q,
                                                                         __nv_bfloat16* __restrict__ s_out, float* __restrict__ ss_out) {
-    __shared__ __align__(16) float part[32];
+    extern __shared__ __align__(16) uint8_t act_smem[];
+    __shared__ float part[32];
     __shared__ uint32_t mxp[32];
     griddep_launch_dependents();
     const int t = blockIdx.x, tid = threadIdx.x;
-    uint4 nw[1] = {make_uint4(0, 0, 0, 0)};
-    if (MODE != ACT_PLAIN && tid * 8 < K) nw[0] = __ldg(reinterpret_cast<const uint4*>(w) + tid);   // weights: before the wait
+    const uint32_t row = smem_u32(act_smem), wrow = row + K * (GATED ? 4 : 2);
+    if (MODE != ACT_PLAIN) act_row_copy(wrow, w, K);   // weights: before the wait
     griddep_wait();   // the activations come from the previous kernel
-    const float s = row_front_end<1, GATED, MODE>(x + (size_t)t * (GATED ? 2 * K : K), nw, eps, K, (int)blockDim.x, part, mxp,
-                                                  MODE == ACT_SCALE_SUMSQ ? ss_out + t : nullptr, [&](int k0, const uint4& v) {
+    const __nv_bfloat16* xr = x + (size_t)t * (GATED ? 2 * K : K);
+    act_row_copy(row, xr, K);
+    if (GATED) act_row_copy(row + K * 2, xr + K, K);
+    const float s = act_row_finish<GATED, MODE>(row, wrow, eps, K, (int)blockDim.x, part, mxp, MODE == ACT_SCALE_SUMSQ ? ss_out + t : nullptr,
+                                                [&](int k0, const uint4& v) {
         if (MODE == ACT_NORM_ONLY) *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(q) + (size_t)t * K + k0) = v;
         else *reinterpret_cast<uint2*>(q + (size_t)t * K + k0) = make_uint2(v.x, v.y);
     });

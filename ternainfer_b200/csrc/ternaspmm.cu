@@ -9,6 +9,7 @@
 #include <stdio.h>
 #include <limits.h>
 #include <stdlib.h>
+#include <math.h>
 
 #include <algorithm>
 #include <vector>
@@ -17,6 +18,7 @@
 #include "ternaspmm.h"
 
 #include "act_quant.cuh"
+#include "attn_decode.cuh"
 #include "dense_pair.cuh"
 #include "dense_prefill.cuh"
 #include "lm_head.cuh"
@@ -646,7 +648,9 @@ static cudaError_t launch_w2_small(W2Params& p, cudaStream_t stream) {
     const int K = p.e.K, KP = w2_pairs(K);
     const int blocks = (p.e.M + MT * 8 - 1) / (MT * 8), tokens = std::min(p.e.M, MT * 8);
     // CTAs: one per SM (fewer when there are fewer strips), so that every SM gets the same share within a strip
-    const int strips = p.e.N / 16, ctas = std::min(strips, std::max(1, device_sm_count() / blocks)), R = (strips + ctas - 1) / ctas;
+    // (at most 40 strips each: the kernel's item index arithmetic)
+    const int strips = p.e.N / 16, ctas = std::min(strips, std::max({1, device_sm_count() / blocks, (strips + 39) / 40}));
+    const int R = (strips + ctas - 1) / ctas;
     p.strips_q = strips / ctas, p.strips_r = strips % ctas;
     // warps: as many as have a block pair of their own, at most ten (two CTAs of that size share the register file, so
     // the next launch's CTA starts beside this one), evenly loaded; at least four for the front-end and the epilogue
@@ -659,10 +663,10 @@ static cudaError_t launch_w2_small(W2Params& p, cudaStream_t stream) {
     const int chunks = groups * ((per + p.chunk_pairs - 1) / p.chunk_pairs), slot_bytes = RG * p.chunk_pairs * 512;
     const int fit = 64 * 1024 / (W * slot_bytes);
     p.slots = std::min(chunks, chunks <= fit && chunks <= kW2MaxSlots ? chunks : 4);
-    p.smem = w2_smem(R, MT, tokens, K, W, p.slots, slot_bytes, XS);
+    p.smem = w2_smem(R, MT, tokens, K, W, p.slots, slot_bytes, XS, FE, p.e.residual != nullptr);
     while (p.smem.total > kW2MaxSmem && p.slots > 1) {
         --p.slots;
-        p.smem = w2_smem(R, MT, tokens, K, W, p.slots, slot_bytes, XS);
+        p.smem = w2_smem(R, MT, tokens, K, W, p.slots, slot_bytes, XS, FE, p.e.residual != nullptr);
     }
     if (p.smem.total > kW2MaxSmem) return cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg = {};
@@ -760,6 +764,49 @@ extern "C" void ternaspmm_w2_linear(void* x, int front_end, __nv_bfloat16* norm_
     checkLastCudaError(__LINE__);
 }
 
+// ---- attention glue of a decode step (attn_decode.cuh) ---------------------------------------------
+template <int GQ>
+static cudaError_t launch_attn_decode(const AttnParams& p, int batch, cudaStream_t stream) {
+    auto kern = attn_decode_kernel<GQ>;
+    // CTAs per key / value head: a power of two up to the portable cluster size, so that all are resident at once (three per SM)
+    int S = 8;
+    while (S > 1 && (long long)batch * p.kv_heads * S > 3ll * device_sm_count()) S >>= 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(S, p.kv_heads, batch);
+    cfg.blockDim = dim3(kAttnWarps * 32, 1, 1);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = S;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = tuning().pdl ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kern, p);
+}
+
+extern "C" int ternaspmm_attn_decode(__nv_bfloat16* qkv, __nv_bfloat16* k_cache, __nv_bfloat16* v_cache, __nv_bfloat16* cos_row,
+                                     __nv_bfloat16* sin_row, long long* pos, __nv_bfloat16* out, int batch, int heads, int kv_heads,
+                                     int head_dim, int max_len, cudaStream_t stream) {
+    t_host_status = ST_OK;
+    const int gq = kv_heads > 0 && heads % kv_heads == 0 ? heads / kv_heads : 0;
+    if (batch < 1 || batch > 65535 || kv_heads < 1 || kv_heads > 65535 || max_len < 1 || head_dim != kAttnD || (gq != 4 && gq != 8)) {
+        t_host_status = ST_BAD_SHAPE;
+        return t_host_status;
+    }
+    const uintptr_t bits = reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache);
+    if (!qkv || !k_cache || !v_cache || !cos_row || !sin_row || !pos || !out || (bits & 15)) {
+        t_host_status = ST_BAD_POINTER;
+        return t_host_status;
+    }
+    AttnParams p = {qkv, k_cache, v_cache, cos_row, sin_row, pos, out, heads, kv_heads, max_len, 1.4426950408889634f / sqrtf((float)head_dim)};
+    if ((gq == 4 ? launch_attn_decode<4>(p, batch, stream) : launch_attn_decode<8>(p, batch, stream)) != cudaSuccess) t_host_status = ST_LAUNCH;
+    checkLastCudaError(__LINE__);
+    return t_host_status;
+}
+
 static void run_norm_quant(bool gated, int mode, __nv_bfloat16* x, __nv_bfloat16* w, float eps, int M, int K,
                            int8_t* q, __nv_bfloat16* s_out, float* ss_out, cudaStream_t stream) {
     t_host_status = ST_OK;
@@ -776,29 +823,29 @@ static void run_norm_quant(bool gated, int mode, __nv_bfloat16* x, __nv_bfloat16
         return;
     }
     typedef void (*Kern)(const __nv_bfloat16*, const __nv_bfloat16*, float, int, int8_t*, __nv_bfloat16*, float*);
-    static const Kern in_regs[5] = {norm_quant_row_kernel<false, ACT_RMSNORM>, norm_quant_row_kernel<false, ACT_SCALE_SUMSQ>,
+    static const Kern by_row[5] = {norm_quant_row_kernel<false, ACT_RMSNORM>, norm_quant_row_kernel<false, ACT_SCALE_SUMSQ>,
                                     norm_quant_row_kernel<false, ACT_PLAIN>, norm_quant_row_kernel<false, ACT_NORM_ONLY>, nullptr};
-    static const Kern in_smem[5] = {norm_quant_kernel<false, ACT_RMSNORM>, norm_quant_kernel<false, ACT_SCALE_SUMSQ>,
+    static const Kern long_row[5] = {norm_quant_kernel<false, ACT_RMSNORM>, norm_quant_kernel<false, ACT_SCALE_SUMSQ>,
                                     norm_quant_kernel<false, ACT_PLAIN>, norm_quant_kernel<false, ACT_NORM_ONLY>, nullptr};
-    const bool row_in_regs = K <= 8 * kActMaxThreads;   // one eight-element vector per thread
-    Kern kern = row_in_regs ? in_regs[mode] : in_smem[mode];
+    const bool short_row = K <= 8 * kActMaxThreads;   // one eight-element vector per thread
+    Kern kern = short_row ? by_row[mode] : long_row[mode];
     if (gated) {
-        if (mode == ACT_RMSNORM) kern = row_in_regs ? norm_quant_row_kernel<true, ACT_RMSNORM> : norm_quant_kernel<true, ACT_RMSNORM>;
-        else kern = row_in_regs ? norm_quant_row_kernel<true, ACT_SCALE_SUMSQ> : norm_quant_kernel<true, ACT_SCALE_SUMSQ>;
+        if (mode == ACT_RMSNORM) kern = short_row ? norm_quant_row_kernel<true, ACT_RMSNORM> : norm_quant_kernel<true, ACT_RMSNORM>;
+        else kern = short_row ? norm_quant_row_kernel<true, ACT_SCALE_SUMSQ> : norm_quant_kernel<true, ACT_SCALE_SUMSQ>;
     }
-    static bool attr_done[64][8] = {};
+    static bool attr_done[2][64][8] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) dev = 0;
     const int slot = (gated ? 4 : 0) + mode;
-    if (!row_in_regs && !attr_done[dev][slot]) {
+    if (!attr_done[short_row][dev][slot]) {
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 56 * 1024);
-        attr_done[dev][slot] = true;
+        attr_done[short_row][dev][slot] = true;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(M, 1, 1);
     cfg.blockDim = dim3(std::min(kActMaxThreads, std::max(64, (K / 8 + 31) / 32 * 32)), 1, 1);   // one vector per thread
-    cfg.dynamicSmemBytes = row_in_regs ? 0 : (size_t)K * 2;
+    cfg.dynamicSmemBytes = short_row ? (size_t)K * (gated ? 6 : (mode == ACT_PLAIN ? 2 : 4)) : (size_t)K * 2;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -42,7 +42,7 @@ constexpr int kW2MaxWarps = 10;
 constexpr uint32_t kW2Mask = 0xC0C0C0C0u;
 
 struct W2Smem {   // shared-memory plan: byte offsets from the base of the dynamic segment
-    int red, xq, ring, total;
+    int red, xq, row, res, ring, total;
     int red_stride, x_stride;
 };
 
@@ -128,7 +128,8 @@ constexpr int kW2Partial = kW2Scale + 48 * 4;                     // two sets (e
 constexpr int kW2ScratchBytes = kW2Partial + 2 * 64 * 4;
 
 // R strips per CTA at most, `tokens` rows of x handled by a CTA (at most MT*8), W warps, ring slots of `slot_bytes`
-inline W2Smem w2_smem(int R, int mt, int tokens, int K, int W, int slots, int slot_bytes, bool x_in_smem) {
+inline W2Smem w2_smem(int R, int mt, int tokens, int K, int W, int slots, int slot_bytes, bool x_in_smem, int front_end,
+                      bool residual) {
     W2Smem s;
     s.red_stride = R * 16 + 4;                       // conflict-free: token stride = 4 mod 16 words
     s.x_stride = (K & 127) ? K : K + 64;             // two tokens' 64-byte pieces on different banks
@@ -138,6 +139,10 @@ inline W2Smem w2_smem(int R, int mt, int tokens, int K, int W, int slots, int sl
     at = (at + 127) & ~127;
     s.xq = at;
     if (x_in_smem) at += ((tokens * s.x_stride + 64 + 127) & ~127);   // (a half pair reads 64 bytes past its row)
+    s.row = at;                                      // a front-end's row (gated: both halves) and norm weight
+    if (front_end != W2_INT8) at += ((K * (front_end == W2_GATED ? 6 : 4) + 127) & ~127);
+    s.res = at;                                      // residual of the CTA's outputs, bf16 [tokens][R * 16]
+    if (residual) at += ((tokens * R * 32 + 127) & ~127);
     s.ring = at;
     at += W * slots * slot_bytes;
     s.total = at;
@@ -188,23 +193,12 @@ __global__ void __launch_bounds__(kW2MaxWarps * 32, MT <= 2 ? 2 : 1) w2_small_ke
         for (int i = 0; i < D && f_gi < NG; ++i) fetch();
     }
     for (int i = tid; i < MT * 8 * L.red_stride; i += nthreads) red[i] = 0;
-    // a front-end's threads (see row_front_end): T virtual threads of eight elements, one or two per thread
-    const int T = FE == W2_INT8 ? 0 : min(kActMaxThreads, max(64, ((K >> 3) + 31) & ~31));
-    constexpr int kNV = 4;
-    uint4 nw[kNV];
-    if (FE != W2_INT8) {
-#pragma unroll
-        for (int j = 0; j < kNV; ++j) {
-            nw[j] = make_uint4(0, 0, 0, 0);
-            if (FE != W2_PLAIN && (tid + j * nthreads) * 8 < K) nw[j] = __ldg(reinterpret_cast<const uint4*>(p.norm_w) + tid + j * nthreads);
-        }
-    }
-    // epilogue items (two columns each) of this thread: tid, tid + nthreads, ...; the first one's place now
-    const int pairs = nstrips * 8, items = mrows * pairs;
+    constexpr bool kGated = FE == W2_GATED;
+    const uint32_t row = base + L.row, wrow = row + K * (kGated ? 4 : 2);
+    if (FE == W2_NORM || FE == W2_GATED) act_row_copy(wrow, p.norm_w, K);
+    const int pairs = nstrips * 8, items = mrows * pairs;     // epilogue items: two columns of a token each
     const uint32_t inv_pairs = ((1u << 22) + pairs - 1) / pairs;   // i / pairs = i * inv >> 22 (i * pairs < 2^22)
-    const int t_first = (int)((uint32_t)tid * inv_pairs >> 22), c_first = (tid - t_first * pairs) * 2;
-    const int grp_first = ws_group(strip0 * 16 + c_first, p.e) | (ws_group(strip0 * 16 + c_first + 1, p.e) << 8);
-    const bool res_ok = p.e.residual != nullptr && (reinterpret_cast<uintptr_t>(p.e.residual) & 3) == 0;
+    const bool res_smem = p.e.residual != nullptr && (reinterpret_cast<uintptr_t>(p.e.residual) & 15) == 0;
     const bool out_ok = (reinterpret_cast<uintptr_t>(p.e.out) & 3) == 0;
 
     __syncwarp();
@@ -221,10 +215,20 @@ __global__ void __launch_bounds__(kW2MaxWarps * 32, MT <= 2 ? 2 : 1) w2_small_ke
             for (int i = lane & 15; i < pieces; i += 16)
                 cp_async_16(base + L.xq + t * L.x_stride + p0 * 128 + i * 16, p.e.x + (size_t)(m0 + t) * K + p0 * 128 + i * 16);
     }
+    if (FE != W2_INT8) {
+        const __nv_bfloat16* xr = p.xb + (size_t)m0 * (kGated ? 2 * K : K);
+        act_row_copy(row, xr, K);
+        if (kGated) act_row_copy(row + K * 2, xr + K, K);
+    }
+    if (res_smem) {
+#pragma unroll 1
+        for (int i = tid; i < mrows * nstrips * 2; i += nthreads) {   // 16 bytes a piece
+            const int t = (int)((uint32_t)(i * 4) * inv_pairs >> 22), c = i * 4 - t * pairs;
+            cp_async_16(base + L.res + (t * pairs + c) * 4, p.e.residual + (size_t)(m0 + t) * N + strip0 * 16 + c * 2);
+        }
+    }
     if (FE == W2_INT8 && tid < mrows && p.e.epilogue != EPI_RAW_I32) scl[tid] = __bfloat162float(p.e.s[m0 + tid]);
     if (tid >= 32 && tid < 36 && p.e.epilogue != EPI_RAW_I32 && p.e.epilogue != EPI_F32_DIV) scl[tid] = __bfloat162float(p.e.ws[tid - 32]);
-    uint32_t res_first = 0;
-    if (res_ok && tid < items) res_first = ld_cg_32(p.e.residual + (size_t)(m0 + t_first) * N + strip0 * 16 + c_first);
     uint4 xn[2 * MT];                                         // direct fragments of the next pair
     auto load_x = [&](int pr, uint4* x) {                     // (columns of absent tokens are not stored)
 #pragma unroll
@@ -244,25 +248,23 @@ __global__ void __launch_bounds__(kW2MaxWarps * 32, MT <= 2 ? 2 : 1) w2_small_ke
         if (!XS && p0 < p1) load_x(p0, xn);
         __syncthreads();                                      // red is zeroed, scales are staged
         if (XS) {
-            cp_async_wait_all();
+            cp_async_wait_all();                              // (the residual too)
             __syncwarp();
         }
     } else {
-        constexpr bool kGated = FE == W2_GATED;
         constexpr int kMode = FE == W2_PLAIN ? ACT_PLAIN : ACT_RMSNORM;
+        const int T = min(kActMaxThreads, max(64, ((K >> 3) + 31) & ~31));   // the fixed order of act_quant.cuh
+#pragma unroll 1
         for (int t = 0; t < mrows; ++t) {
             float* part = reinterpret_cast<float*>(smem + kW2Partial) + (t & 1) * 64;
-            const __nv_bfloat16* xr = p.xb + (size_t)(m0 + t) * (kGated ? 2 * K : K);
-            uint8_t* row = smem + L.xq + t * L.x_stride;
-            auto store = [&](int k0, const uint4& v) { *reinterpret_cast<uint2*>(row + k0) = make_uint2(v.x, v.y); };
-            float s;
-            uint32_t* mxp = reinterpret_cast<uint32_t*>(part + 32);
-            if (K <= 8 * nthreads) {
-                const uint4 one[1] = {nw[0]};
-                s = row_front_end<1, kGated, kMode>(xr, one, p.eps, K, T, part, mxp, nullptr, store);
-            } else {
-                s = row_front_end<kNV, kGated, kMode>(xr, nw, p.eps, K, T, part, mxp, nullptr, store);
+            const uint32_t xrow = base + L.xq + t * L.x_stride;
+            if (t > 0) {                                      // (a thread's own vectors: the previous row's have been used)
+                const __nv_bfloat16* xr = p.xb + (size_t)(m0 + t) * (kGated ? 2 * K : K);
+                act_row_copy(row, xr, K);
+                if (kGated) act_row_copy(row + K * 2, xr + K, K);
             }
+            const float s = act_row_finish<kGated, kMode>(row, wrow, p.eps, K, T, part, reinterpret_cast<uint32_t*>(part + 32), nullptr,
+                                                          [&](int k0, const uint4& v) { sts64(xrow + k0, v.x, v.y); });
             if (tid == 0) scl[t] = s;
         }
         __syncthreads();
@@ -342,49 +344,34 @@ __global__ void __launch_bounds__(kW2MaxWarps * 32, MT <= 2 ? 2 : 1) w2_small_ke
         }
     }
     if (!ok) atomicExch(p.e.status, ST_WAIT_TIMEOUT);
+    if (FE == W2_INT8 && !XS) cp_async_wait_all();            // the residual
     phase_mark(5);
     __syncthreads();
     phase_mark(6);
 
-    // ---- epilogue
-    auto finish = [&](int t, int c, int grp, uint32_t rv) {
-        const int v0 = red[t * L.red_stride + c] >> 6, v1 = red[t * L.red_stride + c + 1] >> 6;
-        const size_t o = (size_t)(m0 + t) * N + strip0 * 16 + c;
+    // ---- epilogue (one loop body: code that runs once is paid for in instruction fetches)
+#pragma unroll 1
+    for (int i = tid; i < items; i += nthreads) {
+        const int t = (int)((uint32_t)i * inv_pairs >> 22), c = (i - t * pairs) * 2, n = strip0 * 16 + c;
+        const int v[2] = {red[t * L.red_stride + c] >> 6, red[t * L.red_stride + c + 1] >> 6};
+        const size_t o = (size_t)(m0 + t) * N + n;
         if (p.e.epilogue == EPI_RAW_I32) {
-            reinterpret_cast<int*>(p.e.out)[o] = v0, reinterpret_cast<int*>(p.e.out)[o + 1] = v1;
+            reinterpret_cast<int*>(p.e.out)[o] = v[0], reinterpret_cast<int*>(p.e.out)[o + 1] = v[1];
         } else if (p.e.epilogue == EPI_F32_DIV) {
             float* out = reinterpret_cast<float*>(p.e.out) + o;
-            out[0] = __fdiv_rn(__int2float_rn(v0), scl[t]), out[1] = __fdiv_rn(__int2float_rn(v1), scl[t]);
+            out[0] = __fdiv_rn(__int2float_rn(v[0]), scl[t]), out[1] = __fdiv_rn(__int2float_rn(v[1]), scl[t]);
         } else {
-            __nv_bfloat16 r0 = scale_epilogue(v0, scl[t], scl[32 + (grp & 0xFF)], p.e.epilogue);
-            __nv_bfloat16 r1 = scale_epilogue(v1, scl[t], scl[32 + (grp >> 8)], p.e.epilogue);
-            if (res_ok) {
-                r0 = __float2bfloat16_rn(__uint_as_float(rv << 16) + __bfloat162float(r0));
-                r1 = __float2bfloat16_rn(__uint_as_float(rv & 0xFFFF0000u) + __bfloat162float(r1));
+            __nv_bfloat16 r[2] = {scale_epilogue(v[0], scl[t], scl[32 + ws_group(n, p.e)], p.e.epilogue),
+                                  scale_epilogue(v[1], scl[t], scl[32 + ws_group(n + 1, p.e)], p.e.epilogue)};
+            if (res_smem) {
+                const uint32_t rv = lds32(base + L.res + i * 4);
+                r[0] = __float2bfloat16_rn(act_lo(rv) + __bfloat162float(r[0])), r[1] = __float2bfloat16_rn(act_hi(rv) + __bfloat162float(r[1]));
             } else if (p.e.residual) {
-                r0 = add_residual(r0, p.e.residual, (long long)o), r1 = add_residual(r1, p.e.residual, (long long)o + 1);
+                r[0] = add_residual(r[0], p.e.residual, (long long)o), r[1] = add_residual(r[1], p.e.residual, (long long)o + 1);
             }
             __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.e.out) + o;
-            if (out_ok) {
-                stg_b32(out, (uint32_t)__bfloat16_as_ushort(r0) | ((uint32_t)__bfloat16_as_ushort(r1) << 16));
-            } else {
-                out[0] = r0, out[1] = r1;
-            }
-        }
-    };
-    if (tid < items) finish(t_first, c_first, grp_first, res_first);
-    for (int i0 = tid + nthreads; i0 < items; i0 += 4 * nthreads) {   // the residuals of four items before their stores
-        uint32_t rv[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int i = i0 + u * nthreads, t = (int)((uint32_t)i * inv_pairs >> 22), c = (i - t * pairs) * 2;
-            rv[u] = (res_ok && i < items) ? ld_cg_32(p.e.residual + (size_t)(m0 + t) * N + strip0 * 16 + c) : 0u;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int i = i0 + u * nthreads, t = (int)((uint32_t)i * inv_pairs >> 22), c = (i - t * pairs) * 2;
-            const int n = strip0 * 16 + c;
-            if (i < items) finish(t, c, ws_group(n, p.e) | (ws_group(n + 1, p.e) << 8), rv[u]);
+            if (out_ok) stg_b32(out, (uint32_t)__bfloat16_as_ushort(r[0]) | ((uint32_t)__bfloat16_as_ushort(r[1]) << 16));
+            else out[0] = r[0], out[1] = r[1];
         }
     }
     phase_mark(7);

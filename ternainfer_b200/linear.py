@@ -110,6 +110,23 @@ def rmsnorm(x: torch.Tensor, norm_weight: torch.Tensor, eps: float) -> torch.Ten
     return y.reshape(x.shape)
 
 
+def attn_decode(qkv, k_cache, v_cache, cos_row, sin_row, pos, heads: int, kv_heads: int):
+    """RoPE, cache append and attention of one new token per sequence in one kernel: qkv bf16 [B, 1, (heads + 2 *
+    kv_heads) * 128], caches bf16 [B, L, kv_heads, 128], ``pos`` int64 [1] on the device, ``cos_row`` / ``sin_row`` bf16
+    [1, 64] the rotation of that position.  bf16 [B, 1, heads * 128], or
+    None where the kernel does not take the shape."""
+    B, D = qkv.shape[0], k_cache.shape[-1]
+    if not (qkv.is_cuda and qkv.dtype == k_cache.dtype == v_cache.dtype == cos_row.dtype == torch.bfloat16 and pos.dtype == torch.int64
+            and D == 128 and heads in (4 * kv_heads, 8 * kv_heads) and cos_row.numel() == sin_row.numel() == 64
+            and qkv.is_contiguous() and k_cache.is_contiguous() and v_cache.is_contiguous()):
+        return None
+    out = torch.empty((B, 1, heads * D), dtype=torch.bfloat16, device=qkv.device)
+    status = load_library().ternaspmm_attn_decode(qkv.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), cos_row.data_ptr(),
+                                                  sin_row.data_ptr(), pos.data_ptr(), out.data_ptr(), B, heads, kv_heads, D,
+                                                  k_cache.shape[1], torch.cuda.current_stream().cuda_stream)
+    return out if status == 0 else None
+
+
 _HEAD_SCRATCH = {}
 
 

@@ -20,7 +20,7 @@ import torch
 from torch import nn
 from torch.nn import functional as F
 
-from .linear import SpBitLinear, quant_input, rmsnorm, lm_head_argmax
+from .linear import SpBitLinear, attn_decode, quant_input, rmsnorm, lm_head_argmax
 
 
 @dataclass
@@ -120,18 +120,24 @@ class Attention(nn.Module):
         o = o.transpose(1, 2).reshape(B, T, H * D)
         return self._project(o, x, fused)
 
-    def forward_flash(self, x, cache: LayerCache, seqlens, cos_tab, sin_tab, fused):
-        """Attention glue through flash_attn's kv-cache kernel (library code, not part of the
-        TernaSpMM path): RoPE on adjacent pairs, cache append and causal attention in one
-        launch.  Cache layout [B, L, Hkv, D]."""
-        from flash_attn import flash_attn_with_kvcache
+    def forward_flash(self, x, cache: LayerCache, pos, rope, rope_row, seqlens, fused):
+        """Attention glue in the cache layout [B, L, Hkv, D]: RoPE on adjacent pairs, cache append and causal
+        attention in one launch - the library's decode kernel for one token per sequence, flash_attn's kv-cache
+        kernel for prompts and for head shapes that the former does not take."""
         B, T = x.shape[0], x.shape[1]
         H, Hkv, D = self.n_heads, self.n_kv_heads, self.head_dim
         qkv = self.wqkv(x) if fused is None else self.wqkv.forward_normed(x, fused[0], fused[1])
+        if rope_row is not None:
+            o = attn_decode(qkv, cache[0], cache[1], *rope_row, pos, H, Hkv)
+            if o is not None:
+                return self._project(o, x, fused)
+        from flash_attn import flash_attn_with_kvcache
         q = qkv[..., : H * D].view(B, T, H, D)
         k = qkv[..., H * D: (H + Hkv) * D].view(B, T, Hkv, D)
         v = qkv[..., (H + Hkv) * D:].view(B, T, Hkv, D)
-        o = flash_attn_with_kvcache(q, cache[0], cache[1], k=k, v=v, rotary_cos=cos_tab, rotary_sin=sin_tab,
+        if seqlens is None:
+            seqlens = pos[:1].to(torch.int32).expand(B).contiguous()
+        o = flash_attn_with_kvcache(q, cache[0], cache[1], k=k, v=v, rotary_cos=rope[0], rotary_sin=rope[1],
                                     cache_seqlens=seqlens, causal=True, rotary_interleaved=True)
         return self._project(o.reshape(B, T, H * D), x, fused)
 
@@ -187,12 +193,12 @@ class TransformerBlock(nn.Module):
             eps = self.attention_norm.eps
             fused = (self.attention_norm.weight, eps)
             if flash is not None:
-                h = self.attention.forward_flash(x, cache, flash[0], flash[1], flash[2], fused)
+                h = self.attention.forward_flash(x, cache, *flash, fused)
             else:
                 h = self.attention(x, cache, pos, cos, sin, mask, fused=fused)
             return self.feed_forward.forward_fused(h, self.ffn_norm.weight, eps)
         if flash is not None:
-            h = x + self.attention.forward_flash(self.attention_norm(x), cache, flash[0], flash[1], flash[2], None)
+            h = x + self.attention.forward_flash(self.attention_norm(x), cache, *flash, None)
         else:
             h = x + self.attention(self.attention_norm(x), cache, pos, cos, sin, mask)
         return h + self.feed_forward(self.ffn_norm(h))
@@ -267,8 +273,9 @@ class Transformer(nn.Module):
         h = self.tok_embeddings(tokens)
         fused = self.args.fused_glue and self.tp == 1
         flash, cos, sin, mask = None, None, None, None
-        if self.flash:   # the kv-cache kernel applies RoPE from the tables and masks by sequence length itself
-            flash = (pos[:1].to(torch.int32).expand(B).contiguous(), self._rope_lp[0], self._rope_lp[1])
+        if self.flash:   # the attention kernels apply RoPE from the tables and mask by position themselves
+            flash = (pos, self._rope_lp, tuple(t.index_select(0, pos) for t in self._rope_lp) if T == 1 else None,
+                     pos[:1].to(torch.int32).expand(B).contiguous() if T > 1 else None)
         else:
             cos, sin = self._rope[0][pos].expand(B, T, -1), self._rope[1][pos].expand(B, T, -1)
             keys = torch.arange(self.max_seq_len, device=tokens.device)

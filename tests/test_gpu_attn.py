@@ -1,0 +1,35 @@
+"""GPU: the attention glue of a decode step against a float64 restatement, at the edges of its split over a cluster and
+of its key tiles."""
+import pytest
+import torch
+
+from ternainfer_b200.linear import attn_decode
+from ternainfer_b200.model import apply_rope, rope_tables
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("H,Hkv", [(20, 5), (64, 8)])
+@pytest.mark.parametrize("B,pos,L", [(1, 0, 8), (1, 1, 8), (2, 7, 8), (1, 9, 64), (1, 127, 640), (3, 600, 640), (8, 255, 300),
+                                     (8, 1100, 1101), (1, 2047, 2500), (1, 2300, 2500), (16, 513, 600), (70, 300, 320)])
+def test_decode_attention(lib, B, pos, L, H, Hkv):
+    D = 128
+    g = torch.Generator(device="cuda").manual_seed(pos + B)
+    qkv = torch.randn((B, 1, (H + 2 * Hkv) * D), generator=g, device="cuda").to(torch.bfloat16)
+    kc, vc = (torch.randn((B, L, Hkv, D), generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    kc[:, pos + 1:], vc[:, pos + 1:] = float('nan'), float('nan')       # rows that hold no token yet
+    k0, v0 = kc.clone(), vc.clone()
+    cos, sin = (t.to(torch.bfloat16) for t in rope_tables(D, L, 500000.0, "cuda"))
+    p = torch.tensor([pos], device="cuda")
+    out = attn_decode(qkv, kc, vc, cos[p], sin[p], p, H, Hkv)
+    q, k, v = (t.view(B, 1, -1, D) for t in qkv.split([H * D, Hkv * D, Hkv * D], -1))
+    c, s = cos[p].float().expand(B, 1, -1), sin[p].float().expand(B, 1, -1)
+    q, k = apply_rope(q, c, s), apply_rope(k, c, s)
+    k0[:, pos], v0[:, pos] = k[:, 0], v[:, 0]
+    assert torch.equal(kc.view(torch.int16), k0.view(torch.int16)) and torch.equal(vc.view(torch.int16), v0.view(torch.int16)), "the caches differ from an append of the rotated key and the value"
+    kk, vv = (t[:, :pos + 1].double().repeat_interleave(H // Hkv, 2) for t in (k0, v0))
+    a = torch.softmax(torch.einsum("bhd,blhd->bhl", q[:, 0].double(), kk) / D ** 0.5, -1)
+    want = torch.einsum("bhl,blhd->bhd", a, vv).reshape(B, 1, H * D)
+    assert ((out.double() - want).norm() / want.norm()).item() < 3e-3
+    assert (out.double() - want).abs().max().item() < 1.2e-2 * want.abs().max().item()
+    assert torch.equal(attn_decode(qkv, kc, vc, cos[p], sin[p], p, H, Hkv), out)
