@@ -21,14 +21,13 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime_api.h>
+#include <limits.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "ternaspmm.h"
 
 namespace {
-
-constexpr int64_t kSmallTokens = 32;   // the mma.sync kernel on two-bit weights; above it the tensor-core paths of the library
 
 PyObject* g_keys[5];                   // interned parameter names, in the order of Weights
 
@@ -102,9 +101,24 @@ bool usable(PyObject* o, at::ScalarType type, int64_t K) {
 
 void run_linear(Layer* self, const Weights& w, void* w2, void* x, int front_end, void* norm_w, float eps, at::Tensor& out, void* s,
                 int64_t M, void* residual, cudaStream_t stream) {
-    ternaspmm_w2_linear(x, front_end, static_cast<ternaspmm_bf16*>(norm_w), eps, w2, static_cast<ternaspmm_bf16*>(out.data_ptr()),
-                        static_cast<ternaspmm_bf16*>(s), static_cast<ternaspmm_bf16*>(w.scale->data_ptr()), self->ws_num, (int)M,
-                        self->out_features, self->in_features, self->seg[0], self->seg[1], self->seg[2], -1,
+    auto* o = static_cast<ternaspmm_bf16*>(out.data_ptr());
+    auto* scale = static_cast<ternaspmm_bf16*>(w.scale->data_ptr());
+    const bool segments = self->seg[0] | self->seg[1] | self->seg[2];
+    if (front_end == 0 && !(segments && residual) && !ternaspmm_w2_pays((int)M, self->out_features, self->in_features)) {
+        auto* bitmap = static_cast<uint64_t*>(w.bitmap->data_ptr());
+        auto* to = static_cast<int*>(w.tile_offsets->data_ptr());
+        auto* qo = static_cast<uint16_t*>(w.quarter_offsets->data_ptr());
+        auto* signs = static_cast<uint32_t*>(w.signs->data_ptr());
+        if (segments)
+            ternaspmm_linear_segments(static_cast<int8_t*>(x), bitmap, to, qo, signs, o, static_cast<ternaspmm_bf16*>(s), scale, self->ws_num,
+                                      (int)M, self->out_features, self->in_features, self->seg[0], self->seg[1], self->seg[2], -1, stream);
+        else
+            bitlinear_TernaSpMM_residual(static_cast<int8_t*>(x), bitmap, to, qo, signs, o, static_cast<ternaspmm_bf16*>(s), scale, self->ws_num,
+                                         (int)M, self->out_features, self->in_features, static_cast<ternaspmm_bf16*>(residual), stream);
+        return;
+    }
+    ternaspmm_w2_linear(x, front_end, static_cast<ternaspmm_bf16*>(norm_w), eps, w2, o, static_cast<ternaspmm_bf16*>(s), scale, self->ws_num,
+                        (int)M, self->out_features, self->in_features, self->seg[0], self->seg[1], self->seg[2], -1,
                         static_cast<ternaspmm_bf16*>(residual), stream);
 }
 
@@ -127,7 +141,7 @@ PyObject* front_and_linear(Layer* self, PyObject* params, PyObject* xo, int fron
     if (!usable(xo, at::kBFloat16, gated ? 2 * K : K)) Py_RETURN_NONE;
     const at::Tensor& x = THPVariable_Unpack(xo);
     const int64_t M = x.numel() / x.size(-1);
-    if (M > kSmallTokens) Py_RETURN_NONE;
+    if (M > INT_MAX / 2) Py_RETURN_NONE;
     void* norm_w = nullptr;
     if (norm_o) {
         if (!usable(norm_o, at::kBFloat16, K) || THPVariable_Unpack(norm_o).numel() != K) Py_RETURN_NONE;
@@ -185,7 +199,7 @@ PyObject* layer_forward_quantized(PyObject* o, PyObject* const* args, Py_ssize_t
     if (!usable(args[1], at::kChar, K) || !THPVariable_Check(args[2])) Py_RETURN_NONE;
     const at::Tensor &x = THPVariable_Unpack(args[1]), &s = THPVariable_Unpack(args[2]);
     const int64_t M = x.numel() / K;
-    if (M > kSmallTokens || s.scalar_type() != at::kBFloat16 || !s.is_contiguous() || s.numel() != M || s.device() != x.device())
+    if (M > INT_MAX / 2 || s.scalar_type() != at::kBFloat16 || !s.is_contiguous() || s.numel() != M || s.device() != x.device())
         Py_RETURN_NONE;
     bool ok;
     void* residual = residual_ptr(args[3], M, self->out_features, ok);

@@ -189,9 +189,19 @@ __device__ __forceinline__ void store_slice16(const SpmmParams& p, const int (&v
 // sixteen of one row.  The residual, if any, is read the same way (16 bytes per lane) and added after the
 // first rounding, as in add_residual().  `o_row0` = index of (first token, the warp's first column);
 // needs a 16-byte aligned output (and residual).
+// Residual of a slice as store_slice16_wide reads it: 16 bytes per lane, rows lane / 4 and lane / 4 + 8.
+__device__ __forceinline__ void load_residual16(const SpmmParams& p, long long o_row0, int live, int lane, uint4 (&res)[2]) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int row = (lane >> 2) + 8 * i;
+        if (row < live) res[i] = ldg_128(p.residual + o_row0 + (long long)row * p.N + (lane & 3) * 8);
+    }
+}
+
+// `ahead`: the residual, already loaded, where the caller has it (an L2 latency per slice otherwise).
 __device__ __forceinline__ void store_slice16_wide(const SpmmParams& p, const int (&v)[16], const float* sc,
                                                    long long o_row0, int live, bool fast, float ws_el, uint32_t stage,
-                                                   int lane) {
+                                                   int lane, const uint4* ahead = nullptr) {
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
         const float scj = sc[j];   // the tokens' scales (or prefill coefficients), in shared memory
@@ -206,8 +216,9 @@ __device__ __forceinline__ void store_slice16_wide(const SpmmParams& p, const in
     for (int i = 0; i < 2; ++i) {
         const int row = (lane >> 2) + 8 * i;
         d[i] = lds128(stage + (uint32_t)(row * 64 + part * 16));
-        if (p.residual && row < live) res[i] = ldg_128(p.residual + o_row0 + (long long)row * p.N + part * 8);
+        if (ahead) res[i] = ahead[i];
     }
+    if (p.residual && !ahead) load_residual16(p, o_row0, live, lane, res);
     if (p.residual) {
 #pragma unroll
         for (int i = 0; i < 2; ++i) {

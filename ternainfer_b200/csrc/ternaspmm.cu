@@ -26,6 +26,7 @@
 #include "spmm_large_m.cuh"
 #include "spmm_list.cuh"
 #include "spmm_small_m.cuh"
+#include "w2_pair.cuh"
 #include "w2_small.cuh"
 
 namespace tsp {
@@ -632,6 +633,9 @@ extern "C" void ternaspmm_linear_segments(int8_t* x, uint64_t* bitmap, int* tile
 
 // ---- linears on two-bit weights (w2_small.cuh) -----------------------------------------------------
 constexpr int kW2MaxSmem = 227 * 1024;
+// Tokens up to which the mma.sync kernel runs (more: tcgen05 on CTA pairs).  Measured, one call in a stream, mma.sync / pairs:
+// 3840 x 2560 at 48 / 64 tokens 8.9 / 10.3, 9.4 / 10.3 us, 2560 x 2560 7.7 / 10.3, 8.5 / 10.3, 13824 x 2560 17.0 / 13.2, 17.1 / 13.2.
+static int w2_small_tokens(int N) { return N <= 32 * device_sm_count() ? 64 : 32; }
 
 template <int MT, int RG, int U, int FE, bool XS>
 static cudaError_t launch_w2_small(W2Params& p, cudaStream_t stream) {
@@ -698,6 +702,46 @@ static cudaError_t launch_w2_int8(W2Params& p, cudaStream_t stream) {
     return xs ? launch_w2_small<4, 2, 1, W2_INT8, true>(p, stream) : launch_w2_small<4, 2, 1, W2_INT8, false>(p, stream);
 }
 
+static cudaError_t launch_w2_pair(const W2Params& p, cudaStream_t stream) {
+    static bool attr_done[64] = {false};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) dev = 0;
+    auto kern = w2_pair_kernel;
+    if (!attr_done[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, W2PairSmem::total);
+        if (e != cudaSuccess) return e;
+        attr_done[dev] = true;
+    }
+    const int pairs = device_sm_count() / 2, RB = (p.e.N + kPairRows - 1) / kPairRows;
+    W2PairParams pp = {p.e, p.w, w2_pair_tile(p.e.M, RB, w2_pairs(p.e.K), pairs), 0};
+    pp.stages = std::min(kW2PairMaxStages, W2PairSmem::stage_bytes / (kPairHalf + pp.nt * kLgKStep / 2));
+    CUtensorMap map;   // each CTA of a pair loads half of the tile's tokens per stage
+    if (!encode_x_map(&map, p.e.x, p.e.M, p.e.K, pp.nt / 2)) return cudaErrorInvalidValue;   // reported as status 3, nothing is launched
+    const long long tiles = (long long)RB * ((p.e.M + pp.nt - 1) / pp.nt);
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(kW2PairThreads, 1, 1);
+    cfg.gridDim = dim3((unsigned)(2 * std::min<long long>(tiles, pairs)), 1, 1);
+    cfg.dynamicSmemBytes = W2PairSmem::total;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = tuning().pdl ? 2 : 1;
+    t_echo = {7, pp.nt, 2, kW2PairThreads / 32, 4, (int)cfg.gridDim.x};
+    return cudaLaunchKernelEx(&cfg, kern, pp, map);
+}
+
+// Whether a call that has both forms of the weight in hand should take the two-bit one.  Deep and narrow layers at 33 to 256
+// tokens fill few pairs, each with a long K loop, which the packed tcgen05 kernel splits over a cluster (2560 x 6912 at 64 / 256
+// tokens: 15.1 / 18.3 us packed, 21.0 / 22.6 us two-bit).
+extern "C" int ternaspmm_w2_pays(int M, int N, int K) { return M <= 32 || M > 256 || K < 5120 || N > 32 * device_sm_count(); }
+
 // Bytes of a weight's two-bit layout.
 extern "C" long long ternaspmm_w2_bytes(int N, int K) { return N < 16 || K < 64 ? 0 : (long long)(N / 16) * w2_pairs(K) * 512; }
 
@@ -756,7 +800,8 @@ extern "C" void ternaspmm_w2_linear(void* x, int front_end, __nv_bfloat16* norm_
     if (front_end == W2_PLAIN) e = launch_w2_fused<W2_PLAIN>(p, stream);
     else if (front_end == W2_NORM) e = launch_w2_fused<W2_NORM>(p, stream);
     else if (front_end == W2_GATED) e = launch_w2_fused<W2_GATED>(p, stream);
-    else e = launch_w2_int8(p, stream);
+    else if (M <= w2_small_tokens(N)) e = launch_w2_int8(p, stream);
+    else e = launch_w2_pair(p, stream);
     if (e != cudaSuccess) {
         fprintf(stderr, "ternaspmm: launch failed: %s\n", cudaGetErrorString(e));
         t_host_status = ST_LAUNCH;

@@ -27,6 +27,10 @@ def w2_of(lib, pk):
                                         (13824, 320, 2), (38464, 128, 2), (9536, 8192, 1)])
 @pytest.mark.parametrize("M", [1, 7, 9, 17, 33, 64, 65, 130])
 def test_linear_on_two_bit_weights(lib, M, N, K, ws_num):
+    check_linear(lib, M, N, K, ws_num)
+
+
+def check_linear(lib, M, N, K, ws_num):
     w = o.make_ternary(N, K, 0.45, N + K)
     pk = Packed(w, [t.cpu().numpy() for t in compress_weight(torch.from_numpy(w).cuda())])
     xq, s = o.make_activations(M, K, M + 1)
@@ -49,6 +53,13 @@ def test_linear_on_two_bit_weights(lib, M, N, K, ws_num):
         got = out.cpu().numpy().view(np.uint16)
         assert (got[:skew] == 0x7B7B).all() and (got[skew + M * N:] == 0x7B7B).all(), "wrote outside the output"
         assert (got[skew:skew + M * N].reshape(M, N) == exp).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(40, 64, 64), (257, 320, 192), (700, 320, 128), (2049, 2560, 192), (1000, 13824, 320), (300, 2560, 6912),
+                                   (1226, 3840, 2560), (4096, 192, 64), (150, 57344, 128)])
+def test_pairs_with_several_tiles_and_ragged_edges(lib, M, N, K):
+    """Tile heights from 32 to 256 tokens, several tiles per pair, a last row block of 64 rows, half a last stage."""
+    check_linear(lib, M, N, K, 2)
 
 
 def make_layer(N, K, ws_num, seed, segments=None):
