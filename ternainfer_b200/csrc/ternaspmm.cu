@@ -23,6 +23,7 @@
 #include "dense_prefill.cuh"
 #include "lm_head.cuh"
 #include "mma_rate_probe.cuh"
+#include "pack_gpu.cuh"
 #include "spmm_large_m.cuh"
 #include "spmm_list.cuh"
 #include "spmm_small_m.cuh"
@@ -1005,6 +1006,56 @@ extern "C" void ternaspmm_tp_allreduce_finish(float** bufs, unsigned int** flags
                            (const __nv_bfloat16*)ws, eps, full_width, M, N, (const __nv_bfloat16*)residual,
                            status, g_wait_limit_ns) != cudaSuccess)
         t_host_status = ST_LAUNCH;
+    checkLastCudaError(__LINE__);
+}
+
+// ---- packer on the GPU (pack_gpu.cuh) --------------------------------------------------------------
+extern "C" long long ternaspmm_pack_gpu_layout(const int8_t* W, int N, int K, uint64_t* bitmap, int* tile_offsets, uint16_t* quarter_offsets,
+                                               cudaStream_t stream) {
+    t_host_status = ST_OK;
+    if (N < 64 || K < 64 || (N % 64) || (K % 64)) {
+        t_host_status = ST_BAD_SHAPE;
+        return -1;
+    }
+    if (!W || !bitmap || !tile_offsets || !quarter_offsets || (reinterpret_cast<uintptr_t>(W) & 15) || (reinterpret_cast<uintptr_t>(bitmap) & 15)) {
+        t_host_status = ST_BAD_POINTER;
+        return -1;
+    }
+    static thread_local long long* total = nullptr;   // pinned, written by the scan kernel; one per thread, kept
+    if (!total && cudaHostAlloc(reinterpret_cast<void**>(&total), sizeof(*total), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+        total = nullptr;
+        cudaGetLastError();
+        t_host_status = ST_LAUNCH;
+        return -1;
+    }
+    const long long tiles = (long long)(N / 64) * (K / 64);
+    const unsigned blocks = (unsigned)((tiles + kPackWarps - 1) / kPackWarps);
+    pack_bitmap_kernel<<<blocks, kPackWarps * 32, 0, stream>>>(W, N, K, reinterpret_cast<uint4*>(bitmap), tile_offsets, quarter_offsets);
+    pack_scan_kernel<<<1, 1024, 0, stream>>>(tile_offsets, tiles, total);
+    if (cudaStreamSynchronize(stream) != cudaSuccess) {
+        t_host_status = ST_LAUNCH;
+        checkLastCudaError(__LINE__);
+        return -1;
+    }
+    if (*total >= (1ll << 31)) {   // offsets are 32-bit
+        t_host_status = ST_BAD_SHAPE;
+        return -1;
+    }
+    return *total / 32;
+}
+
+extern "C" void ternaspmm_pack_gpu_signs(const int8_t* W, int N, int K, const int* tile_offsets, uint32_t* sign_words, cudaStream_t stream) {
+    t_host_status = ST_OK;
+    if (N < 64 || K < 64 || (N % 64) || (K % 64)) {
+        t_host_status = ST_BAD_SHAPE;
+        return;
+    }
+    if (!W || !tile_offsets || !sign_words || (reinterpret_cast<uintptr_t>(W) & 15)) {
+        t_host_status = ST_BAD_POINTER;
+        return;
+    }
+    const long long tiles = (long long)(N / 64) * (K / 64);
+    pack_signs_kernel<<<(unsigned)((tiles + kPackWarps - 1) / kPackWarps), kPackWarps * 32, 0, stream>>>(W, N, K, tile_offsets, sign_words);
     checkLastCudaError(__LINE__);
 }
 
