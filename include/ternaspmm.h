@@ -226,6 +226,14 @@ void ternaspmm_relu2_gate_rmsnorm_quant(ternaspmm_bf16* x13, ternaspmm_bf16* nor
 void ternaspmm_rmsnorm(ternaspmm_bf16* x, ternaspmm_bf16* norm_weight, float eps, int M, int K, ternaspmm_bf16* y,
                        ternaspmm_stream_t stream);
 
+/* Single launches in place of chains of elementwise operators, the same roundings: RoPE on adjacent pairs in fp32 (x bf16
+ * [batch][tokens][heads][128], `ld` elements between two tokens; cos, sin fp32 [tokens][64]; out contiguous), the gate
+ * relu(x1)^2 * x3 (x13 bf16 [M][2K], out bf16 [M][K]) and bf16 -> fp32.  16-byte aligned pointers, ld and K multiples of 8. */
+void ternaspmm_rope(ternaspmm_bf16* x, long long ld, float* cos_t, float* sin_t, ternaspmm_bf16* out, int batch, int tokens,
+                    int heads, ternaspmm_stream_t stream);
+void ternaspmm_relu2_gate(ternaspmm_bf16* x13, ternaspmm_bf16* out, int M, int K, ternaspmm_stream_t stream);
+void ternaspmm_bf16_to_f32(ternaspmm_bf16* x, float* y, long long n, ternaspmm_stream_t stream);
+
 /* Plain per-token absmax quantiser (model.py:120-123) as one kernel. */
 void ternaspmm_quant(ternaspmm_bf16* x, int M, int K, int8_t* q, ternaspmm_bf16* s_out,
                      ternaspmm_stream_t stream);
@@ -294,6 +302,14 @@ void ternaspmm_w2_linear(void* x, int front_end, ternaspmm_bf16* norm_weight, fl
 int ternaspmm_attn_decode(ternaspmm_bf16* qkv, ternaspmm_bf16* k_cache, ternaspmm_bf16* v_cache,
                           ternaspmm_bf16* cos_row, ternaspmm_bf16* sin_row, long long* pos, ternaspmm_bf16* out,
                           int batch, int heads, int kv_heads, int head_dim, int max_len, ternaspmm_stream_t stream);
+
+/* The same for `tokens` consecutive new tokens per sequence, causal, in two launches: qkv bf16 [batch][tokens][(heads +
+ * 2 kv_heads) * head_dim], rotation tables bf16 [max_len][head_dim/2], first position *pos (rows 0 .. *pos - 1 hold
+ * earlier tokens), out bf16 [batch][tokens][heads * head_dim].  head_dim 128, heads / kv_heads a multiple of 4. */
+int ternaspmm_attn_prefill(ternaspmm_bf16* qkv, ternaspmm_bf16* k_cache, ternaspmm_bf16* v_cache,
+                           ternaspmm_bf16* cos_tab, ternaspmm_bf16* sin_tab, long long* pos, ternaspmm_bf16* out,
+                           int batch, int tokens, int heads, int kv_heads, int head_dim, int max_len,
+                           ternaspmm_stream_t stream);
 
 /* ---- work lists: many independent small-batch linears in one persistent launch ------------------
  * One item is what one call of bitlinear_TernaSpMM / ternaspmm_linear_segments /

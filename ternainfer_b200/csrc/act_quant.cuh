@@ -87,6 +87,12 @@ __device__ __forceinline__ uint32_t act_pack(float lo, float hi) {
     return r;
 }
 
+// T of the fixed order
+__host__ __device__ inline int act_row_threads(int K) {
+    const int t = ((K >> 3) + 31) & ~31;
+    return t < 64 ? 64 : (t > kActMaxThreads ? kActMaxThreads : t);
+}
+
 template <bool GATED, int MODE, typename Store>
 __device__ __forceinline__ float act_row_finish(uint32_t row, uint32_t wrow, float eps, int K, int T, float* part, uint32_t* mxp,
                                                 float* ss_out, Store store) {
@@ -181,7 +187,8 @@ __device__ __forceinline__ float act_row_finish(uint32_t row, uint32_t wrow, flo
     return s;
 }
 
-// Rows of at most 8192 elements: one CTA of T threads per row, one vector per thread.  Dynamic shared memory: the row (gated:
+// Rows of at most 8192 elements: one CTA per row, T threads for few rows (a chain of latencies), T / 4 for many (more rows
+// in flight per SM: 1226 gated rows of 6912 17.3 -> 11.5 us).  Dynamic shared memory: the row (gated:
 // both halves) and the norm weight.  x: [M][ld] bf16 (GATED: the row holds [x1 (K) | x3 (K)], ld = 2K), w: [K] bf16 norm
 // weight, q: [M][K] int8, s_out: [M] bf16, ss_out: [M] fp32 (MODE 1).
 template <bool GATED, int MODE>
@@ -199,12 +206,73 @@ __global__ void __launch_bounds__(kActMaxThreads) norm_quant_row_kernel(const __
     const __nv_bfloat16* xr = x + (size_t)t * (GATED ? 2 * K : K);
     act_row_copy(row, xr, K);
     if (GATED) act_row_copy(row + K * 2, xr + K, K);
-    const float s = act_row_finish<GATED, MODE>(row, wrow, eps, K, (int)blockDim.x, part, mxp, MODE == ACT_SCALE_SUMSQ ? ss_out + t : nullptr,
+    const float s = act_row_finish<GATED, MODE>(row, wrow, eps, K, act_row_threads(K), part, mxp, MODE == ACT_SCALE_SUMSQ ? ss_out + t : nullptr,
                                                 [&](int k0, const uint4& v) {
         if (MODE == ACT_NORM_ONLY) *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(q) + (size_t)t * K + k0) = v;
         else *reinterpret_cast<uint2*>(q + (size_t)t * K + k0) = make_uint2(v.x, v.y);
     });
     if (MODE != ACT_NORM_ONLY && tid == 0) s_out[t] = __float2bfloat16_rn(s);
+}
+
+// ---- elementwise kernels of the unfused glue: each replaces a chain of torch operators by one launch with the same
+// roundings -----------------------------------------------------------------------------------------------------------
+// RoPE on adjacent pairs in fp32 (products and difference rounded separately): x [B][T][H][128] with `ld` elements between
+// two tokens, cos / sin fp32 [T][64] (the same for every sequence), out contiguous.  One thread per 8 elements.
+__global__ void __launch_bounds__(256) rope_kernel(const __nv_bfloat16* __restrict__ x, long long ld, const float* __restrict__ cos_t,
+                                                  const float* __restrict__ sin_t, __nv_bfloat16* __restrict__ out, int T, int H,
+                                                  long long items) {
+    griddep_launch_dependents();
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    griddep_wait();
+    if (i >= items) return;
+    const int c = (int)(i & 15), h = (int)((i >> 4) % H);
+    const long long bt = (i >> 4) / H;
+    const int t = (int)(bt % T);
+    const uint4 v = ld_cg_128(x + bt * ld + h * 128 + c * 8);
+    const float4 cs = *reinterpret_cast<const float4*>(cos_t + (size_t)t * 64 + c * 4), sn = *reinterpret_cast<const float4*>(sin_t + (size_t)t * 64 + c * 4);
+    const uint32_t a[4] = {v.x, v.y, v.z, v.w};
+    const float cc[4] = {cs.x, cs.y, cs.z, cs.w}, ss[4] = {sn.x, sn.y, sn.z, sn.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float p = act_lo(a[e]), q = act_hi(a[e]);
+        o[e] = act_pack(__fsub_rn(__fmul_rn(p, cc[e]), __fmul_rn(q, ss[e])), __fadd_rn(__fmul_rn(p, ss[e]), __fmul_rn(q, cc[e])));
+    }
+    *reinterpret_cast<uint4*>(out + i * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+// relu(x1) ** 2 * x3 of rows [x1 (K) | x3 (K)], bf16 after every step.
+__global__ void __launch_bounds__(256) relu2_gate_kernel(const __nv_bfloat16* __restrict__ x13, __nv_bfloat16* __restrict__ out, int K8, long long items) {
+    griddep_launch_dependents();
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    griddep_wait();
+    if (i >= items) return;
+    const long long t = i / K8, c = i - t * K8;
+    const uint4 a = ld_cg_128(x13 + (t * 2 * K8 + c) * 8), b = ld_cg_128(x13 + ((t * 2 + 1) * K8 + c) * 8);
+    const uint32_t av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        uint32_t r;
+        asm("max.NaN.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(av[e]), "r"(0u));
+        o[e] = act_mul2(act_mul2(r, r), bv[e]);
+    }
+    *reinterpret_cast<uint4*>(out + i * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+// bf16 -> fp32, eight values per thread.
+__global__ void __launch_bounds__(256) bf16_to_f32_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ y, long long n) {
+    griddep_launch_dependents();
+    griddep_wait();
+    const long long n8 = n >> 3, stride = (long long)gridDim.x * 256;
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n8; i += stride) {
+        const uint4 v = ld_cg_128(x + i * 8);
+        float4* o = reinterpret_cast<float4*>(y + i * 8);
+        __stcs(o, make_float4(act_lo(v.x), act_hi(v.x), act_lo(v.y), act_hi(v.y)));
+        __stcs(o + 1, make_float4(act_lo(v.z), act_hi(v.z), act_lo(v.w), act_hi(v.w)));
+    }
+    const long long rest = n8 * 8 + (long long)blockIdx.x * 256 + threadIdx.x;
+    if (blockIdx.x == 0 && rest < n) y[rest] = __bfloat162float(x[rest]);
 }
 
 // Longer rows, staged in shared memory: same arguments, dynamic shared memory K bf16.

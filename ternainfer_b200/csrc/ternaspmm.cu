@@ -19,6 +19,7 @@
 
 #include "act_quant.cuh"
 #include "attn_decode.cuh"
+#include "attn_prefill.cuh"
 #include "dense_pair.cuh"
 #include "dense_prefill.cuh"
 #include "lm_head.cuh"
@@ -853,6 +854,54 @@ extern "C" int ternaspmm_attn_decode(__nv_bfloat16* qkv, __nv_bfloat16* k_cache,
     return t_host_status;
 }
 
+extern "C" int ternaspmm_attn_prefill(__nv_bfloat16* qkv, __nv_bfloat16* k_cache, __nv_bfloat16* v_cache, __nv_bfloat16* cos_tab,
+                                      __nv_bfloat16* sin_tab, long long* pos, __nv_bfloat16* out, int batch, int tokens, int heads,
+                                      int kv_heads, int head_dim, int max_len, cudaStream_t stream) {
+    t_host_status = ST_OK;
+    if (batch < 1 || batch > 65535 || tokens < 1 || kv_heads < 1 || heads % kv_heads || (heads / kv_heads) % 4 || heads > 4 * 65535 ||
+        max_len < 1 || head_dim != kAttnD) {
+        t_host_status = ST_BAD_SHAPE;
+        return t_host_status;
+    }
+    const uintptr_t bits = reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache) |
+                           reinterpret_cast<uintptr_t>(cos_tab) | reinterpret_cast<uintptr_t>(sin_tab);
+    if (!qkv || !k_cache || !v_cache || !cos_tab || !sin_tab || !pos || !out || (bits & 15)) {
+        t_host_status = ST_BAD_POINTER;
+        return t_host_status;
+    }
+    static bool attr_done[64] = {false};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) dev = 0;
+    if (!attr_done[dev]) {
+        if (cudaFuncSetAttribute(attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * kPfTile) != cudaSuccess) {
+            t_host_status = ST_LAUNCH;
+            return t_host_status;
+        }
+        attr_done[dev] = true;
+    }
+    const AttnPrefillParams p = {qkv, k_cache, v_cache, cos_tab, sin_tab, pos, out, tokens, heads, kv_heads, max_len,
+                                 1.4426950408889634f / sqrtf((float)head_dim)};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.attrs = attr;
+    cfg.numAttrs = tuning().pdl ? 1 : 0;
+    cfg.stream = stream;
+    const long long items = (long long)batch * tokens * kv_heads * 16;
+    cfg.gridDim = dim3((unsigned)((items + 255) / 256), 1, 1);
+    cfg.blockDim = dim3(256, 1, 1);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, rope_append_kernel, p, items);
+    cfg.gridDim = dim3((tokens + 15) / 16, heads / 4, batch);
+    cfg.blockDim = dim3(128, 1, 1);
+    cfg.dynamicSmemBytes = 4 * kPfTile;
+    if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, attn_prefill_kernel, p);
+    if (e != cudaSuccess) t_host_status = ST_LAUNCH;
+    checkLastCudaError(__LINE__);
+    return t_host_status;
+}
+
 static void run_norm_quant(bool gated, int mode, __nv_bfloat16* x, __nv_bfloat16* w, float eps, int M, int K,
                            int8_t* q, __nv_bfloat16* s_out, float* ss_out, cudaStream_t stream) {
     t_host_status = ST_OK;
@@ -890,7 +939,9 @@ static void run_norm_quant(bool gated, int mode, __nv_bfloat16* x, __nv_bfloat16
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(M, 1, 1);
-    cfg.blockDim = dim3(std::min(kActMaxThreads, std::max(64, (K / 8 + 31) / 32 * 32)), 1, 1);   // one vector per thread
+    // one vector per thread; for more rows than two per SM a quarter of the threads, four vectors each
+    const int T = act_row_threads(K);
+    cfg.blockDim = dim3(short_row && M >= 2 * device_sm_count() ? std::max(64, (T / 4 + 31) / 32 * 32) : T, 1, 1);
     cfg.dynamicSmemBytes = short_row ? (size_t)K * (gated ? 6 : (mode == ACT_PLAIN ? 2 : 4)) : (size_t)K * 2;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -929,6 +980,60 @@ extern "C" void ternaspmm_quant(__nv_bfloat16* x, int M, int K, int8_t* q, __nv_
 extern "C" void ternaspmm_scale_quant_sumsq(__nv_bfloat16* x, __nv_bfloat16* weight, int gated, int M, int K,
                                            int8_t* q, __nv_bfloat16* s_out, float* ss_out, cudaStream_t stream) {
     run_norm_quant(gated != 0, ACT_SCALE_SUMSQ, x, weight, 0.f, M, K, q, s_out, ss_out, stream);
+    checkLastCudaError(__LINE__);
+}
+
+static cudaLaunchConfig_t elementwise_launch(long long items, cudaStream_t stream, cudaLaunchAttribute* attr) {
+    attr->id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr->val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((items + 255) / 256), 1, 1);
+    cfg.blockDim = dim3(256, 1, 1);
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = tuning().pdl ? 1 : 0;
+    return cfg;
+}
+
+extern "C" void ternaspmm_rope(__nv_bfloat16* x, long long ld, float* cos_t, float* sin_t, __nv_bfloat16* out, int batch, int tokens, int heads,
+                               cudaStream_t stream) {
+    t_host_status = ST_OK;
+    const uintptr_t bits = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(cos_t) |
+                           reinterpret_cast<uintptr_t>(sin_t);
+    if (!x || !out || !cos_t || !sin_t || (bits & 15) || (ld & 7) || batch < 1 || tokens < 1 || heads < 1) {
+        t_host_status = ST_BAD_POINTER;
+        return;
+    }
+    const long long items = (long long)batch * tokens * heads * 16;
+    cudaLaunchAttribute attr;
+    cudaLaunchConfig_t cfg = elementwise_launch(items, stream, &attr);
+    if (cudaLaunchKernelEx(&cfg, rope_kernel, (const __nv_bfloat16*)x, ld, (const float*)cos_t, (const float*)sin_t, out, tokens, heads, items) != cudaSuccess)
+        t_host_status = ST_LAUNCH;
+    checkLastCudaError(__LINE__);
+}
+
+extern "C" void ternaspmm_relu2_gate(__nv_bfloat16* x13, __nv_bfloat16* out, int M, int K, cudaStream_t stream) {
+    t_host_status = ST_OK;
+    if (!x13 || !out || ((reinterpret_cast<uintptr_t>(x13) | reinterpret_cast<uintptr_t>(out)) & 15) || M < 1 || K < 8 || (K & 7)) {
+        t_host_status = ST_BAD_POINTER;
+        return;
+    }
+    const long long items = (long long)M * (K / 8);
+    cudaLaunchAttribute attr;
+    cudaLaunchConfig_t cfg = elementwise_launch(items, stream, &attr);
+    if (cudaLaunchKernelEx(&cfg, relu2_gate_kernel, (const __nv_bfloat16*)x13, out, K / 8, items) != cudaSuccess) t_host_status = ST_LAUNCH;
+    checkLastCudaError(__LINE__);
+}
+
+extern "C" void ternaspmm_bf16_to_f32(__nv_bfloat16* x, float* y, long long n, cudaStream_t stream) {
+    t_host_status = ST_OK;
+    if (!x || !y || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) || n < 1) {
+        t_host_status = ST_BAD_POINTER;
+        return;
+    }
+    cudaLaunchAttribute attr;
+    cudaLaunchConfig_t cfg = elementwise_launch(std::min<long long>((n + 7) / 8, 256ll * 16 * device_sm_count()), stream, &attr);
+    if (cudaLaunchKernelEx(&cfg, bf16_to_f32_kernel, (const __nv_bfloat16*)x, y, n) != cudaSuccess) t_host_status = ST_LAUNCH;
     checkLastCudaError(__LINE__);
 }
 

@@ -110,6 +110,43 @@ def rmsnorm(x: torch.Tensor, norm_weight: torch.Tensor, eps: float) -> torch.Ten
     return y.reshape(x.shape)
 
 
+def _stream():
+    return torch.cuda.current_stream().cuda_stream
+
+
+def rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor):
+    """RoPE on adjacent pairs as one kernel: x bf16 [B, T, H, 128] (heads contiguous), cos / sin fp32 [B, T, 64] equal in
+    every sequence (expanded).  None where the kernel does not take the tensors."""
+    B, T, H, D = x.shape
+    if not (x.is_cuda and x.dtype == torch.bfloat16 and cos.dtype == sin.dtype == torch.float32 and D == 128 and x.numel() > 0
+            and x.stride(3) == 1 and x.stride(2) == D and (B == 1 or x.stride(0) == T * x.stride(1)) and x.stride(1) % 8 == 0
+            and x.data_ptr() % 16 == 0 and cos.shape[1:] == sin.shape[1:] == (T, 64) and (B == 1 or cos.stride(0) == sin.stride(0) == 0)
+            and cos.stride()[1:] == sin.stride()[1:] == (64, 1) and cos.data_ptr() % 16 == 0 and sin.data_ptr() % 16 == 0):
+        return None
+    out = torch.empty((B, T, H, D), dtype=torch.bfloat16, device=x.device)
+    load_library().ternaspmm_rope(x.data_ptr(), x.stride(1), cos.data_ptr(), sin.data_ptr(), out.data_ptr(), B, T, H, _stream())
+    return out
+
+
+def relu2_gate(x13: torch.Tensor):
+    """relu(x1)^2 * x3 of bf16 [..., x1 | x3] as one kernel, rounded as the torch operators; None where it does not apply."""
+    K = x13.shape[-1] // 2
+    if not (x13.is_cuda and x13.dtype == torch.bfloat16 and x13.is_contiguous() and K % 8 == 0 and x13.numel() > 0 and x13.data_ptr() % 16 == 0):
+        return None
+    out = torch.empty((*x13.shape[:-1], K), dtype=torch.bfloat16, device=x13.device)
+    load_library().ternaspmm_relu2_gate(x13.data_ptr(), out.data_ptr(), x13.numel() // (2 * K), K, _stream())
+    return out
+
+
+def to_float(x: torch.Tensor) -> torch.Tensor:
+    """x.float(); bf16 on the GPU by the library (at the copy rate; torch's casting kernel reaches a third of it)."""
+    if not (x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous() and x.numel() > 0 and x.data_ptr() % 16 == 0):
+        return x.float()
+    out = torch.empty(x.shape, dtype=torch.float32, device=x.device)
+    load_library().ternaspmm_bf16_to_f32(x.data_ptr(), out.data_ptr(), x.numel(), _stream())
+    return out
+
+
 def attn_decode(qkv, k_cache, v_cache, cos_row, sin_row, pos, heads: int, kv_heads: int):
     """RoPE, cache append and attention of one new token per sequence in one kernel: qkv bf16 [B, 1, (heads + 2 *
     kv_heads) * 128], caches bf16 [B, L, kv_heads, 128], ``pos`` int64 [1] on the device, ``cos_row`` / ``sin_row`` bf16
@@ -124,6 +161,21 @@ def attn_decode(qkv, k_cache, v_cache, cos_row, sin_row, pos, heads: int, kv_hea
     status = load_library().ternaspmm_attn_decode(qkv.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), cos_row.data_ptr(),
                                                   sin_row.data_ptr(), pos.data_ptr(), out.data_ptr(), B, heads, kv_heads, D,
                                                   k_cache.shape[1], torch.cuda.current_stream().cuda_stream)
+    return out if status == 0 else None
+
+
+def attn_prefill(qkv, k_cache, v_cache, cos_tab, sin_tab, pos, heads: int, kv_heads: int):
+    """``attn_decode`` for T new tokens per sequence at consecutive positions (``pos`` int64 [T]), causal: qkv bf16
+    [B, T, (heads + 2 * kv_heads) * 128], tables bf16 [>= L, 64].  bf16 [B, T, heads * 128], or None."""
+    B, T, D = qkv.shape[0], qkv.shape[1], k_cache.shape[-1]
+    if not (qkv.is_cuda and qkv.dtype == k_cache.dtype == v_cache.dtype == cos_tab.dtype == torch.bfloat16 and pos.dtype == torch.int64
+            and D == 128 and heads % (4 * kv_heads) == 0 and k_cache.shape[1] <= cos_tab.shape[0]
+            and qkv.is_contiguous() and k_cache.is_contiguous() and v_cache.is_contiguous()):
+        return None
+    out = torch.empty((B, T, heads * D), dtype=torch.bfloat16, device=qkv.device)
+    status = load_library().ternaspmm_attn_prefill(qkv.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), cos_tab.data_ptr(),
+                                                   sin_tab.data_ptr(), pos.data_ptr(), out.data_ptr(), B, T, heads, kv_heads, D,
+                                                   k_cache.shape[1], torch.cuda.current_stream().cuda_stream)
     return out if status == 0 else None
 
 

@@ -20,7 +20,7 @@ import torch
 from torch import nn
 from torch.nn import functional as F
 
-from .linear import SpBitLinear, attn_decode, quant_input, rmsnorm, lm_head_argmax
+from .linear import SpBitLinear, attn_decode, attn_prefill, lm_head_argmax, quant_input, relu2_gate, rmsnorm, rope, to_float
 
 
 @dataclass
@@ -52,6 +52,9 @@ class RMSNorm(nn.Module):
         self.weight = nn.Parameter(torch.ones(dim))
 
     def forward(self, x):
+        if (x.is_cuda and x.dtype == self.weight.dtype == torch.bfloat16 and x.shape[-1] % 16 == 0 and x.shape[-1] <= 57344 and x.numel() > 0
+                and not torch.is_grad_enabled()):
+            return rmsnorm(x, self.weight, self.eps)       # one launch instead of seven, the fused front-ends' summation order
         xf = x.float()
         y = xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + self.eps)
         return (y * self.weight.float()).to(x.dtype)
@@ -78,6 +81,9 @@ def rope_tables(head_dim: int, max_len: int, theta: float, device):
 
 def apply_rope(x, cos, sin):
     """Rotate adjacent pairs (2i, 2i+1); x [B, T, H, D], cos/sin [B, T, D/2]."""
+    out = rope(x, cos, sin) if not torch.is_grad_enabled() else None
+    if out is not None:
+        return out
     xf = x.float().unflatten(-1, (-1, 2))
     a, b = xf[..., 0], xf[..., 1]
     c, s = cos.unsqueeze(2), sin.unsqueeze(2)
@@ -120,23 +126,24 @@ class Attention(nn.Module):
         o = o.transpose(1, 2).reshape(B, T, H * D)
         return self._project(o, x, fused)
 
-    def forward_flash(self, x, cache: LayerCache, pos, rope, rope_row, seqlens, fused):
+    def forward_flash(self, x, cache: LayerCache, pos, rope, rope_row, fused):
         """Attention glue in the cache layout [B, L, Hkv, D]: RoPE on adjacent pairs, cache append and causal
-        attention in one launch - the library's decode kernel for one token per sequence, flash_attn's kv-cache
-        kernel for prompts and for head shapes that the former does not take."""
+        attention - the library's kernels for one token or a prompt per sequence, flash_attn's kv-cache kernel for head
+        shapes that they do not take."""
         B, T = x.shape[0], x.shape[1]
         H, Hkv, D = self.n_heads, self.n_kv_heads, self.head_dim
         qkv = self.wqkv(x) if fused is None else self.wqkv.forward_normed(x, fused[0], fused[1])
         if rope_row is not None:
             o = attn_decode(qkv, cache[0], cache[1], *rope_row, pos, H, Hkv)
-            if o is not None:
-                return self._project(o, x, fused)
+        else:
+            o = attn_prefill(qkv, cache[0], cache[1], *rope, pos, H, Hkv)
+        if o is not None:
+            return self._project(o, x, fused)
         from flash_attn import flash_attn_with_kvcache
         q = qkv[..., : H * D].view(B, T, H, D)
         k = qkv[..., H * D: (H + Hkv) * D].view(B, T, Hkv, D)
         v = qkv[..., (H + Hkv) * D:].view(B, T, Hkv, D)
-        if seqlens is None:
-            seqlens = pos[:1].to(torch.int32).expand(B).contiguous()
+        seqlens = pos[:1].to(torch.int32).expand(B).contiguous()
         o = flash_attn_with_kvcache(q, cache[0], cache[1], k=k, v=v, rotary_cos=rope[0], rotary_sin=rope[1],
                                     cache_seqlens=seqlens, causal=True, rotary_interleaved=True)
         return self._project(o.reshape(B, T, H * D), x, fused)
@@ -170,8 +177,11 @@ class FeedForward(nn.Module):
         return self.w2.forward_normed(x13, self.ffn_sub_norm.weight, eps, gated=True, residual=h)
 
     def forward(self, x):
-        x1, x3 = self.w13(x).chunk(2, -1)
-        inner = F.relu(x1) ** 2 * x3
+        x13 = self.w13(x)
+        inner = relu2_gate(x13) if not torch.is_grad_enabled() else None
+        if inner is None:
+            x1, x3 = x13.chunk(2, -1)
+            inner = F.relu(x1) ** 2 * x3
         if self.ffn_sub_norm is not None:
             inner = self.ffn_sub_norm(inner)
         return self.w2(inner)
@@ -258,7 +268,8 @@ class Transformer(nn.Module):
         if h.is_cuda and B * T <= 8 and emb.dtype == torch.bfloat16 and h.dtype == torch.bfloat16 and h.shape[-1] % 32 == 0:
             logits, toks = lm_head_argmax(h, emb, want_logits=not greedy, want_argmax=greedy)
             return (None, toks.view(B, T)) if greedy else logits.view(B, T, -1)
-        logits = F.linear(h, emb).float()
+        logits = F.linear(h, emb)
+        logits = logits.float() if greedy else to_float(logits)
         return (None, logits.argmax(-1)) if greedy else logits
 
     def forward(self, tokens: torch.Tensor, cache: List[LayerCache], pos: torch.Tensor, greedy_last: bool = False):
@@ -274,8 +285,7 @@ class Transformer(nn.Module):
         fused = self.args.fused_glue and self.tp == 1
         flash, cos, sin, mask = None, None, None, None
         if self.flash:   # the attention kernels apply RoPE from the tables and mask by position themselves
-            flash = (pos, self._rope_lp, tuple(t.index_select(0, pos) for t in self._rope_lp) if T == 1 else None,
-                     pos[:1].to(torch.int32).expand(B).contiguous() if T > 1 else None)
+            flash = (pos, self._rope_lp, tuple(t.index_select(0, pos) for t in self._rope_lp) if T == 1 else None)
         else:
             cos, sin = self._rope[0][pos].expand(B, T, -1), self._rope[1][pos].expand(B, T, -1)
             keys = torch.arange(self.max_seq_len, device=tokens.device)

@@ -3,7 +3,7 @@ of its key tiles."""
 import pytest
 import torch
 
-from ternainfer_b200.linear import attn_decode
+from ternainfer_b200.linear import attn_decode, attn_prefill
 from ternainfer_b200.model import apply_rope, rope_tables
 
 pytestmark = pytest.mark.gpu
@@ -33,3 +33,29 @@ def test_decode_attention(lib, B, pos, L, H, Hkv):
     assert ((out.double() - want).norm() / want.norm()).item() < 3e-3
     assert (out.double() - want).abs().max().item() < 1.2e-2 * want.abs().max().item()
     assert torch.equal(attn_decode(qkv, kc, vc, cos[p], sin[p], p, H, Hkv), out)
+
+
+@pytest.mark.parametrize("H,Hkv", [(20, 5), (64, 8)])
+@pytest.mark.parametrize("B,T,past,L", [(1, 2, 0, 8), (2, 16, 0, 16), (1, 17, 0, 64), (3, 64, 0, 64), (1, 65, 1, 80), (2, 200, 63, 300), (1, 613, 0, 613),
+                                        (1, 40, 1000, 1040)])
+def test_prompt_attention(lib, B, T, past, L, H, Hkv):
+    D = 128
+    g = torch.Generator(device="cuda").manual_seed(T + past)
+    qkv = torch.randn((B, T, (H + 2 * Hkv) * D), generator=g, device="cuda").to(torch.bfloat16)
+    kc, vc = (torch.randn((B, L, Hkv, D), generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    kc[:, past:], vc[:, past:] = float("nan"), float("nan")
+    k0, v0 = kc.clone(), vc.clone()
+    cos, sin = (t.to(torch.bfloat16) for t in rope_tables(D, L, 500000.0, "cuda"))
+    p = torch.arange(past, past + T, device="cuda")
+    out = attn_prefill(qkv, kc, vc, cos, sin, p, H, Hkv)
+    q, k, v = (t.view(B, T, -1, D) for t in qkv.split([H * D, Hkv * D, Hkv * D], -1))
+    c, s = cos[p].float().expand(B, T, -1), sin[p].float().expand(B, T, -1)
+    q, k = apply_rope(q, c, s), apply_rope(k, c, s)
+    k0[:, past:past + T], v0[:, past:past + T] = k, v
+    assert torch.equal(kc.view(torch.int16), k0.view(torch.int16)) and torch.equal(vc.view(torch.int16), v0.view(torch.int16))
+    kk, vv = (t[:, :past + T].double().repeat_interleave(H // Hkv, 2) for t in (k0, v0))
+    a = torch.einsum("bthd,blhd->bhtl", q.double(), kk) / D ** 0.5
+    a = a.masked_fill(torch.arange(past + T, device="cuda")[None, :] > p[:, None], float("-inf")).softmax(-1)
+    want = torch.einsum("bhtl,blhd->bthd", a, vv).reshape(B, T, H * D)
+    assert ((out.double() - want).norm() / want.norm()).item() < 4e-3
+    assert (out.double() - want).abs().max().item() < 1.2e-2 * want.abs().max().item()
