@@ -662,18 +662,18 @@ static cudaError_t launch_w2_small(W2Params& p, cudaStream_t stream) {
     // the next launch's CTA starts beside this one), evenly loaded; at least four for the front-end and the epilogue
     const int per = (KP + kW2MaxWarps - 1) / kW2MaxWarps, W = std::max(4, (KP + per - 1) / per);
     p.pairs_q = KP / W, p.pairs_r = KP % W;
-    // ring: all of the CTA's weights when they fit 64 KB (two launches' prefetches fit an SM side by side), otherwise
-    // slots of about 32 KB per CTA and up to four of them
-    const int groups = (R + RG - 1) / RG;
-    p.chunk_pairs = std::max(1, std::min(per, 32 * 1024 / (W * RG * 512)));
-    const int chunks = groups * ((per + p.chunk_pairs - 1) / p.chunk_pairs), slot_bytes = RG * p.chunk_pairs * 512;
-    const int fit = 64 * 1024 / (W * slot_bytes);
-    p.slots = std::min(chunks, chunks <= fit && chunks <= kW2MaxSlots ? chunks : 4);
-    p.smem = w2_smem(R, MT, tokens, K, W, p.slots, slot_bytes, XS, FE, p.e.residual != nullptr);
-    while (p.smem.total > kW2MaxSmem && p.slots > 1) {
-        --p.slots;
-        p.smem = w2_smem(R, MT, tokens, K, W, p.slots, slot_bytes, XS, FE, p.e.residual != nullptr);
+    // ring: all of the CTA's weights when they fit 64 KB (two launches' prefetches fit an SM side by side), otherwise two
+    // slots or more with copies of 4 KB (the copy engine takes about 60 cycles for each, whatever its size: 57344 x 8192
+    // at 4 tokens 43 us with copies of 1 KB, 35 with 2 KB, 32 with 3.5 KB)
+    const int groups = (R + RG - 1) / RG, unit = W * RG * 512, room = kW2MaxSmem - w2_smem(R, MT, tokens, K, W, 0, 0, XS, FE, p.e.residual != nullptr).total;
+    if (room < unit) return cudaErrorInvalidValue;
+    p.chunk_pairs = per, p.slots = groups;
+    if (groups > kW2MaxSlots || groups * per * unit > std::min(64 * 1024, room)) {
+        p.chunk_pairs = std::max(1, std::min(std::min(per, 8), room / 2 / unit));
+        const int chunks = groups * ((per + p.chunk_pairs - 1) / p.chunk_pairs);
+        p.slots = std::min(std::min(chunks, kW2MaxSlots), room / (p.chunk_pairs * unit));
     }
+    p.smem = w2_smem(R, MT, tokens, K, W, p.slots, RG * p.chunk_pairs * 512, XS, FE, p.e.residual != nullptr);
     if (p.smem.total > kW2MaxSmem) return cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas, blocks, 1);
@@ -689,16 +689,17 @@ static cudaError_t launch_w2_small(W2Params& p, cudaStream_t stream) {
     return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
-// RG: strips whose accumulators a warp holds at a time; one where a CTA has one or two strips.  XS: activations in shared
+// RG: strips whose accumulators a warp holds at a time; one where a CTA has one or two strips, and where three
+// strips' share of a long K would leave no room for a second ring slot (8192 x 28672 at 1 token 26.9 -> 20.7 us).  XS: activations in shared
 // memory while they leave room for the ring.
 template <int FE>
 static cudaError_t launch_w2_fused(W2Params& p, cudaStream_t stream) {
-    return p.e.N / 16 <= 2 * device_sm_count() ? launch_w2_small<1, 1, 2, FE, true>(p, stream) : launch_w2_small<1, 3, 2, FE, true>(p, stream);
+    return p.e.N / 16 <= 2 * device_sm_count() || p.e.K > 8192 ? launch_w2_small<1, 1, 2, FE, true>(p, stream) : launch_w2_small<1, 3, 2, FE, true>(p, stream);
 }
 
 static cudaError_t launch_w2_int8(W2Params& p, cudaStream_t stream) {
     const int M = p.e.M;
-    const bool xs = (long long)std::min(M, 32) * (p.e.K + 64) <= 96 * 1024;
+    const bool xs = (long long)std::min(M, 32) * (p.e.K + 64) <= 120 * 1024;
     if (M <= 8) return xs ? launch_w2_fused<W2_INT8>(p, stream) : launch_w2_small<1, 3, 1, W2_INT8, false>(p, stream);
     if (M <= 16) return xs ? launch_w2_small<2, 2, 2, W2_INT8, true>(p, stream) : launch_w2_small<2, 2, 1, W2_INT8, false>(p, stream);
     return xs ? launch_w2_small<4, 2, 1, W2_INT8, true>(p, stream) : launch_w2_small<4, 2, 1, W2_INT8, false>(p, stream);

@@ -29,6 +29,8 @@ namespace tsp {
 constexpr int kW2PairDecoders = 8;
 constexpr int kW2PairFirstDecoder = kLgFirstEpi + kPairEpiWarps;
 constexpr int kW2PairThreads = (kW2PairFirstDecoder + kW2PairDecoders + 1) * 32;
+constexpr int kW2OutStride = 80;           // bytes between two tokens of an output slice in shared memory: conflict-free
+constexpr int kW2OutStageBytes = 16 * kW2OutStride;
 constexpr int kW2PairMaxStages = 8;
 constexpr int kW2PairSlots = 2;            // of two-bit weights: 128 rows x 512 k each
 constexpr int kW2PairChunk = 4;            // stages per slot
@@ -45,7 +47,7 @@ struct W2PairSmem {
     static constexpr int abort_flag = 196;
     static constexpr int scl = 256;             // float[64] per epilogue warp
     static constexpr int ostage = scl + kPairEpiWarps * 64 * 4;   // 1 KB per epilogue warp (output staging)
-    static constexpr int w = (ostage + kPairEpiWarps * kOutStageBytes + 1023) / 1024 * 1024;
+    static constexpr int w = (ostage + kPairEpiWarps * kW2OutStageBytes + 1023) / 1024 * 1024;
     static constexpr int stage = w + kW2PairSlots * kW2PairSlotBytes;   // [weights 16 KB][activations NT * 64 bytes] per stage
     static constexpr int total = 227 * 1024;
     static constexpr int stage_bytes = total - 1024 - stage;
@@ -54,6 +56,63 @@ struct W2PairSmem {
 // arrive on a barrier of any CTA of the cluster, ordering this CTA's accesses only
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_bar) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+
+// bf16 epilogue of a slice of 16 tokens x 32 weight rows.  The accumulators come as 8x8 matrix fragments (rows = weight rows,
+// columns = tokens; a lane has two neighbouring tokens of four rows), so that a lane needs four token scales instead of
+// sixteen and stmatrix transposes on the way to shared memory: a third of the instructions of the row-per-lane form
+// (store_slice16_wide).  ws_rows: weight scales of rows 8r + lane / 4; `ahead`: the residual as load_residual16 reads it.
+__device__ __forceinline__ void store_slice16_matrix(const SpmmParams& p, uint32_t tmem, const float* sc, long long o_row0, int live, bool fast,
+                                                     const float (&ws_rows)[4], uint32_t stage, int lane, const uint4 (&ahead)[2]) {
+    int v[2][8];                                             // [16 rows][token half x (row half, token)]
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+        asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(v[h][0]), "=r"(v[h][1]), "=r"(v[h][2]), "=r"(v[h][3]), "=r"(v[h][4]), "=r"(v[h][5]), "=r"(v[h][6]), "=r"(v[h][7])
+                     : "r"(tmem + ((uint32_t)(16 * h) << 16)));
+    const float2 s0 = *reinterpret_cast<const float2*>(sc + 2 * (lane & 3)), s1 = *reinterpret_cast<const float2*>(sc + 8 + 2 * (lane & 3));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    uint32_t m[2][4];                                        // [token half][8 rows]: two tokens
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const int a = v[r >> 1][4 * t + 2 * (r & 1)] >> 6, b = v[r >> 1][4 * t + 2 * (r & 1) + 1] >> 6;   // the operand holds 64 * weight
+            const float sa = t ? s1.x : s0.x, sb = t ? s1.y : s0.y;
+            if (fast) {
+                m[t][r] = act_pack(__fmul_rn(__int2float_rn(a), sa), __fmul_rn(__int2float_rn(b), sb));
+            } else {
+                m[t][r] = (uint32_t)__bfloat16_as_ushort(scale_epilogue(a, sa, ws_rows[r], p.epilogue)) |
+                          ((uint32_t)__bfloat16_as_ushort(scale_epilogue(b, sb, ws_rows[r], p.epilogue)) << 16);
+            }
+        }
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {                            // matrix r -> tokens 8t .. 8t+7, columns 8r .. 8r+7; lane l addresses row l % 8 of matrix l / 8
+        const uint32_t addr = stage + (uint32_t)((8 * t + (lane & 7)) * kW2OutStride + (lane >> 3) * 16);
+        asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(m[t][0]), "r"(m[t][1]), "r"(m[t][2]),
+                     "r"(m[t][3])
+                     : "memory");
+    }
+    __syncwarp();
+    const int part = lane & 3;
+    uint4 d[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) d[i] = lds128(stage + (uint32_t)(((lane >> 2) + 8 * i) * kW2OutStride + part * 16));
+    if (p.residual) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            uint32_t* dv = reinterpret_cast<uint32_t*>(&d[i]);
+            const uint32_t* rv = reinterpret_cast<const uint32_t*>(&ahead[i]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) dv[e] = act_pack(act_lo(rv[e]) + act_lo(dv[e]), act_hi(rv[e]) + act_hi(dv[e]));
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int row = (lane >> 2) + 8 * i;
+        if (row < live) stg_128(reinterpret_cast<__nv_bfloat16*>(p.out) + o_row0 + (long long)row * p.N + part * 8, d[i]);
+    }
+    __syncwarp();   // the staging area is free for the next slice
 }
 
 __device__ __forceinline__ bool elect_one() {
@@ -111,6 +170,7 @@ __global__ void __launch_bounds__(kW2PairThreads, 1)
     const int n_tiles = RB * ((M + NT - 1) / NT);
     const int my_tiles = pair < n_tiles ? (n_tiles - 1 - pair) / npairs + 1 : 0;
 
+    phase_mark(0);
     griddep_launch_dependents();
     if (tid == 0) {
         for (int s = 0; s < ST; ++s) {
@@ -133,11 +193,13 @@ __global__ void __launch_bounds__(kW2PairThreads, 1)
     tc_fence_after();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(rest + L::tmem_slot);
     bool ok = true;
+    phase_mark(1);
 
     if (warp == 0) {
         // ------------------------------------------------ activation loader (both CTAs)
         if (lane == 0) {
             griddep_wait();   // the activations come from earlier kernels of the stream
+            phase_mark(2);
             int s = 0, it = 0;
             for (int ti = 0; ti < my_tiles && ok; ++ti) {
                 const int t0 = ((pair + ti * npairs) / RB) * NT + (int)crank * (NT / 2);   // this CTA's tokens
@@ -171,6 +233,7 @@ __global__ void __launch_bounds__(kW2PairThreads, 1)
                     ok = __all_sync(0xffffffffu, wait_suspended(bar_full(s), it & 1, abort_flag));
                     if (!ok) break;
                     tc_fence_after();
+                    if (ti == 0 && ks == 0 && lane == 0) phase_mark_here(3);
                     const uint32_t off = (uint32_t)s * (stage_bytes >> 4);   // descriptor addresses count 16 bytes
                     if (elected) {
 #pragma unroll
@@ -218,34 +281,47 @@ __global__ void __launch_bounds__(kW2PairThreads, 1)
         for (int ti = 0; ti < my_tiles && ok; ++ti) {
             const bool live = ((pair + ti * npairs) % RB) * (kPairRows / 16) + (int)crank * 8 + strip_in < (N >> 4);
 #pragma unroll 1
-            for (int ks = 0; ks < KS; ++ks) {
+            for (int ks = 0; ks < KS; ks += 2) {         // two stages per turn: one fence, and the latencies overlap
                 const int in_slot = ks & (kW2PairChunk - 1);
+                const bool two = ks + 1 < KS;
                 if (in_slot == 0) {
                     ok = wait_suspended(bar_w(ws), wit & 1, abort_flag);
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                 }
-                uint4 w = make_uint4(0, 0, 0, 0);
-                if (live) w = lds128(w_lane + ws * kW2PairSlotBytes + in_slot * 512);
-                if (odd) w = make_uint4(w.z, w.w, w.x, w.y);
-                uint32_t a[4], b[4], c[4], d[4];
-                w2_decode(w.x, a), w2_decode(w.y, b), w2_decode(w.z, c), w2_decode(w.w, d);
-                if (it > 0) ok = wait_suspended(bar_empty(s), (it - 1) & 1, abort_flag);
+                uint4 w[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
+                if (live) {
+                    w[0] = lds128(w_lane + ws * kW2PairSlotBytes + in_slot * 512);
+                    if (two) w[1] = lds128(w_lane + ws * kW2PairSlotBytes + in_slot * 512 + 512);
+                }
+                const int s0 = s, s1 = s + 1 == ST ? 0 : s + 1, it1 = it + (s + 1 == ST);
+                if (it > 0) ok = wait_suspended(bar_empty(s0), (it - 1) & 1, abort_flag);
+                if (two && it1 > 0) ok = ok && wait_suspended(bar_empty(s1), (it1 - 1) & 1, abort_flag);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
-                const uint32_t off = (uint32_t)s * stage_bytes;
-                sts128(first + off, make_uint4(a[0], a[2], b[0], b[2]));
-                sts128(first + off + 8 * 128, make_uint4(a[1], a[3], b[1], b[3]));
-                sts128(second + off, make_uint4(c[0], c[2], d[0], d[2]));
-                sts128(second + off + 8 * 128, make_uint4(c[1], c[3], d[1], d[3]));
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    if (u == 1 && !two) break;
+                    const uint4 v = odd ? make_uint4(w[u].z, w[u].w, w[u].x, w[u].y) : w[u];
+                    uint32_t a[4], b[4];
+                    const uint32_t off = (uint32_t)(u ? s1 : s0) * stage_bytes;
+                    w2_decode(v.x, a), w2_decode(v.y, b);
+                    sts128(first + off, make_uint4(a[0], a[2], b[0], b[2]));
+                    sts128(first + off + 8 * 128, make_uint4(a[1], a[3], b[1], b[3]));
+                    w2_decode(v.z, a), w2_decode(v.w, b);
+                    sts128(second + off, make_uint4(a[0], a[2], b[0], b[2]));
+                    sts128(second + off + 8 * 128, make_uint4(a[1], a[3], b[1], b[3]));
+                }
                 fence_proxy_async_smem();        // generic-proxy stores -> visible to the tensor cores' async proxy
                 __syncwarp();
-                const bool slot_done = in_slot == kW2PairChunk - 1 || ks == KS - 1;
+                const bool slot_done = in_slot == kW2PairChunk - 2 || ks + 2 >= KS;
                 if (lane == 0) {
-                    mbar_arrive_remote(full0 + 8 * s);
+                    mbar_arrive_remote(full0 + 8 * s0);
+                    if (two) mbar_arrive_remote(full0 + 8 * s1);
                     if (slot_done) mbar_arrive(bar_w_free(ws));
                 }
                 if (++s == ST) s = 0, ++it;
+                if (two && ++s == ST) s = 0, ++it;
                 if (slot_done && ++ws == WS) ws = 0, ++wit;
             }
         }
@@ -255,7 +331,7 @@ __global__ void __launch_bounds__(kW2PairThreads, 1)
         const int quarter = warp & 3;          // the tensor-memory lanes a warp may read: 32 * (warp % 4)
         const int cg = (warp - kLgFirstEpi) >> 2;   // this warp's slices of 16 tokens: cg, cg + 4, ...
         float* s_w = s_s + (warp - kLgFirstEpi) * 64;
-        const uint32_t ostage = sbase + L::ostage + (uint32_t)((warp - kLgFirstEpi) * kOutStageBytes);
+        const uint32_t ostage = sbase + L::ostage + (uint32_t)((warp - kLgFirstEpi) * kW2OutStageBytes);
         const bool wide = ((reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(p.residual)) & 15) == 0;
         for (int ti = 0; ti < my_tiles; ++ti) {
             const int tile = pair + ti * npairs;
@@ -268,6 +344,9 @@ __global__ void __launch_bounds__(kW2PairThreads, 1)
             const int g0 = __shfl_sync(0xffffffffu, gsel, 0);
             const bool fast = p.epilogue == EPI_PREFILL && __all_sync(0xffffffffu, gsel == g0 || gsel < 0);
             const float ws0 = __shfl_sync(0xffffffffu, ws_el, 0);
+            float ws_rows[4];                      // of the rows that store_slice16_matrix gives this lane
+#pragma unroll
+            for (int r = 0; r < 4; ++r) ws_rows[r] = __shfl_sync(0xffffffffu, ws_el, 8 * r + (lane >> 2));
             __syncwarp();                          // the previous tile's scales are no longer read
             for (int i = lane; i < 64; i += 32) {  // token of local slot i: slice cg + 4 (i / 16)
                 const int c = (cg + 4 * (i >> 4)) * 16 + (i & 15);
@@ -287,37 +366,41 @@ __global__ void __launch_bounds__(kW2PairThreads, 1)
             ok = __all_sync(0xffffffffu, ok);   // the tensor-memory loads below are warp-collective
             if (!ok) break;
             tc_fence_after();
+            if (ti == 0 && warp == kLgFirstEpi && lane == 0) phase_mark_here(4);
 #pragma unroll 1
             for (int i = 0; (cg + 4 * i) * 16 < cols; ++i) {
                 const int c0 = (cg + 4 * i) * 16;
-                int v[16];
-                tmem_ld16(tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(buf * 256 + c0), v);
-#pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] >>= 6;   // the operand holds 64 * weight
                 const long long o0 = (long long)(t0 + c0) * N + n;
                 const int live = n_ok ? min(16, M - t0 - c0) : 0;   // (n_ok is uniform over the warp: N is a multiple of 64)
+                const uint32_t tmem = tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(buf * 256 + c0);
                 if (wide) {
                     residual_of(i + 1, res_next);
-                    store_slice16_wide(p, v, s_w + 16 * i, o0 - lane, live, fast, ws_el, ostage, lane, res);
+                    store_slice16_matrix(p, tmem, s_w + 16 * i, o0 - lane, live, fast, ws_rows, ostage, lane, res);
                     res[0] = res_next[0], res[1] = res_next[1];
                 } else {
+                    int v[16];
+                    tmem_ld16(tmem, v);
                     float sc[16];
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) sc[j] = s_w[16 * i + j];
+                    for (int j = 0; j < 16; ++j) v[j] >>= 6, sc[j] = s_w[16 * i + j];   // (the operand holds 64 * weight)
                     store_slice16(p, v, sc, o0, live, fast, ws_el);
                 }
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(map_to_rank(bar_acc_empty(buf), 0));   // the leader may overwrite this buffer
+            // the leader may overwrite this buffer (CTA scope: a cluster release would wait for the output stores)
+            if (lane == 0) mbar_arrive_remote(map_to_rank(bar_acc_empty(buf), 0));
+            if (ti == 0 && warp == kLgFirstEpi && lane == 0) phase_mark_here(5);
         }
     }
+    phase_mark(6);
     if (*abort_flag && tid == 0) atomicExch(p.status, ST_WAIT_TIMEOUT);
     tc_fence_before();
     __syncthreads();
-    cluster_arrive();        // neither CTA frees tensor memory or leaves while the other may still signal it
+    cluster_arrive_relaxed();   // neither CTA frees tensor memory or leaves while the other may still signal it
     cluster_wait();
     if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
+    phase_mark(7);
 }
 
 // Tokens per tile for M tokens, RB row blocks, KS stages and `pairs` resident pairs: the shortest time of the busiest pair.
