@@ -12,9 +12,10 @@
 // of four values and pairs them up with byte permutes.  The scores leave the first product in the registers in which the
 // second one wants its A operand.  Running maximum and sum per warp, one merge per CTA (the new token's own key and
 // value are one more partial result there), one over the cluster.  fp32 everywhere but the inputs, the rotated query,
-// the probabilities of a group and the result.  Measured (10 caches in turn, 5 key / value heads): 1 sequence of 600
-// tokens 5.6 us, 8 of 1100 10.7 us, 16 of 2000 19 us (82 MB: 12.6 us at the copy rate); with value tiles staged in shared
-// memory and a CTA-wide softmax 6.0, 14.8, 32.9 us.
+// the probabilities of a group and the result.  Measured (60 caches in turn, 5 key / value heads): 1 sequence of 600 tokens
+// 5.0 us, 8 of 1100 9.3 us, 16 of 2000 17.8 us (82 MB: 12.6 us at the copy rate); with the cache rows asked for ahead of
+// the projections and a merge of one dimension per thread 5.6, 10.7, 19 us; with value tiles staged in shared memory and a
+// CTA-wide softmax 6.0, 14.8, 32.9 us.
 #pragma once
 #include <cuda_bf16.h>
 
@@ -69,7 +70,8 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 3) attn_decode_kernel(const A
     __shared__ __align__(16) float os[kParts][GQ][kAttnD];
     __shared__ float ms[kParts][8], ls[kParts][8];
     __shared__ __align__(16) __nv_bfloat16 kn[kAttnD];
-    __shared__ float slot_o[kOut], slot_m[8][GQ], slot_l[8][GQ];   // pushed by the cluster's CTAs: [sender][outputs of this CTA], statistics
+    __shared__ __align__(16) float slot_o[kOut];
+    __shared__ float slot_m[8][GQ], slot_l[8][GQ];   // pushed by the cluster's CTAs: [sender][outputs of this CTA], statistics
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
     const int S = gridDim.x, rank = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
 
@@ -103,15 +105,28 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 3) attn_decode_kernel(const A
     phase_mark(1);
     griddep_wait();
     phase_mark(2);
-    // Everything is asked for before the position is known: rows at and beyond it are masked below.
+    // Everything is asked for before the position is known (rows at and beyond it are masked below), the new token's
+    // projections ahead of the cache rows: a warp's loads return in order, and 8 KB of keys and values per warp, 100 KB per SM,
+    // take their time (8 sequences of 1100 tokens: the query was in place 2.8 us after the dependency, before).
     const long long pos_ll = *p.pos;
+    constexpr int kPairs = (GQ + 1) * 64 / kThreads + ((GQ + 1) * 64 % kThreads != 0);   // rotated pairs per thread, query heads and the new key
+    uint32_t xy[kPairs];
+    float rc[kPairs], rs[kPairs];
+#pragma unroll
+    for (int k = 0; k < kPairs; ++k) {
+        const int i = tid + k * kThreads, h = i >> 6, d = i & 63;
+        if (h < GQ + (rank == 0)) {
+            xy[k] = ld_cg_32(qkv + (size_t)(h < GQ ? hk * GQ + h : p.heads + hk) * kAttnD + 2 * d);
+            rc[k] = __bfloat162float(p.cos_row[d]), rs[k] = __bfloat162float(p.sin_row[d]);
+        }
+    }
+    const uint2 vnew = *reinterpret_cast<const uint2*>(qkv + (size_t)(p.heads + p.kv_heads + hk) * kAttnD + lane * 4);
     if (gi * 16 < p.max_len) load_keys(gi), load_values(gi);
-#pragma unroll 1
-    for (int i = tid; i < GQ * 64 + (rank == 0 ? 64 : 0); i += kThreads) {
-        const int h = i >> 6, d = i & 63;                     // pairs of the query heads, then (rank 0) of the new key
-        const uint32_t xy = ld_cg_32(qkv + (size_t)(h < GQ ? hk * GQ + h : p.heads + hk) * kAttnD + 2 * d);
-        const uint32_t r = rope_pair(xy, __bfloat162float(p.cos_row[d]), __bfloat162float(p.sin_row[d]));
-        (h < GQ ? reinterpret_cast<uint32_t*>(qs) + h * kQStride / 2 : reinterpret_cast<uint32_t*>(kn))[d] = r;
+#pragma unroll
+    for (int k = 0; k < kPairs; ++k) {
+        const int i = tid + k * kThreads, h = i >> 6, d = i & 63;
+        if (h < GQ + (rank == 0))
+            (h < GQ ? reinterpret_cast<uint32_t*>(qs) + h * kQStride / 2 : reinterpret_cast<uint32_t*>(kn))[d] = rope_pair(xy[k], rc[k], rs[k]);
     }
     // cached keys 0 .. pos-1, the new one goes to row pos (clamped: a wrong position must not leave the cache)
     const int pos = (int)max(0ll, min(pos_ll, (long long)p.max_len - 1));
@@ -186,7 +201,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 3) attn_decode_kernel(const A
 #pragma unroll
             for (int k = 16; k > 0; k >>= 1) d += __shfl_xor_sync(0xffffffffu, d, k);
             d *= p.scale_log2;
-            const uint2 v = *reinterpret_cast<const uint2*>(qkv + (size_t)(p.heads + p.kv_heads + hk) * kAttnD + lane * 4);
+            const uint2 v = vnew;
             *reinterpret_cast<float4*>(&os[kAttnWarps][h][lane * 4]) = make_float4(bf16_lo(v.x), bf16_hi(v.x), bf16_lo(v.y), bf16_hi(v.y));
             if (h == 0) {
                 *reinterpret_cast<uint2*>(p.k_cache + head0 + (size_t)pos * row + lane * 4) = kv;
@@ -207,21 +222,28 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 3) attn_decode_kernel(const A
     // ---- merge the CTA's parts (a part without keys has maximum -inf and weight 0) and push them to the CTA that finishes them
     const int per = kOut / S, lg = 31 - __clz(per);           // outputs finished by a CTA, a power of two
 #pragma unroll 1
-    for (int h = 0; h < GQ; ++h) {
-        float mk[kParts], top = -INFINITY, sum = 0.f, o = 0.f;
+    for (int h = warp; h < GQ; h += kAttnWarps) {             // a warp per head, four dimensions per lane
+        float mk[kParts], lk[kParts], top = -INFINITY, sum = 0.f;
+        float4 ok[kParts], o = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int k = 0; k < kParts; ++k) mk[k] = ms[k][h], top = fmaxf(top, mk[k]);
+        for (int k = 0; k < kParts; ++k) {
+            mk[k] = ms[k][h], lk[k] = ls[k][h];
+            ok[k] = k < kAttnWarps || rank == 0 ? *reinterpret_cast<const float4*>(&os[k][h][lane * 4]) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int k = 0; k < kParts; ++k) top = fmaxf(top, mk[k]);
 #pragma unroll
         for (int k = 0; k < kParts; ++k) {
             const float w = mk[k] == -INFINITY ? 0.f : exp2f(mk[k] - top);
-            sum += w * ls[k][h];
-            if (k < kAttnWarps || rank == 0) o += w * os[k][h][tid];   // one dimension per thread
+            sum += w * lk[k];
+            o.x += w * ok[k].x, o.y += w * ok[k].y, o.z += w * ok[k].z, o.w += w * ok[k].w;
         }
-        const int i = h * kAttnD + tid;
-        st_cluster_f32(map_to_rank(smem_u32(&slot_o[rank * per + (i & (per - 1))]), i >> lg), o);
-        if (tid < S) {
-            st_cluster_f32(map_to_rank(smem_u32(&slot_m[rank][h]), tid), top);
-            st_cluster_f32(map_to_rank(smem_u32(&slot_l[rank][h]), tid), sum);
+        const int i = h * kAttnD + lane * 4;                  // (per is at least 64: four outputs have one owner)
+        st_cluster_v4(map_to_rank(smem_u32(&slot_o[rank * per + (i & (per - 1))]), i >> lg), __float_as_int(o.x), __float_as_int(o.y),
+                      __float_as_int(o.z), __float_as_int(o.w));
+        if (lane < S) {
+            st_cluster_f32(map_to_rank(smem_u32(&slot_m[rank][h]), lane), top);
+            st_cluster_f32(map_to_rank(smem_u32(&slot_l[rank][h]), lane), sum);
         }
     }
     phase_mark(5);
@@ -230,13 +252,17 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 3) attn_decode_kernel(const A
     phase_mark(6);
     for (int j = tid; j < per; j += kThreads) {
         const int i = rank * per + j, h = i / kAttnD;
-        float top = -INFINITY, l_all = 0.f, o_all = 0.f;
-#pragma unroll 1
-        for (int r = 0; r < S; ++r) top = fmaxf(top, slot_m[r][h]);
-#pragma unroll 4
-        for (int r = 0; r < S; ++r) {
-            const float w = slot_m[r][h] == -INFINITY ? 0.f : exp2f(slot_m[r][h] - top);
-            l_all += w * slot_l[r][h], o_all += w * slot_o[r * per + j];
+        float mr[8], lr[8], orr[8], top = -INFINITY, l_all = 0.f, o_all = 0.f;
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+            if (r < S) mr[r] = slot_m[r][h], lr[r] = slot_l[r][h], orr[r] = slot_o[r * per + j];
+            else mr[r] = -INFINITY, lr[r] = orr[r] = 0.f;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) top = fmaxf(top, mr[r]);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const float w = mr[r] == -INFINITY ? 0.f : exp2f(mr[r] - top);
+            l_all += w * lr[r], o_all += w * orr[r];
         }
         p.out[((size_t)b * p.heads + hk * GQ) * kAttnD + i] = __float2bfloat16_rn(o_all / l_all);
     }

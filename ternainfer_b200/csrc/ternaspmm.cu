@@ -823,15 +823,16 @@ static cudaError_t launch_attn_decode(const AttnParams& p, int batch, cudaStream
     cfg.gridDim = dim3(S, p.kv_heads, batch);
     cfg.blockDim = dim3(kAttnWarps * 32, 1, 1);
     cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
+    cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = S;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    // Not a programmatic dependent of the linear before it: launched early, its CTAs take the places that are left beside that
+    // linear's, unevenly and some of them late (30-layer model, per layer: 7.6 us instead of 5.8 at batch 1 and 600 tokens,
+    // 16.1 instead of 10.5 at batch 8 and 1100).  The kernel after it is one of this kernel's.
     cfg.attrs = attr;
-    cfg.numAttrs = tuning().pdl ? 2 : 1;
+    cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
@@ -897,6 +898,7 @@ extern "C" int ternaspmm_attn_prefill(__nv_bfloat16* qkv, __nv_bfloat16* k_cache
     cfg.gridDim = dim3((tokens + 15) / 16, heads / 4, batch);
     cfg.blockDim = dim3(128, 1, 1);
     cfg.dynamicSmemBytes = 4 * kPfTile;
+    cfg.numAttrs = 0;   // (launched early its CTAs spread unevenly: one prompt of 1024 tokens 57 us instead of 47)
     if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, attn_prefill_kernel, p);
     if (e != cudaSuccess) t_host_status = ST_LAUNCH;
     checkLastCudaError(__LINE__);
