@@ -93,6 +93,27 @@ __host__ __device__ inline int act_row_threads(int K) {
     return t < 64 ? 64 : (t > kActMaxThreads ? kActMaxThreads : t);
 }
 
+// scale of a row whose largest magnitude has the bf16 pattern `top`: 127 / amax as reciprocal * 127, in bf16
+__device__ __forceinline__ float act_scale(uint32_t top_bits) {
+    const float top = __uint_as_float(top_bits << 16);
+    const float amax = bf16_round_f(top < 1e-5f ? 1e-5f : top);
+    return bf16_round_f(bf16_round_f(1.0f / amax) * 127.0f);
+}
+// eight bf16 values times the scale (in both halves of s2), to int8
+__device__ __forceinline__ uint2 act_quant8(const uint4& a, uint32_t s2) {
+    const uint32_t av[4] = {a.x, a.y, a.z, a.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        uint32_t pr = act_mul2(av[i], s2);
+        asm("min.bf16x2 %0, %1, %2;" : "=r"(pr) : "r"(pr), "r"(0x42FE42FEu));   // 127: only +128 can lie outside of int8
+        // adding 1.5 * 2^23 leaves the value rounded half to even in the low bits
+        const uint32_t lo = __float_as_uint(__fadd_rn(act_lo(pr), 12582912.f)), hi = __float_as_uint(__fadd_rn(act_hi(pr), 12582912.f));
+        o[i] = __byte_perm(lo, hi, 0x0040);
+    }
+    return make_uint2(__byte_perm(o[0], o[1], 0x5410), __byte_perm(o[2], o[3], 0x5410));
+}
+
 template <bool GATED, int MODE, typename Store>
 __device__ __forceinline__ float act_row_finish(uint32_t row, uint32_t wrow, float eps, int K, int T, float* part, uint32_t* mxp,
                                                 float* ss_out, Store store) {
@@ -165,32 +186,20 @@ __device__ __forceinline__ float act_row_finish(uint32_t row, uint32_t wrow, flo
     }
     if (MODE == ACT_NORM_ONLY) return 0.f;
     __syncthreads();
-    const float top = __uint_as_float(warp_max_u32(lane < vwarps ? mxp[lane] : 0u) << 16);
-    const float amax = bf16_round_f(top < 1e-5f ? 1e-5f : top);
-    const float s = bf16_round_f(bf16_round_f(1.0f / amax) * 127.0f);   // 127 / amax as reciprocal * 127, in bf16
+    const float s = act_scale(warp_max_u32(lane < vwarps ? mxp[lane] : 0u));
     const uint32_t s2 = (__float_as_uint(s) >> 16) * 0x10001u;
 #pragma unroll 1
     for (int vt = tid; vt * 8 < K; vt += nthreads) {
-        const uint4 a = lds128(row + vt * 16);
-        const uint32_t av[4] = {a.x, a.y, a.z, a.w};
-        uint32_t o[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            uint32_t pr = act_mul2(av[i], s2);
-            asm("min.bf16x2 %0, %1, %2;" : "=r"(pr) : "r"(pr), "r"(0x42FE42FEu));   // 127: only +128 can lie outside of int8
-            // adding 1.5 * 2^23 leaves the value rounded half to even in the low bits
-            const uint32_t lo = __float_as_uint(__fadd_rn(act_lo(pr), 12582912.f)), hi = __float_as_uint(__fadd_rn(act_hi(pr), 12582912.f));
-            o[i] = __byte_perm(lo, hi, 0x0040);
-        }
-        store(vt * 8, make_uint4(__byte_perm(o[0], o[1], 0x5410), __byte_perm(o[2], o[3], 0x5410), 0u, 0u));
+        const uint2 v = act_quant8(lds128(row + vt * 16), s2);
+        store(vt * 8, make_uint4(v.x, v.y, 0u, 0u));
     }
     return s;
 }
 
-// Rows of at most 8192 elements: one CTA per row, T threads for few rows (a chain of latencies), T / 4 for many (more rows
-// in flight per SM: 1226 gated rows of 6912 17.3 -> 11.5 us).  Dynamic shared memory: the row (gated:
-// both halves) and the norm weight.  x: [M][ld] bf16 (GATED: the row holds [x1 (K) | x3 (K)], ld = 2K), w: [K] bf16 norm
-// weight, q: [M][K] int8, s_out: [M] bf16, ss_out: [M] fp32 (MODE 1).
+// Rows of at most 8192 elements: one CTA per row, T threads for few rows (a chain of latencies), T / 4 for many gated rows
+// (more rows in flight per SM: 1226 rows of 6912 17.3 -> 11.5 us; held in registers, as below, 11.4 us alone and 13.0 us between
+// the linears of a prompt).  Dynamic shared memory: the row (gated: both halves) and the norm weight.  x: [M][ld] bf16 (GATED: the
+// row holds [x1 (K) | x3 (K)], ld = 2K), w: [K] bf16 norm weight, q: [M][K] int8, s_out: [M] bf16, ss_out: [M] fp32 (MODE 1).
 template <bool GATED, int MODE>
 __global__ void __launch_bounds__(kActMaxThreads) norm_quant_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                                                                         float eps, int K, int8_t* __restrict__ q,
@@ -212,6 +221,87 @@ __global__ void __launch_bounds__(kActMaxThreads) norm_quant_row_kernel(const __
         else *reinterpret_cast<uint2*>(q + (size_t)t * K + k0) = make_uint2(v.x, v.y);
     });
     if (MODE != ACT_NORM_ONLY && tid == 0) s_out[t] = __float2bfloat16_rn(s);
+}
+
+// The same rows ungated, many of them (two per SM and more): what bounds them is no longer the chain but the instructions, so a
+// CTA of T / 4 threads keeps its row in registers, four vectors per thread, the butterflies of the four virtual warps side by
+// side and one maximum per warp.  Measured between the linears of a prompt, 1226 rows of 2560: 7.8 us through shared
+// memory, 5.2 here (9.4 MB: 1.4 us at the copy rate; what is left is the row's chain, one wave of CTAs long).
+template <int MODE>
+__global__ void __launch_bounds__(kActMaxThreads / 4, 3) norm_quant_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                                                                             float eps, int K, int8_t* __restrict__ q,
+                                                                             __nv_bfloat16* __restrict__ s_out, float* __restrict__ ss_out) {
+    constexpr int V = 4;
+    __shared__ __align__(16) float part[kActMaxThreads / 32];
+    __shared__ uint32_t mxp[kActMaxThreads / V / 32];
+    griddep_launch_dependents();
+    const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, n = blockDim.x;
+    const int vwarps = act_row_threads(K) >> 5;
+    uint4 a[V], wv[V];
+    griddep_wait();                                    // the activations come from the previous kernel
+    const __nv_bfloat16* xr = x + (size_t)t * K;
+#pragma unroll
+    for (int j = 0; j < V; ++j) a[j] = (tid + j * n) * 8 < K ? ld_cg_128(xr + (tid + j * n) * 8) : make_uint4(0, 0, 0, 0);
+    float rstd = 1.f;
+    if (MODE != ACT_PLAIN) {
+        float ss[V];
+#pragma unroll
+        for (int j = 0; j < V; ++j) {
+            const uint32_t av[4] = {a[j].x, a[j].y, a[j].z, a[j].w};
+            ss[j] = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float lo = act_lo(av[i]), hi = act_hi(av[i]);
+                ss[j] = __fadd_rn(ss[j], __fmul_rn(lo, lo));
+                ss[j] = __fadd_rn(ss[j], __fmul_rn(hi, hi));
+            }
+        }
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1)
+#pragma unroll
+            for (int j = 0; j < V; ++j) ss[j] += __shfl_xor_sync(0xffffffffu, ss[j], d);
+#pragma unroll
+        for (int j = 0; j < V; ++j)
+            if (lane == j) part[(tid + j * n) >> 5] = ss[j];   // (at most 32 virtual warps: V * n <= 1024)
+#pragma unroll
+        for (int j = 0; j < V; ++j)                    // (asked for this late to spare registers)
+            if ((tid + j * n) * 8 < K) wv[j] = *reinterpret_cast<const uint4*>(w + (tid + j * n) * 8);
+        __syncthreads();
+        float sum = part[0];
+#pragma unroll 4
+        for (int i = 1; i < vwarps; ++i) sum += part[i];
+        if (MODE == ACT_SCALE_SUMSQ && tid == 0) ss_out[t] = sum;
+        if (MODE != ACT_SCALE_SUMSQ) rstd = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)K), eps)));
+    }
+    uint32_t mx = 0;
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+        if ((tid + j * n) * 8 >= K) continue;
+        uint32_t* av = reinterpret_cast<uint32_t*>(&a[j]);
+        if (MODE != ACT_PLAIN) {
+            const uint32_t wj[4] = {wv[j].x, wv[j].y, wv[j].z, wv[j].w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float lo = MODE == ACT_SCALE_SUMSQ ? act_lo(av[i]) : __fmul_rn(act_lo(av[i]), rstd);
+                const float hi = MODE == ACT_SCALE_SUMSQ ? act_hi(av[i]) : __fmul_rn(act_hi(av[i]), rstd);
+                av[i] = act_pack(__fmul_rn(lo, act_lo(wj[i])), __fmul_rn(hi, act_hi(wj[i])));
+            }
+            if (MODE == ACT_NORM_ONLY) *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(q) + (size_t)t * K + (tid + j * n) * 8) = a[j];
+        }
+        // magnitudes: their bit patterns order like the values, NaN above all
+#pragma unroll
+        for (int i = 0; i < 4; ++i) asm("max.u16x2 %0, %0, %1;" : "+r"(mx) : "r"(av[i] & 0x7FFF7FFFu));
+    }
+    if (MODE == ACT_NORM_ONLY) return;
+    mx = warp_max_u32(max(mx & 0xFFFFu, mx >> 16));
+    if (lane == 0) mxp[tid >> 5] = mx;
+    __syncthreads();
+    const float s = act_scale(warp_max_u32(lane < (n >> 5) ? mxp[lane] : 0u));
+    const uint32_t s2 = (__float_as_uint(s) >> 16) * 0x10001u;
+#pragma unroll
+    for (int j = 0; j < V; ++j)
+        if ((tid + j * n) * 8 < K) *reinterpret_cast<uint2*>(q + (size_t)t * K + (tid + j * n) * 8) = act_quant8(a[j], s2);
+    if (tid == 0) s_out[t] = __float2bfloat16_rn(s);
 }
 
 // ---- elementwise kernels of the unfused glue: each replaces a chain of torch operators by one launch with the same

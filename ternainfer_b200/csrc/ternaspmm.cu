@@ -925,8 +925,12 @@ static void run_norm_quant(bool gated, int mode, __nv_bfloat16* x, __nv_bfloat16
                                     norm_quant_row_kernel<false, ACT_PLAIN>, norm_quant_row_kernel<false, ACT_NORM_ONLY>, nullptr};
     static const Kern long_row[5] = {norm_quant_kernel<false, ACT_RMSNORM>, norm_quant_kernel<false, ACT_SCALE_SUMSQ>,
                                     norm_quant_kernel<false, ACT_PLAIN>, norm_quant_kernel<false, ACT_NORM_ONLY>, nullptr};
+    static const Kern many_rows[5] = {norm_quant_rows_kernel<ACT_RMSNORM>, norm_quant_rows_kernel<ACT_SCALE_SUMSQ>,
+                                      norm_quant_rows_kernel<ACT_PLAIN>, norm_quant_rows_kernel<ACT_NORM_ONLY>, nullptr};
     const bool short_row = K <= 8 * kActMaxThreads;   // one eight-element vector per thread
-    Kern kern = short_row ? by_row[mode] : long_row[mode];
+    // two rows per SM and more: fewer threads per row (below that a row's own chain of latencies is longer with them)
+    const bool many = short_row && M >= 2 * device_sm_count(), in_regs = many && !gated;
+    Kern kern = in_regs ? many_rows[mode] : short_row ? by_row[mode] : long_row[mode];
     if (gated) {
         if (mode == ACT_RMSNORM) kern = short_row ? norm_quant_row_kernel<true, ACT_RMSNORM> : norm_quant_kernel<true, ACT_RMSNORM>;
         else kern = short_row ? norm_quant_row_kernel<true, ACT_SCALE_SUMSQ> : norm_quant_kernel<true, ACT_SCALE_SUMSQ>;
@@ -936,16 +940,15 @@ static void run_norm_quant(bool gated, int mode, __nv_bfloat16* x, __nv_bfloat16
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) dev = 0;
     const int slot = (gated ? 4 : 0) + mode;
-    if (!attr_done[short_row][dev][slot]) {
+    if (!in_regs && !attr_done[short_row][dev][slot]) {
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 56 * 1024);
         attr_done[short_row][dev][slot] = true;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(M, 1, 1);
-    // one vector per thread; for more rows than two per SM a quarter of the threads, four vectors each
-    const int T = act_row_threads(K);
-    cfg.blockDim = dim3(short_row && M >= 2 * device_sm_count() ? std::max(64, (T / 4 + 31) / 32 * 32) : T, 1, 1);
-    cfg.dynamicSmemBytes = short_row ? (size_t)K * (gated ? 6 : (mode == ACT_PLAIN ? 2 : 4)) : (size_t)K * 2;
+    const int T = act_row_threads(K);   // one vector per thread; for many rows four
+    cfg.blockDim = dim3(many ? std::max(64, (T / 4 + 31) / 32 * 32) : T, 1, 1);
+    cfg.dynamicSmemBytes = in_regs ? 0 : short_row ? (size_t)K * (gated ? 6 : (mode == ACT_PLAIN ? 2 : 4)) : (size_t)K * 2;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -116,3 +116,26 @@ def test_layer_follows_its_weights(lib):
         z = layer(x)
     graph.replay()
     assert torch.equal(z, -y) and torch.equal(layer(x), -y)
+
+
+@pytest.mark.parametrize("K", [64, 1040, 2560, 8192])
+def test_norms_of_many_rows_are_the_norms_of_each(lib, K):
+    """From two rows per SM on, a kernel that keeps a row in registers takes over: the same bits as a few rows at a time."""
+    from ternainfer_b200.linear import rmsnorm
+    M = 2 * torch.cuda.get_device_properties(0).multi_processor_count + 3
+    g = torch.Generator(device="cuda").manual_seed(K)
+    x = (torch.randn((M, K), generator=g, device="cuda") * torch.logspace(-3, 3, M, device="cuda")[:, None]).to(torch.bfloat16)
+    x[7, K // 2], x[9] = float("nan"), 0.0
+    w = (1 + 0.1 * torch.randn(K, generator=g, device="cuda")).to(torch.bfloat16)
+
+    def bits(ts):
+        return [t.view(torch.int16) if t.dtype == torch.bfloat16 else t for t in ts]
+
+    for f in (lambda v: rmsnorm_quant(v, w, 1e-5), quant_input, lambda v: (rmsnorm(v, w, 1e-5),)):
+        parts = [bits(f(x[i:i + 50])) for i in range(0, M, 50)]
+        for k, got in enumerate(bits(f(x))):
+            want = torch.cat([p[k] for p in parts])
+            keep = torch.ones(M, dtype=torch.bool, device="cuda")
+            keep[7] = False                                   # (a NaN's payload and its int8 values are not part of the contract)
+            assert torch.equal(got[keep], want[keep])
+    assert torch.isnan(rmsnorm_quant(x, w, 1e-5)[1].reshape(-1)[7]) and torch.isnan(quant_input(x)[1].reshape(-1)[7])
