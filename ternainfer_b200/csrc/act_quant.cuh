@@ -350,18 +350,26 @@ __global__ void __launch_bounds__(256) relu2_gate_kernel(const __nv_bfloat16* __
     *reinterpret_cast<uint4*>(out + i * 8) = make_uint4(o[0], o[1], o[2], o[3]);
 }
 
-// bf16 -> fp32, eight values per thread.
+// bf16 -> fp32.  Four values per lane and access, so that a warp's store covers whole lines (eight per lane: half a sector at a
+// time), four accesses in flight, from the end: the last values of what the kernel before wrote are still in L2.
+// 1226 x 128256 logits: 200 -> 160 us (144 at the copy rate).
 __global__ void __launch_bounds__(256) bf16_to_f32_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ y, long long n) {
+    constexpr int U = 4;
     griddep_launch_dependents();
     griddep_wait();
-    const long long n8 = n >> 3, stride = (long long)gridDim.x * 256;
-    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n8; i += stride) {
-        const uint4 v = ld_cg_128(x + i * 8);
-        float4* o = reinterpret_cast<float4*>(y + i * 8);
-        __stcs(o, make_float4(act_lo(v.x), act_hi(v.x), act_lo(v.y), act_hi(v.y)));
-        __stcs(o + 1, make_float4(act_lo(v.z), act_hi(v.z), act_lo(v.w), act_hi(v.w)));
+    const long long n4 = n >> 2, chunks = (n4 + U * 256 - 1) / (U * 256);
+    for (long long c = chunks - 1 - blockIdx.x; c >= 0; c -= gridDim.x) {
+        const long long i0 = c * (U * 256) + threadIdx.x;
+        uint2 v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (i0 + u * 256 < n4) v[u] = __ldcg(reinterpret_cast<const uint2*>(x) + i0 + u * 256);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (i0 + u * 256 < n4)
+                __stcs(reinterpret_cast<float4*>(y) + i0 + u * 256, make_float4(act_lo(v[u].x), act_hi(v[u].x), act_lo(v[u].y), act_hi(v[u].y)));
     }
-    const long long rest = n8 * 8 + (long long)blockIdx.x * 256 + threadIdx.x;
+    const long long rest = n4 * 4 + threadIdx.x;
     if (blockIdx.x == 0 && rest < n) y[rest] = __bfloat162float(x[rest]);
 }
 

@@ -876,7 +876,8 @@ extern "C" int ternaspmm_attn_prefill(__nv_bfloat16* qkv, __nv_bfloat16* k_cache
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) dev = 0;
     if (!attr_done[dev]) {
-        if (cudaFuncSetAttribute(attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * kPfTile) != cudaSuccess) {
+        if (cudaFuncSetAttribute(attn_prefill_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * kPfTile) != cudaSuccess ||
+            cudaFuncSetAttribute(attn_prefill_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * kPfTile) != cudaSuccess) {
             t_host_status = ST_LAUNCH;
             return t_host_status;
         }
@@ -895,11 +896,20 @@ extern "C" int ternaspmm_attn_prefill(__nv_bfloat16* qkv, __nv_bfloat16* k_cache
     cfg.gridDim = dim3((unsigned)((items + 255) / 256), 1, 1);
     cfg.blockDim = dim3(256, 1, 1);
     cudaError_t e = cudaLaunchKernelEx(&cfg, rope_append_kernel, p, items);
-    cfg.gridDim = dim3((tokens + 15) / 16, heads / 4, batch);
+    const int heads_x_batch = heads / 4 * batch, items_a = (tokens + 15) / 16 * heads_x_batch, key_tiles = (tokens + 63) / 64;
+    // Two CTAs per item where the chain of the longest rows outlasts an SM's share of the work: few items, the more the longer they
+    // are (one prompt of 1024 tokens, 320 items: 30 us instead of 37; of 2048, 640 items: 82 instead of 76; two of 613, 390
+    // items of up to 10 tiles: 30 instead of 27; four of 100, 140 items of two tiles: 10.3 instead of 9.3)
+    const bool split = key_tiles >= 3 && items_a <= device_sm_count() + 12 * key_tiles;
+    cfg.gridDim = dim3(split ? 2 * items_a : items_a, 1, 1);
     cfg.blockDim = dim3(128, 1, 1);
     cfg.dynamicSmemBytes = 4 * kPfTile;
-    cfg.numAttrs = 0;   // (launched early its CTAs spread unevenly: one prompt of 1024 tokens 57 us instead of 47)
-    if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, attn_prefill_kernel, p);
+    // (not a programmatic dependent: launched early its CTAs spread unevenly, one prompt of 1024 tokens 57 us instead of 47)
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.numAttrs = split ? 1 : 0;
+    if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, split ? attn_prefill_kernel<2> : attn_prefill_kernel<1>, p, heads_x_batch);
     if (e != cudaSuccess) t_host_status = ST_LAUNCH;
     checkLastCudaError(__LINE__);
     return t_host_status;
@@ -1038,7 +1048,7 @@ extern "C" void ternaspmm_bf16_to_f32(__nv_bfloat16* x, float* y, long long n, c
         return;
     }
     cudaLaunchAttribute attr;
-    cudaLaunchConfig_t cfg = elementwise_launch(std::min<long long>((n + 7) / 8, 256ll * 16 * device_sm_count()), stream, &attr);
+    cudaLaunchConfig_t cfg = elementwise_launch(std::min<long long>((n + 15) / 16, 256ll * 8 * device_sm_count()), stream, &attr);
     if (cudaLaunchKernelEx(&cfg, bf16_to_f32_kernel, (const __nv_bfloat16*)x, y, n) != cudaSuccess) t_host_status = ST_LAUNCH;
     checkLastCudaError(__LINE__);
 }

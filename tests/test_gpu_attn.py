@@ -37,7 +37,7 @@ def test_decode_attention(lib, B, pos, L, H, Hkv):
 
 @pytest.mark.parametrize("H,Hkv", [(20, 5), (64, 8)])
 @pytest.mark.parametrize("B,T,past,L", [(1, 2, 0, 8), (2, 16, 0, 16), (1, 17, 0, 64), (3, 64, 0, 64), (1, 65, 1, 80), (2, 200, 63, 300), (1, 613, 0, 613),
-                                        (1, 40, 1000, 1040)])
+                                        (1, 40, 1000, 1040), (1, 129, 0, 200), (2, 500, 37, 640)])
 def test_prompt_attention(lib, B, T, past, L, H, Hkv):
     D = 128
     g = torch.Generator(device="cuda").manual_seed(T + past)
