@@ -65,21 +65,11 @@ def _pack_tiles(t: np.ndarray):
 
 def _compress_weight_cuda(weight: torch.Tensor):
     """Same packing by the library's kernels on the GPU (one wait, for the size of the sign stream)."""
-    from ..lib import load_library
-    lib, dev = load_library(), weight.device
-    N, K = weight.shape
-    tiles = N * K // 4096
-    bitmap = torch.empty(N * K // 64, dtype=torch.uint64, device=dev)
-    tile_off = torch.empty(tiles + 1, dtype=torch.int32, device=dev)
-    quarters = torch.empty(3 * tiles, dtype=torch.uint16, device=dev)
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream().cuda_stream
-        words = lib.ternaspmm_pack_gpu_layout(weight.data_ptr(), N, K, bitmap.data_ptr(), tile_off.data_ptr(), quarters.data_ptr(), stream)
-        if words < 0:
-            raise RuntimeError(f"packing a {N} x {K} weight on the GPU failed with status {lib.ternaspmm_last_status()}")
-        signs = torch.empty(words + _PAD_WORDS, dtype=torch.uint32, device=dev)
-        lib.ternaspmm_pack_gpu_signs(weight.data_ptr(), N, K, tile_off.data_ptr(), signs.data_ptr(), stream)
-    return signs, tile_off, quarters, bitmap
+    from ..lib import load_host_call
+    packed = load_host_call().pack(weight)
+    if packed is None:
+        raise RuntimeError(f"a {tuple(weight.shape)} weight cannot be packed on the GPU")
+    return packed
 
 
 def compress_weight(weight: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:

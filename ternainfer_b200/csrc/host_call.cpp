@@ -253,6 +253,35 @@ void layer_dealloc(PyObject* o) {
     Py_TYPE(o)->tp_free(o);
 }
 
+// pack(weight): the four packed tensors of a contiguous, 16-byte aligned int8 CUDA tensor [N][K] whose sizes are multiples of 64.
+PyObject* pack_weight(PyObject*, PyObject* o) {
+    HANDLE_TH_ERRORS
+    if (!THPVariable_Check(o)) Py_RETURN_NONE;
+    const at::Tensor& w = THPVariable_Unpack(o);
+    if (!w.is_cuda() || w.scalar_type() != at::kChar || w.dim() != 2 || !w.is_contiguous() || w.size(0) % 64 || w.size(1) % 64 || !w.numel() ||
+        w.size(0) > INT_MAX || w.size(1) > INT_MAX || (reinterpret_cast<uintptr_t>(w.data_ptr()) & 15))
+        Py_RETURN_NONE;
+    const int64_t N = w.size(0), K = w.size(1), tiles = N / 64 * (K / 64);
+    c10::cuda::CUDAGuard guard(w.device());
+    cudaStream_t stream = c10::cuda::getCurrentCUDAStream();
+    at::Tensor bitmap = at::empty({tiles * 64}, w.options().dtype(at::kUInt64)), tile_off = at::empty({tiles + 1}, w.options().dtype(at::kInt));
+    at::Tensor quarters = at::empty({tiles * 3}, w.options().dtype(at::kUInt16));
+    const auto* src = static_cast<const int8_t*>(w.data_ptr());
+    auto* offsets = static_cast<int*>(tile_off.data_ptr());
+    long long words;
+    Py_BEGIN_ALLOW_THREADS
+    words = ternaspmm_pack_gpu_layout(src, (int)N, (int)K, static_cast<uint64_t*>(bitmap.data_ptr()), offsets,
+                                      static_cast<uint16_t*>(quarters.data_ptr()), stream);
+    Py_END_ALLOW_THREADS
+    TORCH_CHECK(words >= 0, "packing a ", N, " x ", K, " weight on the GPU failed with status ", ternaspmm_last_status());
+    at::Tensor signs = at::empty({words + 4}, w.options().dtype(at::kUInt32));   // four zero words behind the last tile's
+    ternaspmm_pack_gpu_signs(src, (int)N, (int)K, offsets, static_cast<uint32_t*>(signs.data_ptr()), stream);
+    return Py_BuildValue("NNNN", THPVariable_Wrap(signs), THPVariable_Wrap(tile_off), THPVariable_Wrap(quarters), THPVariable_Wrap(bitmap));
+    END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef module_methods[] = {{"pack", pack_weight, METH_O, nullptr}, {nullptr, nullptr, 0, nullptr}};
+
 PyMethodDef layer_methods[] = {
     {"forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(layer_forward)), METH_FASTCALL, nullptr},
     {"forward_normed", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(layer_forward_normed)), METH_FASTCALL, nullptr},
@@ -264,7 +293,7 @@ PyMethodDef layer_methods[] = {
 
 PyTypeObject layer_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
-PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host_call", "Native call site of the ternary linears.", -1, nullptr};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host_call", "Native call sites: the ternary linears and the packer.", -1, module_methods};
 
 }  // namespace
 

@@ -1149,20 +1149,27 @@ extern "C" long long ternaspmm_pack_gpu_layout(const int8_t* W, int N, int K, ui
         t_host_status = ST_LAUNCH;
         return -1;
     }
+    volatile long long* const result = total;
+    *result = -1;
     const long long tiles = (long long)(N / 64) * (K / 64);
     const unsigned blocks = (unsigned)((tiles + kPackWarps - 1) / kPackWarps);
     pack_bitmap_kernel<<<blocks, kPackWarps * 32, 0, stream>>>(W, N, K, reinterpret_cast<uint4*>(bitmap), tile_offsets, quarter_offsets);
     pack_scan_kernel<<<1, 1024, 0, stream>>>(tile_offsets, tiles, total);
-    if (cudaStreamSynchronize(stream) != cudaSuccess) {
-        t_host_status = ST_LAUNCH;
-        checkLastCudaError(__LINE__);
-        return -1;
+    // The number is here a few microseconds before the stream is idle; the stream is asked now and then whether it still runs.
+    for (int i = 1; *result < 0; ++i) {
+        if (i & 4095) continue;
+        const cudaError_t e = cudaStreamQuery(stream);
+        if (e != cudaErrorNotReady && (e != cudaSuccess || *result < 0)) {
+            t_host_status = ST_LAUNCH;
+            checkLastCudaError(__LINE__);
+            return -1;
+        }
     }
-    if (*total >= (1ll << 31)) {   // offsets are 32-bit
+    if (*result >= (1ll << 31)) {   // offsets are 32-bit
         t_host_status = ST_BAD_SHAPE;
         return -1;
     }
-    return *total / 32;
+    return *result / 32;
 }
 
 extern "C" void ternaspmm_pack_gpu_signs(const int8_t* W, int N, int K, const int* tile_offsets, uint32_t* sign_words, cudaStream_t stream) {
