@@ -50,7 +50,14 @@ __device__ __forceinline__ void mma_bf16_full(float (&d)[4], uint32_t a0, uint32
 __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); }
 __device__ __forceinline__ uint32_t bf16_pack(float lo, float hi) {
-    return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(lo)) | ((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(hi)) << 16);
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+__device__ __forceinline__ float ex2_approx(float v) {                 // (weights below 2^-126 are zero)
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
 }
 // (x, y) rotated by the angle whose cosine and sine are c, s
 __device__ __forceinline__ uint32_t rope_pair(uint32_t xy, float c, float s) {
@@ -164,10 +171,10 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 3) attn_decode_kernel(const A
         }
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-        const float r = exp2f(m - mx);                        // (a group holds at least one key: mx is finite)
+        const float r = ex2_approx(m - mx);                        // (a group holds at least one key: mx is finite)
         m = mx, l *= r;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) pr[i] = exp2f(pr[i] - mx), l += pr[i];
+        for (int i = 0; i < 4; ++i) pr[i] = ex2_approx(pr[i] - mx), l += pr[i];
         const uint32_t b0 = bf16_pack(pr[0], pr[1]), b1 = bf16_pack(pr[2], pr[3]);   // as they are: keys x head g
         const float r0 = __shfl_sync(0xffffffffu, r, 8 * q), r1 = __shfl_sync(0xffffffffu, r, 8 * q + 4);
         if (gi * 16 + 16 > pos) {                             // rows that are not keys may hold anything: 0 * NaN
@@ -234,7 +241,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 3) attn_decode_kernel(const A
         for (int k = 0; k < kParts; ++k) top = fmaxf(top, mk[k]);
 #pragma unroll
         for (int k = 0; k < kParts; ++k) {
-            const float w = mk[k] == -INFINITY ? 0.f : exp2f(mk[k] - top);
+            const float w = mk[k] == -INFINITY ? 0.f : ex2_approx(mk[k] - top);
             sum += w * lk[k];
             o.x += w * ok[k].x, o.y += w * ok[k].y, o.z += w * ok[k].z, o.w += w * ok[k].w;
         }
@@ -261,7 +268,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 3) attn_decode_kernel(const A
         for (int r = 0; r < 8; ++r) top = fmaxf(top, mr[r]);
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
-            const float w = mr[r] == -INFINITY ? 0.f : exp2f(mr[r] - top);
+            const float w = mr[r] == -INFINITY ? 0.f : ex2_approx(mr[r] - top);
             l_all += w * lr[r], o_all += w * orr[r];
         }
         p.out[((size_t)b * p.heads + hk * GQ) * kAttnD + i] = __float2bfloat16_rn(o_all / l_all);

@@ -61,12 +61,6 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
 
-__device__ __forceinline__ float ex2_approx(float v) {             // (probabilities below 2^-126 are zero)
-    float r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
-    return r;
-}
-
 // grid: items (16 positions of four query heads of a sequence), longest first, times S.  S = 2: the CTAs of a cluster take every
 // other tile of keys, and each finishes two of the four heads.
 template <int S>
@@ -188,8 +182,8 @@ __global__ void __launch_bounds__(128, 3) attn_prefill_kernel(const AttnPrefillP
         for (int j = 0; j < 8; ++j) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) s[j][e] = ex2_approx(s[j][e] * p.scale_log2 - ms[e >> 1]), l[e >> 1] += s[j][e];
-            pa[j >> 1][2 * (j & 1)] = act_pack(s[j][0], s[j][1]);
-            pa[j >> 1][2 * (j & 1) + 1] = act_pack(s[j][2], s[j][3]);
+            pa[j >> 1][2 * (j & 1)] = bf16_pack(s[j][0], s[j][1]);
+            pa[j >> 1][2 * (j & 1) + 1] = bf16_pack(s[j][2], s[j][3]);
         }
         // ---- values: 16 rows x 128 dimensions
 #pragma unroll
