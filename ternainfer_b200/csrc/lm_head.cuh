@@ -7,10 +7,10 @@
 // separate `torch.argmax` of the generation loop (generate.py:283, :305).
 //
 // HBM-bound: the embedding is read exactly once.  Persistent CTAs, one per SM,
-// each owning a contiguous range of 16-row groups of the embedding; the warps of
+// each owning a contiguous range of groups of R rows of the embedding; the warps of
 // a CTA take groups from that range through a shared-memory counter.  A warp
-// streams its 16 rows with one 128-bit load per lane and row (lane (g, q) reads 8
-// consecutive k of rows g and g+8; k is only a summation index, so the tensor-core
+// streams its R rows with one 128-bit load per lane and row (lane (g, q) reads 8
+// consecutive k of rows g and g+8 (R = 16); k is only a summation index, so the tensor-core
 // fragments are filled straight from those registers with the hidden states
 // permuted the same way), multiplies with mma.sync m16n8k16 bf16 (tokens are the
 // MMA's N = 8) and accumulates in fp32.  The hidden states [8][K] sit in shared
@@ -32,7 +32,15 @@ namespace tsp {
 
 constexpr int kHeadWarps = 16;
 constexpr int kHeadMaxCtas = 1024;              // scratch holds this many candidate slots
-constexpr int kHeadUnroll = 8;                  // k-steps of 32 in flight per warp (16 x 128-bit loads per lane)
+constexpr int kHeadPrefetch = 1024;             // bytes of a row fetched into L2 ahead
+
+// Rows of a group: 8, whose finer steps leave a shorter tail (K = 2560: 128256 rows 108 -> 102 us, of 100 at the copy rate; 8000 rows
+// 17.8 -> 15.8), but 16 where every warp then has one group of 16 and would have one or two of 8 (32000 rows 33.4 -> 31,
+// 20000 23.4 -> 22.4; in groups of 8 33.6 and 27).  The sums of a row are the same either way.
+inline int head_rows(int V, int ctas) {
+    const int per_cta = ((V + 7) / 8 + ctas - 1) / ctas;
+    return per_cta > kHeadWarps && per_cta <= 2 * kHeadWarps ? 16 : 8;
+}
 
 struct HeadCandidate {
     float v;
@@ -72,7 +80,31 @@ __device__ __forceinline__ bool head_better(float v, int i, float bv, int bi) {
     return v > bv || (v == bv && i < bi);
 }
 
+// U k-steps of 32: all loads first
+template <int R, int U>
+__device__ __forceinline__ void head_block(float (&acc)[4], const __nv_bfloat16* e0, const __nv_bfloat16* e1, const uint8_t* hrow) {
+    uint4 a[U], b[R > 8 ? U : 1];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        a[u] = ldg_stream_128(e0 + 32 * u);
+        if (R > 8) b[u] = ldg_stream_128(e1 + 32 * u);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const uint4 x = *reinterpret_cast<const uint4*>(hrow + 64 * u);
+        if constexpr (R > 8) {
+            mma_bf16_16x8x16(acc, a[u].x, b[u].x, a[u].y, b[u].y, x.x, x.y);
+            mma_bf16_16x8x16(acc, a[u].z, b[u].z, a[u].w, b[u].w, x.z, x.w);
+        } else {
+            mma_bf16_16x8x16(acc, a[u].x, 0u, a[u].y, 0u, x.x, x.y);
+            mma_bf16_16x8x16(acc, a[u].z, 0u, a[u].w, 0u, x.z, x.w);
+        }
+    }
+}
+
+template <int R>
 __global__ void __launch_bounds__(kHeadWarps * 32, 1) lm_head_kernel(const HeadParams p) {
+    constexpr int kHeadUnroll = 128 / R;                          // k-steps of 32 in flight per warp (16 x 128-bit loads per lane)
     extern __shared__ __align__(16) uint8_t head_smem[];
     __shared__ int next_group;
     __shared__ HeadCandidate warp_best[kHeadWarps][8];
@@ -81,12 +113,16 @@ __global__ void __launch_bounds__(kHeadWarps * 32, 1) lm_head_kernel(const HeadP
     const int g = lane >> 2, q = lane & 3;
     const int K = p.K, V = p.V;
     const int hs = K * 2 + 64;                                    // bytes per token row in shared memory
-    const int groups = (V + 15) >> 4;
+    const int groups = (V + R - 1) / R;
     const int g0 = (int)(((long long)groups * blockIdx.x) / gridDim.x);
     const int g1 = (int)(((long long)groups * (blockIdx.x + 1)) / gridDim.x);
 
     griddep_launch_dependents();
     if (tid == 0) next_group = g0;
+    // the warps' first groups into L2 while the hidden states arrive (1 to 3 us of these figures)
+    if (lane < R && g0 + warp < g1 && (g0 + warp) * R + lane < V)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(__cvta_generic_to_global(p.emb + (size_t)((g0 + warp) * R + lane) * K)),
+                     "r"(min(K * 2, kHeadPrefetch)) : "memory");
     griddep_wait();                                               // the hidden states come from the previous kernel
     // stage the hidden states (rows beyond M are zero)
     for (int i = tid; i < 8 * (K >> 3); i += blockDim.x) {
@@ -105,35 +141,18 @@ __global__ void __launch_bounds__(kHeadWarps * 32, 1) lm_head_kernel(const HeadP
         if (lane == 0) grp = atomicAdd(&next_group, 1);
         grp = __shfl_sync(0xffffffffu, grp, 0);
         if (grp >= g1) break;
-        const int r0 = grp * 16 + g, r1 = r0 + 8;
-        const bool ok0 = r0 < V, ok1 = r1 < V;
+        const int r0 = grp * R + g, r1 = r0 + 8;                   // (R = 8: no second row)
+        const bool ok0 = r0 < V, ok1 = R > 8 && r1 < V;
         const __nv_bfloat16* e0 = p.emb + (size_t)(ok0 ? r0 : 0) * K + q * 8;
         const __nv_bfloat16* e1 = p.emb + (size_t)(ok1 ? r1 : 0) * K + q * 8;
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
         int k0 = 0;
-        for (; k0 + 32 * kHeadUnroll <= K; k0 += 32 * kHeadUnroll) {
-            uint4 a[kHeadUnroll], b[kHeadUnroll];
-#pragma unroll
-            for (int u = 0; u < kHeadUnroll; ++u) {
-                a[u] = ldg_stream_128(e0 + k0 + 32 * u);
-                b[u] = ldg_stream_128(e1 + k0 + 32 * u);
-            }
-#pragma unroll
-            for (int u = 0; u < kHeadUnroll; ++u) {
-                const uint4 x = *reinterpret_cast<const uint4*>(hrow + (k0 + 32 * u) * 2);
-                mma_bf16_16x8x16(acc, a[u].x, b[u].x, a[u].y, b[u].y, x.x, x.y);
-                mma_bf16_16x8x16(acc, a[u].z, b[u].z, a[u].w, b[u].w, x.z, x.w);
-            }
-        }
-        for (; k0 < K; k0 += 32) {
-            const uint4 a = ldg_stream_128(e0 + k0), b = ldg_stream_128(e1 + k0);
-            const uint4 x = *reinterpret_cast<const uint4*>(hrow + k0 * 2);
-            mma_bf16_16x8x16(acc, a.x, b.x, a.y, b.y, x.x, x.y);
-            mma_bf16_16x8x16(acc, a.z, b.z, a.w, b.w, x.z, x.w);
-        }
+        for (; k0 + 32 * kHeadUnroll <= K; k0 += 32 * kHeadUnroll) head_block<R, kHeadUnroll>(acc, e0 + k0, e1 + k0, hrow + k0 * 2);
+        for (; k0 + 128 <= K; k0 += 128) head_block<R, 4>(acc, e0 + k0, e1 + k0, hrow + k0 * 2);
+        for (; k0 < K; k0 += 32) head_block<R, 1>(acc, e0 + k0, e1 + k0, hrow + k0 * 2);
         // acc[0], acc[1]: row r0, tokens 2q, 2q+1;  acc[2], acc[3]: row r1
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < (R > 8 ? 4 : 2); ++c) {
             const int row = c < 2 ? r0 : r1, tok = 2 * q + (c & 1);
             const bool ok = c < 2 ? ok0 : ok1;
             const float v = p.round_bf16 ? __bfloat162float(__float2bfloat16_rn(acc[c])) : acc[c];

@@ -1372,7 +1372,8 @@ extern "C" void ternaspmm_lm_head_argmax(__nv_bfloat16* h, __nv_bfloat16* embedd
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) dev = 0;
     if (!attr_done[dev]) {
-        if (cudaFuncSetAttribute(lm_head_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * (12288 * 2 + 64)) != cudaSuccess) {
+        if (cudaFuncSetAttribute(lm_head_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * (12288 * 2 + 64)) != cudaSuccess ||
+            cudaFuncSetAttribute(lm_head_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * (12288 * 2 + 64)) != cudaSuccess) {
             t_host_status = ST_LAUNCH;
             return;
         }
@@ -1383,7 +1384,7 @@ extern "C" void ternaspmm_lm_head_argmax(__nv_bfloat16* h, __nv_bfloat16* embedd
     p.counter = reinterpret_cast<unsigned int*>(scratch);
     p.cand = reinterpret_cast<HeadCandidate*>(reinterpret_cast<uint8_t*>(scratch) + 16);
     p.M = M, p.V = V, p.K = K, p.round_bf16 = round_bf16;
-    const int groups = (V + 15) / 16;
+    const int groups = (V + 7) / 8, R = head_rows(V, device_sm_count());
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(std::min(std::min(device_sm_count(), groups), kHeadMaxCtas), 1, 1);
     cfg.blockDim = dim3(kHeadWarps * 32, 1, 1);
@@ -1395,7 +1396,7 @@ extern "C" void ternaspmm_lm_head_argmax(__nv_bfloat16* h, __nv_bfloat16* embedd
     // model, the decoded token took 5 % longer.  In stream order it starts a few microseconds later and
     // runs on an empty chip.
     t_echo = {4, 8, 1, kHeadWarps, 0, (int)cfg.gridDim.x};
-    if (cudaLaunchKernelEx(&cfg, lm_head_kernel, p) != cudaSuccess) t_host_status = ST_LAUNCH;
+    if (cudaLaunchKernelEx(&cfg, R == 8 ? lm_head_kernel<8> : lm_head_kernel<16>, p) != cudaSuccess) t_host_status = ST_LAUNCH;
     checkLastCudaError(__LINE__);
 }
 
@@ -1454,7 +1455,8 @@ extern "C" void ternaspmm_lm_head_argmax_noalloc(__nv_bfloat16* h, __nv_bfloat16
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) dev = 0;
     if (!attr_done[dev]) {
-        if (cudaFuncSetAttribute(lm_head_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * (12288 * 2 + 64)) != cudaSuccess) {
+        if (cudaFuncSetAttribute(lm_head_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * (12288 * 2 + 64)) != cudaSuccess ||
+            cudaFuncSetAttribute(lm_head_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * (12288 * 2 + 64)) != cudaSuccess) {
             t_host_status = ST_LAUNCH;
             return;
         }
@@ -1471,13 +1473,13 @@ extern "C" void ternaspmm_lm_head_argmax_noalloc(__nv_bfloat16* h, __nv_bfloat16
     p.counter = reinterpret_cast<unsigned int*>(scratch);
     p.cand = reinterpret_cast<HeadCandidate*>(reinterpret_cast<uint8_t*>(scratch) + 16);
     p.M = M, p.V = V, p.K = K, p.round_bf16 = round_bf16;
-    const int groups = (V + 15) / 16;
+    const int groups = (V + 7) / 8, R = head_rows(V, device_sm_count());
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(std::min(std::min(device_sm_count(), groups), kHeadStaticCtas), 1, 1);
     cfg.blockDim = dim3(kHeadWarps * 32, 1, 1);
     cfg.dynamicSmemBytes = 8 * (K * 2 + 64);
     cfg.stream = stream;
-    if (cudaLaunchKernelEx(&cfg, lm_head_kernel, p) != cudaSuccess) t_host_status = ST_LAUNCH;
+    if (cudaLaunchKernelEx(&cfg, R == 8 ? lm_head_kernel<8> : lm_head_kernel<16>, p) != cudaSuccess) t_host_status = ST_LAUNCH;
     checkLastCudaError(__LINE__);
 }
 

@@ -117,3 +117,15 @@ def test_python_call_site(lib):
     logits, toks = lm_head_argmax(h.view(8, 1, 2560), emb)
     assert logits.shape == (8, 4096) and toks.shape == (8,)
     assert (toks.cpu().numpy() == np.argmax(logits.cpu().numpy(), axis=1)).all()
+
+
+@pytest.mark.parametrize("edge", [16, 32])
+@pytest.mark.parametrize("more", [0, 1])
+def test_row_groups_of_either_size_give_the_same_bits(lib, edge, more):
+    """At the vocabulary sizes where the kernel goes over to groups of 16 rows and back: as in pieces of 8-row groups."""
+    from ternainfer_b200.linear import lm_head_argmax
+    V = 8 * edge * torch.cuda.get_device_properties(0).multi_processor_count + more
+    h, emb = inputs(5, V, 352, seed=V)
+    logits, toks = lm_head_argmax(h, emb)
+    want = torch.cat([lm_head_argmax(h, emb[i:i + 8000])[0] for i in range(0, V, 8000)], 1)
+    assert torch.equal(logits, want) and torch.equal(toks, want.argmax(1))
