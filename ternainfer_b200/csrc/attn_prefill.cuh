@@ -7,8 +7,9 @@
 // query is rotated on its way into the A fragments.  Tiles arrive by
 // cp.async, double-buffered, in an XOR-swizzled layout that ldmatrix reads without bank conflicts; three CTAs per SM.
 // Probabilities are rounded to bf16 for the second product, everything else accumulates in fp32.
-// What bounds it is instruction issue (three warps per scheduler, each with a tile's softmax beside 128 MMAs, which alone would
-// take half of the time), and for short prompts the chain of the longest rows.  Hence addresses that take one XOR per
+// What bounds it is the chain of each warp at two to three warps per scheduler (tensor pipe 39 % of the active cycles, 58 % on
+// the busiest SM, issue slots 28 %; stalls: fixed latencies, then fragment loads), and for short prompts the chain of the
+// longest rows.  So instructions on that chain count: addresses that take one XOR per
 // fragment, exponentials without range handling, an output that is rescaled only when a maximum has grown by 2^8, CTAs
 // sorted longest first over the whole launch, and two CTAs per item where there are few (ternaspmm_attn_prefill).  Both
 // launches, 20 / 5 heads: 2 prompts of 613 tokens 35.9 -> 27.1 us (flash_attn's kv-cache kernel, which rotates and
