@@ -230,12 +230,6 @@ PyObject* layer_invalidate(PyObject* o, PyObject*) {
     Py_RETURN_NONE;
 }
 
-// copies and pickles carry the sizes; the weights are laid out again where they are used
-PyObject* layer_reduce(PyObject* o, PyObject*) {
-    Layer* self = reinterpret_cast<Layer*>(o);
-    return Py_BuildValue("O(iiiiii)", Py_TYPE(o), self->in_features, self->out_features, self->ws_num, self->seg[0], self->seg[1], self->seg[2]);
-}
-
 PyObject* layer_new(PyTypeObject* type, PyObject* args, PyObject*) {
     Layer* self = reinterpret_cast<Layer*>(type->tp_alloc(type, 0));
     if (!self) return nullptr;
@@ -288,7 +282,6 @@ PyMethodDef layer_methods[] = {
     {"forward_quantized", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(layer_forward_quantized)), METH_FASTCALL, nullptr},
     {"prepare", layer_prepare, METH_O, nullptr},
     {"invalidate", layer_invalidate, METH_NOARGS, nullptr},
-    {"__reduce__", layer_reduce, METH_NOARGS, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 
 PyTypeObject layer_type = {PyVarObject_HEAD_INIT(nullptr, 0)};

@@ -300,12 +300,24 @@ class SpBitLinear(nn.Module):
         self.segments = [int(v) for v in seg] if seg is not None else None
         if self.segments is not None:
             assert sum(self.segments) == out_features and len(self.segments) == self.ws_num
+        self._attach()
+
+    def _attach(self):
+        """The native call site; it keeps the weights in the layout of the small-batch kernel, laid out here once."""
         bounds = [0, 0, 0]
-        if not _builtin_segments(self.segments, out_features, self.ws_num):
+        if not _builtin_segments(self.segments, self.out_features, self.ws_num):
             bounds = [sum(self.segments[:i + 1]) for i in range(len(self.segments) - 1)] + [2 ** 31 - 1] * 3
-        # native call site; it keeps the weights in the layout of the small-batch kernel, laid out here once
-        self._native = load_host_call().Layer(in_features, out_features, self.ws_num, *bounds[:3])
+        self._native = load_host_call().Layer(self.in_features, self.out_features, self.ws_num, *bounds[:3])
         self._native.prepare(self._parameters)
+
+    def __getstate__(self):      # copies and pickles carry what checkpoints carry; the call site is made again from it
+        state = self.__dict__.copy()
+        state.pop("_native", None)
+        return state
+
+    def __setstate__(self, state):
+        super().__setstate__(state)
+        self._attach()
 
     quant_input = staticmethod(quant_input)
 
