@@ -5,12 +5,15 @@
 // arguments, the quantiser as eight torch operators - its host side took 18 us
 // (int8 input) to 85 us (bf16 input).  `Layer` does all of it in one native call.
 //
-// A Layer also keeps the module's weights in the two-bit layout of w2_small.cuh, which
-// is laid out once from the packed checkpoint tensors and again whenever those have
-// changed: their addresses and version counters are compared on every call (tensors
-// made in inference mode have no version counter; SpBitLinear drops the layout when
-// a state dict is loaded into it).  A layout that is out of date while the stream is
-// being captured is not rebuilt there: that call reads the packed tensors.
+// A Layer also keeps the module's weights in the two-bit layout of w2_small.cuh, laid out
+// from the packed checkpoint tensors.  Nothing on a tensor tells whether its values have
+// changed: an address can come back with other values, and a version counter misses
+// writes through .data, by collectives, through raw pointers and of inference mode.  So
+// the copy is used only while nothing outside of the module can write to the packed
+// tensors.  The module keeps its parameters in a dict (linear.py, _OwnedParameters) that
+// invalidates the copy whenever it hands one out; the next call lays the weights out
+// again once the module alone holds every parameter and its storage, and reads the
+// packed tensors until then (and during a capture, where nothing is laid out).
 //
 // Every method returns None where the native path does not apply (other devices,
 // types or sizes); the caller then takes the general path in linear.py.
@@ -30,6 +33,7 @@
 namespace {
 
 PyObject* g_keys[5];                   // interned parameter names, in the order of Weights
+PyObject* g_layer;                     // interned name of the owning dict's attribute
 
 struct Weights {
     const at::Tensor *signs, *tile_offsets, *quarter_offsets, *bitmap, *scale;
@@ -38,13 +42,10 @@ struct Weights {
 struct Layer {
     PyObject_HEAD
     int in_features, out_features, ws_num, seg[3];
-    bool valid;                        // w2 was laid out from the tensors recorded below
-    const void* src_ptr[4];
-    int64_t src_version[4];
+    bool valid;                        // w2 holds the weights, and nothing outside of the module can change them
+    bool captured;                     // a graph reads w2
     at::Tensor* w2;
 };
-
-int64_t version_of(const at::Tensor& t) { return t.is_inference() ? 0 : t._version(); }
 
 bool get_weights(PyObject* params, Weights& w) {
     const at::Tensor** dst[5] = {&w.signs, &w.tile_offsets, &w.quarter_offsets, &w.bitmap, &w.scale};
@@ -62,26 +63,51 @@ bool capturing(cudaStream_t stream) {
     return cudaStreamIsCapturing(stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
 }
 
-// The two-bit weights, up to date; null where there are none (wrong sizes, out of date during a capture).
-void* two_bit(Layer* self, const Weights& w, cudaStream_t stream) {
-    const at::Tensor* src[4] = {w.signs, w.tile_offsets, w.quarter_offsets, w.bitmap};
-    bool fresh = self->valid;
-    for (int i = 0; i < 4 && fresh; ++i)
-        fresh = src[i]->data_ptr() == self->src_ptr[i] && version_of(*src[i]) == self->src_version[i];
-    if (fresh) return self->w2->data_ptr();
-    self->valid = false;
-    const int64_t N = self->out_features, K = self->in_features;
+// Whether `params` is the dict that reports to this layer what it hands out (and not a plain one put in its place).
+bool reports(Layer* self, PyObject* params) {
+    if (PyDict_CheckExact(params)) return false;
+    PyObject* layer = PyObject_GetAttr(params, g_layer);
+    const bool same = layer == reinterpret_cast<PyObject*>(self);
+    if (!layer) PyErr_Clear();
+    Py_XDECREF(layer);
+    return same;
+}
+
+// Whether the dict holds the only reference to each of the packed tensors, and these the only ones to their storage.
+bool exclusive(PyObject* params) {
+    for (int i = 0; i < 4; ++i) {
+        PyObject* o = PyDict_GetItem(params, g_keys[i]);
+        if (!o || !THPVariable_Check(o) || Py_REFCNT(o) != 1) return false;
+        const at::Tensor& t = THPVariable_Unpack(o);
+        if (t.use_count() != 1 || !t.has_storage()) return false;
+        // (a storage that Python has seen keeps its wrapper, which holds the second reference)
+        const c10::StorageImpl* storage = t.storage().unsafeGetStorageImpl();
+        const size_t refs = t.storage().use_count();
+        if (refs != 1 && !(refs == 2 && storage->pyobj_slot()->has_unique_reference())) return false;
+    }
+    return true;
+}
+
+// Writes the two-bit copy.  False where there is none (sizes, a capture under way).
+bool lay_out(Layer* self, const Weights& w, cudaStream_t stream) {
+    const int64_t N = self->out_features, K = self->in_features, tiles = N * K / 4096;
     if (N < 64 || K < 64 || N % 64 || K % 64 || K >= (1 << 18) || w.bitmap->nbytes() < (size_t)(N * K / 8) ||
-        w.tile_offsets->numel() < N * K / 4096 + 1 || capturing(stream))
-        return nullptr;
+        w.tile_offsets->numel() < tiles + 1 || w.quarter_offsets->numel() < 3 * tiles || capturing(stream))
+        return false;
     if (!self->w2->defined() || self->w2->device() != w.bitmap->device())
         *self->w2 = at::empty({ternaspmm_w2_bytes((int)N, (int)K)}, w.bitmap->options().dtype(at::kByte));
     ternaspmm_w2_relayout(static_cast<uint64_t*>(w.bitmap->data_ptr()), static_cast<int*>(w.tile_offsets->data_ptr()),
                           static_cast<uint16_t*>(w.quarter_offsets->data_ptr()), static_cast<uint32_t*>(w.signs->data_ptr()), (int)N,
                           (int)K, self->w2->data_ptr(), stream);
-    if (cudaStreamSynchronize(stream) != cudaSuccess) return nullptr;   // other streams may use the layer next
-    for (int i = 0; i < 4; ++i) self->src_ptr[i] = src[i]->data_ptr(), self->src_version[i] = version_of(*src[i]);
-    self->valid = true;
+    return cudaStreamSynchronize(stream) == cudaSuccess;   // other streams may use the layer next
+}
+
+// The two-bit weights; null where the call reads the packed tensors.
+void* two_bit(Layer* self, PyObject* params, const Weights& w, cudaStream_t stream) {
+    if (!reports(self, params)) return nullptr;
+    if (!self->valid) self->valid = exclusive(params) && lay_out(self, w, stream);
+    if (!self->valid) return nullptr;
+    if (!self->captured) self->captured = capturing(stream);
     return self->w2->data_ptr();
 }
 
@@ -153,7 +179,7 @@ PyObject* front_and_linear(Layer* self, PyObject* params, PyObject* xo, int fron
     if (!ok || !get_weights(params, w) || w.bitmap->device() != x.device()) Py_RETURN_NONE;
     c10::cuda::OptionalCUDAGuard guard(x.device());
     cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
-    void* w2 = two_bit(self, w, stream);
+    void* w2 = two_bit(self, params, w, stream);
     if (!w2) Py_RETURN_NONE;
     at::Tensor out = output_like(x, self->out_features);
     if (M <= ternaspmm_w2_fused_rows((int)K) && M <= (front_end == 1 ? 4 : 1)) {
@@ -207,7 +233,7 @@ PyObject* layer_forward_quantized(PyObject* o, PyObject* const* args, Py_ssize_t
     if (!ok || !get_weights(args[0], w) || w.bitmap->device() != x.device()) Py_RETURN_NONE;
     c10::cuda::OptionalCUDAGuard guard(x.device());
     cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
-    void* w2 = two_bit(self, w, stream);
+    void* w2 = two_bit(self, args[0], w, stream);
     if (!w2) Py_RETURN_NONE;
     at::Tensor out = output_like(x, self->out_features);
     run_linear(self, w, w2, x.data_ptr(), 0, nullptr, 0.f, out, s.data_ptr(), M, residual, stream);
@@ -215,26 +241,50 @@ PyObject* layer_forward_quantized(PyObject* o, PyObject* const* args, Py_ssize_t
     END_HANDLE_TH_ERRORS
 }
 
-// prepare(params): lay the weights out now instead of in the first call
+// prepare(params): lay the weights out now instead of in the first call; without GPU tensors, give the copy back
 PyObject* layer_prepare(PyObject* o, PyObject* params) {
     HANDLE_TH_ERRORS
+    Layer* self = reinterpret_cast<Layer*>(o);
     Weights w;
-    if (!get_weights(params, w)) Py_RETURN_FALSE;
+    if (!get_weights(params, w)) {
+        self->valid = self->captured = false;
+        *self->w2 = at::Tensor();
+        Py_RETURN_FALSE;
+    }
     c10::cuda::OptionalCUDAGuard guard(w.bitmap->device());
-    return PyBool_FromLong(two_bit(reinterpret_cast<Layer*>(o), w, c10::cuda::getCurrentCUDAStream().stream()) != nullptr);
+    return PyBool_FromLong(two_bit(self, params, w, c10::cuda::getCurrentCUDAStream().stream()) != nullptr);
     END_HANDLE_TH_ERRORS
 }
 
+// invalidate(): a parameter has been handed out
 PyObject* layer_invalidate(PyObject* o, PyObject*) {
     reinterpret_cast<Layer*>(o)->valid = false;
     Py_RETURN_NONE;
+}
+
+// forget(): a parameter has been replaced; calls in flight on other streams may still read the copy, so the next one is a
+// new one (a copy that a graph reads stays, and follows the module's weights when these are laid out again)
+PyObject* layer_forget(PyObject* o, PyObject*) {
+    HANDLE_TH_ERRORS
+    Layer* self = reinterpret_cast<Layer*>(o);
+    self->valid = false;
+    if (!self->captured) *self->w2 = at::Tensor();
+    Py_RETURN_NONE;
+    END_HANDLE_TH_ERRORS
+}
+
+// exclusive(params): what the copy depends on
+PyObject* layer_exclusive(PyObject* o, PyObject* params) {
+    HANDLE_TH_ERRORS
+    return PyBool_FromLong(PyDict_Check(params) && reports(reinterpret_cast<Layer*>(o), params) && exclusive(params));
+    END_HANDLE_TH_ERRORS
 }
 
 PyObject* layer_new(PyTypeObject* type, PyObject* args, PyObject*) {
     Layer* self = reinterpret_cast<Layer*>(type->tp_alloc(type, 0));
     if (!self) return nullptr;
     self->w2 = new at::Tensor();
-    self->valid = false;
+    self->valid = self->captured = false;
     if (!PyArg_ParseTuple(args, "iiiiii", &self->in_features, &self->out_features, &self->ws_num, &self->seg[0], &self->seg[1], &self->seg[2])) {
         Py_DECREF(self);
         return nullptr;
@@ -282,6 +332,8 @@ PyMethodDef layer_methods[] = {
     {"forward_quantized", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(layer_forward_quantized)), METH_FASTCALL, nullptr},
     {"prepare", layer_prepare, METH_O, nullptr},
     {"invalidate", layer_invalidate, METH_NOARGS, nullptr},
+    {"forget", layer_forget, METH_NOARGS, nullptr},
+    {"exclusive", layer_exclusive, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 
 PyTypeObject layer_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
@@ -294,6 +346,7 @@ PyMODINIT_FUNC PyInit__host_call() {
     static const char* const names[5] = {"weight_compressed_val", "weight_TileOffsets_global", "weight_TileOffsets_median", "weight_bitmap",
                                          "weight_scale"};
     for (int i = 0; i < 5; ++i) g_keys[i] = PyUnicode_InternFromString(names[i]);
+    g_layer = PyUnicode_InternFromString("layer");
     layer_type.tp_name = "_host_call.Layer";
     layer_type.tp_basicsize = sizeof(Layer);
     layer_type.tp_flags = Py_TPFLAGS_DEFAULT;

@@ -274,23 +274,73 @@ def TernaInfer_linear(input, compressed_val, TileOffsets_global, TileOffsets_med
     return ret.reshape(*out_shape)
 
 
+class _OwnedParameters(dict):
+    """Parameters of an ``SpBitLinear``.  Whatever gets hold of one - an attribute of the module, ``parameters()``,
+    ``state_dict()``, ``to()`` ... - reads it here, and that invalidates the layer's two-bit copy of the weights, since
+    the values may change from then on without a trace.  The next call takes the copy up again when the module alone holds
+    every parameter (host_call.cpp); hence lists instead of views, which would hand parameters out later."""
+
+    __slots__ = ("layer",)
+
+    def __init__(self, layer, items=()):
+        super().__init__(items)
+        self.layer = layer
+
+    def _handing_out(name):
+        read = getattr(dict, name)
+
+        def method(self, *args):
+            self.layer.invalidate()
+            out = read(self, *args)
+            return list(out) if name in ("items", "values") else out
+        method.__name__ = name
+        return method
+
+    def _replacing(name):
+        write = getattr(dict, name)
+
+        def method(self, *args, **kwargs):
+            self.layer.forget()
+            return write(self, *args, **kwargs)
+        method.__name__ = name
+        return method
+
+    for _name in ("__getitem__", "get", "items", "values", "copy", "__or__", "__ror__"):
+        locals()[_name] = _handing_out(_name)
+    for _name in ("__setitem__", "__delitem__", "__ior__", "pop", "popitem", "setdefault", "update", "clear"):
+        locals()[_name] = _replacing(_name)
+    del _name, _handing_out, _replacing
+
+    def __iter__(self):          # (its own, so that dict(self) reads through __getitem__)
+        return super().__iter__()
+
+    def __reduce__(self):
+        return dict, (dict(self),)
+
+
 class SpBitLinear(nn.Module):
     """Ternary linear layer bound to packed checkpoint tensors (model.py:96-133):
     ``<key>.weight_compressed_val`` (uint32), ``_TileOffsets_global`` (int32),
     ``_TileOffsets_median`` (uint16), ``_bitmap`` (uint64), ``.weight_scale``
-    (bf16[4])."""
+    (bf16[4]).
+
+    The packed tensors are parameters, copied from ``dic``; besides them the module keeps the weights in the two-bit
+    layout of its kernels (N*K/4 bytes more).  Calls use that copy while nothing outside of the module holds a parameter
+    or a tensor that shares its memory, and lay it out again after something did; otherwise they read the packed tensors."""
 
     def __init__(self, in_features: int, out_features: int, dic: dict, key: str, bias: bool = False):
         super().__init__()
         self.in_features = in_features
         self.out_features = out_features
         dev = "cuda"
-        self.weight_compressed_val = nn.Parameter(dic[key + ".weight_compressed_val"].to(dev), requires_grad=False)
-        self.weight_TileOffsets_global = nn.Parameter(dic[key + ".weight_TileOffsets_global"].to(dev),
-                                                      requires_grad=False)
-        self.weight_TileOffsets_median = nn.Parameter(dic[key + ".weight_TileOffsets_median"].to(dev),
-                                                      requires_grad=False)
-        self.weight_bitmap = nn.Parameter(dic[key + ".weight_bitmap"].to(dev), requires_grad=False)
+
+        def own(name):           # on the GPU, in memory that nothing else shares
+            t = dic[key + "." + name]
+            return nn.Parameter(t.clone() if t.is_cuda else t.to(dev), requires_grad=False)
+        self.weight_compressed_val = own("weight_compressed_val")
+        self.weight_TileOffsets_global = own("weight_TileOffsets_global")
+        self.weight_TileOffsets_median = own("weight_TileOffsets_median")
+        self.weight_bitmap = own("weight_bitmap")
         ws = dic[key + ".weight_scale"]
         self.weight_scale = nn.Parameter(ws.to(dev), requires_grad=False)
         self.ws_num = int((ws != 0).sum().item())
@@ -308,11 +358,13 @@ class SpBitLinear(nn.Module):
         if not _builtin_segments(self.segments, self.out_features, self.ws_num):
             bounds = [sum(self.segments[:i + 1]) for i in range(len(self.segments) - 1)] + [2 ** 31 - 1] * 3
         self._native = load_host_call().Layer(self.in_features, self.out_features, self.ws_num, *bounds[:3])
+        self.__dict__["_parameters"] = _OwnedParameters(self._native, self._parameters)
         self._native.prepare(self._parameters)
 
     def __getstate__(self):      # copies and pickles carry what checkpoints carry; the call site is made again from it
         state = self.__dict__.copy()
         state.pop("_native", None)
+        state["_parameters"] = dict(self._parameters)
         return state
 
     def __setstate__(self, state):
@@ -321,20 +373,25 @@ class SpBitLinear(nn.Module):
 
     quant_input = staticmethod(quant_input)
 
-    def _load_from_state_dict(self, *args, **kwargs):
-        super()._load_from_state_dict(*args, **kwargs)
-        self._native.invalidate()
+    def _apply(self, fn, recurse=True):
+        super()._apply(fn, recurse)
+        self._native.prepare(self._parameters)
+        return self
+
+    def _weights(self):
+        """The packed tensors and the scale, for a call to read."""
+        names = ("weight_compressed_val", "weight_TileOffsets_global", "weight_TileOffsets_median", "weight_bitmap", "weight_scale")
+        p = self._parameters
+        return [dict.__getitem__(p, n) for n in names] if isinstance(p, _OwnedParameters) else [getattr(self, n) for n in names]
 
     def forward_quantized(self, input_q, s, residual=None):
         """Already quantised input (int8 + per-token scale), optional fused residual add."""
         out = self._native.forward_quantized(self._parameters, input_q, s, residual)
         if out is not None:
             return out
-        return TernaInfer_linear(
-            input_q,
-            self.weight_compressed_val, self.weight_TileOffsets_global, self.weight_TileOffsets_median,
-            self.weight_bitmap, get_global_workspace(input_q.device), s, self.weight_scale, self.ws_num, self.out_features,
-            residual=residual, segments=self.segments)
+        *packed, ws = self._weights()
+        return TernaInfer_linear(input_q, *packed, get_global_workspace(input_q.device), s, ws, self.ws_num, self.out_features,
+                                 residual=residual, segments=self.segments)
 
     def forward_normed(self, x, norm_weight, eps, gated=False, residual=None):
         """forward_quantized(*rmsnorm_quant(x, norm_weight, eps, gated), residual): the front-end runs inside the
@@ -350,11 +407,6 @@ class SpBitLinear(nn.Module):
         if out is not None:
             return out
         input, s = quant_input(input)
-        return TernaInfer_linear(
-            input,
-            self.weight_compressed_val, self.weight_TileOffsets_global, self.weight_TileOffsets_median,
-            self.weight_bitmap,
-            get_global_workspace(input.device),
-            s, self.weight_scale, self.ws_num,
-            self.out_features, segments=self.segments,
-        )
+        *packed, ws = self._weights()
+        return TernaInfer_linear(input, *packed, get_global_workspace(input.device), s, ws, self.ws_num, self.out_features,
+                                 segments=self.segments)

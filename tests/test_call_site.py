@@ -1,4 +1,7 @@
 """CPU: the Python side of the call site - what a module's copies and pickles carry, what its parameters may share."""
+import copy
+import gc
+import io
 import subprocess
 import sys
 
@@ -9,7 +12,6 @@ from torch import nn
 from conftest import ROOT
 import ternaspmm_oracle as o
 from ternainfer_b200.convert import compress_weight
-from ternainfer_b200.lib import load_host_call
 from ternainfer_b200.linear import SpBitLinear
 
 
@@ -23,7 +25,7 @@ def layer(lib):
     for name, t in (("weight_compressed_val", cv), ("weight_TileOffsets_global", tg), ("weight_TileOffsets_median", tm), ("weight_bitmap", bm),
                     ("weight_scale", torch.tensor([0.5, 2.0, 0, 0]).to(torch.bfloat16))):
         m.register_parameter(name, nn.Parameter(t, requires_grad=False))
-    m._native = load_host_call().Layer(192, 128, 2, 0, 0, 0)
+    m._attach()
     return m
 
 
@@ -35,3 +37,49 @@ def test_saved_module_loads_in_a_fresh_process(layer, tmp_path):
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
     assert r.stdout.split() == ["128", "[64,", "64]", str(layer.weight_bitmap.numel()), "False"]
+
+
+HOLDS = {"attribute": lambda m: m.weight_bitmap, "detached": lambda m: m.weight_compressed_val.detach(), "state_dict": lambda m: m.state_dict(),
+         "parameters": lambda m: list(m.parameters()), "iterator": lambda m: iter(m._parameters.items()), "dict": lambda m: dict(m._parameters),
+         "view": lambda m: m.weight_bitmap.view(torch.uint8)[3:], "numpy": lambda m: m.weight_TileOffsets_global.numpy(),
+         "storage": lambda m: m.weight_TileOffsets_median.untyped_storage(), "get": lambda m: m._parameters.get("weight_bitmap"),
+         "unpacked": lambda m: {**m._parameters}, "shallow copy": lambda m: copy.copy(m)}
+
+
+@pytest.mark.parametrize("how", HOLDS)
+def test_a_parameter_in_other_hands_is_noticed(layer, how):
+    """Handing one out invalidates the two-bit copy, and it stays so while the module is not alone with its parameters."""
+    calls = []
+
+    class Spy:
+        def invalidate(self):
+            calls.append(1)
+    own = layer._native
+    assert own.exclusive(layer._parameters)
+    layer._parameters.layer = Spy()
+    held = HOLDS[how](layer)
+    layer._parameters.layer = own
+    assert calls and not own.exclusive(layer._parameters)
+    del held
+    gc.collect()
+    torch.save(layer.state_dict(), io.BytesIO())
+    assert own.exclusive(layer._parameters)
+
+
+def test_replaced_parameters_and_replaced_dicts_are_noticed(layer):
+    calls = []
+
+    class Spy:
+        def invalidate(self):
+            pass
+
+        def forget(self):
+            calls.append(1)
+    own = layer._native
+    layer._parameters.layer = Spy()
+    layer.weight_bitmap = nn.Parameter(torch.zeros(4), requires_grad=False)
+    assert len(calls) == 1
+    layer._parameters.layer = own
+    assert own.exclusive(layer._parameters)
+    assert not own.exclusive(dict(layer._parameters)) and not own.exclusive(copy.deepcopy(layer)._parameters)
+    assert copy.deepcopy(layer)._native.exclusive(layer._parameters) is False

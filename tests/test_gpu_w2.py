@@ -103,8 +103,7 @@ def test_layer_follows_its_weights(lib):
     twin = copy.deepcopy(layer)
     assert torch.equal(twin(x), y)
     signs = layer.weight_compressed_val
-    layer.weight_compressed_val.data.view(torch.int32).copy_(~signs.data.view(torch.int32))      # every sign flipped (seen: same storage ...)
-    layer.weight_compressed_val.view(torch.int32).add_(0)                                        # ... and a version bump)
+    layer.weight_compressed_val.data.view(torch.int32).copy_(~signs.data.view(torch.int32))      # every sign flipped
     assert torch.equal(layer(x), -y)
     assert torch.equal(twin(x), y)
     layer.load_state_dict(other.state_dict())
@@ -116,6 +115,82 @@ def test_layer_follows_its_weights(lib):
         z = layer(x)
     graph.replay()
     assert torch.equal(z, -y) and torch.equal(layer(x), -y)
+
+
+def flip(t):
+    t = t.view(torch.int32)
+    t.copy_(~t)
+
+
+def by_data(layer):
+    flip(layer.weight_compressed_val.data)
+
+
+def in_inference_mode(layer):
+    with torch.inference_mode():
+        flip(layer.weight_compressed_val)
+
+
+def by_state_dict(layer):
+    flip(layer.state_dict()["weight_compressed_val"].data)
+
+
+def by_iteration(layer):
+    for name, p in layer.named_parameters():
+        if name == "weight_compressed_val":
+            flip(p.data)
+
+
+def on_the_way(layer):          # the memory on the GPU is given back and taken again, at the same address as it may be
+    layer.cpu()
+    flip(layer.weight_compressed_val.data)
+    layer.cuda()
+
+
+def by_swap(layer):
+    layer.weight_compressed_val.data = ~layer.weight_compressed_val.data.view(torch.int32)
+    layer.weight_compressed_val.data = layer.weight_compressed_val.data.view(torch.uint32)
+
+
+@pytest.mark.parametrize("write", [by_data, in_inference_mode, by_state_dict, by_iteration, on_the_way, by_swap])
+@pytest.mark.parametrize("inference", [False, True])
+def test_layer_sees_weights_written_in_any_way(lib, write, inference):
+    with torch.inference_mode(inference):
+        layer, _ = make_layer(128, 192, 2, 1)
+        x = torch.randn((5, 192), generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).cuda()
+        y = layer(x)
+        write(layer)
+        assert torch.equal(layer(x), -y)
+        write(layer)
+        assert torch.equal(layer(x), y)
+
+
+def test_layer_sees_writes_through_tensors_that_somebody_keeps(lib):
+    """As long as one is kept there is nothing to tell a write by: the packed tensors are read, in captures too."""
+    layer, dic = make_layer(128, 192, 2, 1)
+    x = torch.randn((5, 192), generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).cuda()
+    y = layer(x)
+    assert layer._native.prepare(layer._parameters)
+    for kept in (layer.weight_compressed_val, layer.weight_compressed_val.detach(), layer.state_dict()["weight_compressed_val"],
+                 torch.from_dlpack(layer.weight_compressed_val.view(torch.int32)), layer.weight_compressed_val.untyped_storage()):
+        assert not layer._native.prepare(layer._parameters)
+        alias = torch.empty(0, dtype=torch.int32, device="cuda").set_(kept) if isinstance(kept, torch.UntypedStorage) else kept.data
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            z = layer(x)
+        flip(alias)
+        graph.replay()
+        assert torch.equal(layer(x), -y) and torch.equal(z, -y)
+        flip(alias)
+        graph.replay()
+        assert torch.equal(layer(x), y) and torch.equal(z, y)
+        del graph, z
+    del kept, alias
+    assert torch.equal(layer(x), y) and layer._native.prepare(layer._parameters)
+    twin = copy.copy(layer)                        # two modules, one set of parameters
+    assert torch.equal(twin(x), y) and not twin._native.prepare(twin._parameters) and not layer._native.prepare(layer._parameters)
+    flip(twin.weight_compressed_val.data)
+    assert torch.equal(layer(x), -y)
 
 
 @pytest.mark.parametrize("K", [64, 1040, 2560, 8192])
