@@ -241,7 +241,8 @@ PyObject* layer_forward_quantized(PyObject* o, PyObject* const* args, Py_ssize_t
     END_HANDLE_TH_ERRORS
 }
 
-// prepare(params): lay the weights out now instead of in the first call; without GPU tensors, give the copy back
+// prepare(params): lay the weights out now instead of in the first call; without GPU tensors, give the copy back.
+// The address of the copy that calls use, 0 where they read the packed tensors.
 PyObject* layer_prepare(PyObject* o, PyObject* params) {
     HANDLE_TH_ERRORS
     Layer* self = reinterpret_cast<Layer*>(o);
@@ -249,10 +250,25 @@ PyObject* layer_prepare(PyObject* o, PyObject* params) {
     if (!get_weights(params, w)) {
         self->valid = self->captured = false;
         *self->w2 = at::Tensor();
-        Py_RETURN_FALSE;
+        return PyLong_FromLong(0);
     }
     c10::cuda::OptionalCUDAGuard guard(w.bitmap->device());
-    return PyBool_FromLong(two_bit(self, params, w, c10::cuda::getCurrentCUDAStream().stream()) != nullptr);
+    return PyLong_FromVoidPtr(two_bit(self, params, w, c10::cuda::getCurrentCUDAStream().stream()));
+    END_HANDLE_TH_ERRORS
+}
+
+// relayout(params): write the copy again from the packed tensors, in place, whoever holds them - captured graphs read it.
+// False where there is none.
+PyObject* layer_relayout(PyObject* o, PyObject* params) {
+    HANDLE_TH_ERRORS
+    Layer* self = reinterpret_cast<Layer*>(o);
+    Weights w;
+    self->valid = false;
+    if (!reports(self, params) || !get_weights(params, w)) Py_RETURN_FALSE;
+    c10::cuda::OptionalCUDAGuard guard(w.bitmap->device());
+    if (!lay_out(self, w, c10::cuda::getCurrentCUDAStream().stream())) Py_RETURN_FALSE;
+    self->valid = exclusive(params);
+    Py_RETURN_TRUE;
     END_HANDLE_TH_ERRORS
 }
 
@@ -331,6 +347,7 @@ PyMethodDef layer_methods[] = {
     {"forward_normed", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(layer_forward_normed)), METH_FASTCALL, nullptr},
     {"forward_quantized", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(layer_forward_quantized)), METH_FASTCALL, nullptr},
     {"prepare", layer_prepare, METH_O, nullptr},
+    {"relayout", layer_relayout, METH_O, nullptr},
     {"invalidate", layer_invalidate, METH_NOARGS, nullptr},
     {"forget", layer_forget, METH_NOARGS, nullptr},
     {"exclusive", layer_exclusive, METH_O, nullptr},

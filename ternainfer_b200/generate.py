@@ -16,6 +16,7 @@ from dataclasses import dataclass
 
 import torch
 
+from .linear import SpBitLinear
 from .model import ModelArgs, Transformer
 
 
@@ -39,6 +40,12 @@ class FastGen:
         self._pos = torch.zeros(1, dtype=torch.long, device=self.device)
         self._prefill_graph = self._decode_graph = None
         self._prefill_next = self._decode_next = None
+        self._linears = [m for m in model.modules() if isinstance(m, SpBitLinear)]
+        self._weights = None
+
+    def _weight_copies(self):
+        """Lays out what has changed since the graphs were captured; where every linear reads its weights."""
+        return [m._native.prepare(m._parameters) for m in self._linears]
 
     @torch.inference_mode()
     def _capture(self):
@@ -54,12 +61,13 @@ class FastGen:
         self._decode_graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self._decode_graph):
             self._decode_next = self.model(self._tokens, self.cache, self._pos, greedy_last=True)
+        self._weights = self._weight_copies()
 
     @torch.inference_mode()
     def generate(self, prompt: torch.Tensor):
         """prompt [B, prompt_length] token ids -> (tokens [B, gen_length], stats)."""
         a = self.args
-        if a.use_cuda_graph and self._decode_graph is None:
+        if a.use_cuda_graph and (self._decode_graph is None or self._weight_copies() != self._weights):
             self._capture()
         out = torch.empty((a.gen_bsz, a.gen_length), dtype=torch.long, device=self.device)
         torch.cuda.synchronize()

@@ -326,7 +326,9 @@ class SpBitLinear(nn.Module):
 
     The packed tensors are parameters, copied from ``dic``; besides them the module keeps the weights in the two-bit
     layout of its kernels (N*K/4 bytes more).  Calls use that copy while nothing outside of the module holds a parameter
-    or a tensor that shares its memory, and lay it out again after something did; otherwise they read the packed tensors."""
+    or a tensor that shares its memory, and lay it out again after something did; otherwise they read the packed tensors.
+    A captured graph goes on reading what it was captured with.  ``load_state_dict`` and ``relayout()`` write the copy in
+    place, so that replays follow; after any other change of the weights, and after writes through a raw pointer, call ``relayout()``."""
 
     def __init__(self, in_features: int, out_features: int, dic: dict, key: str, bias: bool = False):
         super().__init__()
@@ -378,9 +380,25 @@ class SpBitLinear(nn.Module):
         self._native.prepare(self._parameters)
         return self
 
+    def _load_from_state_dict(self, state_dict, prefix, *args):
+        errors, before = args[-1], len(args[-1])
+        super()._load_from_state_dict(state_dict, prefix, *args)
+        # laid out at once, for the sake of captured graphs; a part of the tensors (one shard of several) is not a weight yet
+        if len(errors) == before and all(prefix + n in state_dict for n in self._PACKED):
+            self._native.relayout(self._parameters)
+
+    def relayout(self):
+        """Lay the two-bit copy out again from the packed parameters, which have changed, and wait for it.  In the
+        copy's memory, so that captured graphs follow.  Not while a stream is being captured."""
+        if torch.cuda.is_current_stream_capturing():
+            raise RuntimeError("SpBitLinear.relayout while the stream is being captured")
+        self._native.relayout(self._parameters)
+
+    _PACKED = ("weight_compressed_val", "weight_TileOffsets_global", "weight_TileOffsets_median", "weight_bitmap")
+
     def _weights(self):
         """The packed tensors and the scale, for a call to read."""
-        names = ("weight_compressed_val", "weight_TileOffsets_global", "weight_TileOffsets_median", "weight_bitmap", "weight_scale")
+        names = (*self._PACKED, "weight_scale")
         p = self._parameters
         return [dict.__getitem__(p, n) for n in names] if isinstance(p, _OwnedParameters) else [getattr(self, n) for n in names]
 

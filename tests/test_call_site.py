@@ -36,7 +36,7 @@ def test_saved_module_loads_in_a_fresh_process(layer, tmp_path):
            "print(m.out_features, m.segments, m.weight_bitmap.numel(), m._native.prepare(m._parameters))"
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
-    assert r.stdout.split() == ["128", "[64,", "64]", str(layer.weight_bitmap.numel()), "False"]
+    assert r.stdout.split() == ["128", "[64,", "64]", str(layer.weight_bitmap.numel()), "0"]
 
 
 HOLDS = {"attribute": lambda m: m.weight_bitmap, "detached": lambda m: m.weight_compressed_val.detach(), "state_dict": lambda m: m.state_dict(),

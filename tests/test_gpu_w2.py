@@ -193,6 +193,71 @@ def test_layer_sees_writes_through_tensors_that_somebody_keeps(lib):
     assert torch.equal(layer(x), -y)
 
 
+def test_graphs_follow_loaded_weights(lib):
+    """A replay after load_state_dict and after relayout() computes with the new weights; a part of the tensors, as from
+    one file of several, is not laid out."""
+    layer, _ = make_layer(128, 192, 2, 1)
+    x = torch.randn((5, 192), generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).cuda()
+    y = layer(x)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        z = layer(x)
+    old = {k: v.clone() for k, v in layer.state_dict().items()}
+    new = {k: v.clone() for k, v in old.items()}
+    flip(new["weight_compressed_val"])
+    layer.load_state_dict(new)
+    graph.replay()
+    assert torch.equal(z, -y)
+    kept = layer.weight_compressed_val             # as an optimiser would
+    layer.load_state_dict(old)
+    graph.replay()
+    assert torch.equal(z, y)
+    flip(kept.data)
+    layer.relayout()
+    graph.replay()
+    assert torch.equal(z, -y) and torch.equal(layer(x), -y)
+    del kept
+    layer.load_state_dict({"weight_compressed_val": old["weight_compressed_val"]}, strict=False)
+    graph.replay()
+    assert torch.equal(z, -y) and torch.equal(layer(x), y)
+    layer.weight_bitmap = torch.nn.Parameter(old["weight_bitmap"].clone(), requires_grad=False)   # (the graph's copy stays where it is)
+    assert torch.equal(layer(x), y)
+    graph.replay()
+    assert torch.equal(z, y)
+    with pytest.raises(RuntimeError, match="captured"):
+        with torch.cuda.graph(torch.cuda.CUDAGraph()):
+            layer.relayout()
+
+
+@torch.inference_mode()
+def test_generation_follows_its_weights(lib):
+    """FastGen replays graphs: weights changed in place, and a parameter that somebody keeps, between two prompts."""
+    from ternainfer_b200.generate import FastGen, GenArgs
+    from ternainfer_b200.model import ModelArgs, Transformer
+    from ternainfer_b200.convert.convert_TernaInfer import random_checkpoint
+    args = ModelArgs(n_layers=1, vocab_size=1024, fused_glue=True)
+    dic = random_checkpoint(args.dim, 1, args.n_heads, args.n_kv_heads, args.ffn_dim, 1024, seed=7)
+
+    def model(d):
+        with torch.device("cuda"):
+            return Transformer(args, d, max_seq_len=96).to(torch.bfloat16)
+    a = model(dic)
+    prompt = torch.randint(0, 1024, (2, 64), generator=torch.Generator(device="cuda").manual_seed(3), device="cuda")
+    gen = FastGen(a, GenArgs(16, 2, 64, True))
+    first, _ = gen.generate(prompt)
+    wo = a.layers[0].attention.wo
+    flip(wo.weight_compressed_val.data)
+    b = model(dic)
+    flip(b.layers[0].attention.wo.weight_compressed_val.data)
+    want, _ = FastGen(b, GenArgs(16, 2, 64, False)).generate(prompt)
+    assert torch.equal(gen.generate(prompt)[0], want) and not torch.equal(first, want)
+    kept = wo.weight_compressed_val
+    flip(kept.data)
+    assert torch.equal(gen.generate(prompt)[0], first)
+    flip(kept.data)
+    assert torch.equal(gen.generate(prompt)[0], want)
+
+
 @pytest.mark.parametrize("K", [64, 1040, 2560, 8192])
 def test_norms_of_many_rows_are_the_norms_of_each(lib, K):
     """From two rows per SM on, a kernel that keeps a row in registers takes over: the same bits as a few rows at a time."""
