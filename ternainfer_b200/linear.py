@@ -147,16 +147,25 @@ def to_float(x: torch.Tensor) -> torch.Tensor:
     return out
 
 
+def _attn_takes(qkv, k_cache, v_cache, cos, sin, pos, heads, kv_heads):
+    """What both attention kernels ask of their tensors; they get addresses and can check none of it."""
+    return (qkv.is_cuda and qkv.device == k_cache.device == v_cache.device == cos.device == sin.device == pos.device
+            and qkv.dtype == k_cache.dtype == v_cache.dtype == cos.dtype == sin.dtype == torch.bfloat16 and pos.dtype == torch.int64
+            and qkv.dim() == 3 and k_cache.dim() == 4 and k_cache.shape == v_cache.shape and kv_heads > 0
+            and k_cache.shape[0] == qkv.shape[0] and k_cache.shape[2:] == (kv_heads, 128) and qkv.shape[2] == (heads + 2 * kv_heads) * 128
+            and pos.numel() == qkv.shape[1] <= k_cache.shape[1] and qkv.numel() > 0
+            and all(t.is_contiguous() for t in (qkv, k_cache, v_cache, cos, sin, pos)))
+
+
 def attn_decode(qkv, k_cache, v_cache, cos_row, sin_row, pos, heads: int, kv_heads: int):
     """RoPE, cache append and attention of one new token per sequence in one kernel: qkv bf16 [B, 1, (heads + 2 *
     kv_heads) * 128], caches bf16 [B, L, kv_heads, 128], ``pos`` int64 [1] on the device, ``cos_row`` / ``sin_row`` bf16
     [1, 64] the rotation of that position.  bf16 [B, 1, heads * 128], or
-    None where the kernel does not take the shape."""
-    B, D = qkv.shape[0], k_cache.shape[-1]
-    if not (qkv.is_cuda and qkv.dtype == k_cache.dtype == v_cache.dtype == cos_row.dtype == torch.bfloat16 and pos.dtype == torch.int64
-            and D == 128 and heads in (4 * kv_heads, 8 * kv_heads) and cos_row.numel() == sin_row.numel() == 64
-            and qkv.is_contiguous() and k_cache.is_contiguous() and v_cache.is_contiguous()):
+    None where the kernel does not take the tensors."""
+    if not (_attn_takes(qkv, k_cache, v_cache, cos_row, sin_row, pos, heads, kv_heads) and qkv.shape[1] == 1
+            and heads in (4 * kv_heads, 8 * kv_heads) and cos_row.numel() == sin_row.numel() == 64):
         return None
+    B, D = qkv.shape[0], k_cache.shape[-1]
     out = torch.empty((B, 1, heads * D), dtype=torch.bfloat16, device=qkv.device)
     status = load_library().ternaspmm_attn_decode(qkv.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), cos_row.data_ptr(),
                                                   sin_row.data_ptr(), pos.data_ptr(), out.data_ptr(), B, heads, kv_heads, D,
@@ -167,11 +176,10 @@ def attn_decode(qkv, k_cache, v_cache, cos_row, sin_row, pos, heads: int, kv_hea
 def attn_prefill(qkv, k_cache, v_cache, cos_tab, sin_tab, pos, heads: int, kv_heads: int):
     """``attn_decode`` for T new tokens per sequence at consecutive positions (``pos`` int64 [T]), causal: qkv bf16
     [B, T, (heads + 2 * kv_heads) * 128], tables bf16 [>= L, 64].  bf16 [B, T, heads * 128], or None."""
-    B, T, D = qkv.shape[0], qkv.shape[1], k_cache.shape[-1]
-    if not (qkv.is_cuda and qkv.dtype == k_cache.dtype == v_cache.dtype == cos_tab.dtype == torch.bfloat16 and pos.dtype == torch.int64
-            and D == 128 and heads % (4 * kv_heads) == 0 and k_cache.shape[1] <= cos_tab.shape[0]
-            and qkv.is_contiguous() and k_cache.is_contiguous() and v_cache.is_contiguous()):
+    if not (_attn_takes(qkv, k_cache, v_cache, cos_tab, sin_tab, pos, heads, kv_heads) and heads % (4 * kv_heads) == 0
+            and cos_tab.shape == sin_tab.shape and cos_tab.dim() == 2 and cos_tab.shape[1] == 64 and k_cache.shape[1] <= cos_tab.shape[0]):
         return None
+    B, T, D = qkv.shape[0], qkv.shape[1], k_cache.shape[-1]
     out = torch.empty((B, T, heads * D), dtype=torch.bfloat16, device=qkv.device)
     status = load_library().ternaspmm_attn_prefill(qkv.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), cos_tab.data_ptr(),
                                                    sin_tab.data_ptr(), pos.data_ptr(), out.data_ptr(), B, T, heads, kv_heads, D,

@@ -59,3 +59,33 @@ def test_prompt_attention(lib, B, T, past, L, H, Hkv):
     want = torch.einsum("bhtl,blhd->bthd", a, vv).reshape(B, T, H * D)
     assert ((out.double() - want).norm() / want.norm()).item() < 4e-3
     assert (out.double() - want).abs().max().item() < 1.2e-2 * want.abs().max().item()
+
+
+def test_attention_refuses_what_its_kernels_cannot_check(lib, monkeypatch):
+    """Tensors on other devices, of other shapes or strides: None (and the caller's general path), without a launch."""
+    from ternainfer_b200 import linear
+    H, Hkv, D, B, L = 20, 5, 128, 2, 16
+
+    def args(T, **other):
+        a = dict(qkv=torch.zeros((B, T, (H + 2 * Hkv) * D), dtype=torch.bfloat16, device="cuda"), pos=torch.arange(T, device="cuda"),
+                 k=torch.zeros((B, L, Hkv, D), dtype=torch.bfloat16, device="cuda"), v=torch.zeros((B, L, Hkv, D), dtype=torch.bfloat16, device="cuda"),
+                 cos=torch.zeros((1 if T == 1 else L, 64), dtype=torch.bfloat16, device="cuda"), heads=H, kv_heads=Hkv)
+        a["sin"] = a["cos"].clone()
+        a.update((k, f(a[k])) for k, f in other.items())
+        return a["qkv"], a["k"], a["v"], a["cos"], a["sin"], a["pos"], a["heads"], a["kv_heads"]
+
+    assert attn_decode(*args(1)) is not None and attn_prefill(*args(3)) is not None
+    monkeypatch.setattr(linear, "load_library", lambda: pytest.fail("launched"))
+    bad = [dict(pos=torch.Tensor.cpu), dict(k=torch.Tensor.cpu), dict(v=torch.Tensor.cpu), dict(cos=torch.Tensor.cpu), dict(sin=torch.Tensor.cpu),
+           dict(sin=torch.Tensor.float), dict(pos=torch.Tensor.int), dict(qkv=lambda t: t[..., :-128].contiguous()), dict(qkv=lambda t: t[:1].contiguous()),
+           dict(k=lambda t: t[:1].contiguous()), dict(v=lambda t: t[:, :8].contiguous()), dict(k=lambda t: t[:, :, :4].contiguous(), v=lambda t: t[:, :, :4].contiguous()),
+           dict(v=lambda t: t.transpose(1, 2).contiguous().transpose(1, 2)), dict(pos=lambda t: torch.arange(len(t) + 1, device="cuda")),
+           dict(heads=lambda h: h + 4), dict(kv_heads=lambda h: 0), dict(cos=lambda t: t[:, :32].contiguous(), sin=lambda t: t[:, :32].contiguous()),
+           dict(pos=lambda t: torch.arange(2 * len(t), device="cuda")[::2])]
+    for T, f in ((1, attn_decode), (3, attn_prefill)):
+        for other in bad:
+            if T == 1 and list(other) == ["pos"] and other is bad[-1]:
+                continue                                                    # (one element is contiguous)
+            assert f(*args(T, **other)) is None, (T, list(other))
+    assert attn_prefill(*args(17, cos=lambda t: t[:1].expand(17, 64).contiguous(), sin=lambda t: t[:1].expand(17, 64).contiguous())) is None, "more tokens than rows of the cache"
+    assert attn_decode(*args(2)) is None
