@@ -53,7 +53,7 @@ bool get_weights(PyObject* params, Weights& w) {
         PyObject* o = PyDict_GetItem(params, g_keys[i]);   // borrowed
         if (!o || !THPVariable_Check(o)) return false;
         *dst[i] = &THPVariable_Unpack(o);
-        if (!(*dst[i])->is_cuda() || !(*dst[i])->is_contiguous()) return false;
+        if (!(*dst[i])->is_cuda() || !(*dst[i])->is_contiguous() || (*dst[i])->device() != w.signs->device()) return false;
     }
     return w.scale->scalar_type() == at::kBFloat16 && w.scale->numel() >= 4;
 }
@@ -148,10 +148,10 @@ void run_linear(Layer* self, const Weights& w, void* w2, void* x, int front_end,
                         static_cast<ternaspmm_bf16*>(residual), stream);
 }
 
-void* residual_ptr(PyObject* o, int64_t M, int64_t N, bool& ok) {   // None, or contiguous bf16 of M*N values
+void* residual_ptr(PyObject* o, const at::Tensor& x, int64_t M, int64_t N, bool& ok) {   // None, or contiguous bf16 of M*N values
     ok = true;
     if (o == Py_None) return nullptr;
-    ok = usable(o, at::kBFloat16, N) && THPVariable_Unpack(o).numel() == M * N;
+    ok = usable(o, at::kBFloat16, N) && THPVariable_Unpack(o).numel() == M * N && THPVariable_Unpack(o).device() == x.device();
     return ok ? THPVariable_Unpack(o).data_ptr() : nullptr;
 }
 
@@ -170,11 +170,12 @@ PyObject* front_and_linear(Layer* self, PyObject* params, PyObject* xo, int fron
     if (M > INT_MAX / 2) Py_RETURN_NONE;
     void* norm_w = nullptr;
     if (norm_o) {
-        if (!usable(norm_o, at::kBFloat16, K) || THPVariable_Unpack(norm_o).numel() != K) Py_RETURN_NONE;
+        if (!usable(norm_o, at::kBFloat16, K) || THPVariable_Unpack(norm_o).numel() != K || THPVariable_Unpack(norm_o).device() != x.device())
+            Py_RETURN_NONE;
         norm_w = THPVariable_Unpack(norm_o).data_ptr();
     }
     bool ok;
-    void* residual = residual_ptr(res_o, M, self->out_features, ok);
+    void* residual = residual_ptr(res_o, x, M, self->out_features, ok);
     Weights w;
     if (!ok || !get_weights(params, w) || w.bitmap->device() != x.device()) Py_RETURN_NONE;
     c10::cuda::OptionalCUDAGuard guard(x.device());
@@ -228,7 +229,7 @@ PyObject* layer_forward_quantized(PyObject* o, PyObject* const* args, Py_ssize_t
     if (M > INT_MAX / 2 || s.scalar_type() != at::kBFloat16 || !s.is_contiguous() || s.numel() != M || s.device() != x.device())
         Py_RETURN_NONE;
     bool ok;
-    void* residual = residual_ptr(args[3], M, self->out_features, ok);
+    void* residual = residual_ptr(args[3], x, M, self->out_features, ok);
     Weights w;
     if (!ok || !get_weights(args[0], w) || w.bitmap->device() != x.device()) Py_RETURN_NONE;
     c10::cuda::OptionalCUDAGuard guard(x.device());

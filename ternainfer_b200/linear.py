@@ -14,6 +14,7 @@ CPU path: calling with CPU tensors raises.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 
 import torch
@@ -46,6 +47,18 @@ def get_global_workspace(device="cuda"):
     return ws
 
 
+_SAME_DEVICE = contextlib.nullcontext()
+
+
+def _on(x: torch.Tensor):
+    """Context in which launches go to the device of ``x``, as torch operators do by themselves."""
+    return _SAME_DEVICE if x.device.index == torch.cuda.current_device() else torch.cuda.device(x.device)
+
+
+def _stream():
+    return torch.cuda.current_stream().cuda_stream
+
+
 def quant_input(input: torch.Tensor):
     """Per-token absmax int8 quantisation (model.py:120-123):
     s = 127 / clamp(max|x|, 1e-5); x_q = clamp(round(x*s), -128, 127).  bf16 activations on the GPU take one
@@ -57,8 +70,8 @@ def quant_input(input: torch.Tensor):
         if x.data_ptr() % 16 == 0:
             q = torch.empty(x.shape, dtype=torch.int8, device=x.device)
             s = torch.empty((*x.shape[:-1], 1), dtype=torch.bfloat16, device=x.device)
-            load_library().ternaspmm_quant(x.data_ptr(), x.numel() // K, K, q.data_ptr(), s.data_ptr(),
-                                           torch.cuda.current_stream(x.device).cuda_stream)
+            with _on(x):
+                load_library().ternaspmm_quant(x.data_ptr(), x.numel() // K, K, q.data_ptr(), s.data_ptr(), _stream())
             return q, s
     s = 127 / input.abs().max(dim=-1, keepdim=True).values.clamp_(min=1e-5)
     return (input * s).round().clamp(-128, 127).to(torch.int8), s
@@ -83,8 +96,8 @@ def rmsnorm_quant(x: torch.Tensor, norm_weight: torch.Tensor, eps: float, gated:
     """One fused kernel for RMSNorm(x) * weight followed by ``quant_input``
     (``gated``: x holds [x1 | x3] and the normalised value is relu(x1)^2 * x3).
     bf16 [..., K or 2K] -> (int8 [..., K], bf16 scale [..., 1])."""
-    if not x.is_cuda:
-        raise RuntimeError("rmsnorm_quant needs CUDA tensors: the B200 library has no CPU path")
+    if not x.is_cuda or norm_weight.device != x.device:
+        raise RuntimeError("rmsnorm_quant needs CUDA tensors of one device: the B200 library has no CPU path")
     lib = load_library()
     K = norm_weight.shape[0]
     x2 = x.reshape(-1, x.shape[-1]).contiguous()
@@ -92,39 +105,36 @@ def rmsnorm_quant(x: torch.Tensor, norm_weight: torch.Tensor, eps: float, gated:
     q = torch.empty((M, K), dtype=torch.int8, device=x.device)
     s = torch.empty((M, 1), dtype=torch.bfloat16, device=x.device)
     fn = lib.ternaspmm_relu2_gate_rmsnorm_quant if gated else lib.ternaspmm_rmsnorm_quant
-    fn(x2.data_ptr(), norm_weight.data_ptr(), float(eps), M, K, q.data_ptr(), s.data_ptr(),
-       torch.cuda.current_stream().cuda_stream)
+    with _on(x):
+        fn(x2.data_ptr(), norm_weight.data_ptr(), float(eps), M, K, q.data_ptr(), s.data_ptr(), _stream())
     return q.reshape(*x.shape[:-1], K), s.reshape(*x.shape[:-1], 1)
 
 
 def rmsnorm(x: torch.Tensor, norm_weight: torch.Tensor, eps: float) -> torch.Tensor:
     """RMSNorm(x) * weight in one kernel, in the summation order of ``rmsnorm_quant``; bf16 in, bf16 out."""
-    if not x.is_cuda:
-        raise RuntimeError("rmsnorm needs CUDA tensors: the B200 library has no CPU path")
+    if not x.is_cuda or norm_weight.device != x.device:
+        raise RuntimeError("rmsnorm needs CUDA tensors of one device: the B200 library has no CPU path")
     lib = load_library()
     K = norm_weight.shape[0]
     x2 = x.reshape(-1, K).contiguous()
     y = torch.empty_like(x2)
-    lib.ternaspmm_rmsnorm(x2.data_ptr(), norm_weight.data_ptr(), float(eps), x2.shape[0], K, y.data_ptr(),
-                          torch.cuda.current_stream().cuda_stream)
+    with _on(x):
+        lib.ternaspmm_rmsnorm(x2.data_ptr(), norm_weight.data_ptr(), float(eps), x2.shape[0], K, y.data_ptr(), _stream())
     return y.reshape(x.shape)
-
-
-def _stream():
-    return torch.cuda.current_stream().cuda_stream
 
 
 def rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor):
     """RoPE on adjacent pairs as one kernel: x bf16 [B, T, H, 128] (heads contiguous), cos / sin fp32 [B, T, 64] equal in
     every sequence (expanded).  None where the kernel does not take the tensors."""
     B, T, H, D = x.shape
-    if not (x.is_cuda and x.dtype == torch.bfloat16 and cos.dtype == sin.dtype == torch.float32 and D == 128 and x.numel() > 0
+    if not (x.is_cuda and x.device == cos.device == sin.device and x.dtype == torch.bfloat16 and cos.dtype == sin.dtype == torch.float32 and D == 128 and x.numel() > 0
             and x.stride(3) == 1 and x.stride(2) == D and (B == 1 or x.stride(0) == T * x.stride(1)) and x.stride(1) % 8 == 0
             and x.data_ptr() % 16 == 0 and cos.shape[1:] == sin.shape[1:] == (T, 64) and (B == 1 or cos.stride(0) == sin.stride(0) == 0)
             and cos.stride()[1:] == sin.stride()[1:] == (64, 1) and cos.data_ptr() % 16 == 0 and sin.data_ptr() % 16 == 0):
         return None
     out = torch.empty((B, T, H, D), dtype=torch.bfloat16, device=x.device)
-    load_library().ternaspmm_rope(x.data_ptr(), x.stride(1), cos.data_ptr(), sin.data_ptr(), out.data_ptr(), B, T, H, _stream())
+    with _on(x):
+        load_library().ternaspmm_rope(x.data_ptr(), x.stride(1), cos.data_ptr(), sin.data_ptr(), out.data_ptr(), B, T, H, _stream())
     return out
 
 
@@ -134,7 +144,8 @@ def relu2_gate(x13: torch.Tensor):
     if not (x13.is_cuda and x13.dtype == torch.bfloat16 and x13.is_contiguous() and K % 8 == 0 and x13.numel() > 0 and x13.data_ptr() % 16 == 0):
         return None
     out = torch.empty((*x13.shape[:-1], K), dtype=torch.bfloat16, device=x13.device)
-    load_library().ternaspmm_relu2_gate(x13.data_ptr(), out.data_ptr(), x13.numel() // (2 * K), K, _stream())
+    with _on(x13):
+        load_library().ternaspmm_relu2_gate(x13.data_ptr(), out.data_ptr(), x13.numel() // (2 * K), K, _stream())
     return out
 
 
@@ -143,7 +154,8 @@ def to_float(x: torch.Tensor) -> torch.Tensor:
     if not (x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous() and x.numel() > 0 and x.data_ptr() % 16 == 0):
         return x.float()
     out = torch.empty(x.shape, dtype=torch.float32, device=x.device)
-    load_library().ternaspmm_bf16_to_f32(x.data_ptr(), out.data_ptr(), x.numel(), _stream())
+    with _on(x):
+        load_library().ternaspmm_bf16_to_f32(x.data_ptr(), out.data_ptr(), x.numel(), _stream())
     return out
 
 
@@ -167,9 +179,10 @@ def attn_decode(qkv, k_cache, v_cache, cos_row, sin_row, pos, heads: int, kv_hea
         return None
     B, D = qkv.shape[0], k_cache.shape[-1]
     out = torch.empty((B, 1, heads * D), dtype=torch.bfloat16, device=qkv.device)
-    status = load_library().ternaspmm_attn_decode(qkv.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), cos_row.data_ptr(),
-                                                  sin_row.data_ptr(), pos.data_ptr(), out.data_ptr(), B, heads, kv_heads, D,
-                                                  k_cache.shape[1], torch.cuda.current_stream().cuda_stream)
+    with _on(qkv):
+        status = load_library().ternaspmm_attn_decode(qkv.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), cos_row.data_ptr(),
+                                                      sin_row.data_ptr(), pos.data_ptr(), out.data_ptr(), B, heads, kv_heads, D,
+                                                      k_cache.shape[1], _stream())
     return out if status == 0 else None
 
 
@@ -181,9 +194,10 @@ def attn_prefill(qkv, k_cache, v_cache, cos_tab, sin_tab, pos, heads: int, kv_he
         return None
     B, T, D = qkv.shape[0], qkv.shape[1], k_cache.shape[-1]
     out = torch.empty((B, T, heads * D), dtype=torch.bfloat16, device=qkv.device)
-    status = load_library().ternaspmm_attn_prefill(qkv.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), cos_tab.data_ptr(),
-                                                   sin_tab.data_ptr(), pos.data_ptr(), out.data_ptr(), B, T, heads, kv_heads, D,
-                                                   k_cache.shape[1], torch.cuda.current_stream().cuda_stream)
+    with _on(qkv):
+        status = load_library().ternaspmm_attn_prefill(qkv.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), cos_tab.data_ptr(),
+                                                       sin_tab.data_ptr(), pos.data_ptr(), out.data_ptr(), B, T, heads, kv_heads, D,
+                                                       k_cache.shape[1], _stream())
     return out if status == 0 else None
 
 
@@ -201,16 +215,16 @@ def lm_head_argmax(h: torch.Tensor, embedding: torch.Tensor, want_logits: bool =
     h2 = h.reshape(-1, K).contiguous()
     M = h2.shape[0]
     assert 1 <= M <= 8 and h2.dtype == torch.bfloat16 and embedding.dtype == torch.bfloat16 and embedding.is_contiguous()
+    assert embedding.device == h2.device
     dev = h.device
     scratch = _HEAD_SCRATCH.get(dev)
     if scratch is None:   # one zero-initialised scratch area per device (calls on one device run in stream order)
         scratch = _HEAD_SCRATCH[dev] = torch.zeros(int(lib.ternaspmm_lm_head_scratch_bytes()), dtype=torch.uint8, device=dev)
     logits = torch.empty((M, V), dtype=torch.float32, device=dev) if want_logits else None
     tokens = torch.empty((M,), dtype=torch.int64, device=dev) if want_argmax else None
-    lib.ternaspmm_lm_head_argmax(h2.data_ptr(), embedding.data_ptr(), M, V, K,
-                                 logits.data_ptr() if want_logits else None,
-                                 tokens.data_ptr() if want_argmax else None, 1, scratch.data_ptr(),
-                                 torch.cuda.current_stream().cuda_stream)
+    with _on(h2):
+        lib.ternaspmm_lm_head_argmax(h2.data_ptr(), embedding.data_ptr(), M, V, K, logits.data_ptr() if want_logits else None,
+                                     tokens.data_ptr() if want_argmax else None, 1, scratch.data_ptr(), _stream())
     return logits, tokens
 
 
@@ -224,6 +238,10 @@ def TernaInfer_linear(input, compressed_val, TileOffsets_global, TileOffsets_med
     2560/640/640 for 3840 outputs)."""
     if not input.is_cuda:
         raise RuntimeError("TernaInfer_linear needs CUDA tensors: the B200 library has no CPU path")
+    if input.device.index != torch.cuda.current_device():
+        with torch.cuda.device(input.device):
+            return TernaInfer_linear(input, compressed_val, TileOffsets_global, TileOffsets_median, bitmap, workspace, s, ws, ws_num,
+                                     out_features, mode, residual, segments)
     lib = load_library()
     out_shape = list(input.shape)
     out_shape[-1] = out_features

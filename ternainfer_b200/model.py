@@ -52,8 +52,8 @@ class RMSNorm(nn.Module):
         self.weight = nn.Parameter(torch.ones(dim))
 
     def forward(self, x):
-        if (x.is_cuda and x.dtype == self.weight.dtype == torch.bfloat16 and x.shape[-1] % 16 == 0 and x.shape[-1] <= 57344 and x.numel() > 0
-                and not torch.is_grad_enabled()):
+        if (x.is_cuda and x.device == self.weight.device and x.dtype == self.weight.dtype == torch.bfloat16 and x.shape[-1] % 16 == 0
+                and x.shape[-1] <= 57344 and x.numel() > 0 and not torch.is_grad_enabled()):
             return rmsnorm(x, self.weight, self.eps)       # one launch instead of seven, the fused front-ends' summation order
         xf = x.float()
         y = xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + self.eps)
