@@ -151,7 +151,8 @@ def relu2_gate(x13: torch.Tensor):
 
 def to_float(x: torch.Tensor) -> torch.Tensor:
     """x.float(); bf16 on the GPU by the library (at the copy rate; torch's casting kernel reaches a third of it)."""
-    if not (x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous() and x.numel() > 0 and x.data_ptr() % 16 == 0):
+    if not (x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous() and x.numel() > 0 and x.data_ptr() % 16 == 0
+            and not (x.requires_grad and torch.is_grad_enabled())):
         return x.float()
     out = torch.empty(x.shape, dtype=torch.float32, device=x.device)
     with _on(x):

@@ -18,6 +18,13 @@ def test_bf16_to_fp32(lib, n):
     assert y.dtype == torch.float32 and torch.equal(y, x.float())
 
 
+def test_bf16_to_fp32_keeps_the_gradient(lib):
+    """Logits of a prompt under autograd."""
+    x = torch.randn(4096, device="cuda").to(torch.bfloat16).requires_grad_()
+    to_float(x).sum().backward()
+    assert torch.equal(x.grad, torch.ones_like(x))
+
+
 def calls():
     def t(*shape):
         return torch.zeros(shape, dtype=torch.bfloat16, device="cuda")
