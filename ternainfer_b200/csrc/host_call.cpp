@@ -43,7 +43,7 @@ struct Layer {
     PyObject_HEAD
     int in_features, out_features, ws_num, seg[3];
     bool valid;                        // w2 holds the weights, and nothing outside of the module can change them
-    bool captured;                     // a graph reads w2
+    bool replaced;                     // w2 holds weights that calls in flight on other streams may still read
     at::Tensor* w2;
 };
 
@@ -94,6 +94,14 @@ bool lay_out(Layer* self, const Weights& w, cudaStream_t stream) {
     if (N < 64 || K < 64 || N % 64 || K % 64 || K >= (1 << 18) || w.bitmap->nbytes() < (size_t)(N * K / 8) ||
         w.tile_offsets->numel() < tiles + 1 || w.quarter_offsets->numel() < 3 * tiles || capturing(stream))
         return false;
+    if (self->replaced) {              // (relaxed: another thread may be capturing)
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        const cudaError_t e = cudaDeviceSynchronize();
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) return false;
+        self->replaced = false;
+    }
     if (!self->w2->defined() || self->w2->device() != w.bitmap->device())
         *self->w2 = at::empty({ternaspmm_w2_bytes((int)N, (int)K)}, w.bitmap->options().dtype(at::kByte));
     ternaspmm_w2_relayout(static_cast<uint64_t*>(w.bitmap->data_ptr()), static_cast<int*>(w.tile_offsets->data_ptr()),
@@ -106,9 +114,7 @@ bool lay_out(Layer* self, const Weights& w, cudaStream_t stream) {
 void* two_bit(Layer* self, PyObject* params, const Weights& w, cudaStream_t stream) {
     if (!reports(self, params)) return nullptr;
     if (!self->valid) self->valid = exclusive(params) && lay_out(self, w, stream);
-    if (!self->valid) return nullptr;
-    if (!self->captured) self->captured = capturing(stream);
-    return self->w2->data_ptr();
+    return self->valid ? self->w2->data_ptr() : nullptr;
 }
 
 at::Tensor output_like(const at::Tensor& x, int64_t N) {
@@ -249,7 +255,7 @@ PyObject* layer_prepare(PyObject* o, PyObject* params) {
     Layer* self = reinterpret_cast<Layer*>(o);
     Weights w;
     if (!get_weights(params, w)) {
-        self->valid = self->captured = false;
+        self->valid = self->replaced = false;
         *self->w2 = at::Tensor();
         return PyLong_FromLong(0);
     }
@@ -279,15 +285,11 @@ PyObject* layer_invalidate(PyObject* o, PyObject*) {
     Py_RETURN_NONE;
 }
 
-// forget(): a parameter has been replaced; calls in flight on other streams may still read the copy, so the next one is a
-// new one (a copy that a graph reads stays, and follows the module's weights when these are laid out again)
-PyObject* layer_forget(PyObject* o, PyObject*) {
-    HANDLE_TH_ERRORS
-    Layer* self = reinterpret_cast<Layer*>(o);
-    self->valid = false;
-    if (!self->captured) *self->w2 = at::Tensor();
+// replace(): a parameter has been replaced; the copy follows in the same memory, for the sake of captured graphs
+PyObject* layer_replace(PyObject* o, PyObject*) {
+    reinterpret_cast<Layer*>(o)->valid = false;
+    reinterpret_cast<Layer*>(o)->replaced = true;
     Py_RETURN_NONE;
-    END_HANDLE_TH_ERRORS
 }
 
 // exclusive(params): what the copy depends on
@@ -301,7 +303,7 @@ PyObject* layer_new(PyTypeObject* type, PyObject* args, PyObject*) {
     Layer* self = reinterpret_cast<Layer*>(type->tp_alloc(type, 0));
     if (!self) return nullptr;
     self->w2 = new at::Tensor();
-    self->valid = self->captured = false;
+    self->valid = self->replaced = false;
     if (!PyArg_ParseTuple(args, "iiiiii", &self->in_features, &self->out_features, &self->ws_num, &self->seg[0], &self->seg[1], &self->seg[2])) {
         Py_DECREF(self);
         return nullptr;
@@ -350,7 +352,7 @@ PyMethodDef layer_methods[] = {
     {"prepare", layer_prepare, METH_O, nullptr},
     {"relayout", layer_relayout, METH_O, nullptr},
     {"invalidate", layer_invalidate, METH_NOARGS, nullptr},
-    {"forget", layer_forget, METH_NOARGS, nullptr},
+    {"replace", layer_replace, METH_NOARGS, nullptr},
     {"exclusive", layer_exclusive, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 

@@ -327,7 +327,7 @@ class _OwnedParameters(dict):
         write = getattr(dict, name)
 
         def method(self, *args, **kwargs):
-            self.layer.forget()
+            self.layer.replace()
             return write(self, *args, **kwargs)
         method.__name__ = name
         return method

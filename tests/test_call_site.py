@@ -73,7 +73,7 @@ def test_replaced_parameters_and_replaced_dicts_are_noticed(layer):
         def invalidate(self):
             pass
 
-        def forget(self):
+        def replace(self):
             calls.append(1)
     own = layer._native
     layer._parameters.layer = Spy()
