@@ -283,7 +283,12 @@ void ternaspmm_tp_allreduce_finish(float** bufs, unsigned int** flags, ternaspmm
  * front_end 0: x is int8 [M][K] with its scales s.  1: x is bf16 [M][K], quantised per token in the
  * same kernel (ternaspmm_quant).  2: RMSNorm with norm_weight and eps first (ternaspmm_rmsnorm_quant).
  * 3: x is bf16 [M][2K], gate + RMSNorm first (ternaspmm_relu2_gate_rmsnorm_quant).  Front-ends 1-3
- * ignore s and take at most ternaspmm_w2_fused_rows(K) tokens.  K below 2^18. */
+ * ignore s and take at most ternaspmm_w2_fused_rows(K) tokens.  K below 2^18.
+ * Order: the linear reads w2 as soon as it is resident, which may be before the kernel ahead of it in the stream has
+ * ended (programmatic dependent launch).  A _relayout on the same stream is complete by then; another stream waits
+ * for it through an event or a synchronisation, and so does any stream for a w2 that something else has
+ * written (a kernel that releases its dependents early, say).  The same holds for the packed arrays and the other linears.
+ * norm_weight, x, s and residual are read in stream order. */
 void ternaspmm_w2_relayout(uint64_t* bitmap, int* tile_offsets, uint16_t* quarter_offsets, uint32_t* sign_words,
                            int N, int K, void* w2, ternaspmm_stream_t stream);
 long long ternaspmm_w2_bytes(int N, int K);

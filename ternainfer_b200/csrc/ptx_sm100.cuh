@@ -49,6 +49,8 @@ __device__ __forceinline__ bool mbar_test_suspended(uint32_t bar, uint32_t parit
 __device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(__cvta_generic_to_global(src)) : "memory");
 }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_but_last() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // -------------------------------------------------------- cluster barrier
 __device__ __forceinline__ void cluster_arrive() {

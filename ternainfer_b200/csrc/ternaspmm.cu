@@ -745,6 +745,8 @@ static cudaError_t launch_w2_pair(const W2Params& p, cudaStream_t stream) {
 // tokens: 15.1 / 18.3 us packed, 21.0 / 22.6 us two-bit).
 extern "C" int ternaspmm_w2_pays(int M, int N, int K) { return M <= 32 || M > 256 || K < 5120 || N > 32 * device_sm_count(); }
 
+__global__ void stream_fence_kernel() {}
+
 // Bytes of a weight's two-bit layout.
 extern "C" long long ternaspmm_w2_bytes(int N, int K) { return N < 16 || K < 64 ? 0 : (long long)(N / 16) * w2_pairs(K) * 512; }
 
@@ -765,6 +767,9 @@ extern "C" void ternaspmm_w2_relayout(uint64_t* bitmap, int* tile_offsets, uint1
     p.signs = sign_words, p.N = N, p.K = K;
     const long long tiles = (long long)(N / 64) * (K / 64);
     relayout_w2_kernel<<<(unsigned)((tiles + 7) / 8), 256, 0, stream>>>(p, static_cast<uint8_t*>(w2));
+    // A linear that follows reads w2 ahead of its dependency wait, as early as the kernel before it lets it.  This one begins in
+    // plain stream order, when the layout is complete and visible, and every later kernel of the stream begins after it.
+    stream_fence_kernel<<<1, 32, 0, stream>>>();
     checkLastCudaError(__LINE__);
 }
 

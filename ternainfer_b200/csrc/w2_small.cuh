@@ -174,7 +174,8 @@ __global__ void __launch_bounds__(kW2MaxWarps * 32, MT <= 2 ? 2 : 1) w2_small_ke
 
     phase_mark(0);
     griddep_launch_dependents();
-    // ---- weights: immutable, so the ring fills - and is waited for - before the dependency wait
+    // ---- weights: complete before any kernel that this one may overtake began (ternaspmm_w2_relayout sees to it), so the ring
+    // fills - and is waited for - before the dependency wait
     int f_gi = 0, f_c = p0, f_d = 0;                          // lane 0: the next chunk to fetch and its slot
     auto fetch = [&]() {
         const int c1 = min(f_c + PC, p1), nr = min(RG, nstrips - f_gi * RG);
@@ -195,7 +196,7 @@ __global__ void __launch_bounds__(kW2MaxWarps * 32, MT <= 2 ? 2 : 1) w2_small_ke
     for (int i = tid; i < MT * 8 * L.red_stride; i += nthreads) red[i] = 0;
     constexpr bool kGated = FE == W2_GATED;
     const uint32_t row = base + L.row, wrow = row + K * (kGated ? 4 : 2);
-    if (FE == W2_NORM || FE == W2_GATED) act_row_copy(wrow, p.norm_w, K);
+    if ((FE == W2_NORM || FE == W2_GATED) && tid == 64 && b == 0) act_weight_ahead(p.norm_w, K);
     const int pairs = nstrips * 8, items = mrows * pairs;     // epilogue items: two columns of a token each
     const uint32_t inv_pairs = ((1u << 22) + pairs - 1) / pairs;   // i / pairs = i * inv >> 22 (i * pairs < 2^22)
     const bool res_smem = p.e.residual != nullptr && (reinterpret_cast<uintptr_t>(p.e.residual) & 15) == 0;
@@ -219,6 +220,8 @@ __global__ void __launch_bounds__(kW2MaxWarps * 32, MT <= 2 ? 2 : 1) w2_small_ke
         const __nv_bfloat16* xr = p.xb + (size_t)m0 * (kGated ? 2 * K : K);
         act_row_copy(row, xr, K);
         if (kGated) act_row_copy(row + K * 2, xr + K, K);
+        cp_async_commit();
+        if (FE != W2_PLAIN) act_row_copy(wrow, p.norm_w, K);
     }
     if (res_smem) {
 #pragma unroll 1
@@ -227,6 +230,7 @@ __global__ void __launch_bounds__(kW2MaxWarps * 32, MT <= 2 ? 2 : 1) w2_small_ke
             cp_async_16(base + L.res + (t * pairs + c) * 4, p.e.residual + (size_t)(m0 + t) * N + strip0 * 16 + c * 2);
         }
     }
+    cp_async_commit();
     if (FE == W2_INT8 && tid < mrows && p.e.epilogue != EPI_RAW_I32) scl[tid] = __bfloat162float(p.e.s[m0 + tid]);
     if (tid >= 32 && tid < 36 && p.e.epilogue != EPI_RAW_I32 && p.e.epilogue != EPI_F32_DIV) scl[tid] = __bfloat162float(p.e.ws[tid - 32]);
     uint4 xn[2 * MT];                                         // direct fragments of the next pair
@@ -262,6 +266,8 @@ __global__ void __launch_bounds__(kW2MaxWarps * 32, MT <= 2 ? 2 : 1) w2_small_ke
                 const __nv_bfloat16* xr = p.xb + (size_t)(m0 + t) * (kGated ? 2 * K : K);
                 act_row_copy(row, xr, K);
                 if (kGated) act_row_copy(row + K * 2, xr + K, K);
+                cp_async_commit();
+                cp_async_commit();                            // (no norm weight behind it)
             }
             const float s = act_row_finish<kGated, kMode>(row, wrow, p.eps, K, T, part, reinterpret_cast<uint32_t*>(part + 32), nullptr,
                                                           [&](int k0, const uint4& v) { sts64(xrow + k0, v.x, v.y); });

@@ -62,6 +62,33 @@ def test_pairs_with_several_tiles_and_ragged_edges(lib, M, N, K):
     check_linear(lib, M, N, K, 2)
 
 
+def test_layout_and_linear_on_one_stream(lib):
+    """Two weights and two norm weights in turn through the same memory, layout and linear in stream order: never the other's values."""
+    N, K = 13824, 2560
+    ws = [o.make_ternary(N, K, 0.45, i) for i in (1, 2)]
+    pks = [Packed(w, [t.cpu().numpy() for t in compress_weight(torch.from_numpy(w).cuda())]) for w in ws]
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn((1, K), generator=g, device="cuda").to(torch.bfloat16)
+    norms = [(1 + 0.3 * torch.randn(K, generator=g, device="cuda")).to(torch.bfloat16) for _ in range(2)]
+    scale = torch.tensor([0.5, 2.0, 0, 0], device="cuda").to(torch.bfloat16)
+    w2, norm = torch.empty(lib.ternaspmm_w2_bytes(N, K), dtype=torch.uint8, device="cuda"), torch.empty_like(norms[0])
+    outs = torch.empty((80, 1, N), dtype=torch.bfloat16, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    for i in range(80):
+        pk = pks[i & 1]
+        norm.copy_(norms[i & 1])
+        lib.ternaspmm_w2_relayout(pk.bm.data_ptr(), pk.tg.data_ptr(), pk.tm.data_ptr(), pk.cv.data_ptr(), N, K, w2.data_ptr(), stream)
+        for _ in range(1 + i % 3):
+            lib.ternaspmm_w2_linear(x.data_ptr(), 2, norm.data_ptr(), 1e-5, w2.data_ptr(), outs[i].data_ptr(), None, scale.data_ptr(), 2, 1, N, K,
+                                    0, 0, 0, -1, None, stream)
+    for i in (0, 1):
+        xq, s = rmsnorm_quant(x, norms[i], 1e-5)
+        _, want = c_oracle.ternaspmm(xq.cpu().numpy(), ws[i], s.view(torch.int16).cpu().numpy().view(np.uint16).reshape(-1),
+                                     scale.view(torch.int16).cpu().numpy().view(np.uint16), 2, -1)
+        got = outs[i::2].view(torch.int16).cpu().numpy().view(np.uint16)
+        assert (got == want[None]).all()
+
+
 def make_layer(N, K, ws_num, seed, segments=None):
     w = o.make_ternary(N, K, 0.45, seed)
     cv, tg, tm, bm = compress_weight(torch.from_numpy(w))
