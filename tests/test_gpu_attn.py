@@ -89,3 +89,28 @@ def test_attention_refuses_what_its_kernels_cannot_check(lib, monkeypatch):
             assert f(*args(T, **other)) is None, (T, list(other))
     assert attn_prefill(*args(17, cos=lambda t: t[:1].expand(17, 64).contiguous(), sin=lambda t: t[:1].expand(17, 64).contiguous())) is None, "more tokens than rows of the cache"
     assert attn_decode(*args(2)) is None
+
+
+@pytest.mark.parametrize("B,T,past,L", [(1, 1, 600, 640), (8, 1, 1100, 1101), (2, 613, 0, 613), (1, 200, 1000, 1200), (1, 1024, 0, 1024)])
+def test_attention_is_as_exact_as_flash_attn(lib, B, T, past, L):
+    """Error against float64 beside that of the kernel which the model called before, on the same inputs."""
+    flash_attn = pytest.importorskip("flash_attn")
+    H, Hkv, D = 20, 5, 128
+    g = torch.Generator(device="cuda").manual_seed(T + past)
+    qkv = torch.randn((B, T, (H + 2 * Hkv) * D), generator=g, device="cuda").to(torch.bfloat16)
+    kc, vc = (torch.randn((B, L, Hkv, D), generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    k0, v0 = kc.clone(), vc.clone()
+    cos, sin = (t.to(torch.bfloat16) for t in rope_tables(D, L, 500000.0, "cuda"))
+    p = torch.arange(past, past + T, device="cuda")
+    ours = attn_decode(qkv, kc, vc, cos[p], sin[p], p, H, Hkv) if T == 1 else attn_prefill(qkv, kc, vc, cos, sin, p, H, Hkv)
+    q, k, v = (t.view(B, T, -1, D) for t in qkv.split([H * D, Hkv * D, Hkv * D], -1))
+    theirs = flash_attn.flash_attn_with_kvcache(q, k0, v0, k=k, v=v, rotary_cos=cos, rotary_sin=sin, causal=True, rotary_interleaved=True,
+                                                cache_seqlens=torch.full((B,), past, dtype=torch.int32, device="cuda")).reshape(B, T, H * D)
+    qr = apply_rope(q, cos[p].float().expand(B, T, -1), sin[p].float().expand(B, T, -1)).double()
+    kk, vv = (t[:, :past + T].double().repeat_interleave(H // Hkv, 2) for t in (kc, vc))
+    a = torch.einsum("bthd,blhd->bhtl", qr, kk) / D ** 0.5
+    a = a.masked_fill(torch.arange(past + T, device="cuda")[None, :] > p[:, None], float("-inf")).softmax(-1)
+    want = torch.einsum("bhtl,blhd->bthd", a, vv).reshape(B, T, H * D)
+    e_ours, e_theirs = (((t.double() - want).norm() / want.norm()).item() for t in (ours, theirs))
+    # the same formats (bf16 operands and probabilities, fp32 sums) and 2e5 to 6e6 outputs: the two norms agree to a per cent
+    assert e_ours <= 1.02 * e_theirs
