@@ -376,9 +376,10 @@ long long ternaspmm_pack_i8(const int8_t* W, int N, int K, uint64_t* bitmap,
                             uint32_t* sign_words);
 
 /* The same packer on the GPU (device pointers, W and bitmap 16-byte aligned), in two steps because the size of the
- * sign stream is known only after the first: _layout writes bitmap, tile_offsets and quarter_offsets, waits
- * for the stream and returns the number of sign words (or -1); _signs fills that many words and clears four
- * more behind them.  Not while capturing. */
+ * sign stream is known only after the first: _layout writes bitmap, tile_offsets and quarter_offsets and returns
+ * the number of sign words (or -1) as soon as that is known, while its last kernel may still be running; _signs
+ * fills that many words and clears four more behind them.  All four arrays are complete in stream order: the host and
+ * other streams wait for the stream first.  Not while capturing. */
 long long ternaspmm_pack_gpu_layout(const int8_t* W, int N, int K, uint64_t* bitmap, int* tile_offsets,
                                     uint16_t* quarter_offsets, ternaspmm_stream_t stream);
 void ternaspmm_pack_gpu_signs(const int8_t* W, int N, int K, const int* tile_offsets, uint32_t* sign_words,
