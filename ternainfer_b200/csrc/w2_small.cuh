@@ -231,8 +231,8 @@ __global__ void __launch_bounds__(kW2MaxWarps * 32, MT <= 2 ? 2 : 1) w2_small_ke
         }
     }
     cp_async_commit();
-    if (FE == W2_INT8 && tid < mrows && p.e.epilogue != EPI_RAW_I32) scl[tid] = __bfloat162float(p.e.s[m0 + tid]);
-    if (tid >= 32 && tid < 36 && p.e.epilogue != EPI_RAW_I32 && p.e.epilogue != EPI_F32_DIV) scl[tid] = __bfloat162float(p.e.ws[tid - 32]);
+    if (FE == W2_INT8 && tid < mrows) scl[tid] = __bfloat162float(p.e.s[m0 + tid]);
+    if (tid >= 32 && tid < 36) scl[tid] = __bfloat162float(p.e.ws[tid - 32]);
     uint4 xn[2 * MT];                                         // direct fragments of the next pair
     auto load_x = [&](int pr, uint4* x) {                     // (columns of absent tokens are not stored)
 #pragma unroll
@@ -361,24 +361,17 @@ __global__ void __launch_bounds__(kW2MaxWarps * 32, MT <= 2 ? 2 : 1) w2_small_ke
         const int t = (int)((uint32_t)i * inv_pairs >> 22), c = (i - t * pairs) * 2, n = strip0 * 16 + c;
         const int v[2] = {red[t * L.red_stride + c] >> 6, red[t * L.red_stride + c + 1] >> 6};
         const size_t o = (size_t)(m0 + t) * N + n;
-        if (p.e.epilogue == EPI_RAW_I32) {
-            reinterpret_cast<int*>(p.e.out)[o] = v[0], reinterpret_cast<int*>(p.e.out)[o + 1] = v[1];
-        } else if (p.e.epilogue == EPI_F32_DIV) {
-            float* out = reinterpret_cast<float*>(p.e.out) + o;
-            out[0] = __fdiv_rn(__int2float_rn(v[0]), scl[t]), out[1] = __fdiv_rn(__int2float_rn(v[1]), scl[t]);
-        } else {
-            __nv_bfloat16 r[2] = {scale_epilogue(v[0], scl[t], scl[32 + ws_group(n, p.e)], p.e.epilogue),
-                                  scale_epilogue(v[1], scl[t], scl[32 + ws_group(n + 1, p.e)], p.e.epilogue)};
-            if (res_smem) {
-                const uint32_t rv = lds32(base + L.res + i * 4);
-                r[0] = __float2bfloat16_rn(act_lo(rv) + __bfloat162float(r[0])), r[1] = __float2bfloat16_rn(act_hi(rv) + __bfloat162float(r[1]));
-            } else if (p.e.residual) {
-                r[0] = add_residual(r[0], p.e.residual, (long long)o), r[1] = add_residual(r[1], p.e.residual, (long long)o + 1);
-            }
-            __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.e.out) + o;
-            if (out_ok) stg_b32(out, (uint32_t)__bfloat16_as_ushort(r[0]) | ((uint32_t)__bfloat16_as_ushort(r[1]) << 16));
-            else out[0] = r[0], out[1] = r[1];
+        __nv_bfloat16 r[2] = {scale_epilogue(v[0], scl[t], scl[32 + ws_group(n, p.e)], p.e.epilogue),
+                              scale_epilogue(v[1], scl[t], scl[32 + ws_group(n + 1, p.e)], p.e.epilogue)};
+        if (res_smem) {
+            const uint32_t rv = lds32(base + L.res + i * 4);
+            r[0] = __float2bfloat16_rn(act_lo(rv) + __bfloat162float(r[0])), r[1] = __float2bfloat16_rn(act_hi(rv) + __bfloat162float(r[1]));
+        } else if (p.e.residual) {
+            r[0] = add_residual(r[0], p.e.residual, (long long)o), r[1] = add_residual(r[1], p.e.residual, (long long)o + 1);
         }
+        __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.e.out) + o;
+        if (out_ok) stg_b32(out, (uint32_t)__bfloat16_as_ushort(r[0]) | ((uint32_t)__bfloat16_as_ushort(r[1]) << 16));
+        else out[0] = r[0], out[1] = r[1];
     }
     phase_mark(7);
 }

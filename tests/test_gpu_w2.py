@@ -144,6 +144,29 @@ def test_layer_follows_its_weights(lib):
     assert torch.equal(z, -y) and torch.equal(layer(x), -y)
 
 
+@pytest.mark.parametrize("N,K", [(64, 64), (2560, 2560), (192, 6912), (320, 8128), (13824, 8192)])
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 7, 8])
+def test_front_end_of_several_rows_through_the_c_abi(lib, M, N, K):
+    """Front-ends 1-3 up to ternaspmm_w2_fused_rows(K) tokens, rows of very different size: the values of the separate launch."""
+    assert lib.ternaspmm_w2_fused_rows(K) == 8 and lib.ternaspmm_w2_fused_rows(8256) == 0
+    w = torch.from_numpy(o.make_ternary(N, K, 0.45, N + K)).cuda()
+    pk = Packed(np.empty((N, K), np.int8), [t.cpu().numpy() for t in compress_weight(w)])
+    w2, stream = w2_of(lib, pk), torch.cuda.current_stream().cuda_stream
+    g = torch.Generator(device="cuda").manual_seed(M)
+    norm = (1 + 0.1 * torch.randn(K, generator=g, device="cuda")).to(torch.bfloat16)
+    ws = torch.tensor([0.5, 2.0, 0, 0], device="cuda").to(torch.bfloat16)
+    res = torch.randn((M, N), generator=g, device="cuda").to(torch.bfloat16)
+    size = torch.logspace(-2, 2, M, device="cuda")[:, None]
+    for front_end in (1, 2, 3):
+        x = (torch.randn((M, K if front_end < 3 else 2 * K), generator=g, device="cuda") * size).to(torch.bfloat16)
+        xq, s = quant_input(x) if front_end == 1 else rmsnorm_quant(x, norm, 1e-5, gated=front_end == 3)
+        outs = [torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+        for out, (t, fe, sc) in zip(outs, ((x, front_end, None), (xq, 0, s.data_ptr()))):
+            lib.ternaspmm_w2_linear(t.data_ptr(), fe, norm.data_ptr(), 1e-5, w2.data_ptr(), out.data_ptr(), sc, ws.data_ptr(), 2, M, N, K, 0, 0, 0, -1,
+                                    res.data_ptr() if front_end > 1 else None, stream)
+        assert lib.ternaspmm_last_status() == 0 and torch.equal(*outs)
+
+
 def flip(t):
     t = t.view(torch.int32)
     t.copy_(~t)
