@@ -635,8 +635,11 @@ extern "C" void ternaspmm_linear_segments(int8_t* x, uint64_t* bitmap, int* tile
 
 // ---- linears on two-bit weights (w2_small.cuh) -----------------------------------------------------
 constexpr int kW2MaxSmem = 227 * 1024;
-// Tokens up to which the mma.sync kernel runs (more: tcgen05 on CTA pairs).  Measured, one call in a stream, mma.sync / pairs:
-// 3840 x 2560 at 48 / 64 tokens 8.9 / 10.3, 9.4 / 10.3 us, 2560 x 2560 7.7 / 10.3, 8.5 / 10.3, 13824 x 2560 17.0 / 13.2, 17.1 / 13.2.
+// Tokens up to which the mma.sync kernel runs (more: tcgen05 on CTA pairs).  Its second block of 32 tokens reads the weights again,
+// which pays while the pairs have few tiles, that is up to 32 rows per SM.  us per call in a stream of different weights,
+// mma.sync / pairs: 3840 x 2560 at 48 / 64 tokens 7.5 / 7.5, 7.9 / 7.7, 2560 x 2560 6.9 / 7.5, 7.0 / 7.6, 2560 x 6912 11.8 / 15.6, 12.1 / 15.6,
+// 4096 x 4096 9.1 / 10.3, 8.7 / 10.4; above that line 6400 x 6400 at 64 tokens 16.9 / 17.0, 13824 x 2560 17.2 / 10.6.  (At 32 tokens
+// the widest layers lose a little by it: 13824 x 2560 10.8 / 9.9, 14336 x 4096 15.5 / 13.4.)
 static int w2_small_tokens(int N) { return N <= 32 * device_sm_count() ? 64 : 32; }
 
 template <int MT, int RG, int U, int FE, bool XS>
@@ -740,10 +743,12 @@ static cudaError_t launch_w2_pair(const W2Params& p, cudaStream_t stream) {
     return cudaLaunchKernelEx(&cfg, kern, pp, map);
 }
 
-// Whether a call that has both forms of the weight in hand should take the two-bit one.  Deep and narrow layers at 33 to 256
-// tokens fill few pairs, each with a long K loop, which the packed tcgen05 kernel splits over a cluster (2560 x 6912 at 64 / 256
-// tokens: 15.1 / 18.3 us packed, 21.0 / 22.6 us two-bit).
-extern "C" int ternaspmm_w2_pays(int M, int N, int K) { return M <= 32 || M > 256 || K < 5120 || N > 32 * device_sm_count(); }
+// Whether a call that has both forms of the weight in hand should take the two-bit one.  Deep and narrow layers beyond the mma.sync
+// kernel's reach fill few pairs, each with a long K loop, which the packed tcgen05 kernel splits over a cluster.  us per call,
+// two-bit / packed: 2560 x 6912 at 48 tokens 11.8 / 13.4, at 128 16.7 / 15.7, 256 17.3 / 17.9, 320 17.7 / 24.6; 4096 x 14336 21.3 / 23.3,
+// 32.9 / 25.3, 33.4 / 27.4, 34.0 / 41.4; above the line in rows 6400 x 6400 at 128 17.1 / 22.2, below the one in K
+// 4096 x 4096 12.5 / 14.7.  (Four row blocks stay behind at any size: 1024 x 16384 at 320 tokens 35.0 / 25.2.)
+extern "C" int ternaspmm_w2_pays(int M, int N, int K) { return M <= w2_small_tokens(N) || M > 256 || K < 5120 || N > 32 * device_sm_count(); }
 
 __global__ void stream_fence_kernel() {}
 

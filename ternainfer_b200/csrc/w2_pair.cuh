@@ -405,7 +405,10 @@ __global__ void __launch_bounds__(kW2PairThreads, 1)
 
 // Tokens per tile for M tokens, RB row blocks, KS stages and `pairs` resident pairs: the shortest time of the busiest pair.
 // Fitted to launches of 20 and 54 stages at 160, 192 and 256 tokens: a tile takes KS * (200 + 0.47 NT) + 20 NT ns (stage
-// overheads, tensor cores, epilogue).
+// overheads, tensor cores, epilogue).  Measured since over 32 .. 256 tokens per tile (us per call, chosen / best): within 3 % for
+// 13824 x 2560 from 48 to 512 tokens, and for the narrower layers up to 64 and from 256 on (2560 x 2560 at 512 10.3 / 9.9 is the
+// widest); in between, one round of many small tiles is dearer than it says: 3840 x 2560 at 128 tokens 9.2 / 7.8
+// (30 tiles of 64 instead of 60 of 32), 2560 x 2560 at 192 9.2 / 7.9, 4096 x 4096 at 128 12.5 / 10.5.
 inline int w2_pair_tile(int M, int RB, int KS, int pairs) {
     int best = 32;
     double best_cost = 1e30;

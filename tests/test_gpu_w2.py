@@ -99,8 +99,8 @@ def make_layer(N, K, ws_num, seed, segments=None):
     return SpBitLinear(K, N, dic, "l"), dic
 
 
-@pytest.mark.parametrize("N,K", [(2560, 2560), (64, 64), (192, 6912), (128, 28672), (64, 8256)])
-@pytest.mark.parametrize("M", [1, 2, 3, 8, 20, 64, 70])
+@pytest.mark.parametrize("N,K", [(2560, 2560), (64, 64), (192, 6912), (128, 28672), (64, 8256), (64, 8128), (128, 8192)])
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 8, 20, 64, 70])
 @pytest.mark.parametrize("kind", ["plain", "norm", "gated"])
 def test_front_end_inside_the_linear(lib, M, N, K, kind):
     """bf16 activations: one kernel or two, always the values of the separate front-end followed by the linear."""
