@@ -34,9 +34,11 @@ constexpr int kHeadWarps = 16;
 constexpr int kHeadMaxCtas = 1024;              // scratch holds this many candidate slots
 constexpr int kHeadPrefetch = 1024;             // bytes of a row fetched into L2 ahead
 
-// Rows of a group: 8, whose finer steps leave a shorter tail (K = 2560: 128256 rows 108 -> 102 us, of 100 at the copy rate; 8000 rows
-// 17.8 -> 15.8), but 16 where every warp then has one group of 16 and would have one or two of 8 (32000 rows 33.4 -> 31,
-// 20000 23.4 -> 22.4; in groups of 8 33.6 and 27).  The sums of a row are the same either way.
+// Rows of a group: 8, whose finer steps leave a shorter tail, but 16 where every warp then has one group of 16 and would have one
+// or two of 8.  K = 2560, 3 tokens, us per call in a graph of calls on different embeddings, groups of 16 without the fetch
+// ahead / of 16 / of 8: 128256 rows 110.0 / 106.1 / 103.6 (100 at the copy rate), 64000 58.9 / 55.5 / 57.4, 32000 32.2 / 30.0 / 31.9, 20000
+// 23.0 / 22.0 / 27.0, 8000 17.7 / 17.3 / 15.3.  Called one after the other from the host the largest gains 1.6 % (106.2 -> 104.5 on one
+// card, 108.9 -> 108.4 on another).  The sums of a row are the same either way.
 inline int head_rows(int V, int ctas) {
     const int per_cta = ((V + 7) / 8 + ctas - 1) / ctas;
     return per_cta > kHeadWarps && per_cta <= 2 * kHeadWarps ? 16 : 8;
@@ -119,7 +121,7 @@ __global__ void __launch_bounds__(kHeadWarps * 32, 1) lm_head_kernel(const HeadP
 
     griddep_launch_dependents();
     if (tid == 0) next_group = g0;
-    // the warps' first groups into L2 while the hidden states arrive (1 to 3 us of these figures)
+    // the warps' first groups into L2 while the hidden states arrive (1 to 4 us of these figures)
     if (lane < R && g0 + warp < g1 && (g0 + warp) * R + lane < V)
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(__cvta_generic_to_global(p.emb + (size_t)((g0 + warp) * R + lane) * K)),
                      "r"(min(K * 2, kHeadPrefetch)) : "memory");

@@ -666,8 +666,8 @@ static cudaError_t launch_w2_small(W2Params& p, cudaStream_t stream) {
     const int per = (KP + kW2MaxWarps - 1) / kW2MaxWarps, W = std::max(4, (KP + per - 1) / per);
     p.pairs_q = KP / W, p.pairs_r = KP % W;
     // ring: all of the CTA's weights when they fit 64 KB (two launches' prefetches fit an SM side by side), otherwise two
-    // slots or more with copies of 4 KB (the copy engine takes about 60 cycles for each, whatever its size: 57344 x 8192
-    // at 4 tokens 43 us with copies of 1 KB, 35 with 2 KB, 32 with 3.5 KB)
+    // slots or more with copies of up to 4 KB (the copy engine takes about 60 cycles for each, whatever its size: 57344 x 8192
+    // at 4 tokens 70 us with copies of 0.5 KB, 41 with 1 KB, 32.5 with 2 or 3 KB, 37 with 2.5, which cuts a share of 3.5 unevenly)
     const int groups = (R + RG - 1) / RG, unit = W * RG * 512, room = kW2MaxSmem - w2_smem(R, MT, tokens, K, W, 0, 0, XS, FE, p.e.residual != nullptr).total;
     if (room < unit) return cudaErrorInvalidValue;
     p.chunk_pairs = per, p.slots = groups;

@@ -3,10 +3,13 @@
 Mirrors ``TernaInfer_linear`` / ``SpBitLinear`` / ``get_global_workspace`` of
 the reference's ``model.py`` (:37-133 in Gu-J/TernaInfer): same names, same
 argument meaning, same checkpoint keys.  Differences, all on this side of the
-C ABI: the activation quantiser runs as plain torch ops (no ``torch.compile``,
-hence no Triton); rows are not padded to a power of two because the B200
-library accepts any token count >= 1; the workspace is accepted and ignored
-(the library reduces its K split on chip).
+C ABI: the activation quantiser is a kernel of the library for bf16 activations
+on the GPU and torch operators otherwise (no ``torch.compile``, hence no
+Triton); rows are not padded to a power of two because the B200 library accepts
+any token count >= 1; K splits are reduced on chip, and the workspace serves
+``TernaInfer_linear`` at large token counts (the weight, decoded once per
+call); ``SpBitLinear`` goes through a native call site (host_call.cpp) that reads a
+two-bit copy of its weights, and needs neither in the calls that it takes.
 
 PyTorch is only plumbing here (device memory, the current stream); all
 arithmetic of the linear layer happens in ``libternaspmm.so``.  There is no

@@ -98,7 +98,7 @@ def ordered_norm_quant(x, w, eps, gated=False):
 def build_pair_same_glue(n_layers, vocab, seed=7, max_len=96):
     """(fused-glue model on this library's kernels, the SAME model in eager torch with every ternary
     linear on the exact reference formula and every norm in the fused kernels' stated
-    order).  Both use flash_attn's kv-cache kernel for the attention glue (library code)."""
+    order).  Both use this library's attention kernels (test_gpu_attn.py checks these)."""
     import types
     from ternainfer_b200.model import ModelArgs, Transformer, RMSNorm
     from ternainfer_b200.convert.convert_TernaInfer import random_checkpoint
@@ -216,7 +216,7 @@ def test_fused_norm_quant_bit_exact_against_its_stated_order(lib, gated, M, K):
 @torch.inference_mode()
 def test_fused_glue_model_logits_and_greedy_tokens_identical(lib):
     """The benchmarked decode path (fused norm/gate/quantiser kernels, residual add in the linear
-    epilogue, flash_attn glue) against the eager model on the reference formula with the same glue
+    epilogue, attention kernels on both sides) against the eager model on the reference formula with the same glue
     arithmetic: logits equal bit for bit on a prefill and a decode step, greedy tokens identical."""
     pytest.importorskip("flash_attn")
     from ternainfer_b200.generate import FastGen, GenArgs
@@ -295,8 +295,8 @@ def test_fused_glue_model_close_to_unfused(lib):
 
 @torch.inference_mode()
 def test_fused_glue_with_flash_attention_close_to_unfused(lib):
-    """Same check with the attention glue routed through flash_attn's kv-cache kernel
-    (RoPE + cache append + attention in one library launch), prefill then one decode step."""
+    """Same check with the attention kernels and their cache layout in the fused model (RoPE, cache append and
+    attention), torch's in the other, prefill then one decode step."""
     pytest.importorskip("flash_attn")
     from ternainfer_b200.model import ModelArgs, Transformer
     from ternainfer_b200.convert.convert_TernaInfer import random_checkpoint
