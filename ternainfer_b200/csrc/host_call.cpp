@@ -92,7 +92,8 @@ bool exclusive(PyObject* params) {
 bool lay_out(Layer* self, const Weights& w, cudaStream_t stream) {
     const int64_t N = self->out_features, K = self->in_features, tiles = N * K / 4096;
     if (N < 64 || K < 64 || N % 64 || K % 64 || K >= (1 << 18) || w.bitmap->nbytes() < (size_t)(N * K / 8) ||
-        w.tile_offsets->numel() < tiles + 1 || w.quarter_offsets->numel() < 3 * tiles || capturing(stream))
+        w.tile_offsets->numel() < tiles + 1 || w.quarter_offsets->numel() < 3 * tiles ||
+        (reinterpret_cast<uintptr_t>(w.bitmap->data_ptr()) & 15) || capturing(stream))
         return false;
     if (self->replaced) {              // (relaxed: another thread may be capturing)
         cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;

@@ -243,6 +243,20 @@ def test_layer_sees_writes_through_tensors_that_somebody_keeps(lib):
     assert torch.equal(layer(x), -y)
 
 
+def test_no_copy_of_tensors_that_cannot_be_laid_out(lib):
+    """A bitmap that does not start on 16 bytes, offsets of another size: no copy, instead of one that nothing has written."""
+    layer, _ = make_layer(128, 192, 2, 1)
+    whole = {k: v.clone() for k, v in layer.state_dict().items()}
+    bitmap, offsets, quarters = (whole["weight_" + n] for n in ("bitmap", "TileOffsets_global", "TileOffsets_median"))
+    for name, bad in (("weight_bitmap", lambda: torch.empty(bitmap.numel() + 1, dtype=torch.int64, device="cuda").view(torch.uint64)[1:]),
+                      ("weight_bitmap", lambda: bitmap[:-64].clone()), ("weight_TileOffsets_global", lambda: offsets[:-1].clone()),
+                      ("weight_TileOffsets_median", lambda: quarters[:-1].clone())):
+        setattr(layer, name, torch.nn.Parameter(bad(), requires_grad=False))
+        assert not layer._native.prepare(layer._parameters)
+        setattr(layer, name, torch.nn.Parameter(whole[name].clone(), requires_grad=False))
+        assert layer._native.prepare(layer._parameters)
+
+
 def test_graphs_follow_loaded_weights(lib):
     """A replay after load_state_dict and after relayout() computes with the new weights; a part of the tensors, as from
     one file of several, is not laid out."""
