@@ -136,20 +136,6 @@ void run_linear(Layer* self, const Weights& w, void* w2, void* x, int front_end,
                 int64_t M, void* residual, cudaStream_t stream) {
     auto* o = static_cast<ternaspmm_bf16*>(out.data_ptr());
     auto* scale = static_cast<ternaspmm_bf16*>(w.scale->data_ptr());
-    const bool segments = self->seg[0] | self->seg[1] | self->seg[2];
-    if (front_end == 0 && !(segments && residual) && !ternaspmm_w2_pays((int)M, self->out_features, self->in_features)) {
-        auto* bitmap = static_cast<uint64_t*>(w.bitmap->data_ptr());
-        auto* to = static_cast<int*>(w.tile_offsets->data_ptr());
-        auto* qo = static_cast<uint16_t*>(w.quarter_offsets->data_ptr());
-        auto* signs = static_cast<uint32_t*>(w.signs->data_ptr());
-        if (segments)
-            ternaspmm_linear_segments(static_cast<int8_t*>(x), bitmap, to, qo, signs, o, static_cast<ternaspmm_bf16*>(s), scale, self->ws_num,
-                                      (int)M, self->out_features, self->in_features, self->seg[0], self->seg[1], self->seg[2], -1, stream);
-        else
-            bitlinear_TernaSpMM_residual(static_cast<int8_t*>(x), bitmap, to, qo, signs, o, static_cast<ternaspmm_bf16*>(s), scale, self->ws_num,
-                                         (int)M, self->out_features, self->in_features, static_cast<ternaspmm_bf16*>(residual), stream);
-        return;
-    }
     ternaspmm_w2_linear(x, front_end, static_cast<ternaspmm_bf16*>(norm_w), eps, w2, o, static_cast<ternaspmm_bf16*>(s), scale, self->ws_num,
                         (int)M, self->out_features, self->in_features, self->seg[0], self->seg[1], self->seg[2], -1,
                         static_cast<ternaspmm_bf16*>(residual), stream);

@@ -635,12 +635,9 @@ extern "C" void ternaspmm_linear_segments(int8_t* x, uint64_t* bitmap, int* tile
 
 // ---- linears on two-bit weights (w2_small.cuh) -----------------------------------------------------
 constexpr int kW2MaxSmem = 227 * 1024;
-// Tokens up to which the mma.sync kernel runs (more: tcgen05 on CTA pairs).  Its second block of 32 tokens reads the weights again,
-// which pays while the pairs have few tiles, that is up to 32 rows per SM.  us per call in a stream of different weights,
-// mma.sync / pairs: 3840 x 2560 at 48 / 64 tokens 7.5 / 7.5, 7.9 / 7.7, 2560 x 2560 6.9 / 7.5, 7.0 / 7.6, 2560 x 6912 11.8 / 15.6, 12.1 / 15.6,
-// 4096 x 4096 9.1 / 10.3, 8.7 / 10.4; above that line 6400 x 6400 at 64 tokens 16.9 / 17.0, 13824 x 2560 17.2 / 10.6.  (At 32 tokens
-// the widest layers lose a little by it: 13824 x 2560 10.8 / 9.9, 14336 x 4096 15.5 / 13.4.)
-static int w2_small_tokens(int N) { return N <= 32 * device_sm_count() ? 64 : 32; }
+// Tokens up to which the mma.sync kernel runs.  us per call in a stream of different weights, mma.sync / tensor-memory tiles, at 8 / 12 / 16
+// tokens: 2560 x 2560 2.9 / 3.5, 3.5 / 3.3, 3.7 / 3.2, 13824 x 2560 5.0 / 5.2, 6.9 / 5.2, 6.9 / 5.2, 2560 x 6912 4.0 / 4.4, 5.4 / 4.4, 5.6 / 4.4.
+constexpr int kW2SmallTokens = 8;
 
 template <int MT, int RG, int U, int FE, bool XS>
 static cudaError_t launch_w2_small(W2Params& p, cudaStream_t stream) {
@@ -703,12 +700,46 @@ static cudaError_t launch_w2_fused(W2Params& p, cudaStream_t stream) {
 static cudaError_t launch_w2_int8(W2Params& p, cudaStream_t stream) {
     const int M = p.e.M;
     const bool xs = (long long)std::min(M, 32) * (p.e.K + 64) <= 120 * 1024;
-    if (M <= 8) return xs ? launch_w2_fused<W2_INT8>(p, stream) : launch_w2_small<1, 3, 1, W2_INT8, false>(p, stream);
-    if (M <= 16) return xs ? launch_w2_small<2, 2, 2, W2_INT8, true>(p, stream) : launch_w2_small<2, 2, 1, W2_INT8, false>(p, stream);
-    return xs ? launch_w2_small<4, 2, 1, W2_INT8, true>(p, stream) : launch_w2_small<4, 2, 1, W2_INT8, false>(p, stream);
+    return xs ? launch_w2_fused<W2_INT8>(p, stream) : launch_w2_small<1, 3, 1, W2_INT8, false>(p, stream);
 }
 
-static cudaError_t launch_w2_pair(const W2Params& p, cudaStream_t stream) {
+static cudaError_t launch_w2_tile(const W2Params& p, const W2TilePlan& plan, cudaStream_t stream) {
+    static bool attr_done[64] = {false};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) dev = 0;
+    auto kern = w2_tile_kernel;
+    if (!attr_done[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kW2MaxSmem / 2 - 1024);
+        if (e != cudaSuccess) return e;
+        attr_done[dev] = true;
+    }
+    const int M = p.e.M, tiles = (p.e.N + kTileRows - 1) / kTileRows, S = plan.splits, blocks = (M + plan.nt - 1) / plan.nt;
+    W2TileParams pp = {p.e, p.w, plan.nt, 0, 0};
+    pp.stages = std::min({kTileMaxStages, (kTileCols - pp.nt) / 64, 64 * 1024 / (pp.nt * 256)});
+    pp.slots = pp.nt > 64 ? 2 : kTileSlots;
+    const int smem = 1024 + W2TileSmem::ring + pp.slots * kTileSlotBytes + pp.stages * pp.nt * 256;
+    CUtensorMap map;
+    if (!encode_x_map(&map, p.e.x, M, p.e.K, pp.nt)) return cudaErrorInvalidValue;   // reported as status 3, nothing is launched
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(kTileThreads, 1, 1);
+    cfg.gridDim = dim3(S, tiles, blocks);
+    cfg.dynamicSmemBytes = std::max(smem, 80 * 1024);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = S;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = tuning().pdl ? 2 : 1;
+    t_echo = {9, pp.nt, S, kTileThreads / 32, 1, S * tiles * blocks};
+    return cudaLaunchKernelEx(&cfg, kern, pp, map);
+}
+
+static cudaError_t launch_w2_pair(const W2Params& p, int nt, cudaStream_t stream) {
     static bool attr_done[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -720,8 +751,8 @@ static cudaError_t launch_w2_pair(const W2Params& p, cudaStream_t stream) {
         attr_done[dev] = true;
     }
     const int pairs = device_sm_count() / 2, RB = (p.e.N + kPairRows - 1) / kPairRows;
-    W2PairParams pp = {p.e, p.w, w2_pair_tile(p.e.M, RB, w2_pairs(p.e.K), pairs), 0};
-    pp.stages = std::min(kW2PairMaxStages, W2PairSmem::stage_bytes / (kPairHalf + pp.nt * kLgKStep / 2));
+    W2PairParams pp = {p.e, p.w, nt, 0, 0, 0, 0};
+    w2_pair_plan(pp);
     CUtensorMap map;   // each CTA of a pair loads half of the tile's tokens per stage
     if (!encode_x_map(&map, p.e.x, p.e.M, p.e.K, pp.nt / 2)) return cudaErrorInvalidValue;   // reported as status 3, nothing is launched
     const long long tiles = (long long)RB * ((p.e.M + pp.nt - 1) / pp.nt);
@@ -743,12 +774,10 @@ static cudaError_t launch_w2_pair(const W2Params& p, cudaStream_t stream) {
     return cudaLaunchKernelEx(&cfg, kern, pp, map);
 }
 
-// Whether a call that has both forms of the weight in hand should take the two-bit one.  Deep and narrow layers beyond the mma.sync
-// kernel's reach fill few pairs, each with a long K loop, which the packed tcgen05 kernel splits over a cluster.  us per call,
-// two-bit / packed: 2560 x 6912 at 48 tokens 11.8 / 13.4, at 128 16.7 / 15.7, 256 17.3 / 17.9, 320 17.7 / 24.6; 4096 x 14336 21.3 / 23.3,
-// 32.9 / 25.3, 33.4 / 27.4, 34.0 / 41.4; above the line in rows 6400 x 6400 at 128 17.1 / 22.2, below the one in K
-// 4096 x 4096 12.5 / 14.7.  (Four row blocks stay behind at any size: 1024 x 16384 at 320 tokens 35.0 / 25.2.)
-extern "C" int ternaspmm_w2_pays(int M, int N, int K) { return M <= w2_small_tokens(N) || M > 256 || K < 5120 || N > 32 * device_sm_count(); }
+// Whether a call that has both forms of the weight in hand should take the two-bit one.  It always should, deep and narrow
+// layers included (us per call, two-bit / packed: 2560 x 6912 at 48 tokens 5.4 / 13.4, at 128 6.9 / 15.7, at 256 8.6 / 17.9, 1024 x 16384 at
+// 333 10.0 / 25.2).
+extern "C" int ternaspmm_w2_pays(int, int, int) { return 1; }
 
 __global__ void stream_fence_kernel() {}
 
@@ -813,8 +842,12 @@ extern "C" void ternaspmm_w2_linear(void* x, int front_end, __nv_bfloat16* norm_
     if (front_end == W2_PLAIN) e = launch_w2_fused<W2_PLAIN>(p, stream);
     else if (front_end == W2_NORM) e = launch_w2_fused<W2_NORM>(p, stream);
     else if (front_end == W2_GATED) e = launch_w2_fused<W2_GATED>(p, stream);
-    else if (M <= w2_small_tokens(N)) e = launch_w2_int8(p, stream);
-    else e = launch_w2_pair(p, stream);
+    else if (M <= kW2SmallTokens) e = launch_w2_int8(p, stream);
+    else {
+        const W2TilePlan tile = w2_tile_plan(M, N, K, device_sm_count());
+        const W2PairPlan pair = w2_pair_plan_tile(M, N, K, device_sm_count() / 2);
+        e = tile.us <= pair.us ? launch_w2_tile(p, tile, stream) : launch_w2_pair(p, pair.nt, stream);
+    }
     if (e != cudaSuccess) {
         fprintf(stderr, "ternaspmm: launch failed: %s\n", cudaGetErrorString(e));
         t_host_status = ST_LAUNCH;

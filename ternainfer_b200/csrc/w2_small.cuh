@@ -9,16 +9,14 @@
 // rewrites them as fixed-rate two-bit codes in the order of the int8 MMA's A
 // fragments, which decode with one AND and at most one shift per four weights.
 //
-// Layout.  Strips of 16 weight rows; inside a strip, pairs of 64-column blocks,
-// 512 bytes each: lane l = 4g + q owns the 16 bytes at l*16 = words (block 0:
-// MMA step 0, 1; block 1: step 0, 1).  Step s of a block covers the lane's columns
-// 16q + 8s .. + 7; byte e of the word holds four codes: bits 7:6 row g, column
-// 8s + e; bits 5:4 row g + 8, column 8s + e; bits 3:2 row g, column 8s + 4 + e; bits
-// 1:0 row g + 8, column 8s + 4 + e.  Code = the weight in two's complement.  Where K
-// is an odd multiple of 64 the second block of the last pair is zero.  A strip is
-// ceil(K / 128) * 512 contiguous bytes, so any range of block pairs of a strip is one bulk copy.  Masking a shifted word with 0xC0C0C0C0 leaves 64 * weight in
-// every signed byte, so the accumulators come out as 64 times the result and are
-// shifted back exactly (|acc| < 2^31 for K < 2^18).
+// Layout.  Strips of 16 weight rows; inside a strip, pairs of 64-column blocks, 512 bytes each: the 16 bytes at
+// w2_chunk(g, q) are four words, row g in block 0, row g in block 1, row g + 8 in block 0, row g + 8 in block 1.  A word
+// covers the columns 16q .. 16q + 15 of its block; byte e of it holds, from the top bits down, the codes of columns e, 4 + e, 8 + e and
+// 12 + e.  Code = the weight in two's complement.  Where K is an odd multiple of 64 the second block of the last pair is zero.  A
+// strip is ceil(K / 128) * 512 contiguous bytes, so any range of block pairs of a strip is one bulk copy.  Masking a shifted
+// word with 0xC0C0C0C0 leaves 64 * weight in every signed byte, four neighbouring columns of a row: the A operand of an int8 MMA,
+// as a lane of mma.sync holds it (lane 4g + q) and as a lane of tensor memory does (w2_tile.cuh: a lane per row).  The accumulators come
+// out as 64 times the result and are shifted back exactly (|acc| < 2^31 for K < 2^18).
 //
 // Work split.  A CTA owns R strips for a block of MT*8 tokens and all of K; its
 // warps split K.  Each warp streams its own part of the CTA's strips through its
@@ -62,6 +60,9 @@ struct W2Params {
 // gate + RMSNorm + quantiser.
 enum W2FrontEnd : int { W2_INT8 = 0, W2_PLAIN = 1, W2_NORM = 2, W2_GATED = 3 };
 
+// Byte offset of the chunk of rows g, g + 8 and columns 16q .. of both blocks.  The order of the chunks turns with the row, so that
+// sixteen lanes with a row each and the same q (w2_tile.cuh) meet no bank twice either.
+__device__ __forceinline__ int w2_chunk(int g, int q) { return g * 64 + ((q ^ (g >> 1)) << 4); }
 __host__ __device__ inline int w2_pairs(int K) { return (K + 127) >> 7; }
 
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
@@ -84,7 +85,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity)
     return false;
 }
 
-// Four weights per byte-sized code group -> the A fragments of one m16n8k32 step, 64 * weight per signed byte.
+// Sixteen columns of a row -> four words of four columns each, 64 * weight per signed byte.
 __device__ __forceinline__ void w2_decode(uint32_t w, uint32_t (&a)[4]) {
     a[0] = w & kW2Mask;
     a[1] = (w << 2) & kW2Mask;
@@ -110,14 +111,14 @@ __global__ void __launch_bounds__(256) relayout_w2_kernel(const SpmmParams p, ui
         pos += __popc(bm[r]);
 #pragma unroll
         for (int b = 0; b < 32; ++b) { // nibble b/4 = 4 * step + field, element b%4 = byte
-            if ((bm[r] >> b) & 1u) {
-                out[b >> 4] |= (1u | ((sgn & 1u) << 1)) << (8 * (b & 3) + 6 - 2 * ((b >> 2) & 3));
+            if ((bm[r] >> b) & 1u) {       // (fields of a step: row g, row g + 8, the same four columns on)
+                out[(b >> 2) & 1] |= (1u | ((sgn & 1u) << 1)) << (8 * (b & 3) + 6 - 2 * (2 * (b >> 4) + ((b >> 3) & 1)));
                 sgn >>= 1;
             }
         }
-        uint8_t* dst = w2 + (((size_t)rt * 4 + r) * KP + (kt >> 1)) * 512 + lane * 16 + (kt & 1) * 8;
-        *reinterpret_cast<uint2*>(dst) = make_uint2(out[0], out[1]);
-        if (kt == KT - 1 && (KT & 1)) *reinterpret_cast<uint2*>(dst + 8) = make_uint2(0u, 0u);
+        uint8_t* dst = w2 + (((size_t)rt * 4 + r) * KP + (kt >> 1)) * 512 + w2_chunk(lane >> 2, lane & 3) + (kt & 1) * 4;
+        reinterpret_cast<uint32_t*>(dst)[0] = out[0], reinterpret_cast<uint32_t*>(dst)[2] = out[1];
+        if (kt == KT - 1 && (KT & 1)) reinterpret_cast<uint32_t*>(dst)[1] = reinterpret_cast<uint32_t*>(dst)[3] = 0u;
     }
 }
 
@@ -293,7 +294,7 @@ __global__ void __launch_bounds__(kW2MaxWarps * 32, MT <= 2 ? 2 : 1) w2_small_ke
                     for (int c = 0; c < 4; ++c) acc[u][r][mt][c] = 0;
         for (int c0 = p0; c0 < p1; c0 += PC) {
             if (refilled) ok = ok && mbar_wait_bounded(bars + 8 * d, parity);
-            const uint32_t slot = ring + d * slot_bytes + lane * 16;
+            const uint32_t slot = ring + d * slot_bytes + w2_chunk(g, q);
             const int c1 = min(c0 + PC, p1);
 #pragma unroll 1
             for (int pr = c0; pr < c1; pr += U) {
@@ -320,13 +321,14 @@ __global__ void __launch_bounds__(kW2MaxWarps * 32, MT <= 2 ? 2 : 1) w2_small_ke
 #pragma unroll
                     for (int r = 0; r < RG; ++r)
 #pragma unroll
-                        for (int st = 0; st < 4; ++st) {
-                            uint32_t a[4];
-                            w2_decode(st == 0 ? w[u][r].x : st == 1 ? w[u][r].y : st == 2 ? w[u][r].z : w[u][r].w, a);
+                        for (int blk = 0; blk < 2; ++blk) {
+                            uint32_t a[4], b[4];              // rows g and g + 8
+                            w2_decode(blk ? w[u][r].y : w[u][r].x, a), w2_decode(blk ? w[u][r].w : w[u][r].z, b);
 #pragma unroll
                             for (int mt = 0; mt < MT; ++mt) {
-                                const uint4 xv = x[u][2 * mt + (st >> 1)];
-                                mma_s8_16x8x32(acc[u % AC][r][mt], a[0], a[1], a[2], a[3], (st & 1) ? xv.z : xv.x, (st & 1) ? xv.w : xv.y);
+                                const uint4 xv = x[u][2 * mt + blk];
+                                mma_s8_16x8x32(acc[u % AC][r][mt], a[0], b[0], a[1], b[1], xv.x, xv.y);
+                                mma_s8_16x8x32(acc[u % AC][r][mt], a[2], b[2], a[3], b[3], xv.z, xv.w);
                             }
                         }
             }

@@ -62,6 +62,42 @@ def test_pairs_with_several_tiles_and_ragged_edges(lib, M, N, K):
     check_linear(lib, M, N, K, 2)
 
 
+@pytest.mark.parametrize("M,N,K", [(9, 64, 64), (16, 128, 640), (33, 192, 1088), (64, 2560, 2560), (48, 2560, 6912), (80, 1024, 16384), (129, 1344, 1344),
+                                   (250, 2560, 2560), (190, 320, 8256), (256, 13824, 320), (1025, 128, 192)])
+def test_tiles_in_tensor_memory(lib, M, N, K):
+    """One to eight slices of K (uneven ones, half a last block pair), one to several blocks of tokens, 16 to 128 tokens per tile, half a last row tile."""
+    check_linear(lib, M, N, K, 3)
+
+
+@pytest.mark.parametrize("M,N,K", [(24, 320, 640), (70, 3840, 2560), (600, 320, 640)])
+def test_scales_out_of_the_usual_range_and_segments(lib, M, N, K):
+    """Scales that the epilogue's short division does not take (tiny, huge, zero) beside usual ones; one scale segment, and several inside a row tile."""
+    w = o.make_ternary(N, K, 0.45, N + K)
+    pk = Packed(w, [t.cpu().numpy() for t in compress_weight(torch.from_numpy(w).cuda())])
+    w2, stream = w2_of(lib, pk), torch.cuda.current_stream().cuda_stream
+    xq, s = o.make_activations(M, K, M + 1)
+    s = s.reshape(-1)
+    odd = s.copy()
+    odd[::5], odd[1::7], odd[2::11] = 1e-20, 3e15, 0.0
+    wb = o.f32_to_bf16_bits(o.make_ws(4, M + 2))
+    for scales in (s, odd):
+        for prefill in (0, 1):
+            for seg in ((N, N, N), (40, 104, 200)):
+                sb = o.f32_to_bf16_bits(scales)
+                out = torch.empty((M, N), dtype=torch.int16, device="cuda")
+                x_d, s_d, ws_d = dev(xq), dev(sb), dev(wb)
+                lib.ternaspmm_w2_linear(x_d.data_ptr(), 0, None, 0.0, w2.data_ptr(), out.data_ptr(), s_d.data_ptr(), ws_d.data_ptr(), 4, M, N, K,
+                                        *seg, prefill, None, stream)
+                want = torch.empty_like(out)
+                lib.ternaspmm_linear_segments(x_d.data_ptr(), pk.bm.data_ptr(), pk.tg.data_ptr(), pk.tm.data_ptr(), pk.cv.data_ptr(), want.data_ptr(),
+                                              s_d.data_ptr(), ws_d.data_ptr(), 4, M, N, K, *seg, prefill, stream)
+                torch.cuda.synchronize()
+                assert lib.ternaspmm_last_status() == 0
+                a, b = out.cpu().numpy().view(np.uint16), want.cpu().numpy().view(np.uint16)
+                nan = np.isnan(o.bf16_bits_to_f32(b))
+                assert (np.isnan(o.bf16_bits_to_f32(a)) == nan).all() and (a == b)[~nan].all()
+
+
 def test_layout_and_linear_on_one_stream(lib):
     """Two weights and two norm weights in turn through the same memory, layout and linear in stream order: never the other's values."""
     N, K = 13824, 2560
