@@ -425,7 +425,7 @@ inline W2PairPlan w2_pair_plan_tile(int M, int N, int K, int pairs) {
     for (int nt = 32; nt <= 256; nt += 32) {
         const long long tiles = (long long)RB * ((M + nt - 1) / nt);
         const double rounds = (double)((tiles + pairs - 1) / pairs);
-        const double us = 4.4 + 0.018 * nt + rounds * KS * std::max(0.15 + 0.00018 * nt, 0.00121 * nt) + (rounds - 1) * (nt > 192 ? 4.5 : 0.45);
+        const double us = 3.9 + 0.015 * nt + rounds * KS * std::max(0.15 + 0.00018 * nt, 0.00121 * nt) + (rounds - 1) * (nt > 192 ? 4.5 : 0.45);
         if (us < best.us) best = {nt, us};
     }
     return best;
