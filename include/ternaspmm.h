@@ -308,6 +308,12 @@ int ternaspmm_attn_decode(ternaspmm_bf16* qkv, ternaspmm_bf16* k_cache, ternaspm
                           ternaspmm_bf16* cos_row, ternaspmm_bf16* sin_row, long long* pos, ternaspmm_bf16* out,
                           int batch, int heads, int kv_heads, int head_dim, int max_len, ternaspmm_stream_t stream);
 
+/* The same on caches [batch][kv_heads][max_len][head_dim], with an fp32 rotation whose products are rounded one by one (as
+ * ternaspmm_rope does). */
+int ternaspmm_attn_decode_by_head(ternaspmm_bf16* qkv, ternaspmm_bf16* k_cache, ternaspmm_bf16* v_cache, float* cos_row,
+                                  float* sin_row, long long* pos, ternaspmm_bf16* out, int batch, int heads, int kv_heads,
+                                  int head_dim, int max_len, ternaspmm_stream_t stream);
+
 /* The same for `tokens` consecutive new tokens per sequence, causal, in two launches: qkv bf16 [batch][tokens][(heads +
  * 2 kv_heads) * head_dim], rotation tables bf16 [max_len][head_dim/2], first position *pos (rows 0 .. *pos - 1 hold
  * earlier tokens), out bf16 [batch][tokens][heads * head_dim].  head_dim 128, heads / kv_heads a multiple of 4. */

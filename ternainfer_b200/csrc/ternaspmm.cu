@@ -856,9 +856,9 @@ extern "C" void ternaspmm_w2_linear(void* x, int front_end, __nv_bfloat16* norm_
 }
 
 // ---- attention glue of a decode step (attn_decode.cuh) ---------------------------------------------
-template <int GQ>
+template <int GQ, bool BY_HEAD>
 static cudaError_t launch_attn_decode(const AttnParams& p, int batch, cudaStream_t stream) {
-    auto kern = attn_decode_kernel<GQ>;
+    auto kern = attn_decode_kernel<GQ, BY_HEAD>;
     // CTAs per key / value head: a power of two up to the portable cluster size, so that all are resident at once (three per SM)
     int S = 8;
     while (S > 1 && (long long)batch * p.kv_heads * S > 3ll * device_sm_count()) S >>= 1;
@@ -879,9 +879,10 @@ static cudaError_t launch_attn_decode(const AttnParams& p, int batch, cudaStream
     return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
-extern "C" int ternaspmm_attn_decode(__nv_bfloat16* qkv, __nv_bfloat16* k_cache, __nv_bfloat16* v_cache, __nv_bfloat16* cos_row,
-                                     __nv_bfloat16* sin_row, long long* pos, __nv_bfloat16* out, int batch, int heads, int kv_heads,
-                                     int head_dim, int max_len, cudaStream_t stream) {
+template <bool BY_HEAD>
+static int run_attn_decode(__nv_bfloat16* qkv, __nv_bfloat16* k_cache, __nv_bfloat16* v_cache, const void* cos_row, const void* sin_row,
+                           long long* pos, __nv_bfloat16* out, int batch, int heads, int kv_heads, int head_dim, int max_len,
+                           cudaStream_t stream) {
     t_host_status = ST_OK;
     const int gq = kv_heads > 0 && heads % kv_heads == 0 ? heads / kv_heads : 0;
     if (batch < 1 || batch > 65535 || kv_heads < 1 || kv_heads > 65535 || max_len < 1 || head_dim != kAttnD || (gq != 4 && gq != 8)) {
@@ -894,9 +895,22 @@ extern "C" int ternaspmm_attn_decode(__nv_bfloat16* qkv, __nv_bfloat16* k_cache,
         return t_host_status;
     }
     AttnParams p = {qkv, k_cache, v_cache, cos_row, sin_row, pos, out, heads, kv_heads, max_len, 1.4426950408889634f / sqrtf((float)head_dim)};
-    if ((gq == 4 ? launch_attn_decode<4>(p, batch, stream) : launch_attn_decode<8>(p, batch, stream)) != cudaSuccess) t_host_status = ST_LAUNCH;
+    if ((gq == 4 ? launch_attn_decode<4, BY_HEAD>(p, batch, stream) : launch_attn_decode<8, BY_HEAD>(p, batch, stream)) != cudaSuccess)
+        t_host_status = ST_LAUNCH;
     checkLastCudaError(__LINE__);
     return t_host_status;
+}
+
+extern "C" int ternaspmm_attn_decode(__nv_bfloat16* qkv, __nv_bfloat16* k_cache, __nv_bfloat16* v_cache, __nv_bfloat16* cos_row,
+                                     __nv_bfloat16* sin_row, long long* pos, __nv_bfloat16* out, int batch, int heads, int kv_heads,
+                                     int head_dim, int max_len, cudaStream_t stream) {
+    return run_attn_decode<false>(qkv, k_cache, v_cache, cos_row, sin_row, pos, out, batch, heads, kv_heads, head_dim, max_len, stream);
+}
+
+extern "C" int ternaspmm_attn_decode_by_head(__nv_bfloat16* qkv, __nv_bfloat16* k_cache, __nv_bfloat16* v_cache, float* cos_row, float* sin_row,
+                                             long long* pos, __nv_bfloat16* out, int batch, int heads, int kv_heads, int head_dim,
+                                             int max_len, cudaStream_t stream) {
+    return run_attn_decode<true>(qkv, k_cache, v_cache, cos_row, sin_row, pos, out, batch, heads, kv_heads, head_dim, max_len, stream);
 }
 
 extern "C" int ternaspmm_attn_prefill(__nv_bfloat16* qkv, __nv_bfloat16* k_cache, __nv_bfloat16* v_cache, __nv_bfloat16* cos_tab,

@@ -117,6 +117,8 @@ def load_library() -> ctypes.CDLL:
     lib.ternaspmm_w2_relayout.restype = None
     lib.ternaspmm_attn_decode.argtypes = [_P] * 7 + [_I] * 5 + [_P]
     lib.ternaspmm_attn_decode.restype = _I
+    lib.ternaspmm_attn_decode_by_head.argtypes = [_P] * 7 + [_I] * 5 + [_P]
+    lib.ternaspmm_attn_decode_by_head.restype = _I
     lib.ternaspmm_pack_gpu_layout.argtypes = [_P, _I, _I, _P, _P, _P, _P]
     lib.ternaspmm_pack_gpu_layout.restype = ctypes.c_longlong
     lib.ternaspmm_pack_gpu_signs.argtypes = [_P, _I, _I, _P, _P, _P]
@@ -171,6 +173,6 @@ EXPORTED_SYMBOLS = (
     "ternaspmm_list_plan", "ternaspmm_list_create", "ternaspmm_list_run", "ternaspmm_list_destroy",
     "ternaspmm_accumulate_i32", "ternaspmm_linear_segments", "bitlinear_TernaSpMM_residual", "bitlinear_TernaSpMM_ws", "ternaspmm_quant",
     "ternaspmm_scale_quant_sumsq", "ternaspmm_partial_f32", "ternaspmm_tp_finish", "ternaspmm_tp_allreduce_finish", "ternaspmm_rmsnorm_quant", "ternaspmm_relu2_gate_rmsnorm_quant", "ternaspmm_rmsnorm", "ternaspmm_pack_i8",
-    "ternaspmm_w2_relayout", "ternaspmm_rope", "ternaspmm_relu2_gate", "ternaspmm_bf16_to_f32", "ternaspmm_attn_decode", "ternaspmm_attn_prefill", "ternaspmm_pack_gpu_layout", "ternaspmm_pack_gpu_signs", "ternaspmm_w2_bytes", "ternaspmm_w2_pays", "ternaspmm_w2_fused_rows", "ternaspmm_w2_linear",
+    "ternaspmm_w2_relayout", "ternaspmm_rope", "ternaspmm_relu2_gate", "ternaspmm_bf16_to_f32", "ternaspmm_attn_decode", "ternaspmm_attn_decode_by_head", "ternaspmm_attn_prefill", "ternaspmm_pack_gpu_layout", "ternaspmm_pack_gpu_signs", "ternaspmm_w2_bytes", "ternaspmm_w2_pays", "ternaspmm_w2_fused_rows", "ternaspmm_w2_linear",
     "ternaspmm_unpack_i8", "ternaspmm_transcode_reference_layout",
 )

@@ -130,14 +130,15 @@ def rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor):
     """RoPE on adjacent pairs as one kernel: x bf16 [B, T, H, 128] (heads contiguous), cos / sin fp32 [B, T, 64] equal in
     every sequence (expanded).  None where the kernel does not take the tensors."""
     B, T, H, D = x.shape
+    ld = x.stride(1) if T > 1 else x.stride(0)           # (the stride of a dimension of one is anything)
     if not (x.is_cuda and x.device == cos.device == sin.device and x.dtype == torch.bfloat16 and cos.dtype == sin.dtype == torch.float32 and D == 128 and x.numel() > 0
-            and x.stride(3) == 1 and x.stride(2) == D and (B == 1 or x.stride(0) == T * x.stride(1)) and x.stride(1) % 8 == 0
+            and x.stride(3) == 1 and x.stride(2) == D and (B == 1 or x.stride(0) == T * ld) and ld % 8 == 0
             and x.data_ptr() % 16 == 0 and cos.shape[1:] == sin.shape[1:] == (T, 64) and (B == 1 or cos.stride(0) == sin.stride(0) == 0)
-            and cos.stride()[1:] == sin.stride()[1:] == (64, 1) and cos.data_ptr() % 16 == 0 and sin.data_ptr() % 16 == 0):
+            and (T == 1 or cos.stride(1) == sin.stride(1) == 64) and cos.stride(2) == sin.stride(2) == 1 and cos.data_ptr() % 16 == 0 and sin.data_ptr() % 16 == 0):
         return None
     out = torch.empty((B, T, H, D), dtype=torch.bfloat16, device=x.device)
     with _on(x):
-        load_library().ternaspmm_rope(x.data_ptr(), x.stride(1), cos.data_ptr(), sin.data_ptr(), out.data_ptr(), B, T, H, _stream())
+        load_library().ternaspmm_rope(x.data_ptr(), ld, cos.data_ptr(), sin.data_ptr(), out.data_ptr(), B, T, H, _stream())
     return out
 
 
@@ -187,6 +188,26 @@ def attn_decode(qkv, k_cache, v_cache, cos_row, sin_row, pos, heads: int, kv_hea
         status = load_library().ternaspmm_attn_decode(qkv.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), cos_row.data_ptr(),
                                                       sin_row.data_ptr(), pos.data_ptr(), out.data_ptr(), B, heads, kv_heads, D,
                                                       k_cache.shape[1], _stream())
+    return out if status == 0 else None
+
+
+def attn_decode_by_head(qkv, k_cache, v_cache, cos_row, sin_row, pos, heads: int, kv_heads: int):
+    """``attn_decode`` on caches [B, kv_heads, L, 128], rotation fp32 [64] of that position in the arithmetic of ``rope``: the
+    default glue's RoPE, ``index_copy_`` and masked attention of one new token per sequence.  Not under autograd."""
+    if not (qkv.is_cuda and qkv.device == k_cache.device == v_cache.device == cos_row.device == sin_row.device == pos.device
+            and qkv.dtype == k_cache.dtype == v_cache.dtype == torch.bfloat16 and cos_row.dtype == sin_row.dtype == torch.float32
+            and pos.dtype == torch.int64 and pos.numel() == 1 and qkv.dim() == 3 and qkv.shape[1] == 1 and k_cache.dim() == 4
+            and k_cache.shape == v_cache.shape and k_cache.shape[:2] == (qkv.shape[0], kv_heads) and k_cache.shape[3] == 128
+            and k_cache.numel() > 0 and heads in (4 * kv_heads, 8 * kv_heads) and qkv.shape[2] == (heads + 2 * kv_heads) * 128
+            and cos_row.numel() == sin_row.numel() == 64 and all(t.is_contiguous() for t in (qkv, k_cache, v_cache, cos_row, sin_row))
+            and not torch.is_grad_enabled()):
+        return None
+    B = qkv.shape[0]
+    out = torch.empty((B, 1, heads * 128), dtype=torch.bfloat16, device=qkv.device)
+    with _on(qkv):
+        status = load_library().ternaspmm_attn_decode_by_head(qkv.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), cos_row.data_ptr(),
+                                                              sin_row.data_ptr(), pos.data_ptr(), out.data_ptr(), B, heads, kv_heads, 128,
+                                                              k_cache.shape[2], _stream())
     return out if status == 0 else None
 
 

@@ -20,7 +20,7 @@ import torch
 from torch import nn
 from torch.nn import functional as F
 
-from .linear import SpBitLinear, attn_decode, attn_prefill, lm_head_argmax, quant_input, relu2_gate, rmsnorm, rope, to_float
+from .linear import SpBitLinear, attn_decode, attn_decode_by_head, attn_prefill, lm_head_argmax, quant_input, relu2_gate, rmsnorm, rope, to_float
 
 
 @dataclass
@@ -90,6 +90,15 @@ def apply_rope(x, cos, sin):
     return torch.stack((a * c - b * s, a * s + b * c), dim=-1).flatten(-2).to(x.dtype)
 
 
+CAUSAL = object()                # in place of a mask: every position up to that of the (one) new token
+
+
+def causal_mask(pos, length):
+    """[1, 1, T, L]: the cache positions that queries at ``pos`` attend to."""
+    keys = torch.arange(length, device=pos.device)
+    return (keys[None, :] <= pos[:, None])[None, None]
+
+
 class Attention(nn.Module):
     def __init__(self, args: ModelArgs, dic: dict, prefix: str, linear_cls, tp_group=None, tp: int = 1):
         super().__init__()
@@ -111,10 +120,16 @@ class Attention(nn.Module):
                 self.attn_sub_norm.weight.copy_(dic[prefix + ".attn_sub_norm.weight"])
 
     def forward(self, x, cache: LayerCache, pos, cos, sin, mask, fused=None):
-        """``fused`` = (norm weight, eps): the norm in front of wqkv runs in its front-end, x is wo's residual."""
+        """``fused`` = (norm weight, eps): the norm in front of wqkv runs in its front-end, x is wo's residual.  ``mask``: [1, 1,
+        T, L], or CAUSAL for one token per sequence, all at the same position (rotation, append and attention in one kernel)."""
         B, T = x.shape[0], x.shape[1]
         H, Hkv, D = self.n_heads, self.n_kv_heads, self.head_dim
         qkv = self.wqkv(x) if fused is None else self.wqkv.forward_normed(x, fused[0], fused[1])
+        if mask is CAUSAL:
+            o = attn_decode_by_head(qkv, cache[0], cache[1], cos[0, 0], sin[0, 0], pos, H, Hkv)
+            if o is not None:
+                return self._project(o, x, fused)
+            mask = causal_mask(pos, cache[0].shape[2])
         q = qkv[..., : H * D].view(B, T, H, D)
         k = qkv[..., H * D: (H + Hkv) * D].view(B, T, Hkv, D)
         v = qkv[..., (H + Hkv) * D:].view(B, T, Hkv, D)
@@ -288,8 +303,7 @@ class Transformer(nn.Module):
             flash = (pos, self._rope_lp, tuple(t.index_select(0, pos) for t in self._rope_lp) if T == 1 else None)
         else:
             cos, sin = self._rope[0][pos].expand(B, T, -1), self._rope[1][pos].expand(B, T, -1)
-            keys = torch.arange(self.max_seq_len, device=tokens.device)
-            mask = (keys[None, :] <= pos[:, None])[None, None]      # [1, 1, T, L] causal over cache positions
+            mask = CAUSAL if T == 1 else causal_mask(pos, self.max_seq_len)
         for layer, c in zip(self.layers, cache):
             h = layer(h, c, pos, cos, sin, mask, fused, flash)
         if greedy_last:

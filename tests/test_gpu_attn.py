@@ -36,6 +36,38 @@ def test_decode_attention(lib, B, pos, L, H, Hkv):
 
 
 @pytest.mark.parametrize("H,Hkv", [(20, 5), (64, 8)])
+@pytest.mark.parametrize("B,pos,L", [(1, 0, 8), (3, 7, 8), (2, 127, 640), (3, 333, 461), (8, 1100, 1101), (1, 2300, 2500), (70, 300, 320)])
+@torch.no_grad()
+def test_decode_attention_by_head(lib, B, pos, L, H, Hkv):
+    """On the default glue's caches: bytes appended as torch's rotation and index_copy_ leave them, result as close to float64 as torch's
+    masked attention (both round the probabilities to bf16 and the result once), rows without a token unread."""
+    from ternainfer_b200.linear import attn_decode_by_head
+    from ternainfer_b200.model import causal_mask
+    D = 128
+    g = torch.Generator(device="cuda").manual_seed(pos + B)
+    qkv = torch.randn((B, 1, (H + 2 * Hkv) * D), generator=g, device="cuda").to(torch.bfloat16)
+    kc, vc = (torch.randn((B, Hkv, L, D), generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    k0, v0 = kc.clone(), vc.clone()
+    kc[:, :, pos + 1:], vc[:, :, pos + 1:] = float("nan"), float("nan")
+    cos, sin = rope_tables(D, L, 500000.0, "cuda")
+    p = torch.tensor([pos], device="cuda")
+    out = attn_decode_by_head(qkv, kc, vc, cos[p], sin[p], p, H, Hkv)
+    q, k, v = (t.view(B, 1, -1, D) for t in qkv.split([H * D, Hkv * D, Hkv * D], -1))
+    with torch.enable_grad():                               # (torch's operators)
+        q, k = (apply_rope(t, cos[p].expand(B, 1, -1), sin[p].expand(B, 1, -1)).detach() for t in (q, k))
+    k0[:, :, pos], v0[:, :, pos] = k[:, 0], v[:, 0]
+    assert torch.equal(kc[:, :, :pos + 1], k0[:, :, :pos + 1]) and torch.equal(vc[:, :, :pos + 1], v0[:, :, :pos + 1])
+    assert kc[:, :, pos + 1:].isnan().all() and vc[:, :, pos + 1:].isnan().all()
+    kk, vv = (t[:, :, :pos + 1].double().repeat_interleave(H // Hkv, 1) for t in (k0, v0))
+    a = torch.softmax(torch.einsum("bhd,bhld->bhl", q[:, 0].double(), kk) / D ** 0.5, -1)
+    want = torch.einsum("bhl,bhld->bhd", a, vv).reshape(B, 1, H * D)
+    plain = torch.nn.functional.scaled_dot_product_attention(q.transpose(1, 2), k0, v0, attn_mask=causal_mask(p, L), enable_gqa=True)
+    err, theirs = (((t.double() - want).norm() / want.norm()).item() for t in (out, plain.transpose(1, 2).reshape(B, 1, H * D)))
+    print(f"error against float64 {err:.2e}, torch {theirs:.2e}")
+    assert err < max(1.05 * theirs, 2.1e-3)                 # (one rounding to bf16 is 1.7e-3 of normally distributed values)
+
+
+@pytest.mark.parametrize("H,Hkv", [(20, 5), (64, 8)])
 @pytest.mark.parametrize("B,T,past,L", [(1, 2, 0, 8), (2, 16, 0, 16), (1, 17, 0, 64), (3, 64, 0, 64), (1, 65, 1, 80), (2, 200, 63, 300), (1, 613, 0, 613),
                                         (1, 40, 1000, 1040), (1, 129, 0, 200), (2, 500, 37, 640)])
 def test_prompt_attention(lib, B, T, past, L, H, Hkv):
