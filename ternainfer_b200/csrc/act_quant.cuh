@@ -92,6 +92,19 @@ __device__ __forceinline__ uint32_t act_pack(float lo, float hi) {
     return r;
 }
 
+// acc / s rounded to nearest, for s with 8 significant bits (a bf16) in [2^-30, 2^30] and r = 1 / s rounded.  q0 is within two units
+// in the last place, the remainder is exact (fused, a few bits), and q0 + rem * r errs by 2^-22 units at most before it is rounded.
+// That decides the rounding: acc is a float, so a quotient that is not itself a float differs from the middle m of two floats by
+// |acc - s m| / s with acc and s m whole multiples of one unit of s m, at least 2^-10 units in the last place (and is
+// never such a middle: s m would have 25 significant bits).
+__device__ __forceinline__ float quotient(float acc, float s, float r) {
+    const float q0 = __fmul_rn(acc, r);
+    return __fmaf_rn(__fmaf_rn(-q0, s, acc), r, q0);
+}
+__device__ __forceinline__ float quotient_rcp(float s) {     // 0: out of range
+    return fabsf(s) >= 0x1p-30f && fabsf(s) <= 0x1p30f ? __fdiv_rn(1.0f, s) : 0.f;
+}
+
 // T of the fixed order
 __host__ __device__ inline int act_row_threads(int K) {
     const int t = ((K >> 3) + 31) & ~31;
@@ -201,6 +214,133 @@ __device__ __forceinline__ float act_row_finish(uint32_t row, uint32_t wrow, flo
         store(vt * 8, make_uint4(v.x, v.y, 0u, 0u));
     }
     return s;
+}
+
+// Up to R rows at a time by one CTA, VK vectors of each row per thread, all in registers: the front-end inside a linear's
+// kernel (w2_small.cuh), where every CTA does the same rows and the chain of latencies is all there is.  Every load is asked for
+// at once, the rows' butterflies run side by side, and with several rows their scalar parts (sum, square root, reciprocals)
+// go to a warp each.  `part`, `mxp`: R x 32 words, `rstd_s`: R words; `scl`: scale and its quotient_rcp per row, [0 .. R) and [32 .. ).
+template <bool GATED, int MODE, int VK, int R, typename Store>
+__device__ __forceinline__ void act_rows(const __nv_bfloat16* x, const __nv_bfloat16* w, float eps, int K, int rows, float* part, uint32_t* mxp,
+                                         float* rstd_s, float* scl, Store store) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = blockDim.x;
+    const int T = act_row_threads(K), vwarps = T >> 5;
+    const size_t ld = GATED ? 2 * (size_t)K : (size_t)K;
+    uint4 a[R * VK], b[GATED ? R * VK : 1], wv[VK];
+#pragma unroll
+    for (int i = 0; i < R * VK; ++i) {
+        const int r = i / VK, k0 = (tid + (i % VK) * n) * 8;
+        const bool in = k0 < K && r < rows;
+        a[i] = in ? ld_cg_128(x + r * ld + k0) : make_uint4(0, 0, 0, 0);
+        if (GATED) b[i] = in ? ld_cg_128(x + r * ld + K + k0) : make_uint4(0, 0, 0, 0);
+    }
+    if (MODE != ACT_PLAIN) {
+#pragma unroll
+        for (int j = 0; j < VK; ++j) wv[j] = (tid + j * n) * 8 < K ? ld_cg_128(w + (tid + j * n) * 8) : make_uint4(0, 0, 0, 0);
+    }
+    float rstd = 1.f;
+    if (MODE != ACT_PLAIN) {
+        float ss[R * VK];
+#pragma unroll
+        for (int i = 0; i < R * VK; ++i) {
+            uint32_t* av = reinterpret_cast<uint32_t*>(&a[i]);
+            if (GATED) {
+                const uint32_t* bv = reinterpret_cast<const uint32_t*>(&b[i]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {       // relu(x1) ** 2, bf16; * x3, bf16
+                    uint32_t r;
+                    asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(av[e]), "r"(0u));
+                    av[e] = act_mul2(act_mul2(r, r), bv[e]);
+                }
+            }
+            ss[i] = 0.f;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float lo = act_lo(av[e]), hi = act_hi(av[e]);
+                ss[i] = __fadd_rn(ss[i], __fmul_rn(lo, lo));
+                ss[i] = __fadd_rn(ss[i], __fmul_rn(hi, hi));
+            }
+        }
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1)
+#pragma unroll
+            for (int i = 0; i < R * VK; ++i) ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], d);
+#pragma unroll
+        for (int i = 0; i < R * VK; ++i) {
+            const int vw = warp + (i % VK) * (n >> 5);
+            if (lane == i && vw < vwarps) part[(i / VK) * 32 + vw] = ss[i];
+        }
+        __syncthreads();
+        if (R == 1 || warp < rows) {                   // (at least four warps: rows beyond them below)
+#pragma unroll 1
+            for (int r = R == 1 ? 0 : warp; r < (R == 1 ? 1 : rows); r += n >> 5) {
+                float4 p4[VK == 1 ? 3 : 8];
+#pragma unroll
+                for (int i = 0; i < (VK == 1 ? 3 : 8); ++i)
+                    if (4 * i < vwarps) p4[i] = *reinterpret_cast<const float4*>(part + r * 32 + 4 * i);
+                float sum = p4[0].x;
+#pragma unroll
+                for (int i = 0; i < (VK == 1 ? 3 : 8); ++i) {
+                    if (i > 0 && 4 * i < vwarps) sum += p4[i].x;
+                    if (4 * i + 1 < vwarps) sum += p4[i].y;
+                    if (4 * i + 2 < vwarps) sum += p4[i].z;
+                    if (4 * i + 3 < vwarps) sum += p4[i].w;
+                }
+                rstd = __frcp_rn(__fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)K), eps)));
+                if (R > 1 && lane == 0) rstd_s[r] = rstd;
+            }
+        }
+        if (R > 1) __syncthreads();
+    }
+    uint32_t mx[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        mx[r] = 0;
+        if (R > 1 && MODE != ACT_PLAIN) rstd = rstd_s[r];
+#pragma unroll
+        for (int j = 0; j < VK; ++j) {
+            uint32_t* av = reinterpret_cast<uint32_t*>(&a[r * VK + j]);
+            if (MODE != ACT_PLAIN) {
+                const uint32_t* wj = reinterpret_cast<const uint32_t*>(&wv[j]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    av[e] = act_pack(__fmul_rn(__fmul_rn(act_lo(av[e]), rstd), act_lo(wj[e])), __fmul_rn(__fmul_rn(act_hi(av[e]), rstd), act_hi(wj[e])));
+            }
+            // magnitudes: their bit patterns order like the values, NaN above all (of vectors beyond the row: zeros, or 0 * rstd)
+            if ((tid + j * n) * 8 < K) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) asm("max.u16x2 %0, %0, %1;" : "+r"(mx[r]) : "r"(av[e] & 0x7FFF7FFFu));
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const uint32_t m = warp_max_u32(max(mx[r] & 0xFFFFu, mx[r] >> 16));
+        if (lane == r) mxp[r * 32 + warp] = m;
+    }
+    __syncthreads();
+    float s = 0.f;
+    if (R == 1) {
+        s = act_scale(warp_max_u32(lane < (n >> 5) ? mxp[lane] : 0u));
+        if (tid == 0) scl[0] = s;
+        if (tid == 32) scl[32] = quotient_rcp(s);
+    } else {
+#pragma unroll 1
+        for (int r = warp; r < rows; r += n >> 5) {
+            s = act_scale(warp_max_u32(lane < (n >> 5) ? mxp[r * 32 + lane] : 0u));
+            if (lane == 0) scl[r] = s;
+            if (lane == 1) scl[32 + r] = quotient_rcp(s);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        if (R > 1) s = scl[min(r, rows - 1)];
+        const uint32_t s2 = (__float_as_uint(s) >> 16) * 0x10001u;
+#pragma unroll
+        for (int j = 0; j < VK; ++j)
+            if ((tid + j * n) * 8 < K && r < rows) store(r, (tid + j * n) * 8, act_quant8(a[r * VK + j], s2));
+    }
 }
 
 // Rows of at most 8192 elements: one CTA per row, T threads for few rows (a chain of latencies), T / 4 for many gated rows

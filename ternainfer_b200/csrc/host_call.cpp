@@ -176,12 +176,13 @@ PyObject* front_and_linear(Layer* self, PyObject* params, PyObject* xo, int fron
     void* w2 = two_bit(self, params, w, stream);
     if (!w2) Py_RETURN_NONE;
     at::Tensor out = output_like(x, self->out_features);
-    // The front-end inside the linear's kernel walks over its rows one after the other in every CTA, and takes shared memory from
-    // the ring; a launch of its own costs 1.1 us of the stream and as much of the host.  us per call, inside / separate: quantiser
-    // 2560 x 2560 at 1 / 3 / 4 / 8 rows 2.8 / 4.0, 4.0 / 4.2, 4.7 / 4.3, 7.0 / 4.3, 2560 x 6912 at 1 / 3 4.3 / 5.4, 6.3 / 5.9, 10240 x 8192 at
-    // 1 / 2 10.9 / 10.8, 12.8 / 11.8, 57344 x 8192 at 1 / 4 37.8 / 34.4, 38.9 / 36.0; norm 2560 x 2560 at 1 / 2 / 3 3.3 / 4.4, 4.4 / 4.6,
-    // 5.6 / 4.7, 2560 x 6912 at 1 / 2 (gated) 5.5 / 6.5, 7.9 / 6.8, 10240 x 8192 at 1 12.3 / 11.2.
-    if (M <= ternaspmm_w2_fused_rows((int)K) && K < 8192 && (front_end == 1 ? M * K <= 4 * 2560 : M == 1)) {
+    // The front-end inside the linear's kernel saves a launch of its own, 1.1 us of the stream and as much of the host; every CTA does
+    // it, up to four rows at once where a row is one vector per thread (K up to 2560), one after the other above that.  us per
+    // call, inside / separate: quantiser 2560 x 2560 at 1 / 4 / 8 rows 2.7 / 4.0, 3.2 / 4.3, 5.0 / 4.3, 2560 x 6912 at 1 / 3 4.0 / 5.4, 6.0 / 5.9,
+    // 10240 x 8192 at 1 / 2 8.9 / 10.8, 12.0 / 11.8, 57344 x 8192 at 1 / 4 37.8 / 34.4, 38.9 / 36.0; norm 2560 x 2560 at 1 3.1 / 4.4, 2560 x 6912 at
+    // 1 / 2 (gated) 5.1 / 6.5, 6.8 / 6.8, 10240 x 8192 at 1 12.3 / 11.2.  Norms of 2 to 4 rows gain alone (2560 x 2560 at 4 4.2 / 4.8), but a
+    // separate one overlaps the kernel before it: 30-layer model at batch 2 / 4 1043 / 1126 us a token, so 1009 / 1074.
+    if (M <= ternaspmm_w2_fused_rows((int)K) && K < 8192 && (M == 1 || (front_end == 1 && M <= 4 && K <= 2560))) {
         run_linear(self, w, w2, x.data_ptr(), front_end, norm_w, eps, out, nullptr, M, residual, stream);
         return THPVariable_Wrap(std::move(out));
     }

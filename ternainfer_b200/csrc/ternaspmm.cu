@@ -635,37 +635,38 @@ extern "C" void ternaspmm_linear_segments(int8_t* x, uint64_t* bitmap, int* tile
 
 // ---- linears on two-bit weights (w2_small.cuh) -----------------------------------------------------
 constexpr int kW2MaxSmem = 227 * 1024;
-// Tokens up to which the mma.sync kernel runs.  us per call in a stream of different weights, mma.sync / tensor-memory tiles, at 8 / 12 / 16
-// tokens: 2560 x 2560 2.9 / 3.5, 3.5 / 3.3, 3.7 / 3.2, 13824 x 2560 5.0 / 5.2, 6.9 / 5.2, 6.9 / 5.2, 2560 x 6912 4.0 / 4.4, 5.4 / 4.4, 5.6 / 4.4.
-constexpr int kW2SmallTokens = 8;
+// Whether the mma.sync kernel runs a call on int8 activations: up to 4 tokens, and activations that leave shared memory for a ring.  In
+// a stream of such calls alone the line would be 8 for narrow layers (us per call, mma.sync / tensor-memory tiles, at 4 / 8 / 12 tokens:
+// 2560 x 2560 2.6 / 3.3, 2.8 / 3.3, 3.5 / 3.3, 13824 x 2560 4.4 / 5.2, 5.2 / 5.2, 6.9 / 5.2, 8192 x 28672 14.7 / 15.5, 23.4 / 15.0), but between other
+// kernels the tiles' expansion is done when those end: 30-layer model at batch 8 1180 us a token, with tiles 1148.
+static bool w2_small_takes(int M, int K) { return M <= 4 && (long long)M * (K + 64) <= 120 * 1024; }
 
-template <int MT, int RG, int U, int FE, bool XS>
-static cudaError_t launch_w2_small(W2Params& p, cudaStream_t stream) {
+template <int MW, int RG, int FE, int VK, int VR>
+static cudaError_t launch_w2_strips(W2Params& p, cudaStream_t stream) {
     static bool attr_done[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) dev = 0;
-    auto kern = w2_small_kernel<MT, RG, U, FE, XS>;
+    auto kern = w2_small_kernel<MW, RG, FE, VK, VR>;
     if (!attr_done[dev]) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kW2MaxSmem);
         if (e != cudaSuccess) return e;
         attr_done[dev] = true;
     }
-    const int K = p.e.K, KP = w2_pairs(K);
-    const int blocks = (p.e.M + MT * 8 - 1) / (MT * 8), tokens = std::min(p.e.M, MT * 8);
+    const int K = p.e.K, KP = w2_pairs(K), tokens = p.e.M;
     // CTAs: one per SM (fewer when there are fewer strips), so that every SM gets the same share within a strip
     // (at most 40 strips each: the kernel's item index arithmetic)
-    const int strips = p.e.N / 16, ctas = std::min(strips, std::max({1, device_sm_count() / blocks, (strips + 39) / 40}));
+    const int strips = p.e.N / 16, ctas = std::min(strips, std::max(device_sm_count(), (strips + 39) / 40));
     const int R = (strips + ctas - 1) / ctas;
     p.strips_q = strips / ctas, p.strips_r = strips % ctas;
-    // warps: as many as have a block pair of their own, at most ten (two CTAs of that size share the register file, so
-    // the next launch's CTA starts beside this one), evenly loaded; at least four for the front-end and the epilogue
-    const int per = (KP + kW2MaxWarps - 1) / kW2MaxWarps, W = std::max(4, (KP + per - 1) / per);
+    const int W = w2_warps(K, MW);
     p.pairs_q = KP / W, p.pairs_r = KP % W;
+    const int per = (KP + W - 1) / W;
     // ring: all of the CTA's weights when they fit 64 KB (two launches' prefetches fit an SM side by side), otherwise two
     // slots or more with copies of up to 4 KB (the copy engine takes about 60 cycles for each, whatever its size: 57344 x 8192
     // at 4 tokens 70 us with copies of 0.5 KB, 41 with 1 KB, 32.5 with 2 or 3 KB, 37 with 2.5, which cuts a share of 3.5 unevenly)
-    const int groups = (R + RG - 1) / RG, unit = W * RG * 512, room = kW2MaxSmem - w2_smem(R, MT, tokens, K, W, 0, 0, XS, FE, p.e.residual != nullptr).total;
+    const bool res = p.e.residual != nullptr;
+    const int groups = (R + RG - 1) / RG, unit = W * RG * 512, room = kW2MaxSmem - w2_smem(R, tokens, K, W, 0, 0, res).total;
     if (room < unit) return cudaErrorInvalidValue;
     p.chunk_pairs = per, p.slots = groups;
     if (groups > kW2MaxSlots || groups * per * unit > std::min(64 * 1024, room)) {
@@ -673,10 +674,10 @@ static cudaError_t launch_w2_small(W2Params& p, cudaStream_t stream) {
         const int chunks = groups * ((per + p.chunk_pairs - 1) / p.chunk_pairs);
         p.slots = std::min(std::min(chunks, kW2MaxSlots), room / (p.chunk_pairs * unit));
     }
-    p.smem = w2_smem(R, MT, tokens, K, W, p.slots, RG * p.chunk_pairs * 512, XS, FE, p.e.residual != nullptr);
+    p.smem = w2_smem(R, tokens, K, W, p.slots, RG * p.chunk_pairs * 512, res);
     if (p.smem.total > kW2MaxSmem) return cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ctas, blocks, 1);
+    cfg.gridDim = dim3(ctas, 1, 1);
     cfg.blockDim = dim3(W * 32, 1, 1);
     cfg.dynamicSmemBytes = p.smem.total;
     cfg.stream = stream;
@@ -685,22 +686,32 @@ static cudaError_t launch_w2_small(W2Params& p, cudaStream_t stream) {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = tuning().pdl ? 1 : 0;
-    t_echo = {8, MT * 8, 1, W, R, (int)(cfg.gridDim.x * cfg.gridDim.y)};
+    t_echo = {8, 8, 1, W, R, (int)cfg.gridDim.x};
     return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
-// RG: strips whose accumulators a warp holds at a time; one where a CTA has one or two strips, and where three
-// strips' share of a long K would leave no room for a second ring slot (8192 x 28672 at 1 token 26.9 -> 20.7 us).  XS: activations in shared
-// memory while they leave room for the ring.
+// Strips at a time: one where a CTA has one or two, or up to six of a K that gives a warp more than two block pairs (w2_small.cuh has both
+// sides measured), and where three strips' share of a long K would leave no room for a second ring slot (8192 x 28672 at 1
+// token 26.9 -> 20.7 us).
+template <int FE, int VK, int VR>
+static cudaError_t launch_w2_small(W2Params& p, cudaStream_t stream) {
+    const int strips = p.e.N / 16, sms = device_sm_count(), K = p.e.K;
+    return strips <= 2 * sms || K > 8192 || (strips <= 6 * sms && w2_pairs(K) > 2 * w2_warps(K)) ? launch_w2_strips<kW2Warps, 1, FE, VK, VR>(p, stream) : launch_w2_strips<kW2Warps, 3, FE, VK, VR>(p, stream);
+}
+// Long launches need no place for the next one beside them: twice the warps, a strip at a time.  us per call at 4 tokens, ten / twenty warps:
+// 8192 x 8192 7.1 / 6.7, 8192 x 28672 16.0 / 14.7, 16384 x 16384 17.6 / 16.0, 57344 x 8192 32.3 / 31.9 (at 8 33.4 / 29.9); not 14336 x 8192 11.8 /
+// 12.4, 28672 x 8192 18.3 / 18.9, nor shorter K (13824 x 2560 4.4 / 6.7).
+static cudaError_t launch_w2_int8(W2Params& p, cudaStream_t stream) {
+    const int strips = p.e.N / 16, sms = device_sm_count(), K = p.e.K;
+    const bool longer = K > 8192 || (K > 7168 && (strips <= 4 * sms || strips > 16 * sms));
+    return longer ? launch_w2_strips<kW2MaxWarps, 1, W2_INT8, 1, 1>(p, stream) : launch_w2_small<W2_INT8, 1, 1>(p, stream);
+}
 template <int FE>
 static cudaError_t launch_w2_fused(W2Params& p, cudaStream_t stream) {
-    return p.e.N / 16 <= 2 * device_sm_count() || p.e.K > 8192 ? launch_w2_small<1, 1, 2, FE, true>(p, stream) : launch_w2_small<1, 3, 2, FE, true>(p, stream);
-}
-
-static cudaError_t launch_w2_int8(W2Params& p, cudaStream_t stream) {
-    const int M = p.e.M;
-    const bool xs = (long long)std::min(M, 32) * (p.e.K + 64) <= 120 * 1024;
-    return xs ? launch_w2_fused<W2_INT8>(p, stream) : launch_w2_small<1, 3, 1, W2_INT8, false>(p, stream);
+    // vectors of a row per thread, and rows at a time
+    const int vk = (act_row_threads(p.e.K) / 32 + w2_warps(p.e.K) - 1) / w2_warps(p.e.K), M = p.e.M;
+    if (vk > 1 || FE == W2_GATED) return vk > 3 ? launch_w2_small<FE, 4, 1>(p, stream) : launch_w2_small<FE, 3, 1>(p, stream);
+    return M == 1 ? launch_w2_small<FE, 1, 1>(p, stream) : launch_w2_small<FE, 1, 4>(p, stream);
 }
 
 static cudaError_t launch_w2_tile(const W2Params& p, const W2TilePlan& plan, cudaStream_t stream) {
@@ -807,8 +818,8 @@ extern "C" void ternaspmm_w2_relayout(uint64_t* bitmap, int* tile_offsets, uint1
     checkLastCudaError(__LINE__);
 }
 
-// Rows that a front-end inside the kernel takes: a thread holds at most two eight-element vectors of a row.
-extern "C" int ternaspmm_w2_fused_rows(int K) { return K < 64 || K > 8 * kActMaxThreads ? 0 : kW2MaxFusedRows; }
+// Rows that a front-end inside the kernel takes: a thread holds at most four eight-element vectors of a row.
+extern "C" int ternaspmm_w2_fused_rows(int K) { return K < 64 || K > 8 * kActMaxThreads ? 0 : kW2MaxRows; }
 
 extern "C" void ternaspmm_w2_linear(void* x, int front_end, __nv_bfloat16* norm_weight, float eps, void* w2, __nv_bfloat16* out,
                                     __nv_bfloat16* s, __nv_bfloat16* ws, int ws_num, int M, int N, int K, int seg1, int seg2,
@@ -842,7 +853,7 @@ extern "C" void ternaspmm_w2_linear(void* x, int front_end, __nv_bfloat16* norm_
     if (front_end == W2_PLAIN) e = launch_w2_fused<W2_PLAIN>(p, stream);
     else if (front_end == W2_NORM) e = launch_w2_fused<W2_NORM>(p, stream);
     else if (front_end == W2_GATED) e = launch_w2_fused<W2_GATED>(p, stream);
-    else if (M <= kW2SmallTokens) e = launch_w2_int8(p, stream);
+    else if (w2_small_takes(M, K)) e = launch_w2_int8(p, stream);
     else {
         const W2TilePlan tile = w2_tile_plan(M, N, K, device_sm_count());
         const W2PairPlan pair = w2_pair_plan_tile(M, N, K, device_sm_count() / 2);

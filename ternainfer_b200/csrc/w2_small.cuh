@@ -1,13 +1,13 @@
-// Ternary linears on weights laid out once in two bits, for sm_100a: up to a few
-// dozen tokens per pass, with the activation front-end (RMSNorm, gate, int8
-// quantiser) optionally inside the kernel.
+// Ternary linears on weights laid out once in two bits, for sm_100a: up to eight
+// tokens (more: w2_tile.cuh, w2_pair.cuh), with the activation front-end (RMSNorm,
+// gate, int8 quantiser) optionally inside the kernel.
 //
 // The packed checkpoint format (bitmap + sign stream) costs about 0.12 warp
 // instructions per weight to decode, and that, not HBM, is what bounds the
 // kernels that read it (spmm_small_m.cuh, spmm_list.cuh).  A module that keeps its
 // weights for the life of a model can pay for that once: relayout_w2_kernel
-// rewrites them as fixed-rate two-bit codes in the order of the int8 MMA's A
-// fragments, which decode with one AND and at most one shift per four weights.
+// rewrites them as fixed-rate two-bit codes, which decode with one AND and at most one
+// shift per four weights.
 //
 // Layout.  Strips of 16 weight rows; inside a strip, pairs of 64-column blocks, 512 bytes each: the 16 bytes at
 // w2_chunk(g, q) are four words, row g in block 0, row g in block 1, row g + 8 in block 0, row g + 8 in block 1.  A word
@@ -18,7 +18,7 @@
 // as a lane of mma.sync holds it (lane 4g + q) and as a lane of tensor memory does (w2_tile.cuh: a lane per row).  The accumulators come
 // out as 64 times the result and are shifted back exactly (|acc| < 2^31 for K < 2^18).
 //
-// Work split.  A CTA owns R strips for a block of MT*8 tokens and all of K; its
+// Work split.  A CTA owns R strips and all of K; its
 // warps split K.  Each warp streams its own part of the CTA's strips through its
 // own ring of shared-memory slots by cp.async.bulk, so the weights of BitNet-2B-sized
 // layers (10 - 60 KB per SM) are on chip before the programmatic-dependency wait
@@ -27,21 +27,29 @@
 // After the wait a call is one chain of latencies: read the activations, norm and quantise
 // them, MMAs, one reduction over the warps, store.  Hence the front-end in the kernel
 // for the smallest calls: every CTA repeats it (a few microseconds of one row's
-// arithmetic would cost more as a launch of its own than as redundant work).
+// arithmetic would cost more as a launch of its own than as redundant work).  At one token the
+// chain of 3840 x 2560 is 5000 cycles: activations 460, norm and quantiser 2000, MMAs 1800, reduction and epilogue 750.  Partial
+// sums go to a set per warp instead of shared atomics and quotients need no division where the scale allows it (us per call, before
+// and now: 3840 x 2560 with the norm 3.5 / 3.3, 2560 x 6912 gated 5.5 / 5.1, quantiser and 4 rows 4.7 / 3.2, 8192 x 8192 at 4 rows 7.8 / 6.7).
+// Measured and no better: the expansion without shifts into unsigned fields, a dry run of the code ahead of the dependency wait,
+// twenty warps for K = 2560.
 #pragma once
 #include <cuda_bf16.h>
+
+#include <algorithm>
 
 #include "act_quant.cuh"
 #include "spmm_small_m.cuh"
 
 namespace tsp {
 
-constexpr int kW2MaxWarps = 10;
+constexpr int kW2Warps = 10, kW2MaxWarps = 20;   // of a CTA that shares its SM with the next launch's, and of one that does not
 constexpr uint32_t kW2Mask = 0xC0C0C0C0u;
 
 struct W2Smem {   // shared-memory plan: byte offsets from the base of the dynamic segment
-    int red, xq, row, res, ring, total;
+    int red, xq, res, ring, total;
     int red_stride, x_stride;
+    int red_sets;     // partial sums: a set per warp, or one that the warps add to
 };
 
 struct W2Params {
@@ -55,6 +63,14 @@ struct W2Params {
     int slots, chunk_pairs;           // ring slots per warp, block pairs per slot
     W2Smem smem;
 };
+
+// Warps of a CTA: as many as have a block pair of their own, at most ten (two CTAs of that size share the register file, so the
+// next launch's CTA starts beside this one), evenly loaded; at least four for the front-end and the epilogue.  Up to twenty where a
+// launch is long.
+inline int w2_warps(int K, int most = kW2Warps) {
+    const int KP = (K + 127) >> 7, per = (KP + most - 1) / most;
+    return std::max(4, (KP + per - 1) / per);
+}
 
 // Front-end inside the kernel: none (int8 activations and scales given), the plain quantiser, RMSNorm + quantiser,
 // gate + RMSNorm + quantiser.
@@ -123,25 +139,23 @@ __global__ void __launch_bounds__(256) relayout_w2_kernel(const SpmmParams p, ui
 }
 
 constexpr int kW2MaxSlots = 8;                       // ring slots per warp
-constexpr int kW2MaxFusedRows = 8;                   // rows a front-end inside the kernel takes
-constexpr int kW2Scale = kW2MaxWarps * kW2MaxSlots * 8;           // float s[32], ws[4] behind the mbarriers
-constexpr int kW2Partial = kW2Scale + 48 * 4;                     // two sets (even and odd rows) of 32 partial sums, 32 maxima
-constexpr int kW2ScratchBytes = kW2Partial + 2 * 64 * 4;
+constexpr int kW2MaxRows = 8;                        // tokens per call of this kernel (the columns of an MMA)
+constexpr int kW2Scale = kW2MaxWarps * kW2MaxSlots * 8;           // behind the mbarriers: float s[32], quotient_rcp(s)[32], ws[4]
+constexpr int kW2Partial = kW2Scale + 80 * 4;                     // of the front-ends: 8 x 32 partial sums, 8 x 32 maxima, 8 factors
+constexpr int kW2ScratchBytes = kW2Partial + (2 * kW2MaxRows * 32 + kW2MaxRows) * 4;
 
-// R strips per CTA at most, `tokens` rows of x handled by a CTA (at most MT*8), W warps, ring slots of `slot_bytes`
-inline W2Smem w2_smem(int R, int mt, int tokens, int K, int W, int slots, int slot_bytes, bool x_in_smem, int front_end,
-                      bool residual) {
+// R strips per CTA at most, `tokens` rows of x, W warps, ring slots of `slot_bytes`
+inline W2Smem w2_smem(int R, int tokens, int K, int W, int slots, int slot_bytes, bool residual) {
     W2Smem s;
     s.red_stride = R * 16 + 4;                       // conflict-free: token stride = 4 mod 16 words
     s.x_stride = (K & 127) ? K : K + 64;             // two tokens' 64-byte pieces on different banks
-    int at = kW2ScratchBytes;
+    s.red_sets = W * tokens * s.red_stride * 4 <= 16 * 1024 ? W : 1;
+    int at = (kW2ScratchBytes + 127) & ~127;
     s.red = at;
-    at += mt * 8 * s.red_stride * 4;
+    at += s.red_sets * tokens * s.red_stride * 4;
     at = (at + 127) & ~127;
     s.xq = at;
-    if (x_in_smem) at += ((tokens * s.x_stride + 64 + 127) & ~127);   // (a half pair reads 64 bytes past its row)
-    s.row = at;                                      // a front-end's row (gated: both halves) and norm weight
-    if (front_end != W2_INT8) at += ((K * (front_end == W2_GATED ? 6 : 4) + 127) & ~127);
+    at += ((tokens * s.x_stride + 64 + 127) & ~127);   // (a half pair reads 64 bytes past its row)
     s.res = at;                                      // residual of the CTA's outputs, bf16 [tokens][R * 16]
     if (residual) at += ((tokens * R * 32 + 127) & ~127);
     s.ring = at;
@@ -150,28 +164,37 @@ inline W2Smem w2_smem(int R, int mt, int tokens, int K, int W, int slots, int sl
     return s;
 }
 
-// XS: the CTA's int8 activations sit in shared memory (always with a front-end); otherwise fragments come straight from L2.
-// Block pairs are taken U at a time, all their shared-memory loads first.  No branches inside: a group's absent strips and
-// an absent second pair are computed from whatever the ring holds and from zeros, and not stored.
-template <int MT, int RG, int U, int FE, bool XS>
-__global__ void __launch_bounds__(kW2MaxWarps * 32, MT <= 2 ? 2 : 1) w2_small_kernel(const __grid_constant__ W2Params p) {
-    static_assert(XS || FE == W2_INT8, "a front-end writes to shared memory");
-    static_assert(XS || U == 1, "fragments from L2 are prefetched one pair ahead instead");
+// Four MMAs of a block pair of a strip: rows g, g + 8 of the strip by the tokens.
+__device__ __forceinline__ void w2_mma_pair(int (&acc0)[4], int (&acc1)[4], const uint4& w, const uint4& x0, const uint4& x1) {
+    uint32_t a[4], c[4];
+    w2_decode(w.x, a), w2_decode(w.z, c);
+    mma_s8_16x8x32(acc0, a[0], c[0], a[1], c[1], x0.x, x0.y);
+    mma_s8_16x8x32(acc0, a[2], c[2], a[3], c[3], x0.z, x0.w);
+    w2_decode(w.y, a), w2_decode(w.w, c);
+    mma_s8_16x8x32(acc1, a[0], c[0], a[1], c[1], x1.x, x1.y);
+    mma_s8_16x8x32(acc1, a[2], c[2], a[3], c[3], x1.z, x1.w);
+}
+
+// MW: warps at most.  RG: strips at a time, three where a CTA has that many and a long enough ring for them.  VK, VR: vectors of a row per thread and rows at a
+// time in the front-end.
+template <int MW, int RG, int FE, int VK, int VR>
+__global__ void __launch_bounds__(MW * 32, MW > kW2Warps ? 1 : 2) w2_small_kernel(const __grid_constant__ W2Params p) {
     extern __shared__ __align__(128) uint8_t smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthreads = blockDim.x;
     const int g = lane >> 2, q = lane & 3;
     const int K = p.e.K, N = p.e.N, D = p.slots;
-    const int m0 = blockIdx.y * (MT * 8), mrows = min(p.e.M - m0, MT * 8);
+    const int mrows = p.e.M;
     const int b = blockIdx.x, strip0 = b * p.strips_q + min(b, p.strips_r), nstrips = p.strips_q + (b < p.strips_r);
     const int KP = w2_pairs(K), PC = p.chunk_pairs;           // block pairs of K, at most PC per ring slot
     const int p0 = warp * p.pairs_q + min(warp, p.pairs_r), p1 = p0 + p.pairs_q + (warp < p.pairs_r);
     const int slot_bytes = RG * PC * 512;
+    const int NG = (nstrips + RG - 1) / RG;                   // groups of RG strips
     const W2Smem& L = p.smem;
     const uint32_t base = smem_u32(smem);
     int* red = reinterpret_cast<int*>(smem + L.red);
     float* scl = reinterpret_cast<float*>(smem + kW2Scale);
     const uint32_t bars = base + warp * (kW2MaxSlots * 8), ring = base + L.ring + warp * D * slot_bytes;
-    const int NG = (nstrips + RG - 1) / RG;                   // groups of RG strips
+    const int red_stride = L.red_stride, red_sets = L.red_sets;
 
     phase_mark(0);
     griddep_launch_dependents();
@@ -194,9 +217,10 @@ __global__ void __launch_bounds__(kW2MaxWarps * 32, MT <= 2 ? 2 : 1) w2_small_ke
         mbar_fence_init();
         for (int i = 0; i < D && f_gi < NG; ++i) fetch();
     }
-    for (int i = tid; i < MT * 8 * L.red_stride; i += nthreads) red[i] = 0;
+    if (red_sets == 1 || p0 >= p1)                            // (a warp without a share of K leaves zeros)
+        for (int i = red_sets == 1 ? tid : lane; i < mrows * red_stride; i += red_sets == 1 ? nthreads : 32)
+            red[(red_sets == 1 ? 0 : warp * mrows * red_stride) + i] = 0;
     constexpr bool kGated = FE == W2_GATED;
-    const uint32_t row = base + L.row, wrow = row + K * (kGated ? 4 : 2);
     if ((FE == W2_NORM || FE == W2_GATED) && tid == 64 && b == 0) act_weight_ahead(p.norm_w, K);
     const int pairs = nstrips * 8, items = mrows * pairs;     // epilogue items: two columns of a token each
     const uint32_t inv_pairs = ((1u << 22) + pairs - 1) / pairs;   // i / pairs = i * inv >> 22 (i * pairs < 2^22)
@@ -211,68 +235,41 @@ __global__ void __launch_bounds__(kW2MaxWarps * 32, MT <= 2 ? 2 : 1) w2_small_ke
     griddep_wait();
     phase_mark(2);
     // ---- activations, scales, residual: everything is asked for before anything is waited for
-    if (XS && FE == W2_INT8) {                                // this warp's columns of the rows, 16 bytes a piece
+    if (FE == W2_INT8) {                                // this warp's columns of the rows, 16 bytes a piece
         const int pieces = (min(p1 * 128, K) - p0 * 128) >> 4;
         for (int t = lane >> 4; t < mrows; t += 2)
             for (int i = lane & 15; i < pieces; i += 16)
-                cp_async_16(base + L.xq + t * L.x_stride + p0 * 128 + i * 16, p.e.x + (size_t)(m0 + t) * K + p0 * 128 + i * 16);
-    }
-    if (FE != W2_INT8) {
-        const __nv_bfloat16* xr = p.xb + (size_t)m0 * (kGated ? 2 * K : K);
-        act_row_copy(row, xr, K);
-        if (kGated) act_row_copy(row + K * 2, xr + K, K);
-        cp_async_commit();
-        if (FE != W2_PLAIN) act_row_copy(wrow, p.norm_w, K);
+                cp_async_16(base + L.xq + t * L.x_stride + p0 * 128 + i * 16, p.e.x + (size_t)t * K + p0 * 128 + i * 16);
     }
     if (res_smem) {
 #pragma unroll 1
         for (int i = tid; i < mrows * nstrips * 2; i += nthreads) {   // 16 bytes a piece
             const int t = (int)((uint32_t)(i * 4) * inv_pairs >> 22), c = i * 4 - t * pairs;
-            cp_async_16(base + L.res + (t * pairs + c) * 4, p.e.residual + (size_t)(m0 + t) * N + strip0 * 16 + c * 2);
+            cp_async_16(base + L.res + (t * pairs + c) * 4, p.e.residual + (size_t)t * N + strip0 * 16 + c * 2);
         }
     }
     cp_async_commit();
-    if (FE == W2_INT8 && tid < mrows) scl[tid] = __bfloat162float(p.e.s[m0 + tid]);
-    if (tid >= 32 && tid < 36) scl[tid] = __bfloat162float(p.e.ws[tid - 32]);
-    uint4 xn[2 * MT];                                         // direct fragments of the next pair
-    auto load_x = [&](int pr, uint4* x) {                     // (columns of absent tokens are not stored)
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-            if (XS) {
-                const uint32_t src = base + L.xq + min(mt * 8 + g, mrows - 1) * L.x_stride + pr * 128 + q * 16;
-                x[2 * mt] = lds128(src);
-                x[2 * mt + 1] = lds128(src + 64);
-            } else {
-                const int8_t* src = p.e.x + (size_t)(m0 + min(mt * 8 + g, mrows - 1)) * K + pr * 128 + q * 16;
-                x[2 * mt] = ld_cg_128(src);
-                x[2 * mt + 1] = ld_cg_128(src + (pr * 128 + 64 < K ? 64 : 0));   // (a half pair's second block has zero weights)
-            }
-        }
-    };
+    if (FE == W2_INT8 && tid < mrows) {
+        const float s = __bfloat162float(p.e.s[tid]);
+        scl[tid] = s, scl[32 + tid] = quotient_rcp(s);
+    }
+    if (tid >= 32 && tid < 36) scl[32 + tid] = __bfloat162float(p.e.ws[tid - 32]);
+    const uint32_t x_lane = base + L.xq + min(g, mrows - 1) * L.x_stride + q * 16;   // (columns of absent tokens are not stored)
     if (FE == W2_INT8) {
-        if (!XS && p0 < p1) load_x(p0, xn);
-        __syncthreads();                                      // red is zeroed, scales are staged
-        if (XS) {
-            cp_async_wait_all();                              // (the residual too)
-            __syncwarp();
-        }
+        cp_async_wait_all();                                  // (the residual too)
+        __syncwarp();                                         // (a warp reads the columns that it copied)
+        if (red_sets == 1) __syncthreads();                   // red is zeroed
     } else {
         constexpr int kMode = FE == W2_PLAIN ? ACT_PLAIN : ACT_RMSNORM;
-        const int T = min(kActMaxThreads, max(64, ((K >> 3) + 31) & ~31));   // the fixed order of act_quant.cuh
+        float* part = reinterpret_cast<float*>(smem + kW2Partial);
+        uint32_t* mxp = reinterpret_cast<uint32_t*>(part + kW2MaxRows * 32);
+        float* rstd = reinterpret_cast<float*>(mxp + kW2MaxRows * 32);
 #pragma unroll 1
-        for (int t = 0; t < mrows; ++t) {
-            float* part = reinterpret_cast<float*>(smem + kW2Partial) + (t & 1) * 64;
+        for (int t = 0; t < mrows; t += VR) {
             const uint32_t xrow = base + L.xq + t * L.x_stride;
-            if (t > 0) {                                      // (a thread's own vectors: the previous row's have been used)
-                const __nv_bfloat16* xr = p.xb + (size_t)(m0 + t) * (kGated ? 2 * K : K);
-                act_row_copy(row, xr, K);
-                if (kGated) act_row_copy(row + K * 2, xr + K, K);
-                cp_async_commit();
-                cp_async_commit();                            // (no norm weight behind it)
-            }
-            const float s = act_row_finish<kGated, kMode>(row, wrow, p.eps, K, T, part, reinterpret_cast<uint32_t*>(part + 32), nullptr,
-                                                          [&](int k0, const uint4& v) { sts64(xrow + k0, v.x, v.y); });
-            if (tid == 0) scl[t] = s;
+            act_rows<kGated, kMode, VK, VR>(p.xb + (size_t)t * (kGated ? 2 * K : K), p.norm_w, p.eps, K, min(VR, mrows - t), part,
+                                            mxp + (VR == 1 ? (t & 1) * 32 : 0), rstd, scl + t,
+                                            [&](int r, int k0, const uint2& v) { sts64(xrow + r * L.x_stride + k0, v.x, v.y); });
         }
         __syncthreads();
     }
@@ -281,78 +278,103 @@ __global__ void __launch_bounds__(kW2MaxWarps * 32, MT <= 2 ? 2 : 1) w2_small_ke
     int d = 0;
     uint32_t parity = 0;
     bool refilled = false;                                    // the slots of the first round have been waited for
-    for (int gi = 0; gi < NG && p0 < p1; ++gi) {
-        constexpr int AC = RG * MT < 3 ? U : 1;               // separate accumulators per pair where there are few chains
-        int acc[AC][RG][MT][4];
+    int* dst = red + (red_sets == 1 ? 0 : warp * mrows * red_stride) + 2 * q * red_stride + g;
+    const bool t0_ok = 2 * q < mrows, t1_ok = 2 * q + 1 < mrows;
+    const uint32_t w_lane = ring + w2_chunk(g, q);
+    auto put = [&](const int (&a)[4], const int (&b)[4]) {    // (rows of absent tokens are not stored)
 #pragma unroll
-        for (int u = 0; u < AC; ++u)
-#pragma unroll
-            for (int r = 0; r < RG; ++r)
-#pragma unroll
-                for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) acc[u][r][mt][c] = 0;
-        for (int c0 = p0; c0 < p1; c0 += PC) {
-            if (refilled) ok = ok && mbar_wait_bounded(bars + 8 * d, parity);
-            const uint32_t slot = ring + d * slot_bytes + w2_chunk(g, q);
-            const int c1 = min(c0 + PC, p1);
-#pragma unroll 1
-            for (int pr = c0; pr < c1; pr += U) {
-                uint4 x[U][2 * MT], w[U][RG];
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int pu = u == 0 ? pr : min(pr + u, c1 - 1);
-                    if (XS) {
-                        load_x(pu, x[u]);
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 2 * MT; ++i) x[u][i] = xn[i];
-                        if (p1 - p0 > 1) load_x(pr + 1 < p1 ? pr + 1 : p0, xn);
-                    }
-#pragma unroll
-                    for (int r = 0; r < RG; ++r) w[u][r] = lds128(slot + (pu - c0) * 512 + r * PC * 512);
-                    if (u > 0 && pr + u >= c1) {              // no second pair: zero activations
-#pragma unroll
-                        for (int i = 0; i < 2 * MT; ++i) x[u][i] = make_uint4(0, 0, 0, 0);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-#pragma unroll
-                    for (int r = 0; r < RG; ++r)
-#pragma unroll
-                        for (int blk = 0; blk < 2; ++blk) {
-                            uint32_t a[4], b[4];              // rows g and g + 8
-                            w2_decode(blk ? w[u][r].y : w[u][r].x, a), w2_decode(blk ? w[u][r].w : w[u][r].z, b);
-#pragma unroll
-                            for (int mt = 0; mt < MT; ++mt) {
-                                const uint4 xv = x[u][2 * mt + blk];
-                                mma_s8_16x8x32(acc[u % AC][r][mt], a[0], b[0], a[1], b[1], xv.x, xv.y);
-                                mma_s8_16x8x32(acc[u % AC][r][mt], a[2], b[2], a[3], b[3], xv.z, xv.w);
-                            }
-                        }
+        for (int c = 0; c < 4; ++c) {
+            int* at = dst + (c & 1) * red_stride + 8 * (c >> 1);
+            if ((c & 1) ? t1_ok : t0_ok) {
+                if (red_sets == 1) atomicAdd(at, a[c] + b[c]);
+                else *at = a[c] + b[c];
             }
-            __syncwarp();
-            if (lane == 0 && f_gi < NG) fetch();              // into the slot just read
-            if (++d == D) d = 0, parity ^= 1u, refilled = true;
         }
+        dst += 16;
+    };
+    auto next_slot = [&]() {                                  // after the last read of a slot: refill it, go on to the next
+        __syncwarp();
+        if (lane == 0 && f_gi < NG) fetch();
+        if (++d == D) d = 0, parity ^= 1u, refilled = true;
+    };
+    const uint4 none = make_uint4(0, 0, 0, 0);
+    // What a turn of a loop costs is its warps' chains and, the first time, its fetch (some 35 cycles for eight instructions).  So
+    // few strips are done one at a time - at once where a warp's share of K is one or two block pairs, whose activations stay in
+    // registers, else a block pair per turn (the next one's operands asked for ahead of it: 3 to 8 % slower) - and more strips
+    // three at a time, two block pairs per turn.  (us per call, three / one at a time: 2560 x 2560 with the norm 3.3 / 3.1, 8192 x 8192 at 4
+    // tokens 7.8 / 7.2, 10240 x 8192 at 8 9.3 / 8.5, 13824 x 2560 at 8 tokens 5.3 / 5.7, 57344 x 8192 at 4 32.6 / 34.2.)
+    if (RG == 1 && p1 - p0 <= 2 && p1 - p0 <= PC && p0 < p1) {
+        const bool two = p1 - p0 == 2;
+        const uint4 x0 = lds128(x_lane + p0 * 128), x1 = lds128(x_lane + p0 * 128 + 64);
+        const uint4 x2 = two ? lds128(x_lane + p0 * 128 + 128) : none, x3 = two ? lds128(x_lane + p0 * 128 + 192) : none;
+        const uint32_t second = two ? 512 : 0;
+        uint4 w0 = lds128(w_lane), w1 = lds128(w_lane + second);
+#pragma unroll 1
+        for (int st = 0; st < nstrips; ++st) {
+            next_slot();
+            if (refilled && st + 1 < nstrips) ok = ok && mbar_wait_bounded(bars + 8 * d, parity);
+            const uint4 n0 = lds128(w_lane + d * slot_bytes), n1 = lds128(w_lane + d * slot_bytes + second);
+            int acc[4][4] = {};
+            w2_mma_pair(acc[0], acc[1], w0, x0, x1);
+            w2_mma_pair(acc[2], acc[3], w1, x2, x3);
 #pragma unroll
-        for (int r = 0; r < RG; ++r) {
-            const int strip = gi * RG + r;
-            if (strip >= nstrips) break;
-            int* dst = red + strip * 16 + g + 2 * q * L.red_stride;
+            for (int c = 0; c < 4; ++c) acc[0][c] += acc[2][c], acc[1][c] += acc[3][c];
+            put(acc[0], acc[1]);
+            w0 = n0, w1 = n1;
+        }
+    } else if (RG == 1) {
+#pragma unroll 1
+        for (int st = 0; st < nstrips && p0 < p1; ++st) {
+            int acc[2][4] = {};
+#pragma unroll 1
+            for (int c0 = p0; c0 < p1; c0 += PC) {
+                if (refilled) ok = ok && mbar_wait_bounded(bars + 8 * d, parity);
+                uint32_t slot = w_lane + d * slot_bytes, xa = x_lane + c0 * 128;
+                const uint32_t end = xa + min(PC, p1 - c0) * 128;
+#pragma unroll 1
+                for (; xa < end; slot += 512, xa += 128) w2_mma_pair(acc[0], acc[1], lds128(slot), lds128(xa), lds128(xa + 64));
+                next_slot();
+            }
+            put(acc[0], acc[1]);
+        }
+    } else {
+        // (a group's absent strips are computed from whatever the ring holds, an absent second pair from zeros, and neither is stored)
+#pragma unroll 1
+        for (int gi = 0; gi < NG && p0 < p1; ++gi) {
+            int acc[RG][4] = {};
+#pragma unroll 1
+            for (int c0 = p0; c0 < p1; c0 += PC) {
+                if (refilled) ok = ok && mbar_wait_bounded(bars + 8 * d, parity);
+                const uint32_t slot = w_lane + d * slot_bytes;
+                const int c1 = min(c0 + PC, p1);
+#pragma unroll 1
+                for (int pr = c0; pr < c1; pr += 2) {
+                    uint4 x[2][2], w[2][RG];
 #pragma unroll
-            for (int mt = 0; mt < MT; ++mt)
+                    for (int u = 0; u < 2; ++u) {
+                        const int pu = u == 0 ? pr : min(pr + 1, c1 - 1);
+                        x[u][0] = lds128(x_lane + pu * 128), x[u][1] = lds128(x_lane + pu * 128 + 64);
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    int v = acc[0][r][mt][c];
-                    if (AC > 1) v += acc[AC - 1][r][mt][c];
-                    if (mt * 8 + 2 * q + (c & 1) < mrows) atomicAdd(dst + (mt * 8 + (c & 1)) * L.red_stride + 8 * (c >> 1), v);
+                        for (int r = 0; r < RG; ++r) w[u][r] = lds128(slot + (pu - c0) * 512 + r * PC * 512);
+                        if (u > 0 && pr + 1 >= c1) x[u][0] = x[u][1] = none;
+                    }
+#pragma unroll
+                    for (int u = 0; u < 2; ++u)
+#pragma unroll
+                        for (int r = 0; r < RG; ++r) w2_mma_pair(acc[r], acc[r], w[u][r], x[u][0], x[u][1]);
                 }
+                next_slot();
+            }
+            const int nothing[4] = {};
+#pragma unroll
+            for (int r = 0; r < RG; ++r) {
+                if (gi * RG + r >= nstrips) break;
+                put(acc[r], nothing);
+            }
         }
     }
     if (!ok) atomicExch(p.e.status, ST_WAIT_TIMEOUT);
-    if (FE == W2_INT8 && !XS) cp_async_wait_all();            // the residual
+    cp_async_wait_all();                                      // the residual
     phase_mark(5);
     __syncthreads();
     phase_mark(6);
@@ -361,10 +383,23 @@ __global__ void __launch_bounds__(kW2MaxWarps * 32, MT <= 2 ? 2 : 1) w2_small_ke
 #pragma unroll 1
     for (int i = tid; i < items; i += nthreads) {
         const int t = (int)((uint32_t)i * inv_pairs >> 22), c = (i - t * pairs) * 2, n = strip0 * 16 + c;
-        const int v[2] = {red[t * L.red_stride + c] >> 6, red[t * L.red_stride + c + 1] >> 6};
-        const size_t o = (size_t)(m0 + t) * N + n;
-        __nv_bfloat16 r[2] = {scale_epilogue(v[0], scl[t], scl[32 + ws_group(n, p.e)], p.e.epilogue),
-                              scale_epilogue(v[1], scl[t], scl[32 + ws_group(n + 1, p.e)], p.e.epilogue)};
+        const int* src = red + t * red_stride + c;
+        int2 v = make_int2(0, 0);
+#pragma unroll 5
+        for (int k = 0; k < red_sets; ++k) {
+            const int2 o = *reinterpret_cast<const int2*>(src + k * mrows * red_stride);
+            v.x += o.x, v.y += o.y;
+        }
+        v.x >>= 6, v.y >>= 6;
+        const size_t o = (size_t)t * N + n;
+        const float s = scl[t], rc = scl[32 + t], ws0 = scl[64 + ws_group(n, p.e)], ws1 = scl[64 + ws_group(n + 1, p.e)];
+        __nv_bfloat16 r[2];
+        if (p.e.epilogue == EPI_DECODE && rc != 0.f) {
+            r[0] = __float2bfloat16_rn(__fmul_rn(quotient(__int2float_rn(v.x), s, rc), ws0));
+            r[1] = __float2bfloat16_rn(__fmul_rn(quotient(__int2float_rn(v.y), s, rc), ws1));
+        } else {
+            r[0] = scale_epilogue(v.x, s, ws0, p.e.epilogue), r[1] = scale_epilogue(v.y, s, ws1, p.e.epilogue);
+        }
         if (res_smem) {
             const uint32_t rv = lds32(base + L.res + i * 4);
             r[0] = __float2bfloat16_rn(act_lo(rv) + __bfloat162float(r[0])), r[1] = __float2bfloat16_rn(act_hi(rv) + __bfloat162float(r[1]));

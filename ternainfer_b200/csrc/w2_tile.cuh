@@ -59,16 +59,7 @@ struct W2TileParams {
     int nt, stages, slots;                 // tokens per tile, ring slots, slots of codes
 };
 
-// acc / s rounded to nearest, for s with 8 significant bits (a bf16) in [2^-30, 2^30] and r = 1 / s rounded.  q0 is within two units
-// in the last place, the remainder is exact (fused, a few bits), and q0 + rem * r errs by 2^-22 units at most before it is rounded.
-// That decides the rounding: acc is a float, so a quotient that is not itself a float differs from the middle m of two floats by
-// |acc - s m| / s with acc and s m whole multiples of one unit of s m, at least 2^-10 units in the last place (and is
-// never such a middle: s m would have 25 significant bits).
-__device__ __forceinline__ float quotient(float acc, float s, float r) {
-    const float q0 = __fmul_rn(acc, r);
-    return __fmaf_rn(__fmaf_rn(-q0, s, acc), r, q0);
-}
-// the same for two quotients, in packed instructions; the products with a factor each
+// Pairs of fp32 values in packed instructions; quotient() of two.
 __device__ __forceinline__ unsigned long long f32x2(float x, float y) {
     unsigned long long r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
@@ -92,10 +83,6 @@ __device__ __forceinline__ float2 quotient2(float2 acc, float2 s, float2 r) {
     const float2 q0 = f32x2_mul(acc, r);
     return f32x2_fma(f32x2_fma(make_float2(-q0.x, -q0.y), s, acc), r, q0);
 }
-__device__ __forceinline__ float quotient_rcp(float s) {     // 0: out of range
-    return fabsf(s) >= 0x1p-30f && fabsf(s) <= 0x1p30f ? __fdiv_rn(1.0f, s) : 0.f;
-}
-
 // D[tmem] (+)= A[tmem] * B[smem]; M = 128
 __device__ __forceinline__ void umma_i8_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
