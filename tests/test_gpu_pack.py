@@ -19,6 +19,21 @@ def test_gpu_packer_equals_host_packer(lib, N, K, p_zero):
         assert np.array_equal(got.cpu().numpy(), want.numpy())
 
 
+def test_gpu_packer_in_two_steps_without_scratch(lib):
+    """The entry points that extract the signs at their places: the same arrays."""
+    N, K = 192, 4160
+    w = torch.from_numpy(o.make_ternary(N, K, 0.45, 5)).cuda()
+    cv, tg, tm, bm = compress_weight(w)
+    a, b, c = torch.empty_like(bm), torch.empty_like(tg), torch.empty_like(tm)
+    stream = torch.cuda.current_stream().cuda_stream
+    words = lib.ternaspmm_pack_gpu_layout(w.data_ptr(), N, K, a.data_ptr(), b.data_ptr(), c.data_ptr(), stream)
+    assert words + 4 == cv.numel()
+    d = torch.empty_like(cv)
+    lib.ternaspmm_pack_gpu_signs(w.data_ptr(), N, K, b.data_ptr(), d.data_ptr(), stream)
+    for x, y in ((a, bm), (b, tg), (c, tm), (d, cv)):
+        assert torch.equal(x.view(torch.int8), y.view(torch.int8))
+
+
 def test_gpu_packer_takes_views(lib):
     w = torch.from_numpy(o.make_ternary(129, 128, 0.45, 3)).cuda()
     a, b = compress_weight(w[1:]), compress_weight(w.t().contiguous().t()[1:])
