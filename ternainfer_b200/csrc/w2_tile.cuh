@@ -490,10 +490,10 @@ __global__ void __launch_bounds__(kTileThreads, 2)
 }
 
 // Tokens per tile and K slices of a call, and the time it takes, in us.  The CTAs of up to 256 (two to an SM; clusters leave some
-// places empty) run at once, each KB = K / 128 / S block pairs long, 0.15 us each, 0.22 with two CTAs on an SM's tensor cores; a
+// places empty) run at once, each KB = K / 128 / S block pairs long, 0.15 us each, 0.2 with two CTAs on an SM's tensor cores; a
 // cluster's exchange grows with S.  Measured, us per call in a stream of
 // different weights, S = 1 / 2 / 4 / 6 / 8: 2560 x 2560 at 48 tokens 5.2 / 4.4 / 4.1 / 4.4 / 5.4, 2560 x 6912 at 16 tokens 9.5 / 6.2 / 5.0 / 4.5 /
-// 4.6, 1024 x 16384 at 16 19.5 / 11.1 / 7.1 / 6.1 / 5.3, 8192 x 8192 at 16 11.2 / 8.6 / 7.0 / 10.6 / 11.8 (384 CTAs with six slices).  Tiles of more
+// 4.6, 1024 x 16384 at 16 19.5 / 11.1 / 7.1 / 6.1 / 5.3, 8192 x 8192 at 16 11.2 / 8.6 / 7.0 / 10.6 / 11.8 (384 CTAs with six slices), 13824 x 2560 at 48 6.7 / 6.0 / 10.2.  Tiles of more
 // than 64 tokens have room for two stages only (0.30 to 0.34 us per block pair) and pay where they save a round
 // of CTAs: 13824 x 2560 at 256 tokens 11.3, in tiles of 64 13.9.
 struct W2TilePlan { int nt, splits; double us; };
@@ -506,10 +506,10 @@ inline W2TilePlan w2_tile_plan(int M, int N, int K, int sms) {
         for (int S = 1; S <= (nt > 64 ? 1 : std::min(8, KP)); ++S) {
             const long long ctas = (long long)tiles * blocks * S, at_once = sms * 2 - sms / 4;
             const long long rounds = (ctas + at_once - 1) / at_once, last = ctas - (rounds - 1) * at_once;
-            const double KB = (KP + S - 1) / S, alone = nt > 64 ? 0.30 : 0.152, two = nt > 64 ? 0.34 : 0.225;
+            const double KB = (KP + S - 1) / S, alone = nt > 64 ? 0.30 : 0.152, two = nt > 64 ? 0.34 : 0.205;
             if (rounds > 1 && S > 1) break;                  // (a second round of clusters waits for whole ones to end)
             const double us = 1.3 + (nt > 64 ? 0.03 : 0.018) * nt + KB * ((rounds - 1) * two + (last > sms ? two : alone)) + (rounds - 1) * 2.0 +
-                              (S > 1 ? 0.3 * S : 0.0) + (ctas > sms ? 0.4 : 0.0);
+                              (S > 1 ? 0.3 * S : 0.0) + (ctas > sms ? 0.1 : 0.0);
             if (us < best.us) best = {nt, S, us};
         }
     }
