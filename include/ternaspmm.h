@@ -153,7 +153,8 @@ double ternaspmm_debug_int8_mma_rate(int iters, ternaspmm_stream_t stream);
  * kernel, thin CTAs; 3 = tcgen05 kernel; 4 = output head; 5 = work list; 6 = tcgen05 kernel
  * on dense weights from the workspace, single CTAs; 7 = tcgen05 kernel on CTA pairs (dense
  * weights from the workspace, or two-bit weights expanded on chip); 8 = small-batch kernel
- * on two-bit weights: splits = 1, row tiles = strips of 16 rows per CTA), tokens per pass, K split (cluster
+ * on two-bit weights: splits = 1, row tiles = strips of 16 rows per CTA; 9 = tcgen05 kernel on
+ * two-bit weights, single CTAs of 128 rows), tokens per pass, K split (cluster
  * size), warps per CTA, 64-row tiles per CTA, CTAs}. */
 void ternaspmm_last_launch_shape(int* out6);
 
@@ -293,7 +294,7 @@ void ternaspmm_w2_relayout(uint64_t* bitmap, int* tile_offsets, uint16_t* quarte
                            int N, int K, void* w2, ternaspmm_stream_t stream);
 long long ternaspmm_w2_bytes(int N, int K);
 int ternaspmm_w2_fused_rows(int K);
-int ternaspmm_w2_pays(int M, int N, int K); /* 0: the packed entry points are faster for this call */
+int ternaspmm_w2_pays(int M, int N, int K); /* 0: the packed entry points are faster for this call (they never are any more) */
 void ternaspmm_w2_linear(void* x, int front_end, ternaspmm_bf16* norm_weight, float eps, void* w2, ternaspmm_bf16* out,
                          ternaspmm_bf16* s, ternaspmm_bf16* ws, int ws_num, int M, int N, int K, int seg1, int seg2,
                          int seg3, int prefill_form, ternaspmm_bf16* residual, ternaspmm_stream_t stream);
