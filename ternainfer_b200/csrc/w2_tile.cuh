@@ -207,7 +207,7 @@ __device__ __noinline__ void tile_store_general(const SpmmParams& p, float ws_el
     for (int j = 0; j < n_tokens; ++j) {
         const long long o = at + (long long)j * p.N;
         if (live) stg_b16(reinterpret_cast<__nv_bfloat16*>(p.out) + o,
-                          __bfloat16_as_ushort(add_residual(scale_epilogue(v[j] >> 6, scl[j] * 0.015625f, ws_el, p.epilogue), p.residual, o)));
+                          __bfloat16_as_ushort(add_residual(scale_epilogue(v[j] >> 6, scl[j], ws_el, p.epilogue), p.residual, o)));
     }
 }
 template <int U>
@@ -222,13 +222,14 @@ __device__ __forceinline__ void tile_store(const SpmmParams& p, const TileOut& o
         return;
     }
     uint32_t f[U][4];                                        // tokens 2j, 2j + 1, rounded
-    const float2 ws2 = make_float2(o.ws_el, o.ws_el);
+    // The accumulators are 64 times the sums.  The quotient comes out 64 times too large and the weight scale takes that back: exact, as
+    // a quotient is below 2^61 here and a bf16 divided by 64 is a float (a scale times 64 may not be: from 2^122 on it is infinite).
+    const float2 ws2 = make_float2(o.ws_el * 0.015625f, o.ws_el * 0.015625f);
 #pragma unroll
     for (int u = 0; u < U; ++u)
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             const float4 aux = *reinterpret_cast<const float4*>(scl + kTileMaxTokens + 8 * u + 4 * j);
-            // 64 times the sums, as the scales are
             float2 a = make_float2(__int2float_rn(v[u][4 * j]), __int2float_rn(v[u][4 * j + 1]));
             float2 b = make_float2(__int2float_rn(v[u][4 * j + 2]), __int2float_rn(v[u][4 * j + 3]));
             if (o.form == FORM_FACTOR) {
@@ -334,15 +335,15 @@ __global__ void __launch_bounds__(kTileThreads, 2)
             const float ws0 = __bfloat162float(p.ws[ws_group(n0, p)]);
             bool in_range = true;
             for (int t = lane; t < NT; t += 32) {
-                // times 64 and 1 / 64, for sums that are 64 times theirs: exact in the range that tile_store takes
                 const float sv = t < cols ? __bfloat162float(p.s[t0 + t]) : 1.f;
                 float aux = quotient_rcp(sv);
                 if (p.epilogue == EPI_PREFILL) {
                     aux = sv != 0.f ? __fdiv_rn(ws0, sv) : 0.f;
-                    if (!(fabsf(aux) >= 0x1p-60f && fabsf(aux) <= 0x1p60f)) aux = 0.f;
+                    // over 64, for sums that are 64 times theirs: exact in this range
+                    aux = fabsf(aux) >= 0x1p-60f && fabsf(aux) <= 0x1p60f ? aux * 0.015625f : 0.f;
                 }
                 float* dst = reinterpret_cast<float*>(rest + L::scl) + t;
-                dst[0] = sv * 64.f, dst[kTileMaxTokens] = aux * 0.015625f;
+                dst[0] = sv, dst[kTileMaxTokens] = aux;
                 in_range &= aux != 0.f;
             }
             in_range = __all_sync(0xffffffffu, in_range);

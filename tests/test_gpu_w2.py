@@ -98,6 +98,35 @@ def test_scales_out_of_the_usual_range_and_segments(lib, M, N, K):
                 assert (np.isnan(o.bf16_bits_to_f32(a)) == nan).all() and (a == b)[~nan].all()
 
 
+@pytest.mark.parametrize("M,N,K", [(3, 320, 640), (6, 192, 1088), (24, 320, 640), (70, 3840, 2560), (1000, 13824, 320)])
+@pytest.mark.parametrize("skew", [0, 1])
+def test_scales_at_the_ends_of_the_number_range(lib, M, N, K, skew):
+    """Every scale that bf16 has is a valid one: the largest, infinity and subnormals beside usual ones, by each kernel, with outputs at odd
+    addresses too: the quotient of the packed kernels, bit for bit."""
+    w = o.make_ternary(N, K, 0.45, N + K)
+    pk = Packed(w, [t.cpu().numpy() for t in compress_weight(torch.from_numpy(w).cuda())])
+    w2, stream = w2_of(lib, pk), torch.cuda.current_stream().cuda_stream
+    xq, s = o.make_activations(M, K, M + 1)
+    s = s.reshape(-1).copy()
+    s[::3], s[1::7], s[2::11], s[-1] = 1e37, np.finfo(np.float32).max / 2, 1e-39, np.inf
+    ws = o.make_ws(2, M + 2)
+    ws[:2] *= 1e30                                     # (so that outputs under the largest scales are not zero)
+    x_d, s_d, ws_d = dev(xq), dev(o.f32_to_bf16_bits(s)), dev(o.f32_to_bf16_bits(ws))
+    for prefill in (0, 1):
+        for seg in ((N, N, N), (40, 104, 200)):
+            got, want = (torch.empty(M * N + 8, dtype=torch.int16, device="cuda")[skew:skew + M * N] for _ in range(2))
+            lib.ternaspmm_w2_linear(x_d.data_ptr(), 0, None, 0.0, w2.data_ptr(), got.data_ptr(), s_d.data_ptr(), ws_d.data_ptr(), 2, M, N, K,
+                                    *seg, prefill, None, stream)
+            lib.ternaspmm_linear_segments(x_d.data_ptr(), pk.bm.data_ptr(), pk.tg.data_ptr(), pk.tm.data_ptr(), pk.cv.data_ptr(), want.data_ptr(),
+                                          s_d.data_ptr(), ws_d.data_ptr(), 2, M, N, K, *seg, prefill, stream)
+            torch.cuda.synchronize()
+            assert lib.ternaspmm_last_status() == 0
+            a, b = got.cpu().numpy().view(np.uint16), want.cpu().numpy().view(np.uint16)
+            nan = np.isnan(o.bf16_bits_to_f32(b))
+            assert (np.isnan(o.bf16_bits_to_f32(a)) == nan).all() and (a == b)[~nan].all()
+            assert ((b.reshape(M, N)[::3] & 0x7FFF) != 0).any()
+
+
 def test_layout_and_linear_on_one_stream(lib):
     """Two weights and two norm weights in turn through the same memory, layout and linear in stream order: never the other's values."""
     N, K = 13824, 2560
