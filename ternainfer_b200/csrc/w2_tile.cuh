@@ -348,6 +348,7 @@ __global__ void __launch_bounds__(kTileThreads, 2)
             }
             in_range = __all_sync(0xffffffffu, in_range);
             if (lane == 0) *reinterpret_cast<int*>(rest + L::scl_ok) = in_range;
+            __syncwarp();                                    // (a vote orders no memory: the other lanes' scales, before lane 0 releases them)
             if (lane == 0) mbar_arrive(bar_scl);
         }
         for (int kb = WS * kTileChunk; kb < KB; kb += kTileChunk) {
