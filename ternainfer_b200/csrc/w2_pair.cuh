@@ -360,6 +360,7 @@ __global__ void __launch_bounds__(kW2PairThreads, 1)
                 in_range &= rv != 0.f;
             }
             in_range = __all_sync(0xffffffffu, in_range);
+            __syncwarp();                          // (a vote orders no memory: the lanes read each other's scales)
             const int cols = min(NT, M - t0);
             uint4 res[2], res_next[2];          // the residual is read one slice ahead
             auto residual_of = [&](int i, uint4 (&r)[2]) {
