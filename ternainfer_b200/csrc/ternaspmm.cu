@@ -633,6 +633,21 @@ extern "C" void ternaspmm_linear_segments(int8_t* x, uint64_t* bitmap, int* tile
     checkLastCudaError(__LINE__);
 }
 
+// The tcgen05 kernels release the next launch before they allocate tensor memory, and tcgen05.alloc waits without a limit.  So the CTAs
+// that shared memory lets onto one SM must never ask for more columns than it has: a later launch that took them first would wait for
+// an earlier one that waits for the columns.
+struct TmemUse { int smem, columns; };
+constexpr TmemUse kTmemUse[] = {{LargeMSmem<64>::total, 2 * 64}, {LargeMSmem<128>::total, 2 * 128}, {LargeMSmem<256>::total, 2 * 256},
+                                {LargeMSmem<128, true>::total, 2 * 128}, {LargeMSmem<256, true>::total, 2 * 256}, {PairSmem::total, 2 * kPairNT},
+                                {W2PairSmem::total, 512}, {kTileMinSmem, kTileCols}};
+constexpr int most_tmem_columns(int smem) {          // of CTAs of these kernels that fit this much shared memory, 1 KB each for the system
+    int most = 0;
+    for (const TmemUse& k : kTmemUse)
+        if (k.smem + 1024 <= smem) most = std::max(most, k.columns + most_tmem_columns(smem - k.smem - 1024));
+    return most;
+}
+static_assert(most_tmem_columns(228 * 1024) <= 512, "CTAs that fit an SM side by side would compete for tensor memory");
+
 // ---- linears on two-bit weights (w2_small.cuh) -----------------------------------------------------
 constexpr int kW2MaxSmem = 227 * 1024;
 // Whether the mma.sync kernel runs a call on int8 activations: up to 4 tokens, and activations that leave shared memory for a ring.  In
@@ -735,7 +750,7 @@ static cudaError_t launch_w2_tile(const W2Params& p, const W2TilePlan& plan, cud
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(kTileThreads, 1, 1);
     cfg.gridDim = dim3(S, tiles, blocks);
-    cfg.dynamicSmemBytes = std::max(smem, 80 * 1024);
+    cfg.dynamicSmemBytes = std::max(smem, kTileMinSmem);
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;

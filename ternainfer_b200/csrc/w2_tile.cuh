@@ -12,7 +12,7 @@
 // MMAs.  A stage's columns and activations share a ring slot, one barrier and one commit.  With S > 1 the partial sums are
 // reduce-scattered through distributed shared memory in units of 8 tokens (st.async, counted by a barrier of the owner; a cluster
 // barrier with release and acquire took three times as long), which their owners scale and store.  Every wait is bounded
-// (status 4).  Shared memory is at least 80 KB, so that no third CTA competes for tensor memory.
+// (status 4).  Shared memory is at least kTileMinSmem, so that no third CTA competes for tensor memory.
 //
 // What bounds it: an MMA of 128 rows x 32 k takes 50 cycles up to 64 tokens and a commit 150, so 270 cycles per 128 k of a CTA; around that
 // the activations' first load, the exchange and the epilogue, each a chain of latencies.  us per call in a stream of different
@@ -35,6 +35,7 @@ constexpr int kTileChunk = 4;              // block pairs (128 k) per copy of co
 constexpr int kTileSlots = 3;              // of codes, at most
 constexpr int kTileSlotBytes = 8 * kTileChunk * 512;
 constexpr int kTileMaxTokens = 128;
+constexpr int kTileMinSmem = 80 * 1024;    // dynamic shared memory of a launch at least (ternaspmm.cu: most_tmem_columns)
 
 constexpr int kTilePart = 8 * kTileRows * 4;   // bytes of a unit's partial sums
 
