@@ -310,7 +310,8 @@ int ternaspmm_attn_decode(ternaspmm_bf16* qkv, ternaspmm_bf16* k_cache, ternaspm
                           int batch, int heads, int kv_heads, int head_dim, int max_len, ternaspmm_stream_t stream);
 
 /* The same on caches [batch][kv_heads][max_len][head_dim], with an fp32 rotation whose products are rounded one by one (as
- * ternaspmm_rope does). */
+ * ternaspmm_rope does).  A position outside of the cache is refused by the kernel: ternaspmm_last_status() returns 1, the caches
+ * stay as they are and out is filled with NaN. */
 int ternaspmm_attn_decode_by_head(ternaspmm_bf16* qkv, ternaspmm_bf16* k_cache, ternaspmm_bf16* v_cache, float* cos_row,
                                   float* sin_row, long long* pos, ternaspmm_bf16* out, int batch, int heads, int kv_heads,
                                   int head_dim, int max_len, ternaspmm_stream_t stream);

@@ -34,6 +34,7 @@ struct AttnParams {
     __nv_bfloat16* out;                    // [B][H * D]
     int heads, kv_heads, max_len;
     float scale_log2;                      // log2(e) / sqrt(D)
+    int* status;                           // BY_HEAD: told of a position outside of the cache
 };
 
 // D(16x8) += A(16x16) * B(16x8), bf16; rows8: rows 8-15 of A are zero
@@ -74,7 +75,8 @@ __device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
 }
 
 // BY_HEAD: caches [B][Hkv][L][D] and an fp32 rotation whose products are rounded one by one: the layout and arithmetic of the
-// default glue, which ran 27 torch kernels here (10 layers at 3 x 333 tokens: 932 us a token with them, 500 so).
+// default glue, which ran 27 torch kernels here (10 layers at 3 x 333 tokens: 932 us a token with them, 500 so).  index_copy_ refused a
+// position outside of the cache, and so does this form: status 1, caches as they were, results NaN.
 template <int GQ, bool BY_HEAD>
 __global__ void __launch_bounds__(kAttnWarps * 32, 3) attn_decode_kernel(const AttnParams p) {
     constexpr int kParts = kAttnWarps + 1;                    // the warps' partial results and the new token's
@@ -146,6 +148,8 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 3) attn_decode_kernel(const A
     }
     // cached keys 0 .. pos-1, the new one goes to row pos (clamped: a wrong position must not leave the cache)
     const int pos = (int)max(0ll, min(pos_ll, (long long)p.max_len - 1));
+    const bool refused = BY_HEAD && pos_ll != pos;
+    if (refused && tid == 0) atomicExch(p.status, ST_BAD_SHAPE);
     const int groups = (pos + 15) >> 4;
     __syncthreads();
     phase_mark(3);
@@ -219,7 +223,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 3) attn_decode_kernel(const A
             d *= p.scale_log2;
             const uint2 v = vnew;
             *reinterpret_cast<float4*>(&os[kAttnWarps][h][lane * 4]) = make_float4(bf16_lo(v.x), bf16_hi(v.x), bf16_lo(v.y), bf16_hi(v.y));
-            if (h == 0) {
+            if (h == 0 && !refused) {
                 *reinterpret_cast<uint2*>(p.k_cache + head0 + (size_t)pos * row + lane * 4) = kv;
                 *reinterpret_cast<uint2*>(p.v_cache + head0 + (size_t)pos * row + lane * 4) = v;
             }
@@ -280,7 +284,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 3) attn_decode_kernel(const A
             const float w = mr[r] == -INFINITY ? 0.f : ex2_approx(mr[r] - top);
             l_all += w * lr[r], o_all += w * orr[r];
         }
-        p.out[((size_t)b * p.heads + hk * GQ) * kAttnD + i] = __float2bfloat16_rn(o_all / l_all);
+        p.out[((size_t)b * p.heads + hk * GQ) * kAttnD + i] = __float2bfloat16_rn(refused ? NAN : o_all / l_all);
     }
     phase_mark(7);
 }

@@ -920,7 +920,12 @@ static int run_attn_decode(__nv_bfloat16* qkv, __nv_bfloat16* k_cache, __nv_bflo
         t_host_status = ST_BAD_POINTER;
         return t_host_status;
     }
-    AttnParams p = {qkv, k_cache, v_cache, cos_row, sin_row, pos, out, heads, kv_heads, max_len, 1.4426950408889634f / sqrtf((float)head_dim)};
+    AttnParams p = {qkv, k_cache, v_cache, cos_row, sin_row, pos, out, heads, kv_heads, max_len, 1.4426950408889634f / sqrtf((float)head_dim),
+                    BY_HEAD ? status_device_ptr() : nullptr};
+    if (BY_HEAD && !p.status) {
+        t_host_status = ST_LAUNCH;
+        return t_host_status;
+    }
     if ((gq == 4 ? launch_attn_decode<4, BY_HEAD>(p, batch, stream) : launch_attn_decode<8, BY_HEAD>(p, batch, stream)) != cudaSuccess)
         t_host_status = ST_LAUNCH;
     checkLastCudaError(__LINE__);

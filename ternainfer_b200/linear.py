@@ -193,7 +193,8 @@ def attn_decode(qkv, k_cache, v_cache, cos_row, sin_row, pos, heads: int, kv_hea
 
 def attn_decode_by_head(qkv, k_cache, v_cache, cos_row, sin_row, pos, heads: int, kv_heads: int):
     """``attn_decode`` on caches [B, kv_heads, L, 128], rotation fp32 [64] of that position in the arithmetic of ``rope``: the
-    default glue's RoPE, ``index_copy_`` and masked attention of one new token per sequence.  Not under autograd."""
+    default glue's RoPE, ``index_copy_`` and masked attention of one new token per sequence.  Not under autograd.  A position outside of the
+    cache gives NaN and leaves the caches as they are (status 1 of the library)."""
     if not (qkv.is_cuda and qkv.device == k_cache.device == v_cache.device == cos_row.device == sin_row.device == pos.device
             and qkv.dtype == k_cache.dtype == v_cache.dtype == torch.bfloat16 and cos_row.dtype == sin_row.dtype == torch.float32
             and pos.dtype == torch.int64 and pos.numel() == 1 and qkv.dim() == 3 and qkv.shape[1] == 1 and k_cache.dim() == 4

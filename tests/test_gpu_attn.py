@@ -67,6 +67,23 @@ def test_decode_attention_by_head(lib, B, pos, L, H, Hkv):
     assert err < max(1.05 * theirs, 2.1e-3)                 # (one rounding to bf16 is 1.7e-3 of normally distributed values)
 
 
+@pytest.mark.parametrize("B,pos,L", [(1, 8, 8), (3, -1, 40), (2, 2 ** 40, 600), (1, -2 ** 33, 16)])
+@torch.no_grad()
+def test_decode_attention_by_head_refuses_a_position_outside_of_the_cache(lib, B, pos, L):
+    """As index_copy_ did: nothing is written, the result is no number, and the library says so once."""
+    from ternainfer_b200.linear import attn_decode_by_head
+    H, Hkv, D = 20, 5, 128
+    qkv = torch.randn((B, 1, (H + 2 * Hkv) * D), device="cuda").to(torch.bfloat16)
+    kc, vc = (torch.randn((B, Hkv, L, D), device="cuda").to(torch.bfloat16) for _ in range(2))
+    k0, v0 = kc.clone(), vc.clone()
+    cos, sin = (t[0] for t in rope_tables(D, L, 500000.0, "cuda"))
+    out = attn_decode_by_head(qkv, kc, vc, cos, sin, torch.tensor([pos], device="cuda"), H, Hkv)
+    assert lib.ternaspmm_last_status() == 1 and lib.ternaspmm_last_status() == 0
+    assert out.isnan().all() and torch.equal(kc, k0) and torch.equal(vc, v0)
+    out = attn_decode_by_head(qkv, kc, vc, cos, sin, torch.tensor([L - 1], device="cuda"), H, Hkv)
+    assert lib.ternaspmm_last_status() == 0 and not out.isnan().any()
+
+
 @pytest.mark.parametrize("H,Hkv", [(20, 5), (64, 8)])
 @pytest.mark.parametrize("B,T,past,L", [(1, 2, 0, 8), (2, 16, 0, 16), (1, 17, 0, 64), (3, 64, 0, 64), (1, 65, 1, 80), (2, 200, 63, 300), (1, 613, 0, 613),
                                         (1, 40, 1000, 1040), (1, 129, 0, 200), (2, 500, 37, 640)])
