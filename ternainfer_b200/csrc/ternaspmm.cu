@@ -650,11 +650,17 @@ static_assert(most_tmem_columns(228 * 1024) <= 512, "CTAs that fit an SM side by
 
 // ---- linears on two-bit weights (w2_small.cuh) -----------------------------------------------------
 constexpr int kW2MaxSmem = 227 * 1024;
-// Whether the mma.sync kernel runs a call on int8 activations: up to 4 tokens, and activations that leave shared memory for a ring.  In
-// a stream of such calls alone the line would be 8 for narrow layers (us per call, mma.sync / tensor-memory tiles, at 4 / 8 / 12 tokens:
-// 2560 x 2560 2.6 / 3.3, 2.8 / 3.3, 3.5 / 3.3, 13824 x 2560 4.4 / 5.2, 5.2 / 5.2, 6.9 / 5.2, 8192 x 28672 14.7 / 15.5, 23.4 / 15.0), but between other
-// kernels the tiles' expansion is done when those end: 30-layer model at batch 8 1180 us a token, with tiles 1148.
-static bool w2_small_takes(int M, int K) { return M <= 4 && (long long)M * (K + 64) <= 120 * 1024; }
+// Whether the mma.sync kernel runs a call on int8 activations: up to 4 tokens, up to 8 where a CTA has three strips at most, and
+// activations that leave shared memory for a ring.  A narrow layer's tiles pay for the exchange between K slices, and a call of them
+// for a tensor map and a search on the host.  us per call in a stream of such calls, mma.sync / tensor-memory tiles, at 5 and 8 tokens: 2560 x 2560
+// 2.4 / 3.2, 2.7 / 3.2, 2560 x 6912 3.8 / 4.4, 4.0 / 4.4, 5120 x 4096 3.8 / 4.3, 4.0 / 4.3, 6912 x 2560 3.0 / 3.9, 3.4 / 3.8; eager module calls of 2560 x 2560 at 8
+// 8.6 / 9.3.  Not where K is short as well (2560 x 256 2.2 / 2.3, 2.4 / 2.3; 6912 x 1024 2.7 / 2.9, 3.0 / 2.9) and not on wider layers: alone they are even (13824 x
+// 2560 5.1 / 5.2, 5.2 / 5.1, 8192 x 8192 7.4 / 7.0), but between other kernels the tiles' expansion is done when those end (30-layer model at
+// batch 8: all by tiles 1147 us a token, narrow layers by mma.sync 1133, gate-up too 1164).
+static bool w2_small_takes(int M, int N, int K) {
+    const int strips = N / 16, sms = device_sm_count();
+    return (M <= 4 || (M <= 8 && K >= 640 && strips <= (K > 1024 ? 3 : 2) * sms)) && (long long)M * (K + 64) <= 120 * 1024;
+}
 
 template <int MW, int RG, int FE, int VK, int VR>
 static cudaError_t launch_w2_strips(W2Params& p, cudaStream_t stream) {
@@ -868,7 +874,7 @@ extern "C" void ternaspmm_w2_linear(void* x, int front_end, __nv_bfloat16* norm_
     if (front_end == W2_PLAIN) e = launch_w2_fused<W2_PLAIN>(p, stream);
     else if (front_end == W2_NORM) e = launch_w2_fused<W2_NORM>(p, stream);
     else if (front_end == W2_GATED) e = launch_w2_fused<W2_GATED>(p, stream);
-    else if (w2_small_takes(M, K)) e = launch_w2_int8(p, stream);
+    else if (w2_small_takes(M, N, K)) e = launch_w2_int8(p, stream);
     else {
         const W2TilePlan tile = w2_tile_plan(M, N, K, device_sm_count());
         const W2PairPlan pair = w2_pair_plan_tile(M, N, K, device_sm_count() / 2);

@@ -2,6 +2,7 @@
 the kernel's tiles: odd numbers of 64-column blocks, fewer blocks than warps, one strip group too many, token blocks with
 one row, weights larger than the shared-memory ring."""
 import copy
+import ctypes
 
 import numpy as np
 import pytest
@@ -125,6 +126,16 @@ def test_scales_at_the_ends_of_the_number_range(lib, M, N, K, skew):
             nan = np.isnan(o.bf16_bits_to_f32(b))
             assert (np.isnan(o.bf16_bits_to_f32(a)) == nan).all() and (a == b)[~nan].all()
             assert ((b.reshape(M, N)[::3] & 0x7FFF) != 0).any()
+
+
+@pytest.mark.parametrize("M,N,K,kernel", [(5, 64, 640, 8), (5, 64, 576, 9), (8, 4736, 1024, 8), (8, 4800, 1024, 9), (6, 7104, 1088, 8), (6, 7168, 1088, 9), (9, 64, 640, 9),
+                                          (7, 128, 17408, 8), (7, 128, 17536, 9), (5, 192, 2496, 8), (4, 7168, 256, 8)])
+def test_five_to_eight_tokens_by_either_kernel(lib, M, N, K, kernel):
+    """Either side of each line of the rule (on 148 SMs): the kernel that was measured to be the faster one there, and the oracle's bits."""
+    check_linear(lib, M, N, K, 2)
+    shape = (ctypes.c_int * 6)()
+    lib.ternaspmm_last_launch_shape(shape)
+    assert shape[0] == kernel or torch.cuda.get_device_properties(0).multi_processor_count != 148
 
 
 def test_layout_and_linear_on_one_stream(lib):
