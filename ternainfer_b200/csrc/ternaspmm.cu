@@ -711,13 +711,15 @@ static cudaError_t launch_w2_strips(W2Params& p, cudaStream_t stream) {
     return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
-// Strips at a time: one where a CTA has one or two, or up to six of a K that gives a warp more than two block pairs (w2_small.cuh has both
-// sides measured), and where three strips' share of a long K would leave no room for a second ring slot (8192 x 28672 at 1
-// token 26.9 -> 20.7 us).
+// Strips at a time: three, whose chains overlap, where that wastes little of a CTA's last group - it has three, or six and more - and
+// their share of K leaves room for the ring (not 8192 x 28672: 26.9 us at 1 token, one at a time 20.7); one otherwise.  One / three at a time, mean over
+// the quantised entry and the front-ends, separate or inside, at 1 to 4 tokens: three strips 5120 x 5120 1.02 to 1.08, 6912 x 4096 1.09 to 1.13; four 8192 x 2560
+// 0.90 to 0.92, 8192 x 6912 0.93 to 0.95; five 10240 x 2048 0.93 to 0.98, 10240 x 6912 0.96 to 0.99; six 13824 x 2560 1.04 to 1.06, 13824 x 4096 1.14 to 1.19; seven
+// 14336 x 8192 11.4 / 9.0 us.
 template <int FE, int VK, int VR>
 static cudaError_t launch_w2_small(W2Params& p, cudaStream_t stream) {
-    const int strips = p.e.N / 16, sms = device_sm_count(), K = p.e.K;
-    return strips <= 2 * sms || K > 8192 || (strips <= 6 * sms && w2_pairs(K) > 2 * w2_warps(K)) ? launch_w2_strips<kW2Warps, 1, FE, VK, VR>(p, stream) : launch_w2_strips<kW2Warps, 3, FE, VK, VR>(p, stream);
+    const int sms = device_sm_count(), R = (p.e.N / 16 + sms - 1) / sms;
+    return p.e.K > 8192 || R <= 2 || R == 4 || R == 5 ? launch_w2_strips<kW2Warps, 1, FE, VK, VR>(p, stream) : launch_w2_strips<kW2Warps, 3, FE, VK, VR>(p, stream);
 }
 // Long launches need no place for the next one beside them: twice the warps, a strip at a time.  us per call at 4 tokens, ten / twenty warps:
 // 8192 x 8192 7.1 / 6.7, 8192 x 28672 16.0 / 14.7, 16384 x 16384 17.6 / 16.0, 57344 x 8192 32.3 / 31.9 (at 8 33.4 / 29.9); not 14336 x 8192 11.8 /

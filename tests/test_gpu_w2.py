@@ -138,6 +138,30 @@ def test_five_to_eight_tokens_by_either_kernel(lib, M, N, K, kernel):
     assert shape[0] == kernel or torch.cuda.get_device_properties(0).multi_processor_count != 148
 
 
+def check_against_packed(lib, M, N, K):
+    g = torch.Generator(device="cuda").manual_seed(N + K + M)
+    w = torch.randint(-1, 2, (N, K), generator=g, device="cuda", dtype=torch.int8)
+    pk = Packed(np.empty((N, K), np.int8), [t.cpu().numpy() for t in compress_weight(w)])
+    w2, stream = w2_of(lib, pk), torch.cuda.current_stream().cuda_stream
+    x = torch.randint(-128, 128, (M, K), generator=g, device="cuda", dtype=torch.int8)
+    s = (20 + 10 * torch.rand(M, generator=g, device="cuda")).to(torch.bfloat16)
+    ws = torch.tensor([0.5, 2.0, 0, 0], device="cuda").to(torch.bfloat16)
+    got, want = (torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    lib.ternaspmm_w2_linear(x.data_ptr(), 0, None, 0.0, w2.data_ptr(), got.data_ptr(), s.data_ptr(), ws.data_ptr(), 2, M, N, K, 0, 0, 0, -1, None, stream)
+    shape = (ctypes.c_int * 6)()
+    lib.ternaspmm_last_launch_shape(shape)
+    lib.bitlinear_TernaSpMM(x.data_ptr(), pk.bm.data_ptr(), pk.tg.data_ptr(), pk.tm.data_ptr(), pk.cv.data_ptr(), want.data_ptr(), s.data_ptr(),
+                            ws.data_ptr(), 2, M, N, K, 1, None, stream)
+    assert lib.ternaspmm_last_status() == 0 and torch.equal(got, want)
+    return list(shape)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 4800, 3072), (4, 7104, 3072), (4, 7168, 384), (2, 9536, 2624), (3, 11840, 640), (4, 11904, 4096), (1, 14208, 2560), (2, 14272, 7680), (3, 4800, 8256)])
+def test_strips_at_a_time(lib, M, N, K):
+    """CTAs of three to seven strips, some with one less, one and three strips at a time: the bits of the packed kernels."""
+    check_against_packed(lib, M, N, K)
+
+
 def test_layout_and_linear_on_one_stream(lib):
     """Two weights and two norm weights in turn through the same memory, layout and linear in stream order: never the other's values."""
     N, K = 13824, 2560
