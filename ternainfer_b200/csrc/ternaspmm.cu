@@ -721,13 +721,18 @@ static cudaError_t launch_w2_small(W2Params& p, cudaStream_t stream) {
     const int sms = device_sm_count(), R = (p.e.N / 16 + sms - 1) / sms;
     return p.e.K > 8192 || R <= 2 || R == 4 || R == 5 ? launch_w2_strips<kW2Warps, 1, FE, VK, VR>(p, stream) : launch_w2_strips<kW2Warps, 3, FE, VK, VR>(p, stream);
 }
-// Long launches need no place for the next one beside them: twice the warps, a strip at a time.  us per call at 4 tokens, ten / twenty warps:
-// 8192 x 8192 7.1 / 6.7, 8192 x 28672 16.0 / 14.7, 16384 x 16384 17.6 / 16.0, 57344 x 8192 32.3 / 31.9 (at 8 33.4 / 29.9); not 14336 x 8192 11.8 /
-// 12.4, 28672 x 8192 18.3 / 18.9, nor shorter K (13824 x 2560 4.4 / 6.7).
+// Twice the warps, a strip at a time, shorten a strip's chain, but leave no place beside them: the next launch's CTAs wait for this one's, and
+// these for a front-end's, 1 to 2 us once per launch.  Where a CTA has up to five strips, whose chains are most of the call, that pays from 8192
+// columns on; more strips, which ten warps take three at a time, from 12288 on - or from 8192 where there are many of them and four tokens,
+// whose sums cost the ten warps 10 % more than one token's and the twenty nothing.  us per call, ten / twenty warps, in a stream of such calls (and behind
+// the quantiser), at 1 and 4 tokens: 2560 x 8192 3.8 / 3.5 (5.7 / 5.1), 4.0 / 3.7 (6.1 / 5.3), 10240 x 8192 7.2 / 7.2 (8.6 / 8.2), 7.5 / 7.9 (9.5 / 9.2), 14336 x 8192 9.6 /
+// 13.6 (12.1 / 13.8), 11.4 / 13.4 (14.1 / 14.3), 14336 x 10240 13.1 / 15.0 (16.1 / 16.0), 13.0 / 14.1 (16.8 / 17.6), 28672 x 8192 17.0 / 19.0 (18.9 / 19.1), 18.7 / 19.1
+// (21.2 / 20.4), 57344 x 8192 30.1 / 33.3 (32.6 / 33.8), 33.3 / 33.2 (36.6 / 34.6), 28672 x 12288 24.4 / 23.6 (28.6 / 25.3), 26.3 / 22.5 (32.3 / 27.6), 14336 x 16384 16.9 /
+// 13.9 (21.1 / 18.3), 17.4 / 15.3 (24.5 / 22.5); shorter K 57344 x 7680 at 4 28.3 / 34.5 (31.7 / 36.0).
 static cudaError_t launch_w2_int8(W2Params& p, cudaStream_t stream) {
-    const int strips = p.e.N / 16, sms = device_sm_count(), K = p.e.K;
-    const bool longer = K > 8192 || (K > 7168 && (strips <= 4 * sms || strips > 16 * sms));
-    return longer ? launch_w2_strips<kW2MaxWarps, 1, W2_INT8, 1, 1>(p, stream) : launch_w2_small<W2_INT8, 1, 1>(p, stream);
+    const int strips = p.e.N / 16, sms = device_sm_count();
+    const bool twice = p.e.K >= (strips <= 5 * sms || (strips > 8 * sms && p.e.M > 3) ? 8192 : 12288);
+    return twice ? launch_w2_strips<kW2MaxWarps, 1, W2_INT8, 1, 1>(p, stream) : launch_w2_small<W2_INT8, 1, 1>(p, stream);
 }
 template <int FE>
 static cudaError_t launch_w2_fused(W2Params& p, cudaStream_t stream) {

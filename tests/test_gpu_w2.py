@@ -162,6 +162,14 @@ def test_strips_at_a_time(lib, M, N, K):
     check_against_packed(lib, M, N, K)
 
 
+@pytest.mark.parametrize("M,N,K,warps", [(1, 11840, 8192, 16), (2, 11840, 8128, 10), (2, 11904, 8192, 10), (4, 11904, 8192, 10), (3, 19008, 8192, 10), (4, 19008, 8192, 16), (4, 18944, 8192, 10),
+                                         (1, 11904, 12288, 20), (1, 11904, 12224, 10), (3, 128, 28672, 19)])
+def test_ten_and_twenty_warps(lib, M, N, K, warps):
+    """Either side of each line of the rule (on 148 SMs): the warps that were measured to be faster there, the bits of the packed kernels."""
+    shape = check_against_packed(lib, M, N, K)
+    assert shape[0] == 8 and (shape[3] == warps or torch.cuda.get_device_properties(0).multi_processor_count != 148)
+
+
 def test_layout_and_linear_on_one_stream(lib):
     """Two weights and two norm weights in turn through the same memory, layout and linear in stream order: never the other's values."""
     N, K = 13824, 2560
