@@ -650,16 +650,19 @@ static_assert(most_tmem_columns(228 * 1024) <= 512, "CTAs that fit an SM side by
 
 // ---- linears on two-bit weights (w2_small.cuh) -----------------------------------------------------
 constexpr int kW2MaxSmem = 227 * 1024;
-// Whether the mma.sync kernel runs a call on int8 activations: up to 4 tokens, up to 8 where a CTA has three strips at most, and
-// activations that leave shared memory for a ring.  A narrow layer's tiles pay for the exchange between K slices, and a call of them
-// for a tensor map and a search on the host.  us per call in a stream of such calls, mma.sync / tensor-memory tiles, at 5 and 8 tokens: 2560 x 2560
-// 2.4 / 3.2, 2.7 / 3.2, 2560 x 6912 3.8 / 4.4, 4.0 / 4.4, 5120 x 4096 3.8 / 4.3, 4.0 / 4.3, 6912 x 2560 3.0 / 3.9, 3.4 / 3.8; eager module calls of 2560 x 2560 at 8
-// 8.6 / 9.3.  Not where K is short as well (2560 x 256 2.2 / 2.3, 2.4 / 2.3; 6912 x 1024 2.7 / 2.9, 3.0 / 2.9) and not on wider layers: alone they are even (13824 x
-// 2560 5.1 / 5.2, 5.2 / 5.1, 8192 x 8192 7.4 / 7.0), but between other kernels the tiles' expansion is done when those end (30-layer model at
-// batch 8: all by tiles 1147 us a token, narrow layers by mma.sync 1133, gate-up too 1164).
+// Whether the mma.sync kernel runs a call on int8 activations: up to 4 tokens, up to 8 where a CTA has three strips at most, and activations that
+// leave shared memory for a ring - from five tokens on, where an SM has more than one strip, a small part of it, so that the next launch's CTA or
+// a front-end's finds room.  A narrow layer's tiles pay for the exchange between K slices, and a call of them for a tensor map and a search on the
+// host.  us per call in a stream of such calls, mma.sync / tensor-memory tiles, at 5 and 8 tokens: 2560 x 2560 2.5 / 3.2, 2.7 / 3.2, 2560 x 6912 3.8 / 4.3,
+// 4.1 / 4.4, 5120 x 5120 4.1 / 4.8, 4.6 / 4.9, 1280 x 8192 at 8 3.5 / 4.4; eager module calls of 2560 x 2560 at 5 8.9 / 9.4.  Not with longer rows (behind a norm
+// 2560 x 10240 at 8 12.6 / 10.2; but 2560 x 6912 at 8 inside the 30-layer model, where other kernels stand between: 1123 us a token, 1142 with tiles),
+// nor where K is short (2560 x 256 2.2 / 2.3, 2.4 / 2.3; 6912 x 1024 behind the quantiser at 8 25 % more), nor on wider layers: alone they are even
+// (13824 x 2560 5.1 / 5.2, 5.2 / 5.1), but between other kernels the tiles' expansion is done when those end (that model at batch 8 with gate-up by
+// mma.sync 1164).
 static bool w2_small_takes(int M, int N, int K) {
     const int strips = N / 16, sms = device_sm_count();
-    return (M <= 4 || (M <= 8 && K >= 640 && strips <= (K > 1024 ? 3 : 2) * sms)) && (long long)M * (K + 64) <= 120 * 1024;
+    const long long bytes = (long long)M * (K + 64);
+    return bytes <= 120 * 1024 && (M <= 4 || (M <= 8 && K >= 640 && strips <= (K > 1024 ? 3 : 2) * sms && (strips <= sms || bytes <= 56 * 1024)));
 }
 
 template <int MW, int RG, int FE, int VK, int VR>

@@ -129,7 +129,7 @@ def test_scales_at_the_ends_of_the_number_range(lib, M, N, K, skew):
 
 
 @pytest.mark.parametrize("M,N,K,kernel", [(5, 64, 640, 8), (5, 64, 576, 9), (8, 4736, 1024, 8), (8, 4800, 1024, 9), (6, 7104, 1088, 8), (6, 7168, 1088, 9), (9, 64, 640, 9),
-                                          (7, 128, 17408, 8), (7, 128, 17536, 9), (5, 192, 2496, 8), (4, 7168, 256, 8)])
+                                          (7, 128, 17408, 8), (7, 128, 17536, 9), (5, 192, 2496, 8), (4, 7168, 256, 8), (8, 2432, 7104, 8), (8, 2432, 7168, 9), (8, 2368, 7168, 8)])
 def test_five_to_eight_tokens_by_either_kernel(lib, M, N, K, kernel):
     """Either side of each line of the rule (on 148 SMs): the kernel that was measured to be the faster one there, and the oracle's bits."""
     check_linear(lib, M, N, K, 2)
