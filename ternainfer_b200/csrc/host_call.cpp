@@ -177,12 +177,13 @@ PyObject* front_and_linear(Layer* self, PyObject* params, PyObject* xo, int fron
     if (!w2) Py_RETURN_NONE;
     at::Tensor out = output_like(x, self->out_features);
     // The front-end inside the linear's kernel saves a launch of its own, 1.1 us of the stream and as much of the host; every CTA does
-    // it, up to four rows at once where a row is one vector per thread (K up to 2560), one after the other above that.  us per
-    // call, inside / separate: quantiser 2560 x 2560 at 1 / 4 / 8 rows 2.7 / 4.0, 3.2 / 4.3, 5.0 / 4.3, 2560 x 6912 at 1 / 3 4.0 / 5.4, 6.0 / 5.9,
+    // it, up to four rows at once where a row is one vector per thread (K up to 2560), one after the other above that.  That pays up to 10240
+    // values.  us per call, inside / separate: quantiser 2560 x 2560 at 1 / 4 / 8 rows 2.7 / 4.0, 3.2 / 4.3, 5.0 / 4.3, 5120 x 5120 at 2 4.7 / 5.9,
+    // 5120 x 4096 at 2 4.2 / 5.9, 2560 x 3072 at 3 4.2 / 4.7 (called eagerly 5.1 / 8.4), 2560 x 6912 at 1 / 3 4.0 / 5.4, 6.0 / 5.9,
     // 10240 x 8192 at 1 / 2 8.9 / 10.8, 12.0 / 11.8, 57344 x 8192 at 1 / 4 37.8 / 34.4, 38.9 / 36.0; norm 2560 x 2560 at 1 3.1 / 4.4, 2560 x 6912 at
     // 1 / 2 (gated) 5.1 / 6.5, 6.8 / 6.8, 10240 x 8192 at 1 12.3 / 11.2.  Norms of 2 to 4 rows gain alone (2560 x 2560 at 4 4.2 / 4.8), but a
     // separate one overlaps the kernel before it: 30-layer model at batch 2 / 4 1043 / 1126 us a token, so 1009 / 1074.
-    if (M <= ternaspmm_w2_fused_rows((int)K) && K < 8192 && (M == 1 || (front_end == 1 && M <= 4 && K <= 2560))) {
+    if (M <= ternaspmm_w2_fused_rows((int)K) && K < 8192 && (M == 1 || (front_end == 1 && M <= 4 && M * K <= 10240))) {
         run_linear(self, w, w2, x.data_ptr(), front_end, norm_w, eps, out, nullptr, M, residual, stream);
         return THPVariable_Wrap(std::move(out));
     }

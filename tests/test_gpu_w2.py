@@ -229,6 +229,15 @@ def test_front_end_inside_the_linear(lib, M, N, K, kind):
     assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("M,N,K", [(2, 64, 5120), (2, 64, 5184), (2, 4800, 4096), (3, 64, 3392), (3, 128, 3456), (4, 64, 2560), (4, 64, 2624)])
+def test_quantiser_inside_the_linear_or_before_it(lib, M, N, K):
+    """Either side of the line up to which a few rows are quantised inside: the values of the separate launch."""
+    layer, _ = make_layer(N, K, 1, N + K)
+    x = torch.randn((M, K), generator=torch.Generator(device="cuda").manual_seed(M), device="cuda").to(torch.bfloat16)
+    x[-1] *= 100
+    assert torch.equal(layer(x), layer.forward_quantized(*quant_input(x)))
+
+
 def test_layer_follows_its_weights(lib):
     """New values in place, a loaded state dict, a replaced parameter and copies: the layout is never stale."""
     layer, dic = make_layer(128, 192, 2, 1, segments=[64, 64])
