@@ -147,7 +147,7 @@ __device__ __forceinline__ void store_slice16_matrix(const SpmmParams& p, SliceA
 struct W2PairParams {
     SpmmParams e;
     const uint8_t* w;                      // two-bit weights
-    int nt, stages;                        // tokens per tile: a multiple of 32, at most 256; ring slots
+    int nt, stages;                        // tokens per tile: a multiple of 32 from 96 to 256; ring slots
     int a_stages;                          // of them, slots of weights in tensor memory
     int acc_bufs, acc_cols;                // accumulator buffers in tensor memory and the columns between them
 };
@@ -420,18 +420,17 @@ __global__ void __launch_bounds__(kW2PairThreads, 1)
 }
 
 // Tokens per tile of a call and the time it takes, in us: KS stages at the rate of the decoders and barriers (small tiles) or of the
-// tensor cores, for each round of tiles over the pairs of the chip, and once what a launch needs around them.  Fitted to one tile per
-// pair of 32 and 128 stages (NT 64 / 128 / 192 / 256: 0.164 / 0.174 / 0.234 / 0.30 us per stage, 5.5 / 6.3 / 7.5 / 8.6 us around them) and to
-// 13824 x 2560 at 1226 tokens (NT 128 / 160 / 192 / 256: 37.1 / 33.0 / 33.6 / 41.9 us).  Above 192 tokens there is one accumulator buffer,
+// tensor cores, for each round of tiles over the pairs of the chip, and once what a launch needs around them (fitted with w2_tile_plan;
+// 13824 x 2560 at 1226 tokens in tiles of 128 / 160 / 192 / 256: 37.1 / 33.0 / 33.6 / 41.9 us).  Above 192 tokens there is one accumulator buffer,
 // and a tile's epilogue holds the next one up.
 struct W2PairPlan { int nt; double us; };
 inline W2PairPlan w2_pair_plan_tile(int M, int N, int K, int pairs) {
     const int RB = (N + kPairRows - 1) / kPairRows, KS = w2_pairs(K);
     W2PairPlan best = {0, 1e30};
-    for (int nt = 32; nt <= 256; nt += 32) {
+    for (int nt = 96; nt <= 256; nt += 32) {              // (smaller ones never beat single tiles)
         const long long tiles = (long long)RB * ((M + nt - 1) / nt);
         const double rounds = (double)((tiles + pairs - 1) / pairs);
-        const double us = 3.9 + 0.015 * nt + rounds * KS * std::max(0.15 + 0.00018 * nt, 0.00121 * nt) + (rounds - 1) * (nt > 192 ? 4.5 : 0.45);
+        const double us = 3.34 + 0.0158 * nt + rounds * KS * std::max(0.153 + 0.00017 * nt, 0.00106 * nt) + (rounds - 1) * (nt > 192 ? 4.7 : 0.68);
         if (us < best.us) best = {nt, us};
     }
     return best;

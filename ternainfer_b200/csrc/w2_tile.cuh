@@ -492,13 +492,14 @@ __global__ void __launch_bounds__(kTileThreads, 2)
     phase_mark(7);
 }
 
-// Tokens per tile and K slices of a call, and the time it takes, in us.  The CTAs of up to 256 (two to an SM; clusters leave some
-// places empty) run at once, each KB = K / 128 / S block pairs long, 0.15 us each, 0.2 with two CTAs on an SM's tensor cores; a
-// cluster's exchange grows with S.  Measured, us per call in a stream of
-// different weights, S = 1 / 2 / 4 / 6 / 8: 2560 x 2560 at 48 tokens 5.2 / 4.4 / 4.1 / 4.4 / 5.4, 2560 x 6912 at 16 tokens 9.5 / 6.2 / 5.0 / 4.5 /
-// 4.6, 1024 x 16384 at 16 19.5 / 11.1 / 7.1 / 6.1 / 5.3, 8192 x 8192 at 16 11.2 / 8.6 / 7.0 / 10.6 / 11.8 (384 CTAs with six slices), 13824 x 2560 at 48 6.7 / 6.0 / 10.2.  Tiles of more
-// than 64 tokens have room for two stages only (0.30 to 0.34 us per block pair) and pay where they save a round
-// of CTAs: 13824 x 2560 at 256 tokens 11.3, in tiles of 64 13.9.
+// Tokens per tile and K slices of a call, and the time it takes, in us.  The CTAs of two to an SM (clusters leave some places empty) run
+// at once, each KB = K / 128 / S block pairs long, 0.15 us each, 0.22 with two CTAs on an SM's tensor cores; a further round of CTAs costs
+// its own start and end, and a cluster's exchange grows with S.  Tiles of more than 64 tokens have room for two stages only, 0.34 us per block
+// pair, and pay where they save a round.  The constants of this and of w2_pair_plan_tile are fitted to 8700 measured plans of 582 calls of 9 to
+// 4096 tokens (the layers of both models, their shards, and sizes drawn over the range): the plan chosen is 1.0 % slower than the best one in the mean,
+// 1.1 % on calls that were left out of a fit.  us per call, S = 1 / 2 / 4 / 6 / 8: 2560 x 2560 at 48 tokens 5.2 / 4.4 / 4.1 / 4.4 / 5.4, 2560 x 6912 at 16 9.5 / 6.2 /
+// 5.0 / 4.5 / 4.6, 1024 x 16384 at 16 19.5 / 11.1 / 7.1 / 6.1 / 5.3, 8192 x 8192 at 16 11.2 / 8.6 / 7.0 / 10.6 / 11.8 (384 CTAs with six slices); tiles of up to 64 / 128
+// tokens: 2560 x 2560 at 1600 15.7 / 11.6, 8192 x 1024 at 512 10.9 / 7.7, 13824 x 2560 at 256 13.9 / 11.3.
 struct W2TilePlan { int nt, splits; double us; };
 inline W2TilePlan w2_tile_plan(int M, int N, int K, int sms) {
     const int tiles = (N + kTileRows - 1) / kTileRows, KP = w2_pairs(K);
@@ -507,12 +508,13 @@ inline W2TilePlan w2_tile_plan(int M, int N, int K, int sms) {
         const int blocks = (M + most - 1) / most, nt = ((M + blocks - 1) / blocks + 15) & ~15;
         if (blocks > 65535 || tiles > 65535) continue;      // (the limits of a grid)
         for (int S = 1; S <= (nt > 64 ? 1 : std::min(8, KP)); ++S) {
-            const long long ctas = (long long)tiles * blocks * S, at_once = sms * 2 - sms / 4;
+            const long long ctas = (long long)tiles * blocks * S, at_once = S > 1 ? sms * 2 - sms / 4 : sms * 2;
             const long long rounds = (ctas + at_once - 1) / at_once, last = ctas - (rounds - 1) * at_once;
-            const double KB = (KP + S - 1) / S, alone = nt > 64 ? 0.30 : 0.152, two = nt > 64 ? 0.34 : 0.205;
+            const bool big = nt > 64;
+            const double KB = (KP + S - 1) / S, alone = big ? 0.338 : 0.154, two = big ? 0.355 : 0.216;
             if (rounds > 1 && S > 1) break;                  // (a second round of clusters waits for whole ones to end)
-            const double us = 1.3 + (nt > 64 ? 0.03 : 0.018) * nt + KB * ((rounds - 1) * two + (last > sms ? two : alone)) + (rounds - 1) * 2.0 +
-                              (S > 1 ? 0.3 * S : 0.0) + (ctas > sms ? 0.1 : 0.0);
+            const double us = (big ? 0.75 + 0.0212 * nt : 1.3 + 0.025 * nt) + KB * ((rounds - 1) * two + (last > sms ? two : alone)) + (rounds - 1) * 3.05 +
+                              (S > 1 ? 0.233 * S : 0.0) + (ctas > sms ? 0.27 : 0.0);
             if (us < best.us) best = {nt, S, us};
         }
     }

@@ -59,14 +59,14 @@ def check_linear(lib, M, N, K, ws_num):
 @pytest.mark.parametrize("M,N,K", [(40, 64, 64), (257, 320, 192), (700, 320, 128), (2049, 2560, 192), (1000, 13824, 320), (300, 2560, 6912),
                                    (1226, 3840, 2560), (4096, 192, 64), (150, 57344, 128)])
 def test_pairs_with_several_tiles_and_ragged_edges(lib, M, N, K):
-    """Tile heights from 32 to 256 tokens, several tiles per pair, a last row block of 64 rows, half a last stage."""
+    """Several tiles per pair, a last row block of 64 rows, half a last stage; small and deep layers, which single tiles take (heights: below)."""
     check_linear(lib, M, N, K, 2)
 
 
 @pytest.mark.parametrize("M,N,K", [(9, 64, 64), (16, 128, 640), (33, 192, 1088), (64, 2560, 2560), (48, 2560, 6912), (80, 1024, 16384), (129, 1344, 1344),
                                    (250, 2560, 2560), (190, 320, 8256), (256, 13824, 320), (1025, 128, 192)])
 def test_tiles_in_tensor_memory(lib, M, N, K):
-    """One to eight slices of K (uneven ones, half a last block pair), one to several blocks of tokens, 16 to 128 tokens per tile, half a last row tile."""
+    """One to eight slices of K (uneven ones, half a last block pair), one to several blocks of tokens, half a last row tile (heights: below)."""
     check_linear(lib, M, N, K, 3)
 
 
@@ -150,9 +150,11 @@ def check_against_packed(lib, M, N, K):
     lib.ternaspmm_w2_linear(x.data_ptr(), 0, None, 0.0, w2.data_ptr(), got.data_ptr(), s.data_ptr(), ws.data_ptr(), 2, M, N, K, 0, 0, 0, -1, None, stream)
     shape = (ctypes.c_int * 6)()
     lib.ternaspmm_last_launch_shape(shape)
+    res, summed = torch.randn((M, N), generator=g, device="cuda").to(torch.bfloat16), torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda")
+    lib.ternaspmm_w2_linear(x.data_ptr(), 0, None, 0.0, w2.data_ptr(), summed.data_ptr(), s.data_ptr(), ws.data_ptr(), 2, M, N, K, 0, 0, 0, -1, res.data_ptr(), stream)
     lib.bitlinear_TernaSpMM(x.data_ptr(), pk.bm.data_ptr(), pk.tg.data_ptr(), pk.tm.data_ptr(), pk.cv.data_ptr(), want.data_ptr(), s.data_ptr(),
                             ws.data_ptr(), 2, M, N, K, 1, None, stream)
-    assert lib.ternaspmm_last_status() == 0 and torch.equal(got, want)
+    assert lib.ternaspmm_last_status() == 0 and torch.equal(got, want) and torch.equal(summed, (res.float() + want.float()).to(torch.bfloat16))
     return list(shape)
 
 
@@ -168,6 +170,24 @@ def test_ten_and_twenty_warps(lib, M, N, K, warps):
     """Either side of each line of the rule (on 148 SMs): the warps that were measured to be faster there, the bits of the packed kernels."""
     shape = check_against_packed(lib, M, N, K)
     assert shape[0] == 8 and (shape[3] == warps or torch.cuda.get_device_properties(0).multi_processor_count != 148)
+
+
+@pytest.mark.parametrize("M,N,K,tokens", [(65, 38208, 1216, 96), (4170, 1088, 64, 96), (2691, 2368, 1216, 128), (1807, 2496, 1216, 160), (2249, 2368, 1216, 192), (1603, 1600, 2368, 192),
+                                          (1926, 1600, 4544, 224), (193, 28800, 3264, 224), (1541, 2560, 6912, 224), (2249, 1600, 9152, 256), (225, 28800, 4544, 256), (2402, 3392, 9152, 256)])
+def test_pairs_by_tokens_per_tile(lib, M, N, K, tokens):
+    """Every height of the pair kernel's tiles (on 148 SMs), one tile per pair and several, one accumulator buffer and two, ragged in every dimension: the
+    bits of the packed kernels."""
+    shape = check_against_packed(lib, M, N, K)
+    assert shape[:2] == [7, tokens] or torch.cuda.get_device_properties(0).multi_processor_count != 148
+
+
+@pytest.mark.parametrize("M,N,K,tokens,slices", [(9, 64, 64, 16, 1), (17, 320, 1216, 32, 2), (577, 448, 2368, 64, 3), (33, 192, 1984, 48, 4), (257, 576, 9152, 64, 5), (1569, 64, 5184, 64, 5),
+                                                 (100, 448, 5184, 64, 6), (9, 64, 7104, 16, 7), (23, 192, 16448, 32, 8), (129, 13120, 1216, 80, 1), (257, 7616, 1216, 96, 1),
+                                                 (770, 2880, 1216, 112, 1), (1671, 1344, 1216, 128, 1), (5000, 448, 64, 128, 1)])
+def test_tiles_by_tokens_and_slices(lib, M, N, K, tokens, slices):
+    """Every height of the tile kernel's tiles and every number of K slices (on 148 SMs), the bits of the packed kernels."""
+    shape = check_against_packed(lib, M, N, K)
+    assert shape[:3] == [9, tokens, slices] or torch.cuda.get_device_properties(0).multi_processor_count != 148
 
 
 def test_layout_and_linear_on_one_stream(lib):
