@@ -163,3 +163,55 @@ def test_attention_is_as_exact_as_flash_attn(lib, B, T, past, L):
     e_ours, e_theirs = (((t.double() - want).norm() / want.norm()).item() for t in (ours, theirs))
     # the same formats (bf16 operands and probabilities, fp32 sums) and 2e5 to 6e6 outputs: the two norms agree to a per cent
     assert e_ours <= 1.02 * e_theirs
+
+
+@pytest.mark.parametrize("B,pos,L", [(2, 17, 40), (3, 333, 461), (8, 1100, 1101), (1, 2300, 2500)])
+@torch.no_grad()
+def test_default_glue_attention_is_no_less_exact_than_torch(lib, B, pos, L):
+    """Error against float64 beside that of the operators which the model called before, on the same inputs: both round the rotated query, the
+    probabilities and the result to bf16, torch its intermediate sums as well, so the kernel's is the smaller one (2.0e-3 and 2.2e-3)."""
+    from ternainfer_b200.linear import attn_decode_by_head
+    from ternainfer_b200.model import causal_mask
+    H, Hkv, D = 20, 5, 128
+    g = torch.Generator(device="cuda").manual_seed(7 * pos + B)
+    qkv = torch.randn((B, 1, (H + 2 * Hkv) * D), generator=g, device="cuda").to(torch.bfloat16)
+    kc, vc = (torch.randn((B, Hkv, L, D), generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    cos, sin = rope_tables(D, L, 500000.0, "cuda")
+    p = torch.tensor([pos], device="cuda")
+    ours = attn_decode_by_head(qkv, kc, vc, cos[p], sin[p], p, H, Hkv)
+    q = apply_rope(qkv[..., :H * D].view(B, 1, H, D), cos[p].expand(B, 1, -1), sin[p].expand(B, 1, -1))
+    theirs = torch.nn.functional.scaled_dot_product_attention(q.transpose(1, 2), kc, vc, attn_mask=causal_mask(p, L), enable_gqa=True).transpose(1, 2).reshape(B, 1, H * D)
+    kk, vv = (t[:, :, :pos + 1].double().repeat_interleave(H // Hkv, 1) for t in (kc, vc))
+    a = torch.softmax(torch.einsum("bhd,bhld->bhl", q[:, 0].double(), kk) / D ** 0.5, -1)
+    want = torch.einsum("bhl,bhld->bhd", a, vv).reshape(B, 1, H * D)
+    e_ours, e_theirs = (((t.double() - want).norm() / want.norm()).item() for t in (ours, theirs))
+    assert e_ours <= e_theirs
+
+
+def test_default_glue_attention_refuses_what_its_kernel_cannot_check(lib, monkeypatch):
+    """Tensors on other devices, of other types, shapes or strides, and under autograd: None (and the caller's general path), without a launch."""
+    from ternainfer_b200 import linear
+    H, Hkv, D, B, L = 20, 5, 128, 2, 16
+
+    def args(**other):
+        a = dict(qkv=torch.zeros((B, 1, (H + 2 * Hkv) * D), dtype=torch.bfloat16, device="cuda"), k=torch.zeros((B, Hkv, L, D), dtype=torch.bfloat16, device="cuda"),
+                 v=torch.zeros((B, Hkv, L, D), dtype=torch.bfloat16, device="cuda"), cos=torch.zeros(64, device="cuda"), sin=torch.zeros(64, device="cuda"),
+                 pos=torch.arange(1, device="cuda"), heads=H, kv_heads=Hkv)
+        a.update((k, f(a[k])) for k, f in other.items())
+        return a.values()
+
+    with torch.no_grad():
+        assert linear.attn_decode_by_head(*args()) is not None
+    monkeypatch.setattr(linear, "load_library", lambda: pytest.fail("launched"))
+    assert linear.attn_decode_by_head(*args()) is None, "under autograd"
+    bad = [dict(pos=torch.Tensor.cpu), dict(k=torch.Tensor.cpu), dict(v=torch.Tensor.cpu), dict(cos=torch.Tensor.cpu), dict(sin=torch.Tensor.cpu),
+           dict(cos=torch.Tensor.bfloat16), dict(sin=torch.Tensor.double), dict(k=torch.Tensor.float), dict(v=torch.Tensor.half), dict(qkv=torch.Tensor.float),
+           dict(pos=torch.Tensor.int), dict(pos=lambda t: torch.arange(2, device="cuda")), dict(qkv=lambda t: t[..., :-128].contiguous()),
+           dict(qkv=lambda t: t[:1].contiguous()), dict(qkv=lambda t: torch.cat([t, t], 1)), dict(qkv=lambda t: t[:, 0]), dict(k=lambda t: t[:1].contiguous()),
+           dict(v=lambda t: t[:, :, :8].contiguous()), dict(k=lambda t: t[:, :4].contiguous(), v=lambda t: t[:, :4].contiguous()),
+           dict(k=lambda t: t[..., :64].contiguous(), v=lambda t: t[..., :64].contiguous()), dict(k=lambda t: t[:, :, :0], v=lambda t: t[:, :, :0]),
+           dict(v=lambda t: t.transpose(1, 2).contiguous().transpose(1, 2)), dict(cos=lambda t: t[:32], sin=lambda t: t[:32]),
+           dict(cos=lambda t: torch.zeros(128, device="cuda")[::2]), dict(heads=lambda h: h + 4), dict(kv_heads=lambda h: 4), dict(kv_heads=lambda h: 0)]
+    with torch.no_grad():
+        for other in bad:
+            assert linear.attn_decode_by_head(*args(**other)) is None, list(other)

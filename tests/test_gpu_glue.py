@@ -34,13 +34,14 @@ def calls():
             "rmsnorm": lambda: linear.rmsnorm(t(1, 64), t(64), 1e-5), "RMSNorm": lambda: RMSNorm(64).to("cuda", torch.bfloat16)(t(1, 64)),
             "rope": lambda: linear.rope(t(1, 1, 1, 128), t(1, 1, 64).float(), t(1, 1, 64).float()), "relu2_gate": lambda: linear.relu2_gate(t(1, 128)),
             "to_float": lambda: to_float(t(1, 64)), "attn_decode": lambda: linear.attn_decode(qkv, kv, kv, t(1, 64), t(1, 64), pos, 20, 5),
+            "attn_decode_by_head": lambda: linear.attn_decode_by_head(qkv, kv.transpose(1, 2).contiguous(), kv.transpose(1, 2).contiguous(), t(64).float(), t(64).float(), pos, 20, 5),
             "attn_prefill": lambda: linear.attn_prefill(qkv, kv, kv, t(8, 64), t(8, 64), pos, 20, 5),
             "lm_head_argmax": lambda: linear.lm_head_argmax(t(1, 64), t(128, 64)),
             "TernaInfer_linear": lambda: linear.TernaInfer_linear(torch.zeros((1, 64), dtype=torch.int8, device="cuda"), cv, tg, tm, bm, None, t(1), t(4), 1, 64)}
 
 
 @pytest.mark.parametrize("name", ["quant_input", "rmsnorm_quant", "rmsnorm", "RMSNorm", "rope", "relu2_gate", "to_float", "attn_decode", "attn_prefill",
-                                  "lm_head_argmax", "TernaInfer_linear"])
+                                  "lm_head_argmax", "TernaInfer_linear", "attn_decode_by_head"])
 def test_launches_go_to_the_device_of_the_tensors(lib, monkeypatch, name):
     """With another device current (here by its number only), a call switches to its tensors' device, as torch operators do."""
     call, entered, real = calls()[name], [], torch.cuda.current_device()
