@@ -294,7 +294,7 @@ void ternaspmm_w2_relayout(uint64_t* bitmap, int* tile_offsets, uint16_t* quarte
                            int N, int K, void* w2, ternaspmm_stream_t stream);
 long long ternaspmm_w2_bytes(int N, int K);
 int ternaspmm_w2_fused_rows(int K);
-int ternaspmm_w2_pays(int M, int N, int K); /* 0: the packed entry points are faster for this call (they never are any more) */
+int ternaspmm_w2_pays(int M, int N, int K); /* whether a caller with both forms in hand should take the two-bit one: 1 for every size */
 void ternaspmm_w2_linear(void* x, int front_end, ternaspmm_bf16* norm_weight, float eps, void* w2, ternaspmm_bf16* out,
                          ternaspmm_bf16* s, ternaspmm_bf16* ws, int ws_num, int M, int N, int K, int seg1, int seg2,
                          int seg3, int prefill_form, ternaspmm_bf16* residual, ternaspmm_stream_t stream);

@@ -1,6 +1,7 @@
 // Ternary linears on weights laid out once in two bits, for sm_100a: up to eight
-// tokens (more: w2_tile.cuh, w2_pair.cuh), with the activation front-end (RMSNorm,
-// gate, int8 quantiser) optionally inside the kernel.
+// tokens with the activation front-end (RMSNorm, gate, int8 quantiser) inside the
+// kernel; on int8 activations up to four, and up to eight for narrow layers (the others
+// and more tokens: w2_tile.cuh, w2_pair.cuh).
 //
 // The packed checkpoint format (bitmap + sign stream) costs about 0.12 warp
 // instructions per weight to decode, and that, not HBM, is what bounds the
@@ -175,8 +176,8 @@ __device__ __forceinline__ void w2_mma_pair(int (&acc0)[4], int (&acc1)[4], cons
     mma_s8_16x8x32(acc1, a[2], c[2], a[3], c[3], x1.z, x1.w);
 }
 
-// MW: warps at most.  RG: strips at a time, three where a CTA has that many and a long enough ring for them.  VK, VR: vectors of a row per thread and rows at a
-// time in the front-end.
+// MW: warps at most.  RG: strips at a time, one or three (ternaspmm.cu has both rules).  VK, VR: vectors of a row per thread and rows at a time in
+// the front-end.
 template <int MW, int RG, int FE, int VK, int VR>
 __global__ void __launch_bounds__(MW * 32, MW > kW2Warps ? 1 : 2) w2_small_kernel(const __grid_constant__ W2Params p) {
     extern __shared__ __align__(128) uint8_t smem[];
@@ -298,11 +299,11 @@ __global__ void __launch_bounds__(MW * 32, MW > kW2Warps ? 1 : 2) w2_small_kerne
         if (++d == D) d = 0, parity ^= 1u, refilled = true;
     };
     const uint4 none = make_uint4(0, 0, 0, 0);
-    // What a turn of a loop costs is its warps' chains and, the first time, its fetch (some 35 cycles for eight instructions).  So
-    // few strips are done one at a time - at once where a warp's share of K is one or two block pairs, whose activations stay in
-    // registers, else a block pair per turn (the next one's operands asked for ahead of it: 3 to 8 % slower) - and more strips
-    // three at a time, two block pairs per turn.  (us per call, three / one at a time: 2560 x 2560 with the norm 3.3 / 3.1, 8192 x 8192 at 4
-    // tokens 7.8 / 7.2, 10240 x 8192 at 8 9.3 / 8.5, 13824 x 2560 at 8 tokens 5.3 / 5.7, 57344 x 8192 at 4 32.6 / 34.2.)
+    // What a turn of a loop costs is its warps' chains and, the first time, its fetch (some 35 cycles for eight instructions).  One strip at a
+    // time: at once where a warp's share of K is one or two block pairs, whose activations stay in registers, else a block pair per
+    // turn (the next one's operands asked for ahead of it: 3 to 8 % slower; two per turn with accumulators of their own: no gain).  Three at a
+    // time: two block pairs per turn.  (us per call, three / one at a time: 2560 x 2560 with the norm 3.3 / 3.1, 13824 x 2560 at 4 tokens
+    // 4.3 / 4.5, 57344 x 8192 at 4 32.6 / 34.2.)
     if (RG == 1 && p1 - p0 <= 2 && p1 - p0 <= PC && p0 < p1) {
         const bool two = p1 - p0 == 2;
         const uint4 x0 = lds128(x_lane + p0 * 128), x1 = lds128(x_lane + p0 * 128 + 64);
