@@ -495,7 +495,7 @@ __global__ void __launch_bounds__(kTileThreads, 2)
 // Tokens per tile and K slices of a call, and the time it takes, in us.  The CTAs of two to an SM (clusters leave some places empty) run
 // at once, each KB = K / 128 / S block pairs long, 0.15 us each, 0.22 with two CTAs on an SM's tensor cores; a further round of CTAs costs
 // its own start and end, and a cluster's exchange grows with S.  Tiles of more than 64 tokens have room for two stages only, 0.34 us per block
-// pair, and pay where they save a round.  The constants of this and of w2_pair_plan_tile are fitted to 8700 measured plans of 582 calls of 9 to
+// pair, and pay where they save a round.  The constants of this and of w2_pair_plan_tile are fitted to 5400 measured plans of 582 calls of 9 to
 // 4096 tokens (the layers of both models, their shards, and sizes drawn over the range): the plan chosen is 1.0 % slower than the best one in the mean,
 // 1.1 % on calls that were left out of a fit.  us per call, S = 1 / 2 / 4 / 6 / 8: 2560 x 2560 at 48 tokens 5.2 / 4.4 / 4.1 / 4.4 / 5.4, 2560 x 6912 at 16 9.5 / 6.2 /
 // 5.0 / 4.5 / 4.6, 1024 x 16384 at 16 19.5 / 11.1 / 7.1 / 6.1 / 5.3, 8192 x 8192 at 16 11.2 / 8.6 / 7.0 / 10.6 / 11.8 (384 CTAs with six slices); tiles of up to 64 / 128
